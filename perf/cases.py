@@ -1,0 +1,353 @@
+"""The work a user of this framework has it do, as cases that can be timed: EXL3 linear layers from one row to a prefill
+chunk, paged attention over fp16 and quantised pools, and whole steps of a model.
+
+A case is a dict of plain values.  `listed()` names twelve; `draw(rng)` gives others of the same ranges; `prepare` makes what
+a program holds before the call (weights, pools, descriptors, a captured graph); `run` makes one call through the public
+API and returns everything it wrote."""
+import math
+import os
+import random
+import sys
+
+import torch
+
+sys.path.insert(0, os.path.join(os.getcwd(), "exllamav3-rs_b200"))      # the package of the tree it is run in
+
+import exl3b200  # noqa: E402
+from exl3b200.step import SyntheticModel  # noqa: E402
+
+PAGE = 256
+CODEBOOKS = {"3inst": 0, "mcg": 1, "mul1": 2}
+
+# Model shapes of the repository's benchmark and tests.
+SHAPES = {
+    "0.6b": dict(hidden=1024, nq=16, nkv=8, inter=3072, vocab=151936),
+    "27b": dict(hidden=5120, nq=40, nkv=8, inter=17408, vocab=151936),
+}
+
+_ctx = None
+
+
+def context():
+    """One context per process and device, as a serving program keeps it."""
+    global _ctx
+    if _ctx is None:
+        _ctx = exl3b200.Ctx(0, workspace_bytes=1 << 30)
+    return _ctx
+
+
+# ---------------------------------------------------------------------------------------------------------------- cases
+
+def _linear(name, m, k, n, bits, codebook="mcg", out="fp16"):
+    return dict(name=name, kind="linear", m=m, k=k, n=n, bits=bits, codebook=codebook, out=out)
+
+
+def _attention(name, kv, decode, chunks, chunk_len, ctx_lo, ctx_hi, nq=40, nkv=8):
+    return dict(name=name, kind="attention", kv=kv, decode=decode, chunks=chunks, chunk_len=chunk_len, ctx_lo=ctx_lo,
+                ctx_hi=ctx_hi, nq=nq, nkv=nkv)
+
+
+def _step(name, shape, layers, bits, kv, decode, chunks, chunk_len, ctx_lo, ctx_hi, graph, all_rows=False, codebook="mcg"):
+    return dict(name=name, kind="step", shape=shape, layers=layers, bits=bits, codebook=codebook, kv=kv, decode=decode,
+                chunks=chunks, chunk_len=chunk_len, ctx_lo=ctx_lo, ctx_hi=ctx_hi, graph=graph, all_rows=all_rows)
+
+
+def listed():
+    return [
+        # one token of one conversation through a projection of a small model: the smallest call there is
+        _linear("linear-small-1row", 1, 1024, 3072, 8),
+        # one token through gate_proj of a 27B-class model: single-user decoding
+        _linear("linear-decode-1row", 1, 5120, 17408, 4),
+        # a continuous batch of thirteen sequences through down_proj, a low-bit quantisation in the default codebook
+        _linear("linear-decode-13rows", 13, 17408, 5120, 3, "3inst"),
+        # a speculative-verify or many-user batch through gate_proj
+        _linear("linear-verify-52rows", 52, 5120, 17408, 4),
+        # a prefill chunk of 2048 tokens through gate_proj: the largest contraction
+        _linear("linear-prefill-2048rows", 2048, 5120, 17408, 4),
+        # decode attention of 64 users with contexts from a prompt to a long document, fp16 pool
+        _attention("attention-decode-fp16", "fp16", 64, 0, 0, 128, 32768),
+        # the same users with the 4-bit pool, which is what makes such contexts fit
+        _attention("attention-decode-4bit", "q4", 64, 0, 0, 128, 32768),
+        # fewer users, 8-bit pool
+        _attention("attention-decode-8bit", "q8", 24, 0, 0, 512, 16384),
+        # four prefill chunks of 256 tokens behind contexts of different lengths
+        _attention("attention-prefill-fp16", "fp16", 0, 4, 256, 512, 16384),
+        # a whole decode step of a small model for eight users, launched call by call: latency and launches count
+        _step("step-small-decode", "0.6b", 28, 8, "fp16", 8, 0, 0, 64, 1024, False),
+        # a whole speculative-verify round of a 27B-class model over 4-bit pools: 4 sequences x 8 draft rows, one graph
+        _step("step-verify-27b", "27b", 64, 4, "q4", 0, 4, 8, 1024, 32768, True, True),
+        # continuous batching: 28 users decode while four prompts are prefilled, the layers of four pipeline positions
+        _step("step-mixed-27b", "27b", 4, 4, "fp16", 28, 4, 256, 512, 16384, False),
+    ]
+
+
+def _log_int(rng, lo, hi):
+    return int(round(math.exp(rng.uniform(math.log(lo), math.log(hi)))))
+
+
+def _draw_linear(rng):
+    k, n = rng.choice([(1024, 3072), (2048, 1024), (5120, 5120), (5120, 1024), (5120, 17408), (17408, 5120),
+                       (128 * _log_int(rng, 8, 96), 128 * _log_int(rng, 4, 160))])
+    m = _log_int(rng, 1, 2048)
+    bits = rng.choice([2, 3, 4, 4, 4, 5, 6, 8])
+    c = _linear(None, m, k, n, bits, rng.choice(["mcg", "mcg", "3inst", "mul1"]), rng.choice(["fp16", "fp16", "fp16", "fp32"]))
+    del c["name"]
+    return c
+
+
+def _draw_attention(rng):
+    nq, nkv = rng.choice([(40, 8), (40, 8), (16, 8), (32, 8), (32, 4)])
+    kv = rng.choice(["fp16", "fp16", "q4", "q4", "q8", "q6"])
+    lo = _log_int(rng, 64, 1024)
+    hi = lo * _log_int(rng, 2, 24)
+    mode = rng.choice(["decode", "decode", "verify", "prefill", "mixed"])
+    decode, chunks, chunk_len = 0, 0, 0
+    if mode in ("decode", "mixed"):
+        decode = _log_int(rng, 1, 64)
+    if mode == "verify":
+        chunks, chunk_len = _log_int(rng, 1, 32), rng.randint(2, 12)
+    if mode in ("prefill", "mixed"):
+        chunks, chunk_len = rng.randint(1, 3), _log_int(rng, 24, 384)
+        if kv != "fp16":
+            chunk_len, hi = min(chunk_len, 128), min(hi, 4096 + lo)
+    c = _attention(None, kv, decode, chunks, chunk_len, lo, hi, nq, nkv)
+    del c["name"]
+    return c
+
+
+def _draw_step(rng):
+    small = rng.random() < 0.6
+    layers = rng.randint(6, 28) if small else rng.randint(2, 6)
+    kv = rng.choice(["fp16", "fp16", "q4", "q8"])
+    mode = rng.choice(["decode", "decode", "verify", "mixed"])
+    decode, chunks, chunk_len = 0, 0, 0
+    if mode in ("decode", "mixed"):
+        decode = _log_int(rng, 1, 48)
+    if mode == "verify":
+        chunks, chunk_len = rng.randint(1, 6), rng.randint(2, 8)
+    if mode == "mixed":
+        chunks, chunk_len = rng.randint(1, 3), _log_int(rng, 24, 256)
+    lo = _log_int(rng, 64, 512)
+    c = _step(None, "0.6b" if small else "27b", layers, rng.choice([3, 4, 4, 5, 6, 8]), kv, decode, chunks, chunk_len, lo,
+              lo * _log_int(rng, 2, 8), rng.random() < 0.5, mode == "verify", rng.choice(["mcg", "mcg", "3inst", "mul1"]))
+    del c["name"]
+    return c
+
+
+def draw(rng):
+    return rng.choice([_draw_linear, _draw_linear, _draw_attention, _draw_attention, _draw_step])(rng)
+
+
+# ----------------------------------------------------------------------------------------------------------- batch shapes
+
+def _lengths(case):
+    """(query rows, cached tokens) of every sequence.  They belong to the case: contexts spread over the logarithm of the
+    case's range, in a mixed-up order."""
+    q = [1] * case["decode"] + [case["chunk_len"]] * case["chunks"]
+    r = random.Random("%d %d %d %d %d" % (case["decode"], case["chunks"], case["chunk_len"], case["ctx_lo"], case["ctx_hi"]))
+    lo, hi, n = math.log(case["ctx_lo"]), math.log(case["ctx_hi"]), len(q)
+    ctx = [int(math.exp(lo + (hi - lo) * (i + r.random()) / n)) for i in range(n)]
+    r.shuffle(ctx)
+    return q, ctx
+
+
+def _kv_bits(case):
+    return 0 if case["kv"] == "fp16" else int(case["kv"][1:])
+
+
+def _kv_token_bytes(case, nkv):
+    """bytes of one token's keys and values of one layer"""
+    bits = _kv_bits(case)
+    return nkv * 128 * 4 if bits == 0 else 2 * (nkv * 4) * (4 * bits + 2)
+
+
+# ------------------------------------------------------------------------------------------------------------------ inputs
+
+def _gen(seed):
+    g = torch.Generator(device="cuda")
+    g.manual_seed(seed)
+    return g
+
+
+def _signs(n, g):
+    return (torch.randint(0, 2, (n,), device="cuda", generator=g) * 2 - 1).to(torch.float16)
+
+
+def _normal(shape, g, std=1.0):
+    return (torch.randn(shape, device="cuda", generator=g) * std).to(torch.float16)
+
+
+class _Pools:
+    """KV planes of all layers in one tensor per plane, filled with a synthetic context: N(0, 0.5^2) values in fp16 pools,
+    random codes with group scales of the same magnitude in quantised ones."""
+
+    def __init__(self, layers, pages, nkv, bits, g):
+        self.bits, groups = bits, nkv * 4
+        if bits == 0:
+            self.planes = [torch.empty((layers, pages, PAGE, nkv, 128), dtype=torch.float16, device="cuda") for _ in range(2)]
+            for t in self.planes:
+                flat = t.view(-1)
+                for i in range(0, flat.numel(), 1 << 28):
+                    part = flat[i:i + (1 << 28)]
+                    part.normal_(0.0, 0.5, generator=g)
+        else:
+            codes = [torch.empty((layers, pages, PAGE, groups * bits), dtype=torch.int32, device="cuda") for _ in range(2)]
+            scales = [torch.empty((layers, pages, PAGE, groups), dtype=torch.float16, device="cuda") for _ in range(2)]
+            for t in codes:
+                t.random_(-2 ** 31, 2 ** 31 - 1, generator=g)
+            for t in scales:
+                t.uniform_(0.01, 0.06, generator=g)
+            self.planes = codes + scales
+
+    def layer(self, i):
+        """device addresses (k, v, sk, sv) of one layer, as exl3b200.Pool.layer gives them"""
+        p = [t[i].data_ptr() for t in self.planes]
+        return tuple(p) if self.bits else (p[0], p[1], 0, 0)
+
+
+def _block_table(q, ctx, seed):
+    need = [(c + x + PAGE - 1) // PAGE for c, x in zip(ctx, q)]
+    pages = sum(need) + 1
+    perm = list(range(pages))
+    random.Random(seed).shuffle(perm)
+    table = torch.zeros((len(q), max(need)), dtype=torch.int32)
+    at = 0
+    for b, cnt in enumerate(need):
+        table[b, :cnt] = torch.tensor(perm[at:at + cnt], dtype=torch.int32)
+        at += cnt
+    return table.cuda(), pages
+
+
+def _prepare_linear(case, seed):
+    g = _gen(seed)
+    m, k, n, bits = case["m"], case["k"], case["n"], case["bits"]
+    return dict(
+        kind="linear", ctx=context(), x=_normal((m, k), g), suh=_signs(k, g),
+        trellis=torch.randint(-32768, 32768, (k // 16, n // 16, 16 * bits), dtype=torch.int16, device="cuda", generator=g),
+        svh=(_signs(n, g).float() / math.sqrt(k)).to(torch.float16),
+        y=torch.zeros((m, n), dtype=torch.float16 if case["out"] == "fp16" else torch.float32, device="cuda"),
+        mcg=case["codebook"] == "mcg", mul1=case["codebook"] == "mul1")
+
+
+def _prepare_attention(case, seed):
+    g = _gen(seed)
+    q_lens, ctx_lens = _lengths(case)
+    nq, nkv, bits = case["nq"], case["nkv"], _kv_bits(case)
+    table, pages = _block_table(q_lens, ctx_lens, seed)
+    rows = sum(q_lens)
+    ragged = case["decode"] > 0 and case["chunks"] > 0
+    lead = (rows,) if ragged else (len(q_lens), q_lens[0])
+    cu = [0]
+    for x in q_lens:
+        cu.append(cu[-1] + x)
+    return dict(
+        kind="attention", ctx=context(), bits=bits, nkv=nkv, pools=_Pools(1, pages, nkv, bits, g), table=table,
+        q=_normal(lead + (nq, 128), g), k=_normal(lead + (nkv, 128), g, 0.5), v=_normal(lead + (nkv, 128), g, 0.5),
+        o=torch.zeros(lead + (nq, 128), dtype=torch.float16, device="cuda"),
+        seqlens=torch.tensor(ctx_lens, dtype=torch.int32, device="cuda"),
+        cu_q=torch.tensor(cu, dtype=torch.int32, device="cuda") if ragged else None, max_q=max(q_lens))
+
+
+def _prepare_step(case, seed):
+    g = _gen(seed)
+    q_lens, ctx_lens = _lengths(case)
+    s, bits = SHAPES[case["shape"]], _kv_bits(case)
+    table, pages = _block_table(q_lens, ctx_lens, seed)
+    pools = _Pools(case["layers"], pages, s["nkv"], bits, g)
+    model = SyntheticModel(case["layers"], s["hidden"], s["nq"], s["nkv"], 128, s["inter"], s["vocab"], K=case["bits"],
+                           cb=CODEBOOKS[case["codebook"]], pages=pages, kv_bits=bits, seed=seed, pool=pools)
+    rows = sum(q_lens)
+    st = dict(
+        kind="step", ctx=context(), model=model, pools=pools, table=table, max_q=max(q_lens), all_rows=case["all_rows"],
+        ids=torch.randint(0, s["vocab"], (rows,), dtype=torch.int64, device="cuda", generator=g),
+        q_lens=torch.tensor(q_lens, dtype=torch.int32, device="cuda"),
+        seqlens=torch.tensor(ctx_lens, dtype=torch.int32, device="cuda"), graph=None,
+        tokens=torch.zeros(rows if case["all_rows"] else len(q_lens), dtype=torch.int64, device="cuda"))
+    if case["graph"]:
+        # a decode loop with fixed buffers captures its step once, after a first call that sets everything up
+        _step_call(st)
+        torch.cuda.synchronize()
+        graph = exl3b200.CudaGraph(st["ctx"])
+        graph.capture_begin()
+        st["logits"] = _step_call(st, stream=graph.side_stream())
+        graph.capture_end()
+        st["graph"] = graph
+    return st
+
+
+def prepare(case, seed):
+    return {"linear": _prepare_linear, "attention": _prepare_attention, "step": _prepare_step}[case["kind"]](case, seed)
+
+
+# -------------------------------------------------------------------------------------------------------------- the calls
+
+def _step_call(s, stream=None):
+    _, logits = s["model"].step(s["ctx"], s["ids"], s["q_lens"], s["seqlens"], s["table"], s["max_q"], want_logits=True,
+                                stream=stream, tokens_out=s["tokens"], all_rows=s["all_rows"])
+    return logits
+
+
+def run(s):
+    ctx = s["ctx"]
+    if s["kind"] == "linear":
+        ctx.exl3_gemm(s["x"], s["trellis"], s["y"], s["suh"], None, s["svh"], mcg=s["mcg"], mul1=s["mul1"])
+        return s["y"]
+    planes = s["pools"].planes
+    if s["kind"] == "attention":
+        p = [t[0] for t in planes]
+        if s["bits"] == 0:
+            ctx.bighead_attn_paged(s["q"], s["k"], s["v"], p[0], p[1], s["table"], s["seqlens"], s["o"], cu_q=s["cu_q"],
+                                   max_q_len=s["max_q"])
+        else:
+            ctx.bighead_attn_paged_q(s["q"], s["k"], s["v"], p[0], p[2], p[1], p[3], s["table"], s["seqlens"], s["o"],
+                                     s["nkv"], cu_q=s["cu_q"], max_q_len=s["max_q"])
+        return [s["o"]] + planes
+    # The greedy token is the logits' argmax; between two logits closer than fp16 rounding it may fall either way, so
+    # the logits stand for it.
+    if s["graph"] is not None:
+        s["graph"].replay()
+        return [s["logits"]] + planes
+    return [_step_call(s)] + planes
+
+
+# ---------------------------------------------------------------------------------------------------- what a pass requires
+
+def _attention_work(case, nq, nkv):
+    q, ctx = _lengths(case)
+    tok = _kv_token_bytes(case, nkv)
+    nbytes = sum(c * tok + x * (nkv * 128 * 4 + tok + 2 * nq * 128 * 2) for x, c in zip(q, ctx))
+    flops = sum(4 * nq * 128 * (x * c + x * (x + 1) // 2) for x, c in zip(q, ctx))
+    return nbytes, flops
+
+
+def work(case):
+    if case["kind"] == "linear":
+        m, k, n = case["m"], case["k"], case["n"]
+        return {"bytes": k * n * case["bits"] / 8 + 2 * (k + n) + 2 * m * k + m * n * (2 if case["out"] == "fp16" else 4),
+                "flops": 2.0 * m * k * n}
+    if case["kind"] == "attention":
+        nbytes, flops = _attention_work(case, case["nq"], case["nkv"])
+        return {"bytes": nbytes, "flops": flops}
+    s = SHAPES[case["shape"]]
+    q, _ = _lengths(case)
+    rows, heads = sum(q), sum(q) if case["all_rows"] else len(q)
+    qd, kd = s["nq"] * 128, s["nkv"] * 128
+    per_layer = s["hidden"] * (2 * qd + 2 * kd) + 3 * s["hidden"] * s["inter"]
+    nbytes, flops = _attention_work(case, s["nq"], s["nkv"])
+    # weights, the pools and their appended rows; embedding rows in, logits out (activations can stay on the chip)
+    return {"bytes": case["layers"] * (per_layer * case["bits"] / 8 + nbytes - rows * (kd * 4 + 2 * qd * 2)) +
+            s["hidden"] * s["vocab"] * case["bits"] / 8 + rows * s["hidden"] * 2 + heads * s["vocab"] * 4,
+            "flops": case["layers"] * (2.0 * rows * per_layer + flops) + 2.0 * heads * s["hidden"] * s["vocab"]}
+
+
+def tolerance(case):
+    # fp16 operands with fp32 sums: the transformed activations and the weights are each rounded to fp16 once, and so is
+    # the result
+    if case["kind"] == "linear":
+        return {"rel": 2e-3}
+    # softmax weights are rounded to fp16 before the second product; in quantised pools the decoded keys and values are too
+    if case["kind"] == "attention":
+        return {"rel": 2e-3 if case["kv"] == "fp16" else 4e-3, "differ": 1e-4}
+    # a stack of such layers, where every rounding goes through the layers behind it; a new key or value on the border of
+    # two codes may be stored as either
+    return {"rel": 1e-2, "differ": 1e-2}
