@@ -351,3 +351,109 @@ def tolerance(case):
     # a stack of such layers, where every rounding goes through the layers behind it; a new key or value on the border of
     # two codes may be stored as either
     return {"rel": 1e-2, "differ": 1e-2}
+
+
+# ---------------------------------------------------------------------------------------------- the same in 64 bits
+
+def _hadamard(n):
+    h = torch.ones((1, 1), dtype=torch.float64, device="cuda")
+    while h.shape[0] < n:
+        h = torch.cat([torch.cat([h, h], 1), torch.cat([h, -h], 1)], 0)
+    return h / math.sqrt(n)
+
+
+def _codebook(name):
+    """the fp16 weights of all 16-bit states"""
+    x = torch.arange(65536, dtype=torch.int64, device="cuda")
+    if name == "mul1":
+        x = (x * 0x83DCD12D) & 0xFFFFFFFF
+        s = 1024 + (x & 255) + ((x >> 8) & 255) + ((x >> 16) & 255) + (x >> 24)
+        inv, bias = (torch.tensor([v], dtype=torch.int16, device="cuda").view(torch.float16).double() for v in (0x1EEE, 0xC931 - 65536))
+        return (s.double() * inv + bias).to(torch.float16).double()
+    x = (x * 89226354 + 64248484 if name == "3inst" else x * 0xCBAC1FED) & 0xFFFFFFFF
+    x = (x & 0x8FFF8FFF) ^ 0x3B603B60
+    lo, hi = (((v & 0xFFFF) ^ 0x8000) - 0x8000 for v in (x, x >> 16))
+    return (lo.to(torch.int16).view(torch.float16).double() + hi.to(torch.int16).view(torch.float16).double()).to(torch.float16).double()
+
+
+def _weights(trellis, bits, codebook):
+    kt, nt, _ = trellis.shape
+    words, nw = trellis.view(torch.int32), 8 * bits
+    book = _codebook(codebook)
+    at = torch.empty(256, dtype=torch.int64, device="cuda")            # position in the tile of every ring position
+    first, second, shift = [], [], []
+    for t in range(256):
+        lane, j = t // 8, t % 8
+        at[t] = (2 * (lane & 3) + (0, 1, 8, 9)[j & 3]) * 16 + (lane >> 2) + 8 * (j >> 2)
+        b = t * bits + bits - 16 + 256 * bits
+        first.append(b // 32 % nw)
+        second.append((b + 15) // 32 % nw)
+        shift.append(((b + 15) // 32 + 1) * 32 - b - 16)
+    first, second, shift = (torch.tensor(v, dtype=torch.int64, device="cuda") for v in (first, second, shift))
+    w = torch.empty((kt * 16, nt * 16), dtype=torch.float64, device="cuda")
+    for i in range(0, kt, 64):
+        x = words[i:i + 64].long() & 0xFFFFFFFF
+        states = ((((x[..., first] & 0xFFFF) << 32) | x[..., second]) >> shift) & 0xFFFF
+        tiles = torch.empty(states.shape, dtype=torch.float64, device="cuda")
+        tiles[..., at] = book[states]
+        w[16 * i:16 * i + 16 * x.shape[0]] = tiles.view(-1, nt, 16, 16).transpose(1, 2).reshape(-1, nt * 16)
+    return w
+
+
+def _exact_linear(case, s):
+    h = _hadamard(128)
+    x = ((s["x"].double() * s["suh"].double()).view(-1, 128) @ h).view(case["m"], case["k"])
+    y = x @ _weights(s["trellis"], case["bits"], case["codebook"])
+    return (y.view(-1, 128) @ h).view(case["m"], case["n"]) * s["svh"].double()
+
+
+def _dequantised(codes, scales, bits):
+    """[tokens, groups * bits] words and [tokens, groups] scales to [tokens, groups * 32] values"""
+    x = (codes.long() & 0xFFFFFFFF).view(codes.shape[0], -1, bits)
+    q, at = 0, 0
+    for w in (8, 4, 2, 1):
+        if bits & w:
+            off = torch.arange(32, device="cuda") * w
+            q = (q << w) | ((x[..., at + off // 32] >> (off % 32)) & ((1 << w) - 1))
+            at += w
+    m = 1 << (bits - 1)
+    return (((q - (m - 0.5)) * (scales.double() / m)[..., None]) @ _hadamard(32)).view(codes.shape[0], -1)
+
+
+def _requantised(x, bits):
+    """what a quantised pool makes of new rows [tokens, width]"""
+    v = x.double().view(x.shape[0], -1, 32) @ _hadamard(32)
+    s = v.abs().amax(-1, keepdim=True) + 1e-10
+    m = 1 << (bits - 1)
+    q = torch.clamp(torch.floor(v / s * m + m), 0, 2 * m - 1)
+    return (((q - (m - 0.5)) * (s.to(torch.float16).double() / m)) @ _hadamard(32)).view(x.shape[0], -1)
+
+
+def _exact_attention(case, s):
+    q_lens, ctx_lens = _lengths(case)
+    nq, nkv, bits, planes = case["nq"], case["nkv"], s["bits"], s["pools"].planes
+    q, new = s["q"].reshape(-1, nkv, nq // nkv, 128).double(), [s[x].reshape(-1, nkv * 128) for x in "kv"]
+    out, at = torch.empty_like(q), 0
+    for b, (ql, cl) in enumerate(zip(q_lens, ctx_lens)):
+        pages = s["table"][b, :(cl + PAGE - 1) // PAGE].long()
+        kv = []
+        for i in (0, 1):
+            rows = [p[0][pages].flatten(0, 1)[:cl].flatten(1) for p in planes[i::2]]
+            old = _dequantised(rows[0], rows[1], bits) if bits else rows[0].double()
+            add = new[i][at:at + ql]
+            kv.append(torch.cat([old, _requantised(add, bits) if bits else add.double()]).view(cl + ql, nkv, 128))
+        hidden = torch.arange(cl + ql, device="cuda")[None, :] > cl + torch.arange(ql, device="cuda")[:, None]
+        for h in range(nkv):
+            score = torch.einsum("igd,kd->gik", q[at:at + ql, h], kv[0][:, h]) / math.sqrt(128)
+            prob = torch.softmax(score.masked_fill(hidden, -math.inf), -1)
+            out[at:at + ql, h] = torch.einsum("gik,kd->igd", prob, kv[1][:, h])
+        at += ql
+    return [out.view(s["o"].shape)] + [None] * len(planes)
+
+
+def exact(case, seed):
+    # A step has no such value here: it is a stack of the calls above, each of which has.
+    if case["kind"] == "step":
+        return None
+    s = prepare(case, seed)
+    return _exact_linear(case, s) if case["kind"] == "linear" else _exact_attention(case, s)
