@@ -3,7 +3,7 @@
 #include "attn_paged.cuh"
 #include "attn_tc.cuh"
 #include "attn_tc2.cuh"
-#include "attn_q4.cuh"
+#include "attn_qdec.cuh"
 
 namespace {
 
@@ -310,9 +310,10 @@ cudaError_t launch_attn_tc2(exl3_ctx* ctx, const AttnParams& p, int max_items, c
     return cudaPeekAtLastError();
 }
 
-// decode-class kernel over 4-bit pools: tensor maps over the code planes ([tokens][nkv * 16] words) and the scale planes
-// ([tokens][nkv * 4] halves, copied in 16-byte pairs of heads)
-cudaError_t launch_attn_q4(const AttnParams& p, dim3 grid, cudaStream_t st)
+// decode-class kernel over 4-bit and 8-bit pools: tensor maps over the code planes ([tokens][nkv * 4 * bits] words, copied in
+// the swizzle of a head's 64 or 128 bytes) and the scale planes ([tokens][nkv * 4] halves, copied in 16-byte pairs of heads)
+template <int B, int NB>
+cudaError_t launch_attn_qdec(const AttnParams& p, dim3 grid, cudaStream_t st)
 {
     EncodeTiledFn enc = attn_encode_tiled();
     if (!enc) return cudaErrorNotSupported;
@@ -321,28 +322,31 @@ cudaError_t launch_attn_q4(const AttnParams& p, dim3 grid, cudaStream_t st)
     const cuuint64_t tokens = (cuuint64_t)p.pages * EXL3_PAGE;
     for (int i = 0; i < 4; ++i) {
         const bool codes = i < 2;
-        cuuint64_t dims[2] = {(cuuint64_t)p.nkv * (codes ? 16 : 4), tokens};
-        cuuint64_t strides[1] = {(cuuint64_t)p.nkv * (codes ? 64 : 8)};
-        cuuint32_t box[2] = {codes ? 16u : 8u, (cuuint32_t)AQ_TK};
+        cuuint64_t dims[2] = {(cuuint64_t)p.nkv * (codes ? 4 * B : 4), tokens};
+        cuuint64_t strides[1] = {(cuuint64_t)p.nkv * (codes ? 16 * B : 8)};
+        cuuint32_t box[2] = {codes ? 4u * B : 8u, (cuuint32_t)QD_TK};
         cuuint32_t estr[2] = {1, 1};
         if (enc(&maps[i], codes ? CU_TENSOR_MAP_DATA_TYPE_UINT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(planes[i]),
-                dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                !codes ? CU_TENSOR_MAP_SWIZZLE_NONE : (B == 4 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B),
                 CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
             return cudaErrorInvalidValue;
     }
+    constexpr int bytes = QdSmem<B, NB>::BYTES;
+    auto kern = attn_qdec_kernel<B, NB>;
     static bool configured[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64 || !configured[dev]) {
-        cudaError_t e = cudaFuncSetAttribute(attn_q4_decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, AQ_SMEM);
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
         if (e != cudaSuccess) return e;
         if (dev >= 0 && dev < 64) configured[dev] = true;
     }
-    attn_q4_decode_kernel<<<grid, AQ_THREADS, AQ_SMEM, st>>>(maps[0], maps[1], maps[2], maps[3], p);
+    kern<<<grid, QD_THREADS, bytes, st>>>(maps[0], maps[1], maps[2], maps[3], p);
     return cudaPeekAtLastError();
 }
 
-bool q4_decode_kernel_applies(const AttnParams& p, bool quant);
+bool qdec_kernel_applies(const AttnParams& p, bool quant);
 
 // One pass = plan + attention + combine over the sequences whose packed row count lies in (rows_lo, rows_hi].
 int attn_pass(exl3_ctx* ctx, cudaStream_t st, AttnParams p, int total_rows, int max_rows, int rows_lo, int rows_hi,
@@ -358,15 +362,16 @@ int attn_pass(exl3_ctx* ctx, cudaStream_t st, AttnParams p, int total_rows, int 
     const bool use_tc = !decode_shape && !quant && ctx->mma_attn != 0 && p.scale_log2 > 0.f && !p.contig_kv;
     // two arrangements of the tcgen05 kernel: 128-row items with two softmax threads per row (default), 256-row items
     static const bool tc_256 = getenv("EXL3_B200_ATTN_TC256") != nullptr;
-    const int rows_per_cta = decode_shape ? 16 : (use_tc ? (tc_256 ? ATC_CTA_ROWS : A2_ROWS) : 64);
+    // 4-bit and 8-bit pools, decode class: the kernel that builds its operands from the codes (its scale copies are 16 bytes
+    // wide = two heads, so the kv head count must be even and the planes 16-byte aligned).  Row blocks of 8 where no
+    // sequence has more rows (a decode batch), else of 16, whose second half costs nothing where it is empty.
+    const bool use_qdec = decode_shape && qdec_kernel_applies(p, quant);
+    const int rows_per_cta = decode_shape ? (use_qdec && max_rows <= 8 ? 8 : 16) : (use_tc ? (tc_256 ? ATC_CTA_ROWS : A2_ROWS) : 64);
     const int rb_max = (max_rows + rows_per_cta - 1) / rows_per_cta;
     // resident CTAs per SM over all kv heads: about 3 for the mma.sync kernels, 1 for the tcgen05 kernel (all of TMEM)
     // (rounded down: one CTA more than fits would run alone in a second wave after all the others have finished)
-    // 4-bit pools, decode class: the kernel that builds the K operand from the codes (its scale copies are 16 bytes wide =
-    // two heads, so the kv head count must be even and the planes 16-byte aligned)
-    const bool use_q4 = decode_shape && q4_decode_kernel_applies(p, quant);
     int per_sm = 1;
-    if (use_q4) per_sm = 3;
+    if (use_qdec) per_sm = qd_ctas(p.k_bits, rows_per_cta / 8);
     else if (!use_tc) {
         // CTAs of the mma.sync kernel that fit on an SM (bounded by shared memory: stages x 34.8 KB for fp16 pools)
         const size_t smem = quant ? (q4 ? AttnSmem<128, 4>::BYTES : AttnSmem<128, 8>::BYTES) : AttnSmem<128, 0>::BYTES;
@@ -379,11 +384,10 @@ int attn_pass(exl3_ctx* ctx, cudaStream_t st, AttnParams p, int total_rows, int 
     // mma.sync kernels (units handed out dynamically, 8 KB partials): see below.
     static const int tc_items = getenv("EXL3_TUNE_TC_ITEMS") ? atoi(getenv("EXL3_TUNE_TC_ITEMS")) : 0;
     // With the units handed out longest first, fewer and longer items win on the mma.sync kernels too (64 decode
-    // sequences at 1 / 2 / 3 / 4 items per slot: fp16 pools 242 / 234 / 237 / 242 us, 4-bit pools 195 / 202 / 209 / 212 us;
-    // the 4-sequence verify step 21.5 / 22.0 / 22.6 / 23.2 ms; 8-bit pools on the generic kernel 532 / 548 / 550 us at 2 / 3 /
-    // 4): two, and one for the 4-bit kernel.
+    // sequences over fp16 pools at 1 / 2 / 3 / 4 items per slot: 242 / 234 / 237 / 242 us): two, and one for the kernel over
+    // quantised pools, whose units start with the rotation of their queries.
     static const int dec_items = getenv("EXL3_TUNE_DEC_ITEMS") ? atoi(getenv("EXL3_TUNE_DEC_ITEMS")) : 0;
-    const int target_items = grid_x * (use_tc ? (tc_items ? tc_items : 2) : (dec_items ? dec_items : (use_q4 ? 1 : 2)));
+    const int target_items = grid_x * (use_tc ? (tc_items ? tc_items : 2) : (dec_items ? dec_items : (use_qdec ? 1 : 2)));
     // items <= target + sum of row blocks (every (sequence, row block) rounds its split count up once); the row blocks are
     // bounded by bsz * rb_max and, usually much tighter for ragged batches, by total_rows * G / rows_per_cta + bsz
     const long long rb_sum = std::min((long long)p.bsz * rb_max, ((long long)total_rows * G + rows_per_cta - 1) / rows_per_cta + p.bsz);
@@ -431,7 +435,9 @@ int attn_pass(exl3_ctx* ctx, cudaStream_t st, AttnParams p, int total_rows, int 
     if (!use_tc && cudaMemsetAsync(&plan->next, 0, sizeof(int), st) != cudaSuccess)      // the persistent kernel's work counter
         return exl3_fail(ctx, EXL3_ERR_CUDA, "attention: cudaMemsetAsync failed");
     if (use_tc) e = tc_256 ? launch_attn_tc(ctx, p, max_items, st) : launch_attn_tc2(ctx, p, max_items, st);
-    else if (use_q4) e = launch_attn_q4(p, grid, st);
+    else if (use_qdec)
+        e = q4 ? (rows_per_cta == 8 ? launch_attn_qdec<4, 1>(p, grid, st) : launch_attn_qdec<4, 2>(p, grid, st))
+               : (rows_per_cta == 8 ? launch_attn_qdec<8, 1>(p, grid, st) : launch_attn_qdec<8, 2>(p, grid, st));
     else if (q4)    e = decode_shape ? launch_attn<128, 1, 4, 4>(p, grid, st) : launch_attn<128, 4, 1, 4>(p, grid, st);
     else if (quant) e = decode_shape ? launch_attn<128, 1, 4, 8>(p, grid, st) : launch_attn<128, 4, 1, 8>(p, grid, st);
     else            e = decode_shape ? launch_attn<128, 1, 4, 0>(p, grid, st) : launch_attn<128, 4, 1, 0>(p, grid, st);
@@ -446,11 +452,11 @@ int attn_pass(exl3_ctx* ctx, cudaStream_t st, AttnParams p, int total_rows, int 
 // Sequences with at most 16 packed (query, head) rows (decode, short verify) take the kernel that spreads the keys of a
 // tile over the four warps; longer ones (verify with many heads, prefill chunks) the one with a 16-row tile per warp.
 // A ragged batch that holds both kinds runs one pass for each.
-// true when attn_pass will take the 4-bit decode-class kernel for these pools
-bool q4_decode_kernel_applies(const AttnParams& p, bool quant)
+// true when attn_pass will take the decode-class kernel for quantised pools (attn_qdec.cuh)
+bool qdec_kernel_applies(const AttnParams& p, bool quant)
 {
     static const bool no_q4 = getenv("EXL3_B200_NO_Q4_ATTN") != nullptr;
-    return quant && p.k_bits == 4 && p.v_bits == 4 && !no_q4 && p.nkv % 2 == 0 && aligned16(p.qk) && aligned16(p.qv) &&
+    return quant && (p.k_bits == 4 || p.k_bits == 8) && p.v_bits == p.k_bits && !no_q4 && p.nkv % 2 == 0 && aligned16(p.qk) && aligned16(p.qv) &&
            aligned16(p.sk) && aligned16(p.sv);
 }
 
@@ -459,12 +465,12 @@ int attn_impl(exl3_ctx* ctx, cudaStream_t st, AttnParams p, int total_rows, int 
     const int G = p.nq / p.nkv;
     const int max_rows = max_q_len * G;
     size_t off = 0;
-    // Decode class = sequences with at most 16 packed rows.  Over 4-bit pools it also takes up to 48 rows (speculative
-    // verify: 8 query rows x 5 heads) as row blocks of 16 that each walk the codes again: the kernel that builds its
-    // operands from the codes is that much cheaper per key than the generic one (4 verify sequences: 90 us per layer there).
+    // Decode class = sequences with at most 16 packed rows.  Over 4-bit and 8-bit pools it also takes up to 48 rows
+    // (speculative verify: 8 query rows x 5 heads) as row blocks of 16 that each walk the codes again: the kernel that
+    // builds its operands from the codes is that much cheaper per key than the generic one.
     // (Sending the decode rows of a ragged fp16 batch through the tcgen05 kernel as well, as items of 128 rows with 5 in
     // use, was measured on the benchmark step: the attention stage takes the same 28.0 ms of the step's 83.)
-    const int dec_rows = q4_decode_kernel_applies(p, quant) ? 48 : 16;
+    const int dec_rows = qdec_kernel_applies(p, quant) ? 48 : 16;
     if (max_rows <= dec_rows) return attn_pass(ctx, st, p, total_rows, max_rows, 0, dec_rows, true, quant, &off);
     if (!p.cu_q) return attn_pass(ctx, st, p, total_rows, max_rows, 0, 1 << 30, false, quant, &off);
     // Ragged batch with both classes: the decode-class pass (bound by HBM) is issued on the context's second stream and

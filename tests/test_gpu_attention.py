@@ -306,3 +306,36 @@ def test_attention_many_short_sequences(ctx):
     worst = float((np.abs(g - w) / allowed).max())
     print(f"worst violation of the per-sequence bar: {worst:.3f}")
     assert worst <= 1.0
+
+
+@pytest.mark.parametrize("bits", [4, 8])
+@pytest.mark.parametrize("q_len,nq,nkv", [(1, 16, 2), (1, 40, 8), (2, 40, 8), (1, 32, 2), (9, 40, 8), (3, 10, 10)])
+def test_attention_quantised_decode_edges(ctx, bits, q_len, nq, nkv):
+    """The decode-class kernel over 4- and 8-bit pools at the edges of its tiles: contexts around the 16 keys of a warp, the
+    64 of a tile and the 256 of a page; row blocks of 8 that are full, partial and several; every row of a page past a
+    sequence holds scales that are not numbers.  Bar: the repository's for quantised pools."""
+    from oracle import oracle as O
+    torch = _torch()
+    hd, bsz = 128, 13
+    c = _make_case(4000 + 10 * bits + q_len + nq, [0, 1, 14, 15, 16, 17, 62, 63, 64, 65, 255, 256, 3000], q_len, nq, nkv)
+    groups, pages = nkv * hd // 32, c["kc"].shape[0]
+    pools = []
+    for x in ("kc", "vc"):
+        codes, scales = O.quant_groups(c[x].reshape(-1), bits)
+        pools += [codes.reshape(pages, 256, groups * bits).copy(), scales.reshape(pages, 256, groups).copy()]
+    live = np.zeros((pages, 256), bool)
+    for b in range(bsz):
+        for pos in range(int(c["seqlens"][b]) + q_len):
+            live[c["block_table"][b, pos // 256], pos % 256] = True
+    for i in (1, 3):
+        pools[i][~live] = np.nan
+    d = [H.to_dev(x.view(np.int32) if x.dtype == np.uint32 else x) for x in pools]
+    o = torch.full(c["q"].shape, float("nan"), dtype=torch.float16, device="cuda")
+    ctx.bighead_attn_paged_q(H.to_dev(c["q"]), H.to_dev(c["k"]), H.to_dev(c["v"]), *d, H.to_dev(c["block_table"]),
+                             H.to_dev(c["seqlens"]), o, nkv)
+    ctx.poll_status()
+    got = o.cpu().numpy()
+    O.quant_cache_paged(c["k"], pools[0], pools[1], c["v"], pools[2], pools[3], c["seqlens"], c["block_table"], bits, bits)
+    want = O.attn_paged(c["q"], None, None, c["block_table"], c["seqlens"], nkv=nkv, quant=(*pools, bits))
+    assert np.isfinite(got).all()
+    assert _close(got, want, TOL_QUANT) <= 1.0
