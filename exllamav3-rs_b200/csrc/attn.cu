@@ -9,6 +9,27 @@ namespace {
 
 using namespace exl3;
 
+// Inclusive scan over the 1024 threads of the block: three barriers instead of the twenty of a scan through shared memory
+// (the list is built in one block in front of the attention kernel, so its latency is the call's).
+__device__ __forceinline__ int plan_scan(int v, int* s_warp)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    #pragma unroll
+    for (int o = 1; o < 32; o <<= 1) { const int u = __shfl_up_sync(0xffffffffu, v, o); if (lane >= o) v += u; }
+    if (lane == 31) s_warp[warp] = v;
+    __syncthreads();
+    if (warp == 0) {
+        int w = s_warp[lane];
+        #pragma unroll
+        for (int o = 1; o < 32; o <<= 1) { const int u = __shfl_up_sync(0xffffffffu, w, o); if (lane >= o) w += u; }
+        s_warp[lane] = w;
+    }
+    __syncthreads();
+    if (warp > 0) v += s_warp[warp - 1];
+    __syncthreads();
+    return v;
+}
+
 // Builds the split-KV work list from the REAL sequence lengths (one CTA; bsz is small next to the KV walk).
 // Each sequence gets ceil(total_k / chunk) splits per row block, with chunk sized so that the list has about
 // `target_items` entries; the reference sizes its splits from the padded block-table width instead
@@ -20,9 +41,11 @@ __global__ void __launch_bounds__(1024) attn_plan_kernel(const int32_t* __restri
                                                          int max_items, AttnPlan* plan, AttnItem* items, int* seq_base,
                                                          int* seq_splits, int* order, int causal, int slots, int* status)
 {
+    pdl_enter();
     __shared__ long long s_total;
     __shared__ int s_scan[1024];
     __shared__ int s_cursor[1024];
+    __shared__ int s_warp[32];
     __shared__ int s_carry, s_chunk;
     const int tid = threadIdx.x;
     if (tid == 0) { s_total = 0; s_carry = 0; }
@@ -83,15 +106,8 @@ __global__ void __launch_bounds__(1024) attn_plan_kernel(const int32_t* __restri
             sp = (rb > 0 && tk > 0) ? (tk + chunk - 1) / chunk : 1;
         }
         const int cnt = rb * sp;
-        s_scan[tid] = cnt;
-        __syncthreads();
-        for (int o = 1; o < 1024; o <<= 1) {                   // inclusive Hillis-Steele scan
-            int v = tid >= o ? s_scan[tid - o] : 0;
-            __syncthreads();
-            s_scan[tid] += v;
-            __syncthreads();
-        }
-        const int base = s_carry + s_scan[tid] - cnt;
+        const int incl = plan_scan(cnt, s_warp);
+        const int base = s_carry + incl - cnt;
         if (b < bsz) {
             seq_base[b] = base;
             seq_splits[b] = sp;
@@ -101,7 +117,7 @@ __global__ void __launch_bounds__(1024) attn_plan_kernel(const int32_t* __restri
             }
         }
         __syncthreads();
-        if (tid == 1023) s_carry += s_scan[1023];
+        if (tid == 1023) s_carry += incl;
         __syncthreads();
     }
     // Launch order: longest items first (counting sort by key tiles, most first).  Items differ in length - last splits,
@@ -126,15 +142,7 @@ __global__ void __launch_bounds__(1024) attn_plan_kernel(const int32_t* __restri
     __syncthreads();
     {
         const int cnt = s_scan[tid];
-        __syncthreads();
-        for (int o = 1; o < 1024; o <<= 1) {                   // inclusive scan over the bins
-            int v = tid >= o ? s_scan[tid - o] : 0;
-            __syncthreads();
-            s_scan[tid] += v;
-            __syncthreads();
-        }
-        const int excl = s_scan[tid] - cnt;
-        __syncthreads();
+        const int excl = plan_scan(cnt, s_warp) - cnt;
         s_scan[tid] = excl;                                    // first position of bin tid
         __syncthreads();
     }
@@ -144,6 +152,7 @@ __global__ void __launch_bounds__(1024) attn_plan_kernel(const int32_t* __restri
     }
     if (tid == 0) {
         plan->n_items = n_items;
+        plan->next = 0;
         plan->chunk = chunk;
         // the host sizes the list from bounds on the batch; a list that does not fit would silently drop work, so it is
         // reported through the status word like a device-side wait that ran out
@@ -155,7 +164,10 @@ __global__ void __launch_bounds__(1024) attn_plan_kernel(const int32_t* __restri
 template <int D>
 __global__ void __launch_bounds__(256) attn_combine_kernel(const AttnParams p, int rows_per_cta, int total_rows)
 {
+    pdl_enter();
     const int lane = threadIdx.x & 31;
+    // the attention kernel in front has handed out all its units: the work list is ready for the next layer's
+    if (blockIdx.x == 0 && threadIdx.x == 0) const_cast<AttnPlan*>(p.plan)->next = 0;
     const long long w = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
     if (w >= (long long)total_rows * p.nq) return;
     const int row = (int)(w / p.nq), head = (int)(w % p.nq);
@@ -214,7 +226,7 @@ __global__ void __launch_bounds__(256) attn_combine_kernel(const AttnParams p, i
 }
 
 template <int D, int WM, int WN, int QB>
-cudaError_t launch_attn(const AttnParams& p, dim3 grid, cudaStream_t st)
+cudaError_t launch_attn(exl3_ctx* ctx, const AttnParams& p, dim3 grid, cudaStream_t st)
 {
     constexpr int bytes = AttnSmem<D, QB>::BYTES;
     auto kern = attn_paged_kernel<D, WM, WN, QB>;
@@ -226,8 +238,7 @@ cudaError_t launch_attn(const AttnParams& p, dim3 grid, cudaStream_t st)
         if (e != cudaSuccess) return e;
         if (dev >= 0 && dev < 64) configured[dev] = true;
     }
-    kern<<<grid, AT_THREADS, bytes, st>>>(p);
-    return cudaPeekAtLastError();
+    return exl3_launch(ctx, kern, grid, AT_THREADS, bytes, st, p);
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
@@ -313,7 +324,7 @@ cudaError_t launch_attn_tc2(exl3_ctx* ctx, const AttnParams& p, int max_items, c
 // decode-class kernel over 4-bit and 8-bit pools: tensor maps over the code planes ([tokens][nkv * 4 * bits] words, copied in
 // the swizzle of a head's 64 or 128 bytes) and the scale planes ([tokens][nkv * 4] halves, copied in 16-byte pairs of heads)
 template <int B, int NB>
-cudaError_t launch_attn_qdec(const AttnParams& p, dim3 grid, cudaStream_t st)
+cudaError_t launch_attn_qdec(exl3_ctx* ctx, const AttnParams& p, dim3 grid, cudaStream_t st)
 {
     EncodeTiledFn enc = attn_encode_tiled();
     if (!enc) return cudaErrorNotSupported;
@@ -342,8 +353,7 @@ cudaError_t launch_attn_qdec(const AttnParams& p, dim3 grid, cudaStream_t st)
         if (e != cudaSuccess) return e;
         if (dev >= 0 && dev < 64) configured[dev] = true;
     }
-    kern<<<grid, QD_THREADS, bytes, st>>>(maps[0], maps[1], maps[2], maps[3], p);
-    return cudaPeekAtLastError();
+    return exl3_launch(ctx, kern, grid, QD_THREADS, bytes, st, maps[0], maps[1], maps[2], maps[3], p);
 }
 
 bool qdec_kernel_applies(const AttnParams& p, bool quant);
@@ -424,27 +434,26 @@ int attn_pass(exl3_ctx* ctx, cudaStream_t st, AttnParams p, int total_rows, int 
 
     static const bool no_lpt = getenv("EXL3_TUNE_NO_LPT") != nullptr;
     if (!(keep && ctx->plan_valid[cls])) {
-        attn_plan_kernel<<<1, 1024, 0, st>>>(p.seqlens, p.cu_q, p.bsz, p.q_len, p.kv_append, G, rows_per_cta, rows_lo, rows_hi,
+        exl3_launch(ctx, attn_plan_kernel, 1, 1024, 0, st, p.seqlens, p.cu_q, p.bsz, p.q_len, p.kv_append, G, rows_per_cta, rows_lo, rows_hi,
                                               use_tc ? ATC_TN : AT_TK, target_items, max_items, plan, items, seq_base, seq_splits, order, no_lpt ? -1 : (p.causal ? 1 : 0),
                                               (use_tc && !tc_items) ? grid_x : 0, ctx->status);
         ctx->launches++;
         if (keep) ctx->plan_valid[cls] = 1;
     }
+    exl3_chain_scope chain(ctx);
     dim3 grid(grid_x, p.nkv);
     cudaError_t e;
-    if (!use_tc && cudaMemsetAsync(&plan->next, 0, sizeof(int), st) != cudaSuccess)      // the persistent kernel's work counter
-        return exl3_fail(ctx, EXL3_ERR_CUDA, "attention: cudaMemsetAsync failed");
     if (use_tc) e = tc_256 ? launch_attn_tc(ctx, p, max_items, st) : launch_attn_tc2(ctx, p, max_items, st);
     else if (use_qdec)
-        e = q4 ? (rows_per_cta == 8 ? launch_attn_qdec<4, 1>(p, grid, st) : launch_attn_qdec<4, 2>(p, grid, st))
-               : (rows_per_cta == 8 ? launch_attn_qdec<8, 1>(p, grid, st) : launch_attn_qdec<8, 2>(p, grid, st));
-    else if (q4)    e = decode_shape ? launch_attn<128, 1, 4, 4>(p, grid, st) : launch_attn<128, 4, 1, 4>(p, grid, st);
-    else if (quant) e = decode_shape ? launch_attn<128, 1, 4, 8>(p, grid, st) : launch_attn<128, 4, 1, 8>(p, grid, st);
-    else            e = decode_shape ? launch_attn<128, 1, 4, 0>(p, grid, st) : launch_attn<128, 4, 1, 0>(p, grid, st);
+        e = q4 ? (rows_per_cta == 8 ? launch_attn_qdec<4, 1>(ctx, p, grid, st) : launch_attn_qdec<4, 2>(ctx, p, grid, st))
+               : (rows_per_cta == 8 ? launch_attn_qdec<8, 1>(ctx, p, grid, st) : launch_attn_qdec<8, 2>(ctx, p, grid, st));
+    else if (q4)    e = decode_shape ? launch_attn<128, 1, 4, 4>(ctx, p, grid, st) : launch_attn<128, 4, 1, 4>(ctx, p, grid, st);
+    else if (quant) e = decode_shape ? launch_attn<128, 1, 4, 8>(ctx, p, grid, st) : launch_attn<128, 4, 1, 8>(ctx, p, grid, st);
+    else            e = decode_shape ? launch_attn<128, 1, 4, 0>(ctx, p, grid, st) : launch_attn<128, 4, 1, 0>(ctx, p, grid, st);
     ctx->launches++;
     if (e != cudaSuccess) { cudaGetLastError(); return exl3_fail(ctx, EXL3_ERR_CUDA, cudaGetErrorString(e)); }
     const long long warps = (long long)total_rows * p.nq;
-    attn_combine_kernel<128><<<(unsigned)((warps + 7) / 8), 256, 0, st>>>(p, rows_per_cta, total_rows);
+    exl3_launch(ctx, attn_combine_kernel<128>, (unsigned)((warps + 7) / 8), 256, 0, st, p, rows_per_cta, total_rows);
     ctx->launches++;
     return exl3_check_launch(ctx, "attention");
 }
@@ -481,8 +490,11 @@ int attn_impl(exl3_ctx* ctx, cudaStream_t st, AttnParams p, int total_rows, int 
     // step the attention stage takes the sum of the two kernels' times).
     if (cudaEventRecord(ctx->ev_fork, st) != cudaSuccess || cudaStreamWaitEvent(ctx->aux_stream, ctx->ev_fork, 0) != cudaSuccess)
         return exl3_fail(ctx, EXL3_ERR_CUDA, "attention: stream fork failed");
+    ctx->chain_break = 1;
     int rc = attn_pass(ctx, ctx->aux_stream, p, total_rows, dec_rows, 0, dec_rows, true, quant, &off);
+    ctx->chain_break = 1;
     int rc2 = rc == EXL3_OK ? attn_pass(ctx, st, p, total_rows, max_rows, dec_rows, 1 << 30, false, quant, &off) : rc;
+    ctx->chain_break = 1;
     // always join, also after an error, so that a capture in progress stays well-formed
     if (cudaEventRecord(ctx->ev_join, ctx->aux_stream) != cudaSuccess || cudaStreamWaitEvent(st, ctx->ev_join, 0) != cudaSuccess)
         return exl3_fail(ctx, EXL3_ERR_CUDA, "attention: stream join failed");
@@ -522,6 +534,7 @@ extern "C" int exl3_bighead_attn_paged(exl3_ctx* ctx, exl3_stream stream, const 
                                         nkv, hd, pages, pages_per_seq);
         if (rc) return rc;
     }
+    exl3_chain_scope chain(ctx, append > 0);
     AttnParams p;
     memset(&p, 0, sizeof(p));
     p.q = (const half*)q; p.o = (half*)o; p.kc = (const half*)k_cache; p.vc = (const half*)v_cache;
@@ -554,6 +567,7 @@ extern "C" int exl3_bighead_attn_paged_q(exl3_ctx* ctx, exl3_stream stream, cons
                                     nkv * hd, pages, pages_per_seq, k_bits, v_bits, EXL3_PAGE, 0.0f, 1);
         if (rc) return rc;
     }
+    exl3_chain_scope chain(ctx, append > 0);
     AttnParams p;
     memset(&p, 0, sizeof(p));
     p.q = (const half*)q; p.o = (half*)o;

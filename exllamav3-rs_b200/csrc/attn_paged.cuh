@@ -103,6 +103,7 @@ struct AttnSmem {
 template <int D, int WM, int WN, int QB>
 __global__ void __launch_bounds__(AT_THREADS, (QB == 4 && WN == 4) ? AT_Q4_DECODE_BLOCKS : 1) attn_paged_kernel(const AttnParams p)
 {
+    pdl_enter();
     using SM = AttnSmem<D, QB>;
     constexpr bool QUANT = QB > 0;
     constexpr int ROWS = 16 * WM;

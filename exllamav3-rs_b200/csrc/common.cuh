@@ -42,7 +42,47 @@ struct exl3_ctx {
     size_t plan_slot_bytes;
     int plan_keep;
     int plan_valid[2];
+    // Programmatic dependent launches (exl3_launch): set while the work in front of a launch on its stream is known to be a
+    // kernel of this library - inside a step, and after the first launch of a call of several - and broken for one launch
+    // where a stream forks or joins.
+    int chain, chain_break;
     char err[256];
+};
+
+// Every kernel that exl3_launch starts begins with this: it lets the next kernel of the chain be set up on the SMs that fall
+// free, and waits until the kernels before it are complete and their writes visible.  Nothing of global memory is touched
+// before it (weights excepted, which no kernel of a chain writes).
+__device__ __forceinline__ void pdl_enter()
+{
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+// Launch as a programmatic dependent of the previous kernel where the context says that there is one: the launch then
+// overlaps the tail of its predecessor.  A decode step of a small model is some fifteen kernels of 3 to 10 us per layer
+// (28 layers, hidden 1024, 8 rows: 2.79 -> 2.23 ms; verify step of 64 layers at 32 rows: 20.55 -> 20.11 ms).
+static inline bool exl3_chained(exl3_ctx* ctx)
+{
+    const bool on = ctx->chain && !ctx->chain_break;
+    ctx->chain_break = 0;
+    return on;
+}
+template <typename... P, typename... A>
+static inline cudaError_t exl3_launch(exl3_ctx* ctx, void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr; cfg.numAttrs = exl3_chained(ctx) ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+}
+// Marks the launches of a scope as a chain.
+struct exl3_chain_scope {
+    exl3_ctx* c; int old;
+    explicit exl3_chain_scope(exl3_ctx* ctx, bool on = true) : c(ctx), old(ctx->chain) { if (on) c->chain = 1; }
+    ~exl3_chain_scope() { c->chain = old; }
 };
 
 static inline int exl3_fail(exl3_ctx* ctx, int code, const char* msg)

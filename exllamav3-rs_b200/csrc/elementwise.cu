@@ -102,6 +102,7 @@ __global__ void __launch_bounds__(1024) rms_norm_kernel(const TI* __restrict__ x
                                                         TO* __restrict__ y, float* __restrict__ r, float eps,
                                                         float cbias, float cscale, int dim)
 {
+    pdl_enter();
     __shared__ float sh[32];
     const int cols = dim >> 2;
     const size_t row = blockIdx.x;
@@ -186,6 +187,7 @@ template <typename TI, bool RES_IN>
 __global__ void __launch_bounds__(1024) rms_norm_had_kernel(const TI* __restrict__ x, const half* __restrict__ w, float* __restrict__ r,
                                                             float eps, float cbias, float cscale, int dim, const exl3_pre_act pre)
 {
+    pdl_enter();
     __shared__ float sh[32];
     const int cols = dim >> 2, lane = threadIdx.x & 31;
     const size_t row = blockIdx.x;
@@ -248,6 +250,7 @@ __global__ void __launch_bounds__(256) rope_kernel(const half* q, const half* k,
                                                    const half* __restrict__ k_norm, float norm_eps, float norm_cbias,
                                                    int rope_mode, float attn_factor, int rows, int seq, int nq, int nk)
 {
+    pdl_enter();
     constexpr int HD = EPL * 32;
     const int lane = threadIdx.x & 31;
     const long long gw = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
@@ -321,6 +324,7 @@ __global__ void __launch_bounds__(256) rope_kernel(const half* q, const half* k,
 __global__ void __launch_bounds__(256) silu_mul_kernel(const half2* __restrict__ x, const half2* __restrict__ y,
                                                        half2* __restrict__ z, long long n4)
 {
+    pdl_enter();
     long long i = (long long)blockIdx.x * 256 + threadIdx.x;
     if (i >= n4) return;
     uint4 xr = reinterpret_cast<const uint4*>(x)[i], yr = reinterpret_cast<const uint4*>(y)[i], o;
@@ -352,6 +356,7 @@ constexpr int SH_BLOCKS = 4;          // 128-blocks per warp: their loads are al
 __global__ void __launch_bounds__(256) silu_mul_had_kernel(const half* __restrict__ x, const half* __restrict__ y,
                                                            const half* __restrict__ suh, half* __restrict__ a_had, long long blocks, int bpr)
 {
+    pdl_enter();
     const int lane = threadIdx.x & 31;
     const long long blk0 = ((long long)blockIdx.x * 8 + (threadIdx.x >> 5)) * SH_BLOCKS;
     if (blk0 >= blocks) return;
@@ -484,8 +489,8 @@ static int rms_norm_impl(exl3_ctx* ctx, exl3_stream stream, const void* x, int x
     const half* wp = (const half*)w;
 #define RN_LAUNCH(TI, TO)                                                                                              \
     do {                                                                                                               \
-        if (r) rms_norm_kernel<TI, TO, true><<<rows, threads, 0, st>>>((const TI*)x, wp, (TO*)y, r, eps, cbias, cscale, dim); \
-        else   rms_norm_kernel<TI, TO, false><<<rows, threads, 0, st>>>((const TI*)x, wp, (TO*)y, r, eps, cbias, cscale, dim); \
+        if (r) exl3_launch(ctx, rms_norm_kernel<TI, TO, true>, rows, threads, 0, st, (const TI*)x, wp, (TO*)y, r, eps, cbias, cscale, dim); \
+        else   exl3_launch(ctx, rms_norm_kernel<TI, TO, false>, rows, threads, 0, st, (const TI*)x, wp, (TO*)y, r, eps, cbias, cscale, dim); \
     } while (0)
     if (x_fp32 && y_fp32) RN_LAUNCH(float, float);
     else if (x_fp32)      RN_LAUNCH(float, half);
@@ -531,7 +536,7 @@ extern "C" int exl3_rope(exl3_ctx* ctx, exl3_stream stream, void* q, void* out_q
     cudaStream_t st = (cudaStream_t)stream;
     const int nk_eff = k ? nk : 0;
 #define ROPE_LAUNCH(E)                                                                                                 \
-    rope_kernel<E><<<grid, 256, 0, st>>>((const half*)q, (const half*)k, (half*)(out_q ? out_q : q), (half*)(out_k ? out_k : k), inv_freq, n_freq, position, positions, row_pos, \
+    exl3_launch(ctx, rope_kernel<E>, grid, 256, 0, st, (const half*)q, (const half*)k, (half*)(out_q ? out_q : q), (half*)(out_k ? out_k : k), inv_freq, n_freq, position, positions, row_pos, \
                                          (const half*)q_norm, (const half*)k_norm, norm_eps, norm_constant_bias,       \
                                          rope_mode, attn_factor, rows, seq, nq, nk_eff)
     if (hd == 64) ROPE_LAUNCH(2); else if (hd == 128) ROPE_LAUNCH(4); else ROPE_LAUNCH(8);
@@ -550,7 +555,7 @@ extern "C" int exl3_silu_mul(exl3_ctx* ctx, exl3_stream stream, const void* x, c
     cudaStream_t st = (cudaStream_t)stream;
     const long long n8 = numel / 8;
     if (n8) {
-        silu_mul_kernel<<<(unsigned)((n8 + 255) / 256), 256, 0, st>>>((const half2*)x, (const half2*)y, (half2*)z, n8);
+        exl3_launch(ctx, silu_mul_kernel, (unsigned)((n8 + 255) / 256), 256, 0, st, (const half2*)x, (const half2*)y, (half2*)z, n8);
         ctx->launches++;
     }
     if (numel % 8) {
@@ -612,11 +617,11 @@ int exl3_rms_norm_pre(exl3_ctx* ctx, exl3_stream stream, const void* x, int x_fp
     cudaStream_t st = (cudaStream_t)stream;
     const half* wp = (const half*)w;
     if (x_fp32) {
-        if (r) rms_norm_had_kernel<float, true><<<rows, threads, 0, st>>>((const float*)x, wp, r, eps, cbias, cscale, dim, *pre);
-        else   rms_norm_had_kernel<float, false><<<rows, threads, 0, st>>>((const float*)x, wp, r, eps, cbias, cscale, dim, *pre);
+        if (r) exl3_launch(ctx, rms_norm_had_kernel<float, true>, rows, threads, 0, st, (const float*)x, wp, r, eps, cbias, cscale, dim, *pre);
+        else   exl3_launch(ctx, rms_norm_had_kernel<float, false>, rows, threads, 0, st, (const float*)x, wp, r, eps, cbias, cscale, dim, *pre);
     } else {
-        if (r) rms_norm_had_kernel<half, true><<<rows, threads, 0, st>>>((const half*)x, wp, r, eps, cbias, cscale, dim, *pre);
-        else   rms_norm_had_kernel<half, false><<<rows, threads, 0, st>>>((const half*)x, wp, r, eps, cbias, cscale, dim, *pre);
+        if (r) exl3_launch(ctx, rms_norm_had_kernel<half, true>, rows, threads, 0, st, (const half*)x, wp, r, eps, cbias, cscale, dim, *pre);
+        else   exl3_launch(ctx, rms_norm_had_kernel<half, false>, rows, threads, 0, st, (const half*)x, wp, r, eps, cbias, cscale, dim, *pre);
     }
     ctx->launches++;
     return exl3_check_launch(ctx, "rms_norm (fused transform)");
@@ -629,7 +634,7 @@ int exl3_silu_mul_pre(exl3_ctx* ctx, exl3_stream stream, const void* x, const vo
     EXL3_REQUIRE(aligned16(x) && aligned16(y), "silu_mul (fused transform): pointers must be 16-byte aligned");
     if (rows == 0) return EXL3_OK;
     const long long blocks = (long long)rows * (dim / 128);
-    silu_mul_had_kernel<<<(unsigned)((blocks + 8 * SH_BLOCKS - 1) / (8 * SH_BLOCKS)), 256, 0, (cudaStream_t)stream>>>((const half*)x, (const half*)y, pre->suh[0], pre->a_had[0],
+    exl3_launch(ctx, silu_mul_had_kernel, (unsigned)((blocks + 8 * SH_BLOCKS - 1) / (8 * SH_BLOCKS)), 256, 0, (cudaStream_t)stream, (const half*)x, (const half*)y, pre->suh[0], pre->a_had[0],
                                                                                       blocks, dim / 128);
     ctx->launches++;
     return exl3_check_launch(ctx, "silu_mul (fused transform)");

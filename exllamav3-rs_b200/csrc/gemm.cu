@@ -131,6 +131,7 @@ struct ProloguePlainArgs { const half* suh[TC_MAX_SEG]; half* a_had[TC_MAX_SEG];
 
 __global__ void __launch_bounds__(256) gemm_prologue_plain_kernel(const half* __restrict__ A, const ProloguePlainArgs args, int k)
 {
+    pdl_enter();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const size_t row = blockIdx.x;
     const half* __restrict__ suh = args.suh[blockIdx.y];
@@ -186,6 +187,7 @@ constexpr int GP_PAIRS = 4;          // block pairs per warp: their loads are al
 __global__ void __launch_bounds__(256) gemm_prologue_mma_kernel(const half* __restrict__ A, const ProloguePlainArgs args, int k,
                                                                 long long pairs_total)
 {
+    pdl_enter();
     __shared__ __align__(16) uint8_t stage[8][512];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, t = lane & 3;
@@ -307,11 +309,14 @@ cudaError_t launch_tc(const CUtensorMap* amap, const CUtensorMap* rmap, const CU
     cfg.blockDim = dim3(TC_THREADS);
     cfg.dynamicSmemBytes = bytes;
     cfg.stream = st;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = CTAS; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    // a programmatic dependent of the kernel that writes the transformed activations, which directly precedes it
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = 2;
     return cudaLaunchKernelEx(&cfg, kern, amap[0], amap[1], amap[2], rmap[0], rmap[1], rmap[2], cmap[0], cmap[1], cmap[2], p);
 }
 
@@ -414,9 +419,9 @@ int gemm_tc_rows(exl3_ctx* ctx, cudaStream_t st, const half* A, int nseg, const 
         // nothing to launch
     } else if (k % 256 == 0 && all_signed) {
         const long long pairs = (long long)m * (k / 256);
-        gemm_prologue_mma_kernel<<<dim3((unsigned)((pairs + 8 * GP_PAIRS - 1) / (8 * GP_PAIRS)), nseg), 256, 0, st>>>(A, pa, k, pairs);
+        exl3_launch(ctx, gemm_prologue_mma_kernel, dim3((unsigned)((pairs + 8 * GP_PAIRS - 1) / (8 * GP_PAIRS)), nseg), 256, 0, st, A, pa, k, pairs);
     } else
-        gemm_prologue_plain_kernel<<<dim3(m, nseg), 256, 0, st>>>(A, pa, k);
+        exl3_launch(ctx, gemm_prologue_plain_kernel, dim3(m, nseg), 256, 0, st, A, pa, k);
     if (!pre) ctx->launches++;
     p.status = ctx->status; p.m = m; p.k = k; p.c_fp32 = c_fp32;
     cudaError_t e = launch_tc_k(K, cb, ctx->use_pair != 0, bn, amap, rmap, cmap, p, blocks, st);
@@ -533,7 +538,7 @@ int gemm_decode_rows(exl3_ctx* ctx, cudaStream_t st, const half* A, int nseg, co
     if (!p.partial) return exl3_fail(ctx, EXL3_ERR_WORKSPACE, "exl3_gemm: context scratch too small for the partial sums");
     p.counters = ctx->counters; p.status = ctx->status; p.m = m; p.k = k; p.c_fp32 = c_fp32;
     p.rowsum_parts = GD_PRO_SPLIT;
-    gemm_decode_prologue_kernel<<<dim3(8 * mt, nseg, GD_PRO_SPLIT), 256, 0, st>>>(A, pa, m, k);
+    exl3_launch(ctx, gemm_decode_prologue_kernel, dim3(8 * mt, nseg, GD_PRO_SPLIT), 256, 0, st, A, pa, m, k);
     ctx->launches++;
     cudaError_t e = launch_decode_k(K, cb, mt, rmap, p, grid, st);
     ctx->launches++;

@@ -221,7 +221,7 @@ __device__ __forceinline__ void gd_prologue_row(const half* __restrict__ Arow, c
 static __global__ void __launch_bounds__(256) gemm_decode_prologue_kernel(const half* __restrict__ A, const GemmDecodePrologueArgs args,
                                                                    int m, int k)
 {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    pdl_enter();
     const int b = blockIdx.x, seg = blockIdx.y;
     gd_prologue_row(A + (size_t)b * k, args.suh[seg], args.a_frag[seg], args.rowsum[seg], b, b < m, k, blockIdx.z, gridDim.z);
 }
@@ -299,6 +299,7 @@ __global__ void __launch_bounds__(GD_THREADS, 1) gemm_decode_kernel(const __grid
                                                                    const GemmDecodeParams p)
 {
     using SM = GdSmem<K, MT>;
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     extern __shared__ uint8_t gd_smem_unaligned[];
     uint8_t* smem = gd_smem_unaligned + ((128u - (smem_u32(gd_smem_unaligned) & 127u)) & 127u);
     float* red = reinterpret_cast<float*>(smem + SM::OFF_RED);

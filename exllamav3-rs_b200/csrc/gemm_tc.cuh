@@ -267,6 +267,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const __grid_con
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + SM::OFF_TMEM);
     __shared__ int s_failed;
 
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int rank = PAIR ? (int)cluster_ctarank() : 0;                  // 0 = leader of the pair
     const int slab = PAIR ? (int)(blockIdx.x >> 1) : (int)blockIdx.x;
@@ -327,6 +328,9 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const __grid_con
         // ===== activation producer: one or two tiled TMA loads per K step
         if (lane == 0) {
             const uint32_t a_bytes = (two_tiles ? 2u : 1u) * TC_A_TILE * CTAS;     // what lands on the leader's barrier
+            // The set-up above and the codes (the other producer) do not depend on the kernel that writes the activations;
+            // everything this kernel writes depends on the activations.
+            asm volatile("griddepcontrol.wait;" ::: "memory");
             int sa = 0;
             uint32_t par_ae = 1;                                  // a_empty is waited from the second round on
             for (int ks = 0; ks < ksteps; ++ks) {

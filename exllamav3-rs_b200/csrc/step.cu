@@ -199,6 +199,7 @@ static int step_forward_impl(exl3_ctx* ctx, exl3_stream stream, const exl3_model
     STEP_TRY(exl3_embed(ctx, stream, b->ids, m->embed, s.resid, rows, hidden, m->vocab));
 
     STAGE(0);                           // descriptors and embedding
+    exl3_chain_scope chain(ctx);        // from here on every launch follows one of this library
     const half* pending = nullptr;      // output of the previous block's MLP, added to the residual by the next norm
     // (measured on the 27B-class shard: 84.6 against 85.3 ms at 1052 rows, but 22.7 against 22.5 ms at 32 rows, where the norm's
     // one CTA per row leaves the three transforms of a row to 32 CTAs: fused from 128 rows on)
