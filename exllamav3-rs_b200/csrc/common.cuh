@@ -109,9 +109,11 @@ static inline bool aligned16(const void* p) { return (((uintptr_t)p) & 15) == 0;
 
 // Transformed activations of up to three EXL3 tensors that share an input, written by the kernel that produces the input
 // (norm, activation) instead of by the GEMM's own transform launch: where each tensor's copy goes and its sign vector.
-struct exl3_pre_act { const half* suh[3]; half* a_had[3]; int nseg; };
-// gemm.cu: fills `pre` and returns true when exl3_gemm_fanout_pre can run these tensors at m rows (tensor-core path)
-bool exl3_tc_pre_buffers(exl3_ctx* ctx, int count, const exl3_linear* const* w, int m, exl3_pre_act* pre);
+// frag_rows = 0: rows of a_had, for the tensor-core GEMM.  frag_rows = 8 or 16: the decode GEMM's fragment order in a_frag,
+// where row slots from `rows` on are zero-filled.
+struct exl3_pre_act { const half* suh[3]; half* a_had[3]; uint32_t* a_frag[3]; int nseg, rows, frag_rows; };
+// gemm.cu: fills `pre` and returns true when exl3_gemm_fanout_pre can run these tensors at m rows
+bool exl3_pre_buffers(exl3_ctx* ctx, int count, const exl3_linear* const* w, int m, exl3_pre_act* pre);
 int exl3_gemm_fanout_pre(exl3_ctx* ctx, exl3_stream stream, int count, const exl3_linear* const* w, void* const* C, int m, int c_fp32);
 // elementwise.cu
 int exl3_rms_norm_pre(exl3_ctx* ctx, exl3_stream stream, const void* x, int x_fp32, const void* w, float* r, float eps,

@@ -351,7 +351,7 @@ cudaError_t launch_tc_k(int K, int cb, bool pair, int bn, const CUtensorMap* ama
 
 // Tensor-core path for rows [0, m) and `nseg` weight tensors that share the activations, k, bits and codebook:
 // one launch of the input transforms (each tensor has its own suh) and one of the tcgen05 kernel.
-// With `pre` the transformed activations are already in place (written into the buffers exl3_tc_pre_buffers named, by the
+// With `pre` the transformed activations are already in place (written into the buffers exl3_pre_buffers named, by the
 // kernel that produced the input), and the transform launch is skipped.
 int gemm_tc_rows(exl3_ctx* ctx, cudaStream_t st, const half* A, int nseg, const void* const* trellis, void* const* C,
                  const half* const* suh, const half* const* svh, const int* n, int m, int k, int K, int c_fp32, int cb,
@@ -488,7 +488,8 @@ cudaError_t launch_decode_k(int K, int cb, int mt, const CUtensorMap* rmap, cons
 // Decode path for m <= 16 rows and `nseg` weight tensors that share the activations, k, bits and codebook: one launch of
 // the input transforms (fragment order, one per tensor) and one of the streaming kernel over all their column blocks.
 int gemm_decode_rows(exl3_ctx* ctx, cudaStream_t st, const half* A, int nseg, const void* const* trellis, void* const* C,
-                     const half* const* suh, const half* const* svh, const int* n, int m, int k, int K, int c_fp32, int cb)
+                     const half* const* suh, const half* const* svh, const int* n, int m, int k, int K, int c_fp32, int cb,
+                     bool pre = false)
 {
     EncodeTiledFn enc = get_encode_tiled();
     if (!enc) return exl3_fail(ctx, EXL3_ERR_CUDA, "exl3_gemm: cuTensorMapEncodeTiled is not available from this driver");
@@ -538,8 +539,10 @@ int gemm_decode_rows(exl3_ctx* ctx, cudaStream_t st, const half* A, int nseg, co
     if (!p.partial) return exl3_fail(ctx, EXL3_ERR_WORKSPACE, "exl3_gemm: context scratch too small for the partial sums");
     p.counters = ctx->counters; p.status = ctx->status; p.m = m; p.k = k; p.c_fp32 = c_fp32;
     p.rowsum_parts = GD_PRO_SPLIT;
-    exl3_launch(ctx, gemm_decode_prologue_kernel, dim3(8 * mt, nseg, GD_PRO_SPLIT), 256, 0, st, A, pa, m, k);
-    ctx->launches++;
+    if (!pre) {
+        exl3_launch(ctx, gemm_decode_prologue_kernel, dim3(8 * mt, nseg, GD_PRO_SPLIT), 256, 0, st, A, pa, m, k);
+        ctx->launches++;
+    }
     cudaError_t e = launch_decode_k(K, cb, mt, rmap, p, grid, st);
     ctx->launches++;
     if (e != cudaSuccess) { cudaGetLastError(); return exl3_fail(ctx, EXL3_ERR_CUDA, cudaGetErrorString(e)); }
@@ -656,11 +659,37 @@ static bool tc_pre_applies(exl3_ctx* ctx, int count, const exl3_linear* const* w
     return true;
 }
 
-bool exl3_tc_pre_buffers(exl3_ctx* ctx, int count, const exl3_linear* const* w, int m, exl3_pre_act* pre)
+// The same for the decode GEMM (gemm_decode_rows).  Codebook 2 also needs the row sums of the transformed activations, which
+// the producers do not form; it keeps the separate transform.
+static bool decode_pre_applies(exl3_ctx* ctx, int count, const exl3_linear* const* w, int m)
 {
-    if (!tc_pre_applies(ctx, count, w, m)) return false;
+    if (!ctx || !w || count < 1 || count > GD_MAX_SEG || m < 1 || m > GD_MAX_M || !ctx->use_decode) return false;
+    for (int i = 0; i < count; ++i) {
+        if (!w[i] || !w[i]->trellis || !w[i]->suh || w[i]->cb == 2) return false;
+        if (w[i]->k != w[0]->k || w[i]->K != w[0]->K || w[i]->cb != w[0]->cb) return false;
+        if (w[i]->k % 128 != 0 || w[i]->n % (count > 1 ? TC_BN : 128) != 0) return false;
+        if (w[i]->K < 1 || w[i]->K > 8 || !aligned16(w[i]->trellis) || !aligned16(w[i]->suh) || !aligned16(w[i]->svh)) return false;
+    }
+    return true;
+}
+
+bool exl3_pre_buffers(exl3_ctx* ctx, int count, const exl3_linear* const* w, int m, exl3_pre_act* pre)
+{
     size_t off = 0;
-    pre->nseg = count;
+    pre->nseg = count; pre->rows = m; pre->frag_rows = 0;
+    for (int i = 0; i < 3; ++i) pre->a_frag[i] = nullptr;
+    if (decode_pre_applies(ctx, count, w, m)) {
+        const int mt = m <= 8 ? 1 : 2;
+        pre->frag_rows = 8 * mt;
+        for (int i = 0; i < 3; ++i) { pre->suh[i] = nullptr; pre->a_had[i] = nullptr; }
+        for (int i = 0; i < count; ++i) {
+            pre->a_frag[i] = (uint32_t*)exl3_ws_take(ctx, &off, (size_t)mt * w[0]->k * 32);
+            if (!exl3_ws_take(ctx, &off, (size_t)GD_PRO_SPLIT * mt * 8 * 4) || !pre->a_frag[i]) return false;
+            pre->suh[i] = (const half*)w[i]->suh;
+        }
+        return true;
+    }
+    if (!tc_pre_applies(ctx, count, w, m)) return false;
     for (int i = 0; i < 3; ++i) { pre->suh[i] = nullptr; pre->a_had[i] = nullptr; }
     for (int i = 0; i < count; ++i) {
         pre->a_had[i] = (half*)exl3_ws_take(ctx, &off, (size_t)m * w[0]->k * 2);
@@ -672,12 +701,14 @@ bool exl3_tc_pre_buffers(exl3_ctx* ctx, int count, const exl3_linear* const* w, 
 
 int exl3_gemm_fanout_pre(exl3_ctx* ctx, exl3_stream stream, int count, const exl3_linear* const* w, void* const* C, int m, int c_fp32)
 {
-    EXL3_REQUIRE(tc_pre_applies(ctx, count, w, m) && C, "exl3_gemm (activations transformed by the producer): not applicable to these tensors");
+    const bool decode = decode_pre_applies(ctx, count, w, m);
+    EXL3_REQUIRE((decode || tc_pre_applies(ctx, count, w, m)) && C, "exl3_gemm (activations transformed by the producer): not applicable to these tensors");
     const void* tr[TC_MAX_SEG]; const half* suh[TC_MAX_SEG]; const half* svh[TC_MAX_SEG]; int n[TC_MAX_SEG];
     for (int i = 0; i < count; ++i) {
         EXL3_REQUIRE(C[i] && aligned16(C[i]), "exl3_gemm: bad output pointer");
         tr[i] = w[i]->trellis; suh[i] = (const half*)w[i]->suh; svh[i] = (const half*)w[i]->svh; n[i] = w[i]->n;
     }
+    if (decode) return gemm_decode_rows(ctx, (cudaStream_t)stream, nullptr, count, tr, C, suh, svh, n, m, w[0]->k, w[0]->K, c_fp32, w[0]->cb, true);
     return gemm_tc_rows(ctx, (cudaStream_t)stream, nullptr, count, tr, C, suh, svh, n, m, w[0]->k, w[0]->K, c_fp32, w[0]->cb, true);
 }
 

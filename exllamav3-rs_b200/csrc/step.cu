@@ -202,8 +202,14 @@ static int step_forward_impl(exl3_ctx* ctx, exl3_stream stream, const exl3_model
     exl3_chain_scope chain(ctx);        // from here on every launch follows one of this library
     const half* pending = nullptr;      // output of the previous block's MLP, added to the residual by the next norm
     // (measured on the 27B-class shard: 84.6 against 85.3 ms at 1052 rows, but 22.7 against 22.5 ms at 32 rows, where the norm's
-    // one CTA per row leaves the three transforms of a row to 32 CTAs: fused from 128 rows on)
-    const bool fuse_pre = ctx->fuse_transform != 0 && rows >= 128;
+    // one CTA per row leaves the three transforms of a row to 32 CTAs: fused from 128 rows on.)  Up to 16 rows, where every
+    // kernel of a layer is a few microseconds of latency, the launches that drop out count: the activation, which has a warp
+    // per 128-block, always writes the transform, the norms up to a hidden size of 2048, where a warp of a row's CTA has at
+    // most two blocks (28 layers, hidden 1024, 8 rows: 2.23 -> 2.20 ms; hidden 5120, 2 rows, five blocks per warp and three
+    // transforms of each: 3 % slower than with separate transforms).
+    const bool few = rows <= 16;
+    const bool fuse_pre = ctx->fuse_transform != 0 && (rows >= 128 || (few && hidden <= 2048));
+    const bool fuse_act = ctx->fuse_transform != 0 && (rows >= 128 || few);
     for (int l = 0; l < m->n_layers; ++l) {
         const exl3_layer& L = m->layers[l];
         {
@@ -211,7 +217,7 @@ static int step_forward_impl(exl3_ctx* ctx, exl3_stream stream, const exl3_model
             const exl3_linear* w[3] = {&L.q_proj, &L.k_proj, &L.v_proj};
             void* out[3] = {s.q, s.k, s.v};
             exl3_pre_act pre;
-            if (fuse_pre && exl3_tc_pre_buffers(ctx, 3, w, rows, &pre)) {
+            if (fuse_pre && exl3_pre_buffers(ctx, 3, w, rows, &pre)) {
                 if (pending) STEP_TRY(exl3_rms_norm_pre(ctx, stream, pending, 0, L.attn_norm, s.resid, m->norm_eps, 0.f, 1.f, rows, hidden, &pre));
                 else         STEP_TRY(exl3_rms_norm_pre(ctx, stream, s.resid, 1, L.attn_norm, nullptr, m->norm_eps, 0.f, 1.f, rows, hidden, &pre));
                 STEP_TRY(exl3_gemm_fanout_pre(ctx, stream, 3, w, out, rows, 0));
@@ -240,7 +246,7 @@ static int step_forward_impl(exl3_ctx* ctx, exl3_stream stream, const exl3_model
             const exl3_linear* w[2] = {&L.gate_proj, &L.up_proj};
             void* out[2] = {s.gate, s.up};
             exl3_pre_act pre;
-            if (fuse_pre && exl3_tc_pre_buffers(ctx, 2, w, rows, &pre)) {
+            if (fuse_pre && exl3_pre_buffers(ctx, 2, w, rows, &pre)) {
                 STEP_TRY(exl3_rms_norm_pre(ctx, stream, s.proj, 0, L.mlp_norm, s.resid, m->norm_eps, 0.f, 1.f, rows, hidden, &pre));
                 STEP_TRY(exl3_gemm_fanout_pre(ctx, stream, 2, w, out, rows, 0));
             } else {
@@ -253,7 +259,7 @@ static int step_forward_impl(exl3_ctx* ctx, exl3_stream stream, const exl3_model
             const exl3_linear* w[1] = {&L.down_proj};
             void* out[1] = {s.proj};
             exl3_pre_act pre;
-            if (fuse_pre && exl3_tc_pre_buffers(ctx, 1, w, rows, &pre)) {
+            if (fuse_act && exl3_pre_buffers(ctx, 1, w, rows, &pre)) {
                 STEP_TRY(exl3_silu_mul_pre(ctx, stream, s.gate, s.up, rows, m->inter, &pre));
                 STEP_TRY(exl3_gemm_fanout_pre(ctx, stream, 1, w, out, rows, 0));
             } else {

@@ -223,3 +223,29 @@ def test_multi_step_greedy_generation_with_page_allocator(ctx, kv_bits):
         pool.release(blk)
     assert pool.num_free() == 16
     pool.close()
+
+
+@pytest.mark.parametrize("rows,cb", [(1, 1), (7, 0), (8, 1), (9, 1), (16, 0), (9, 2)])
+def test_decode_step_with_fused_transforms_is_bit_identical(ctx, rows, cb):
+    """Up to 16 rows the norms and the activation write the decode GEMM's operand themselves (codebook 2 keeps the separate
+    transform).  They do the same operations in the same order, so the results are the same bits; 1, 7, 8, 9 and 16 rows
+    leave no, some and many of the operand's 8 or 16 row slots empty."""
+    import os
+    import torch
+    from exl3b200 import Ctx
+    r = H.rng(300 + rows)
+    model, _, ids, q_lens, ctx_lens, bt = _setup(0, 4, cb, [1] * rows, r.integers(3, 400, rows), 70 + rows)
+    os.environ["EXL3_B200_NO_FUSED_TRANSFORM"] = "1"
+    try:
+        plain = Ctx(0)
+    finally:
+        del os.environ["EXL3_B200_NO_FUSED_TRANSFORM"]
+    got = []
+    for c in (ctx, plain):
+        # a larger batch before it leaves other values in the scratch
+        model.step(c, H.to_dev(np.zeros(16, np.int64)), H.to_dev(np.full(1, 16, np.int32)), H.to_dev(np.zeros(1, np.int32)),
+                   H.to_dev(bt[:1]), 16)
+        _, logits = model.step(c, H.to_dev(ids), H.to_dev(q_lens), H.to_dev(ctx_lens), H.to_dev(bt), 1, want_logits=True)
+        c.poll_status()
+        got.append(logits.cpu())
+    assert torch.isfinite(got[0]).all() and torch.equal(got[0], got[1])
