@@ -178,7 +178,6 @@ attn_qdec_kernel(const __grid_constant__ CUtensorMap map_qk, const __grid_consta
     const uint32_t v_off = SM::CODES + (warp * 16 + 2 * t) * SM::ROWB +
                            (B == 4 ? (t << 4) + 4 * (g >> 1) : (((g >> 2) ^ (2 * t)) << 4) + 4 * (g & 3));
     const uint32_t sel_lo = (g & 1) ? 0x3632u : 0x1410u, sel_hi = (g & 1) ? 0x2723u : 0x0501u;
-    const float s_mul = p.scale_log2 / (float)(1 << (B - 1));
 
     __shared__ int s_unit;
     const int n_units = n_items * p.nkv;
@@ -232,33 +231,47 @@ attn_qdec_kernel(const __grid_constant__ CUtensorMap map_qk, const __grid_consta
         // ---- Q as B operands.  Lane (g, t) holds row g of a column block at the eight dims of every group whose codes it
         // unpacks from a key: 4 bits: dims 8t .. 8t+7 (word t of the group), 8 bits: dims 4t .. 4t+3 and 16 + 4t .. (word t
         // of either half).  H32 runs over the lane's eight values and the quad.  cini: minus the exponents' share of a sum.
+        uint32_t w[NB][4][4];
+        half2 qmax = __float2half2_rn(0.f);
+        #pragma unroll
+        for (int nb = 0; nb < NB; ++nb) {
+            const int row = r0 + nb * 8 + g;
+            const int qidx = row / G, head = kvh * G + (row - qidx * G);
+            const half* qp = p.q + ((size_t)(row_base + qidx) * p.nq + head) * D;
+            #pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                uint4 raw = make_uint4(0u, 0u, 0u, 0u);
+                if (row < ql * G) {
+                    if constexpr (B == 4) raw = *reinterpret_cast<const uint4*>(qp + 32 * j + 8 * t);
+                    else {
+                        const uint2 lo = *reinterpret_cast<const uint2*>(qp + 32 * j + 4 * t);
+                        const uint2 hi = *reinterpret_cast<const uint2*>(qp + 32 * j + 16 + 4 * t);
+                        raw = make_uint4(lo.x, lo.y, hi.x, hi.y);
+                    }
+                }
+                w[nb][j][0] = raw.x; w[nb][j][1] = raw.y; w[nb][j][2] = raw.z; w[nb][j][3] = raw.w;
+                #pragma unroll
+                for (int e = 0; e < 4; ++e) qmax = __hmax2(qmax, __habs2(*reinterpret_cast<const half2*>(&w[nb][j][e])));
+            }
+        }
+        // A group that lines up with a row of the transform grows by sqrt(32) and would leave fp16 from 11580 on.  Such queries
+        // are packed at an eighth, which keeps every finite one in range (46 318), and the scores are taken up again.  (Every
+        // warp holds all rows of the block, so the CTA's warps agree.)
+        const bool big = __any_sync(0xffffffffu, fmaxf(__low2float(qmax), __high2float(qmax)) > 11576.f);
+        const float q_mul = big ? 0.125f * R32 : R32;
+        const float s_mul = p.scale_log2 * (big ? 8.f / (float)(1 << (B - 1)) : 1.f / (float)(1 << (B - 1)));
         uint32_t qf[NB][8][2];
         float cini[NB][4][2];
         int lim[NB][2];                                    // keys visible to rows 2t, 2t+1 of the column block
         int wlim = 0x7fffffff;
         #pragma unroll
         for (int nb = 0; nb < NB; ++nb) {
-            const int row = r0 + nb * 8 + g;
-            const int qidx = row / G, head = kvh * G + (row - qidx * G);
-            const bool valid = row < ql * G;
-            const half* qp = p.q + ((size_t)(row_base + qidx) * p.nq + head) * D;
             #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 float v[8];
-                uint32_t w[4] = {0u, 0u, 0u, 0u};
-                if (valid) {
-                    if constexpr (B == 4) {
-                        const uint4 raw = *reinterpret_cast<const uint4*>(qp + 32 * j + 8 * t);
-                        w[0] = raw.x; w[1] = raw.y; w[2] = raw.z; w[3] = raw.w;
-                    } else {
-                        const uint2 lo = *reinterpret_cast<const uint2*>(qp + 32 * j + 4 * t);
-                        const uint2 hi = *reinterpret_cast<const uint2*>(qp + 32 * j + 16 + 4 * t);
-                        w[0] = lo.x; w[1] = lo.y; w[2] = hi.x; w[3] = hi.y;
-                    }
-                }
                 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
-                    const half2 x = *reinterpret_cast<const half2*>(&w[e]);
+                    const half2 x = *reinterpret_cast<const half2*>(&w[nb][j][e]);
                     v[2 * e] = __low2float(x); v[2 * e + 1] = __high2float(x);
                 }
                 #pragma unroll
@@ -276,7 +289,7 @@ attn_qdec_kernel(const __grid_constant__ CUtensorMap map_qk, const __grid_consta
                     }
                 }
                 #pragma unroll
-                for (int e = 0; e < 8; ++e) v[e] *= R32;
+                for (int e = 0; e < 8; ++e) v[e] *= q_mul;
                 if constexpr (B == 4) {                    // pair i of a word: codes i, i + 4
                     #pragma unroll
                     for (int i = 0; i < 4; ++i) qf[nb][2 * j + (i >> 1)][i & 1] = pack_h2(v[i], v[i + 4]);

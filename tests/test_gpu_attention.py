@@ -339,3 +339,33 @@ def test_attention_quantised_decode_edges(ctx, bits, q_len, nq, nkv):
     want = O.attn_paged(c["q"], None, None, c["block_table"], c["seqlens"], nkv=nkv, quant=(*pools, bits))
     assert np.isfinite(got).all()
     assert _close(got, want, TOL_QUANT) <= 1.0
+
+
+@pytest.mark.parametrize("bits", [4, 8])
+@pytest.mark.parametrize("q_len,peak", [(1, 11500.0), (1, 11700.0), (3, 30000.0), (1, 65504.0), (9, 65504.0)])
+def test_attention_quantised_large_queries(ctx, bits, q_len, peak):
+    """Queries of which a group of 32 dims lines up with a row of the codec's transform, so that its rotation is sqrt(32) times
+    as large: every finite one has to come out, from both sides of where the rotation leaves fp16.  Keys are small, so that
+    the scores stay moderate.  Bar: the repository's for quantised pools."""
+    from oracle import oracle as O
+    torch = _torch()
+    nq, nkv, hd = 40, 8, 128
+    c = _make_case(6100 + bits + q_len, [3, 100, 700], q_len, nq, nkv)
+    c["q"][..., 32:64] = peak * np.where(np.arange(32) & 4, -1, 1).astype(np.float16)      # a row of the 32-point transform
+    for x in ("k", "kc"):
+        c[x] = (c[x].astype(np.float32) * (20.0 / peak)).astype(np.float16)
+    groups, pages = nkv * hd // 32, c["kc"].shape[0]
+    pools = []
+    for x in ("kc", "vc"):
+        codes, scales = O.quant_groups(c[x].reshape(-1), bits)
+        pools += [codes.reshape(pages, 256, groups * bits).copy(), scales.reshape(pages, 256, groups).copy()]
+    d = [H.to_dev(x.view(np.int32) if x.dtype == np.uint32 else x) for x in pools]
+    o = torch.full(c["q"].shape, float("nan"), dtype=torch.float16, device="cuda")
+    ctx.bighead_attn_paged_q(H.to_dev(c["q"]), H.to_dev(c["k"]), H.to_dev(c["v"]), *d, H.to_dev(c["block_table"]),
+                             H.to_dev(c["seqlens"]), o, nkv)
+    ctx.poll_status()
+    got = o.cpu().numpy()
+    O.quant_cache_paged(c["k"], pools[0], pools[1], c["v"], pools[2], pools[3], c["seqlens"], c["block_table"], bits, bits)
+    want = O.attn_paged(c["q"], None, None, c["block_table"], c["seqlens"], nkv=nkv, quant=(*pools, bits))
+    assert np.isfinite(got).all()
+    assert _close(got, want, TOL_QUANT) <= 1.0
