@@ -105,16 +105,23 @@ __device__ __forceinline__ uint32_t qd_field(uint32_t x, uint32_t m, uint32_t e)
     asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(y) : "r"(x), "r"(m), "r"(e));
     return y;
 }
-struct QdConst { uint32_t e16, e64, e512, e1024, x64, x4, x2; };
+struct QdConst { uint32_t e16, e256, e512, e1024, x64, x4, x2; };
 
-// K, 4 bits: the four fp16 pairs (n_i, n_{i+4}) of a word: 1024 + n for even i, 64 + n for odd i, with one shift per word.
+// K, 4 bits: the four fp16 pairs (n_i - 7.5, n_{i+4} - 7.5) of a word: 256 + n for even i, 16 + n for odd i, whose fp16 steps
+// are fine enough to take the centre out exactly.  Both words come from one shift and one multiplication.
 __device__ __forceinline__ void qd_pairs4_k(uint32_t w, uint32_t (&x)[4], const QdConst& c)
 {
-    const uint32_t h = w >> 8;
-    x[0] = qd_field(w, 0x000F000Fu, c.e1024);
-    x[1] = qd_field(w, 0x00F000F0u, c.e64);
-    x[2] = qd_field(h, 0x000F000Fu, c.e1024);
-    x[3] = qd_field(h, 0x00F000F0u, c.e64);
+    const uint32_t l = w * c.x4, h = w >> 6;
+    x[0] = qd_field(l, 0x003C003Cu, c.e256);
+    x[1] = qd_field(l, 0x03C003C0u, c.e16);
+    x[2] = qd_field(h, 0x003C003Cu, c.e256);
+    x[3] = qd_field(h, 0x03C003C0u, c.e16);
+    const half2 o256 = __float2half2_rn(263.5f), o16 = __float2half2_rn(23.5f);
+    #pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const half2 a = __hsub2(*reinterpret_cast<const half2*>(&x[i]), (i & 1) ? o16 : o256);
+        x[i] = *reinterpret_cast<const uint32_t*>(&a);
+    }
 }
 // V, 4 bits: fp16 pairs 16 + n of four dims over two keys, from the keys' words (the selectors pick the two bytes that hold
 // the dims).  The left shifts are multiplications, which run beside the logic operations on another pipe.
@@ -168,7 +175,7 @@ attn_qdec_kernel(const __grid_constant__ CUtensorMap map_qk, const __grid_consta
     // stage and parity of the next tile to consume and of the next to request (the same in every thread)
     int c_stage = 0, i_stage = 0;
     uint32_t c_par = 0, i_par = 1;                         // a stage is waited for from its second use on
-    const QdConst cst = {qd_reg(0x4C004C00u), qd_reg(0x54005400u), qd_reg(0x60006000u), qd_reg(0x64006400u), qd_reg(64u), qd_reg(4u), qd_reg(2u)};
+    const QdConst cst = {qd_reg(0x4C004C00u), qd_reg(0x5C005C00u), qd_reg(0x60006000u), qd_reg(0x64006400u), qd_reg(64u), qd_reg(4u), qd_reg(2u)};
     // Byte offsets in a stage of this lane's first word of K and of V.  The chunk index of the copies' swizzle sits in
     // address bits 4.. of a 1024-byte aligned stage, so that chunk c of a row is reached by XOR with c << 4:
     //   K, 4 bits: chunk j ^ (key / 2 % 4), word t; 8 bits: chunk (2 j + h) ^ (key % 8), word t;  keys g and g + 8
@@ -230,7 +237,7 @@ attn_qdec_kernel(const __grid_constant__ CUtensorMap map_qk, const __grid_consta
 
         // ---- Q as B operands.  Lane (g, t) holds row g of a column block at the eight dims of every group whose codes it
         // unpacks from a key: 4 bits: dims 8t .. 8t+7 (word t of the group), 8 bits: dims 4t .. 4t+3 and 16 + 4t .. (word t
-        // of either half).  H32 runs over the lane's eight values and the quad.  cini: minus the exponents' share of a sum.
+        // of either half).  H32 runs over the lane's eight values and the quad.  cini (8 bits): minus the exponents' share of a sum.
         uint32_t w[NB][4][4];
         half2 qmax = __float2half2_rn(0.f);
         #pragma unroll
@@ -297,17 +304,19 @@ attn_qdec_kernel(const __grid_constant__ CUtensorMap map_qk, const __grid_consta
                     #pragma unroll
                     for (int i = 0; i < 4; ++i) qf[nb][2 * j + (i >> 1)][i & 1] = pack_h2(v[4 * (i >> 1) + (i & 1)], v[4 * (i >> 1) + (i & 1) + 2]);
                 }
-                // what the exponents put on the codes add to the products (of the rounded values, which the MMA multiplies)
-                float sum = 0.f;
-                #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const half2 x = *reinterpret_cast<const half2*>(&qf[nb][2 * j + (i >> 1)][i & 1]);
-                    sum = fmaf(B == 8 ? 1151.5f : (i & 1) ? 71.5f : 1031.5f, __low2float(x) + __high2float(x), sum);
+                if constexpr (B == 8) {
+                    // what the exponents put on the codes adds to the products (of the rounded values, which the MMA multiplies)
+                    float sum = 0.f;
+                    #pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const half2 x = *reinterpret_cast<const half2*>(&qf[nb][2 * j + (i >> 1)][i & 1]);
+                        sum = fmaf(1151.5f, __low2float(x) + __high2float(x), sum);
+                    }
+                    sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+                    sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+                    cini[nb][j][0] = -__shfl_sync(0xffffffffu, sum, 8 * t);
+                    cini[nb][j][1] = -__shfl_sync(0xffffffffu, sum, 8 * t + 4);
                 }
-                sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-                sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-                cini[nb][j][0] = -__shfl_sync(0xffffffffu, sum, 8 * t);
-                cini[nb][j][1] = -__shfl_sync(0xffffffffu, sum, 8 * t + 4);
             }
             #pragma unroll
             for (int h = 0; h < 2; ++h) {
@@ -386,7 +395,7 @@ attn_qdec_kernel(const __grid_constant__ CUtensorMap map_qk, const __grid_consta
                         mma_f16(d, xa[2], xb[2], xa[3], xb[3], qf[nb][2 * j + 1][0], qf[nb][2 * j + 1][1]);
                         #pragma unroll
                         for (int e = 0; e < 4; ++e) {
-                            const float v = d[e] + cini[nb][j][e & 1];
+                            const float v = B == 4 ? d[e] : d[e] + cini[nb][j][e & 1];
                             s_acc[nb][e] = j == 0 ? v * (e < 2 ? fa : fb) : fmaf(v, e < 2 ? fa : fb, s_acc[nb][e]);
                         }
                     }
