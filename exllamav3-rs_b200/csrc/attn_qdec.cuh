@@ -167,9 +167,10 @@ attn_qdec_kernel(const __grid_constant__ CUtensorMap map_qk, const __grid_consta
     const int g = lane >> 2, t = lane & 3;
     const int G = p.nq / p.nkv;
     const int n_items = p.plan->n_items, chunk = p.plan->chunk;
+    __shared__ uint32_t s_asked[SM::STAGES];               // parity of the last copy requested into a stage, 2 = none yet
     if (tid == 0) {
         #pragma unroll
-        for (int s = 0; s < SM::STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 4); }
+        for (int s = 0; s < SM::STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 4); s_asked[s] = 2; }
         mbar_fence_init();
     }
     // stage and parity of the next tile to consume and of the next to request (the same in every thread)
@@ -220,6 +221,7 @@ attn_qdec_kernel(const __grid_constant__ CUtensorMap map_qk, const __grid_consta
                 if (!mbar_wait(&empty[i_stage], i_par)) failed = true;
                 else {
                     const uint32_t dst = smem_u32(smem + i_stage * SM::STAGE), bar = smem_u32(&full[i_stage]);
+                    s_asked[i_stage] = i_par ^ 1u;
                     mbar_expect_tx(&full[i_stage], SM::STAGE);
                     qd_tma_2d(dst, &map_qk, kvh * 4 * B, tok0, bar);
                     qd_tma_2d(dst + SM::CODES, &map_qv, kvh * 4 * B, tok0, bar);
@@ -492,6 +494,8 @@ attn_qdec_kernel(const __grid_constant__ CUtensorMap map_qk, const __grid_consta
         // all warps are done with the stages: the merge buffer may overwrite them
         if (__syncthreads_or(failed)) {
             if (tid == 0) atomicCAS(p.status, 0, 4);
+            // no copy may land after the CTA has given its shared memory back (a wait for a phase that has passed returns)
+            if (tid < SM::STAGES && s_asked[tid] < 2u) mbar_wait(&full[tid], s_asked[tid]);
             return;                                                    // uniform: every thread saw the same barrier result
         }
 
