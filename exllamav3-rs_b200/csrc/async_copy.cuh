@@ -45,6 +45,11 @@ __device__ __forceinline__ bool mbar_try_wait_hint(uint64_t* bar, uint32_t parit
         : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity), "r"(ns) : "memory");
     return ok != 0;
 }
+// Waits until the kernels in front of a programmatic dependent launch are complete (at once from then on, and in a plain
+// launch).  A role of a kernel that overlaps them executes it before its first wait for anything that depends on them, so
+// that the wait's bound covers this kernel's own work and not what is left of theirs.  (The decoder warps of the tensor-core
+// GEMM go without: their waits last two seconds, and a test per stage in their loop cost 1 % at 5120 x 17408, 52 rows.)
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // Bounded wait with sleeping polls (about limit * ns nanoseconds at most).
 __device__ __forceinline__ bool mbar_wait_sleep(uint64_t* bar, uint32_t parity, uint32_t limit = (1u << 20), uint32_t ns = 2000)
 {

@@ -392,7 +392,7 @@ __global__ void __launch_bounds__(GD_THREADS, 1) gemm_decode_kernel(const __grid
                     if constexpr (SM::ACT_BYTES > 0) {
                         // The launch may overlap the tail of the kernel that writes the activations (programmatic dependent
                         // launch): the codes above do not depend on it, the activations do.
-                        if (!waited) { asm volatile("griddepcontrol.wait;" ::: "memory"); waited = true; }
+                        if (!waited) { pdl_wait(); waited = true; }
                         const uint4* afr = MULTI ? p.a_frag[0] + (size_t)seg * afrag_slot
                                                  : (seg == 0 ? p.a_frag[0] : (seg == 1 ? p.a_frag[1] : p.a_frag[2]));
                         asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
@@ -408,6 +408,7 @@ __global__ void __launch_bounds__(GD_THREADS, 1) gemm_decode_kernel(const __grid
             }
             // nothing to do for any lane: leave the issue slots to the decoders for a moment; give up after about 4 s
             if (!__any_sync(0xffffffffu, go)) {
+                pdl_wait();                    // what it waits for depends on the activations
                 __nanosleep(200);
                 if (++idle > (1u << 24)) { failed = true; break; }
             } else idle = 0;
@@ -428,7 +429,7 @@ __global__ void __launch_bounds__(GD_THREADS, 1) gemm_decode_kernel(const __grid
                 #pragma unroll
                 for (int e = 0; e < 4; ++e) acc[s][c][e] = 0.0f;
 
-        if constexpr (SM::ACT_BYTES == 0) asm volatile("griddepcontrol.wait;" ::: "memory");      // these warps read the activations themselves
+        pdl_wait();                                         // the slots, or these warps' own loads, hold the activations
 
         const int lane_prev = (lane + 31) & 31;
         int nbg = nbg0, kc = kc0 - 1, slot = 0, par = 0;

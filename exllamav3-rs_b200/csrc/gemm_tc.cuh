@@ -330,7 +330,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const __grid_con
             const uint32_t a_bytes = (two_tiles ? 2u : 1u) * TC_A_TILE * CTAS;     // what lands on the leader's barrier
             // The set-up above and the codes (the other producer) do not depend on the kernel that writes the activations;
             // everything this kernel writes depends on the activations.
-            asm volatile("griddepcontrol.wait;" ::: "memory");
+            pdl_wait();
             int sa = 0;
             uint32_t par_ae = 1;                                  // a_empty is waited from the second round on
             for (int ks = 0; ks < ksteps; ++ks) {
@@ -358,6 +358,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const __grid_con
             int sr = 0;
             uint32_t par_re = 1;                                  // r_empty is waited from the second round on
             for (int kr = 0; kr < ksteps; ++kr) {
+                if (kr == SM::SR) pdl_wait();                     // from here on it waits for what depends on the activations
                 if (kr >= SM::SR && !mbar_wait(&r_empty[sr], par_re)) { failed = true; break; }
                 if (lane == 0) mbar_expect_tx(&r_full[sr], SM::RAW_STAGE);
                 if constexpr (PAIR) {
@@ -381,6 +382,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const __grid_con
             auto mk = [](uint32_t lo) { return ((uint64_t)HI << 32) | lo; };
             int sa = 0, sb = 0;
             uint32_t par_a = 0, par_b = 0;
+            pdl_wait();
             for (int ks = 0; ks < ksteps; ++ks) {
                 bool ok = PAIR ? mbar_spin_cluster(&a_full[sa], par_a) : mbar_wait(&a_full[sa], par_a);
                 ok = ok && (PAIR ? mbar_spin_cluster(&b_full[sb], par_b) : mbar_wait(&b_full[sb], par_b));
@@ -484,6 +486,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const __grid_con
 
     // ===== epilogue (warps 2..17): TMEM -> registers -> output transform -> global.  Each CTA stores its own rows.
     if (warp >= 2 && warp < 2 + TC_DECODERS && !failed) {
+        pdl_wait();
         if (!mbar_wait_warp(acc_full, 0)) failed = true;
         if (!failed) {
             tc_fence_after();
