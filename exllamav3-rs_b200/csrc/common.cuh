@@ -34,7 +34,7 @@ struct exl3_ctx {
     int stage_prof;
     cudaEvent_t* prof_ev; int* prof_stage; int prof_ev_n;
     double stage_ms[EXL3_STAGES]; int stage_steps;
-    int fuse_transform;     // 1: in the step runner the norm / activation kernels write the tensor-core GEMM's transformed activations (default), 0: separate launches
+    int fuse_transform;     // 1: in the step runner the norm / activation kernels write the next GEMM's transformed activations (default), 0: separate launches
     // Work lists of the attention kernels kept across the layers of one exl3_step_forward call (they depend on the batch's
     // lengths only, not on the layer): slot 0 = decode class, slot 1 = long class.  plan_keep is set for the duration of a
     // step; outside of it every attention call builds its list anew.

@@ -201,14 +201,16 @@ static int step_forward_impl(exl3_ctx* ctx, exl3_stream stream, const exl3_model
     STAGE(0);                           // descriptors and embedding
     exl3_chain_scope chain(ctx);        // from here on every launch follows one of this library
     const half* pending = nullptr;      // output of the previous block's MLP, added to the residual by the next norm
-    // (measured on the 27B-class shard: 84.6 against 85.3 ms at 1052 rows, but 22.7 against 22.5 ms at 32 rows, where the norm's
-    // one CTA per row leaves the three transforms of a row to 32 CTAs: fused from 128 rows on.)  Up to 16 rows, where every
-    // kernel of a layer is a few microseconds of latency, the launches that drop out count: the activation, which has a warp
-    // per 128-block, always writes the transform, the norms up to a hidden size of 2048, where a warp of a row's CTA has at
-    // most two blocks (28 layers, hidden 1024, 8 rows: 2.23 -> 2.20 ms; hidden 5120, 2 rows, five blocks per warp and three
-    // transforms of each: 3 % slower than with separate transforms).
+    // Who transforms the activations, a launch of its own or their producer.  Norms, from 128 rows on: 85.3 against 84.6 ms at
+    // 1052 rows of the 27B-class shard, but 22.5 against 22.7 ms at 32, where one CTA per row leaves a row's three transforms
+    // to 32 CTAs.  Up to 16 rows, where every kernel of a layer is a few microseconds of latency, the launches that drop out
+    // count: the activation, which has a warp per 128-block, always writes the transform (16 layers, 8 rows: hidden 1024 1154
+    // against 1132 us, 2048 1394 against 1368, 5120 2650 against 2587); the norms where a warp of a row's CTA has one block,
+    // which is up to hidden 1024 (within 2 % either way at 512 and 1024).  From the second block on the transforms of a
+    // block follow one another in a warp (hidden 1536 1260 against 1317 us, 2048 1368 against 1462, 5120 1329 against 1484
+    // at 8 layers).
     const bool few = rows <= 16;
-    const bool fuse_pre = ctx->fuse_transform != 0 && (rows >= 128 || (few && hidden <= 2048));
+    const bool fuse_pre = ctx->fuse_transform != 0 && (rows >= 128 || (few && hidden <= 1024));
     const bool fuse_act = ctx->fuse_transform != 0 && (rows >= 128 || few);
     for (int l = 0; l < m->n_layers; ++l) {
         const exl3_layer& L = m->layers[l];
