@@ -228,8 +228,8 @@ def test_multi_step_greedy_generation_with_page_allocator(ctx, kv_bits):
 @pytest.mark.parametrize("rows,cb", [(1, 1), (7, 0), (8, 1), (9, 1), (16, 0), (9, 2)])
 def test_decode_step_with_fused_transforms_is_bit_identical(ctx, rows, cb):
     """Up to 16 rows the norms and the activation write the decode GEMM's operand themselves (codebook 2 keeps the separate
-    transform).  They do the same operations in the same order, so the results are the same bits; 1, 7, 8, 9 and 16 rows
-    leave no, some and many of the operand's 8 or 16 row slots empty."""
+    transform).  They do the same operations in the same order, so the results are the same bits, with one and with two
+    groups of eight rows."""
     import os
     import torch
     from exl3b200 import Ctx
@@ -249,3 +249,70 @@ def test_decode_step_with_fused_transforms_is_bit_identical(ctx, rows, cb):
         c.poll_status()
         got.append(logits.cpu())
     assert torch.isfinite(got[0]).all() and torch.equal(got[0], got[1])
+
+
+@pytest.mark.parametrize("hidden,cb,fewer", [(1024, 1, 3), (1024, 2, 0), (1152, 1, 1), (2048, 0, 1), (2176, 1, 1)])
+def test_decode_step_fused_launches(ctx, hidden, cb, fewer):
+    """Which transforms drop out of a step of few rows: q/k/v, gate/up and down_proj up to hidden 1024, above it down_proj's,
+    none in codebook 2; the results are the same bits either way."""
+    import os
+    import torch
+    from exl3b200 import Ctx
+    from exl3b200.step import SyntheticModel
+    r = H.rng(500 + hidden + cb)
+    layers, rows = 2, 9
+    ctx_lens = r.integers(3, 300, rows).astype(np.int32)
+    bt, pages = H.make_paged(r, rows, ctx_lens + 1, 4, 128)
+    model = SyntheticModel(layers, hidden, 8, 4, 128, 1280, 512, K=4, cb=cb, pages=pages, seed=hidden)
+    model.fill_kv()
+    args = (H.to_dev(r.integers(0, 512, rows)), H.to_dev(np.ones(rows, np.int32)), H.to_dev(ctx_lens), H.to_dev(bt), 1)
+    os.environ["EXL3_B200_NO_FUSED_TRANSFORM"] = "1"
+    try:
+        plain = Ctx(0)
+    finally:
+        del os.environ["EXL3_B200_NO_FUSED_TRANSFORM"]
+    logits, launches = [], []
+    for c in (ctx, plain):
+        n0 = c.launch_count()
+        logits.append(model.step(c, *args, want_logits=True)[1].cpu())
+        launches.append(c.launch_count() - n0)
+        c.poll_status()
+    assert torch.isfinite(logits[0]).all() and torch.equal(logits[0], logits[1])
+    assert launches[1] - launches[0] == fewer * layers
+
+
+@pytest.mark.parametrize("kv_bits", [4, 8])
+def test_ragged_step_over_quantised_pools(ctx, kv_bits):
+    """Decode rows, verify rows and a prefill chunk in one step over quantised pools: the two attention passes of every layer
+    share the work lists that the first layer built.  Against the oracle, and replayed from a graph bit for bit."""
+    import torch
+    import exl3b200
+    from exl3b200.step import SyntheticModel
+    from oracle import oracle_model
+    r = H.rng(600 + kv_bits)
+    q_lens, ctx_lens = np.array([1, 8, 40, 1, 9], np.int32), np.array([300, 100, 0, 1000, 64], np.int32)
+    bt, pages = H.make_paged(r, 5, ctx_lens + q_lens, 8, 128)
+    model = SyntheticModel(3, 1024, 40, 8, 128, 2048, 2048, K=4, cb=1, pages=pages, kv_bits=kv_bits, seed=kv_bits)
+    model.fill_kv()
+    nm = oracle_model.model_to_numpy(model)
+    ids = r.integers(0, 2048, int(q_lens.sum())).astype(np.int64)
+    args = (H.to_dev(ids), H.to_dev(q_lens), H.to_dev(ctx_lens), H.to_dev(bt), int(q_lens.max()))
+    tok, logits = model.step(ctx, *args, want_logits=True)
+    ctx.poll_status()
+    _, wlog = oracle_model.step(nm, ids, q_lens, ctx_lens, bt)
+    # A new key or value on the border of two codes may be stored as either, and the rows of the prompt without a context
+    # see few others.  The oracle against itself with norm weights off by up to one fp16 step differs by 1.4e-2 of the
+    # logits' 2-norm at 4 bits and 2.5e-3 at 8 (0.1 and 0.015 at the largest difference over the RMS).  Bar: twice that.
+    err = np.linalg.norm(logits.cpu().numpy() - wlog) / np.linalg.norm(wlog)
+    print(f"{kv_bits} bits: relative 2-norm {err:.2e}")
+    assert err < (2.8e-2 if kv_bits == 4 else 5e-3)
+    g = exl3b200.CudaGraph(ctx)
+    tokens = torch.empty(5, dtype=torch.int64, device="cuda")
+    g.capture_begin()
+    _, replayed = model.step(ctx, *args, want_logits=True, stream=g.side_stream(), tokens_out=tokens)
+    g.capture_end()
+    for _ in range(2):
+        g.replay()
+    assert exl3b200.lib().exl3_sync_side_stream(ctx.handle) == 0
+    ctx.poll_status()
+    assert torch.equal(replayed, logits) and torch.equal(tokens, tok)
