@@ -395,7 +395,8 @@ int attn_pass(exl3_ctx* ctx, cudaStream_t st, AttnParams p, int total_rows, int 
     static const int tc_items = getenv("EXL3_TUNE_TC_ITEMS") ? atoi(getenv("EXL3_TUNE_TC_ITEMS")) : 0;
     // With the units handed out longest first, fewer and longer items win on the mma.sync kernels too (64 decode
     // sequences over fp16 pools at 1 / 2 / 3 / 4 items per slot: 242 / 234 / 237 / 242 us): two, and one for the kernel over
-    // quantised pools, whose units start with the rotation of their queries.
+    // quantised pools, whose units start with the rotation of their queries (24 sequences, contexts 512 .. 16384, 40 / 8
+    // heads, one and two items: 4 bits, 5 rows 68 and 72 us, 40 rows 188 and 193; 8 bits 68 and 75, 188 and 196).
     static const int dec_items = getenv("EXL3_TUNE_DEC_ITEMS") ? atoi(getenv("EXL3_TUNE_DEC_ITEMS")) : 0;
     const int target_items = grid_x * (use_tc ? (tc_items ? tc_items : 2) : (dec_items ? dec_items : (use_qdec ? 1 : 2)));
     // items <= target + sum of row blocks (every (sequence, row block) rounds its split count up once); the row blocks are
@@ -476,7 +477,13 @@ int attn_impl(exl3_ctx* ctx, cudaStream_t st, AttnParams p, int total_rows, int 
     size_t off = 0;
     // Decode class = sequences with at most 16 packed rows.  Over 4-bit and 8-bit pools it also takes up to 48 rows
     // (speculative verify: 8 query rows x 5 heads) as row blocks of 16 that each walk the codes again: the kernel that
-    // builds its operands from the codes is that much cheaper per key than the generic one.
+    // builds its operands from the codes is that much cheaper per key than the generic one.  Against the generic kernel, us,
+    // 40 / 8 heads, 15 / 25 / 40 / 45 rows: 24 sequences, contexts 512 .. 16384, 4 bits 93 / 144 / 188 / 193 against 130 /
+    // 196 / 197 / 197, 8 bits 95 / 148 / 188 / 198 against 216 / 282 / 289 / 280; 64 sequences, contexts 128 .. 4096, 40 and 45
+    // rows, 4 bits 146 / 155 against 158 / 162, 8 bits 149 / 158 against 216 / 221; 4 sequences, contexts 1024 .. 32768, 45
+    // rows, 99 against 126 and 104 against 156.  Behind only on one sequence of 8192 with 40 or more rows at 4 bits (51
+    // against 46).  A ragged batch with longer sequences runs all its decode rows in blocks of 16 (28 of 1 row beside 4 of 64
+    // rows: 4 bits 221 us, 252 with everything on the generic kernel; 8 bits 286 and 374).
     // (Sending the decode rows of a ragged fp16 batch through the tcgen05 kernel as well, as items of 128 rows with 5 in
     // use, was measured on the benchmark step: the attention stage takes the same 28.0 ms of the step's 83.)
     const int dec_rows = qdec_kernel_applies(p, quant) ? 48 : 16;

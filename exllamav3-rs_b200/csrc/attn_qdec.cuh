@@ -13,7 +13,8 @@
 //    in the copy's swizzle of their row width, which makes every load below free of bank conflicts.
 //  * K operands are the codes with an exponent put on them (one logic op or permute per pair).  An MMA pair covers one
 //    group of 32 dims, so the group's scale is applied to the fp32 sum afterwards (one FMA per group and score instead of
-//    one multiplication per code pair), after what the exponents added to the sum, -off * sum(q), has been taken out.
+//    one multiplication per code pair).  4-bit codes get an exponent fine enough to be centred exactly in fp16, once for
+//    all rows; what the exponents add to a sum of 8-bit ones, -off * sum(q), is taken out of the fp32 sum.
 //  * V operands are pairs of one dim over two neighbouring keys, built in registers from the two keys' words (a permute
 //    pairs the bytes); V never goes through shared memory a second time.  Its scales are multiplied into the softmax
 //    weights, per group.  The 4-bit offset 23.5 * sum(P s) comes from one MMA per group against a row of ones; 8-bit codes
@@ -21,11 +22,15 @@
 //  * A row's running maximum is reduced over the warp only in tiles where some score passes it.
 //  * Warps are coupled by a full and an empty mbarrier per stage, not by a CTA barrier per tile, and take turns requesting
 //    tiles.
-// Per 16 keys and warp: 430 instructions, 212 of them on the ALU pipe, whose rate is the bound (62 % of the issue slots
-// under ncu).  Whole calls, 40 / 8 heads: 64 sequences, contexts 128 .. 32768, 4 bits 220 -> 160 us; 24 sequences, contexts
-// 512 .. 16384, 8 bits (the generic kernel before) 219 -> 76 us.  Error against 64 bits: 4 bits 3.0e-4 -> 2.8e-4, 8 bits
-// 3.6e-4 -> 3.3e-4.
-// Queries are rotated by H32 once per work unit (q . H(c) = H(q) . c), output rows once when the warps' parts are merged.
+// Per 16 keys and warp, 4 bits, row blocks of 8: 437 instructions, 204 of them on the ALU pipe, whose rate is the bound (65 %
+// of the issue slots under ncu); 8 bits: 417 and 188.  Whole calls, 40 / 8 heads, before (4 bits: an arrangement with keys
+// on the columns, 8 bits: the generic kernel) and now: 64 sequences, contexts 128 .. 32768, 5 rows each, 222 -> 144 us and
+// 607 -> 160 us; 24 sequences, contexts 512 .. 16384, 4 / 8 bits: 5 rows 95 -> 68 and 221 -> 68 us, 15 rows 102 -> 93 and
+// 223 -> 95, 25 rows 155 -> 144 and 287 -> 147, 45 rows 207 -> 193 and 285 -> 198.
+// Error against 64 bits, value scales 0.01 .. 0.06: 4 bits 3.0e-4 -> 2.8e-4, 8 bits 3.4e-4 -> 3.1e-4.  Softmax weight x value
+// scale is formed in fp16: under scores with a deviation of 6 the error at 8 bits is 6e-4 at value scales of 1, 0.01 and
+// 1e-3 and 7e-4 at 1e-4, where the generic kernel, which rounds scale / 128 to fp16, has 8e-4, 8e-4, 2.2e-3 and 2.0e-2.
+// Queries are rotated by H32 once per work unit (q . H(c) = H(q) . c; those near the end of fp16 are packed at an eighth), output rows once when the warps' parts are merged.
 // Work distribution, split-KV partials and the combine kernel are those of attn_paged.cuh.
 #pragma once
 #include <cuda.h>
