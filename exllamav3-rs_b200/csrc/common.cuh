@@ -112,8 +112,9 @@ static inline bool aligned16(const void* p) { return (((uintptr_t)p) & 15) == 0;
 // frag_rows = 0: rows of a_had, for the tensor-core GEMM.  frag_rows = 8 or 16: the decode GEMM's fragment order in a_frag,
 // where row slots from `rows` on are zero-filled.
 struct exl3_pre_act { const half* suh[3]; half* a_had[3]; uint32_t* a_frag[3]; int nseg, rows, frag_rows; };
-// gemm.cu: fills `pre` and returns true when exl3_gemm_fanout_pre can run these tensors at m rows
-bool exl3_pre_buffers(exl3_ctx* ctx, int count, const exl3_linear* const* w, int m, exl3_pre_act* pre);
+// gemm.cu: fills `pre` and returns true when exl3_gemm_fanout_pre can run these tensors on m rows of `dim` values (a tensor
+// whose k is not the producer's width keeps the separate launches: the buffers are sized by k, the producer fills rows of dim)
+bool exl3_pre_buffers(exl3_ctx* ctx, int count, const exl3_linear* const* w, int m, int dim, exl3_pre_act* pre);
 int exl3_gemm_fanout_pre(exl3_ctx* ctx, exl3_stream stream, int count, const exl3_linear* const* w, void* const* C, int m, int c_fp32);
 // elementwise.cu
 int exl3_rms_norm_pre(exl3_ctx* ctx, exl3_stream stream, const void* x, int x_fp32, const void* w, float* r, float eps,

@@ -673,9 +673,10 @@ static bool decode_pre_applies(exl3_ctx* ctx, int count, const exl3_linear* cons
     return true;
 }
 
-bool exl3_pre_buffers(exl3_ctx* ctx, int count, const exl3_linear* const* w, int m, exl3_pre_act* pre)
+bool exl3_pre_buffers(exl3_ctx* ctx, int count, const exl3_linear* const* w, int m, int dim, exl3_pre_act* pre)
 {
     size_t off = 0;
+    if (!w || count < 1 || !w[0] || w[0]->k != dim) return false;
     pre->nseg = count; pre->rows = m; pre->frag_rows = 0;
     for (int i = 0; i < 3; ++i) pre->a_frag[i] = nullptr;
     if (decode_pre_applies(ctx, count, w, m)) {

@@ -219,7 +219,7 @@ static int step_forward_impl(exl3_ctx* ctx, exl3_stream stream, const exl3_model
             const exl3_linear* w[3] = {&L.q_proj, &L.k_proj, &L.v_proj};
             void* out[3] = {s.q, s.k, s.v};
             exl3_pre_act pre;
-            if (fuse_pre && exl3_pre_buffers(ctx, 3, w, rows, &pre)) {
+            if (fuse_pre && exl3_pre_buffers(ctx, 3, w, rows, hidden, &pre)) {
                 if (pending) STEP_TRY(exl3_rms_norm_pre(ctx, stream, pending, 0, L.attn_norm, s.resid, m->norm_eps, 0.f, 1.f, rows, hidden, &pre));
                 else         STEP_TRY(exl3_rms_norm_pre(ctx, stream, s.resid, 1, L.attn_norm, nullptr, m->norm_eps, 0.f, 1.f, rows, hidden, &pre));
                 STEP_TRY(exl3_gemm_fanout_pre(ctx, stream, 3, w, out, rows, 0));
@@ -248,7 +248,7 @@ static int step_forward_impl(exl3_ctx* ctx, exl3_stream stream, const exl3_model
             const exl3_linear* w[2] = {&L.gate_proj, &L.up_proj};
             void* out[2] = {s.gate, s.up};
             exl3_pre_act pre;
-            if (fuse_pre && exl3_pre_buffers(ctx, 2, w, rows, &pre)) {
+            if (fuse_pre && exl3_pre_buffers(ctx, 2, w, rows, hidden, &pre)) {
                 STEP_TRY(exl3_rms_norm_pre(ctx, stream, s.proj, 0, L.mlp_norm, s.resid, m->norm_eps, 0.f, 1.f, rows, hidden, &pre));
                 STEP_TRY(exl3_gemm_fanout_pre(ctx, stream, 2, w, out, rows, 0));
             } else {
@@ -261,7 +261,7 @@ static int step_forward_impl(exl3_ctx* ctx, exl3_stream stream, const exl3_model
             const exl3_linear* w[1] = {&L.down_proj};
             void* out[1] = {s.proj};
             exl3_pre_act pre;
-            if (fuse_act && exl3_pre_buffers(ctx, 1, w, rows, &pre)) {
+            if (fuse_act && exl3_pre_buffers(ctx, 1, w, rows, m->inter, &pre)) {
                 STEP_TRY(exl3_silu_mul_pre(ctx, stream, s.gate, s.up, rows, m->inter, &pre));
                 STEP_TRY(exl3_gemm_fanout_pre(ctx, stream, 1, w, out, rows, 0));
             } else {

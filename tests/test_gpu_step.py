@@ -316,3 +316,40 @@ def test_ragged_step_over_quantised_pools(ctx, kv_bits):
     assert exl3b200.lib().exl3_sync_side_stream(ctx.handle) == 0
     ctx.poll_status()
     assert torch.equal(replayed, logits) and torch.equal(tokens, tok)
+
+
+@pytest.mark.parametrize("rows", [9, 130])
+def test_step_with_a_narrower_down_proj_keeps_separate_launches(ctx, rows):
+    """A tensor whose k is not the width of the activation (here smaller): its transform buffers are sized by k, so the
+    activation must not write them.  Same bits and launches as with separate transforms."""
+    import os
+    import torch
+    from exl3b200 import Ctx
+    from exl3b200.step import SyntheticLinear, SyntheticModel
+    r = H.rng(700 + rows)
+    ctx_lens = np.array([40], np.int32)
+    bt, pages = H.make_paged(r, 1, ctx_lens + rows, 4, 128)
+    model = SyntheticModel(1, 1152, 8, 4, 128, 1408, 512, K=4, cb=1, pages=pages, seed=rows)
+    model.fill_kv()
+    g = torch.Generator(device="cuda")
+    g.manual_seed(rows)
+    narrow = SyntheticLinear(1280, 1152, 4, 1, g, "cuda")
+    model._layer_array[0].down_proj = narrow.struct()
+    args = (H.to_dev(r.integers(0, 512, rows)), H.to_dev(np.array([rows], np.int32)), H.to_dev(ctx_lens), H.to_dev(bt), rows)
+    os.environ["EXL3_B200_NO_FUSED_TRANSFORM"] = "1"
+    try:
+        plain = Ctx(0)
+    finally:
+        del os.environ["EXL3_B200_NO_FUSED_TRANSFORM"]
+    logits, launches = [], []
+    for c in (ctx, plain):
+        n0 = c.launch_count()
+        logits.append(model.step(c, *args, want_logits=True)[1].cpu())
+        launches.append(c.launch_count() - n0)
+        c.poll_status()
+    assert torch.isfinite(logits[0]).all()
+    if rows == 9:                                       # the norms of 130 rows write q/k/v's and gate/up's operands, in another order of sums
+        assert torch.equal(logits[0], logits[1])
+        assert launches[0] == launches[1]
+    else:
+        assert H.rel_rms_err(logits[0].numpy(), logits[1].numpy()) < 5e-3
