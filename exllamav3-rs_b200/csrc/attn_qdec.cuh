@@ -30,7 +30,8 @@
 // Error against 64 bits, value scales 0.01 .. 0.06: 4 bits 3.0e-4 -> 2.8e-4, 8 bits 3.4e-4 -> 3.1e-4.  Softmax weight x value
 // scale is formed in fp16: under scores with a deviation of 6 the error at 8 bits is 6e-4 at value scales of 1, 0.01 and
 // 1e-3 and 7e-4 at 1e-4, where the generic kernel, which rounds scale / 128 to fp16, has 8e-4, 8e-4, 2.2e-3 and 2.0e-2.
-// Queries are rotated by H32 once per work unit (q . H(c) = H(q) . c; those near the end of fp16 are packed at an eighth), output rows once when the warps' parts are merged.
+// Queries are rotated by H32 once per work unit (q . H(c) = H(q) . c; those near the end of fp16 are packed at an eighth),
+// output rows once when the warps' parts are merged.
 // Work distribution, split-KV partials and the combine kernel are those of attn_paged.cuh.
 #pragma once
 #include <cuda.h>
