@@ -2,6 +2,7 @@
 #include "gemm_small.cuh"
 #include "gemm_tc.cuh"
 #include "gemm_decode.cuh"
+#include "gemm_ts.cuh"
 
 namespace {
 
@@ -349,6 +350,31 @@ cudaError_t launch_tc_k(int K, int cb, bool pair, int bn, const CUtensorMap* ama
     }
 }
 
+// How gemm_ts_kernel's units of (128-column block, 128 k) are dealt out: the grid, and whether every CTA has whole blocks.
+// Costs are in units, about half a microsecond: the longest CTA's share, plus what partial sums cost.  Cutting every block into
+// the same number of parts leaves each CTA one part; an even share of all units over all SMs leaves most CTAs the end of one
+// block and the beginning of the next.  Measured at k = 5120, 32 and 128 rows, us: 1024 columns in 1, 2, 4, 8 parts 21.7, 13.3,
+// 8.8, 7.6 and 24.3, 16.9, 13.1, 12.8; 5120 columns in 3 parts 12.7 and 16.4, even share 13.4 and 18.6; 7168 columns in 2 parts
+// 15.7 and 19.0, even share 17.2 and 20.8; 17408 columns whole 25.8 and 29.3, even share 26.7 and 32.1; at k = 17408, 5120
+// columns in 3 parts 28.8 and 33.4, even share 26.6 and 32.4.  Below five units a part is mostly its own start and end (k = 1024,
+// 3072 columns whole, in 2, 3 parts 6.2, 6.2, 6.6).
+constexpr int TS_MIN_PART = 5;
+
+int ts_split(int sms, int blocks, int units, int m, bool may_share, int* whole)
+{
+    int grid = blocks < sms ? blocks : sms;
+    float best = (float)((blocks + sms - 1) / sms * units);
+    *whole = 1;
+    if (!may_share) return grid;
+    for (int s = 2; s * blocks <= sms && s * TS_MIN_PART <= units; ++s) {
+        const float cost = (units + s - 1) / s + 1.2f + m / 160.0f + s * (0.25f + m / 170.0f);
+        if (cost < best) { best = cost; grid = s * blocks; *whole = 0; }
+    }
+    const long long total = (long long)blocks * units;
+    if (total >= (long long)sms * TS_MIN_PART && (total + sms - 1) / sms + 7.0f + m / 24.0f < best) { grid = sms; *whole = 0; }
+    return grid;
+}
+
 // Tensor-core path for rows [0, m) and `nseg` weight tensors that share the activations, k, bits and codebook:
 // one launch of the input transforms (each tensor has its own suh) and one of the tcgen05 kernel.
 // With `pre` the transformed activations are already in place (written into the buffers exl3_pre_buffers named, by the
@@ -370,7 +396,10 @@ int gemm_tc_rows(exl3_ctx* ctx, cudaStream_t st, const half* A, int nseg, const 
     int blocks256 = 0;
     bool n128 = true;
     for (int i = 0; i < nseg; ++i) { blocks256 += (n[i] + TC_BN - 1) / TC_BN; n128 = n128 && n[i] % 128 == 0; }
-    const int bn = (ctx->use_pair && n128 && m <= 2 * TC_BM && blocks256 * 4 <= ctx->num_sms) ? 128 : TC_BN;
+    // Up to 128 rows the weights go through tensor memory in 128-column blocks (gemm_ts.cuh): at 128 rows 5120 x 17408 takes 35 us
+    // against 47, at more its accumulator does not fit.
+    const bool ts = n128 && m <= TS_MAX_N;
+    const int bn = ts || (ctx->use_pair && n128 && m <= 2 * TC_BM && blocks256 * 4 <= ctx->num_sms) ? 128 : TC_BN;
     int blocks = 0;
     for (int i = 0; i < TC_MAX_SEG; ++i) {
         const int j = i < nseg ? i : nseg - 1;              // unused slots repeat the last tensor (never selected)
@@ -381,7 +410,7 @@ int gemm_tc_rows(exl3_ctx* ctx, cudaStream_t st, const half* A, int nseg, const 
             blocks += (n[i] + bn - 1) / bn;                // a trailing 128-column half slab counts (CTA pairs only)
             cuuint64_t dims[2] = {(cuuint64_t)k, (cuuint64_t)m};
             cuuint64_t strides[1] = {(cuuint64_t)k * 2};
-            cuuint32_t box[2] = {(cuuint32_t)TC_BK, 128u};
+            cuuint32_t box[2] = {(cuuint32_t)TC_BK, ts ? (cuuint32_t)((m + 15) & ~15) : 128u};
             cuuint32_t estr[2] = {1, 1};
             CUresult r = enc(&amap[i], CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, pa.a_had[i], dims, strides, box, estr,
                              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -391,13 +420,13 @@ int gemm_tc_rows(exl3_ctx* ctx, cudaStream_t st, const half* A, int nseg, const 
             // half slab (4 tile rows x 8 tiles x 32K bytes) as one box
             cuuint64_t rdims[2] = {(cuuint64_t)(n[i] / 16) * 4 * K, (cuuint64_t)(k / 16)};
             cuuint64_t rstrides[1] = {(cuuint64_t)(n[i] / 16) * 32 * K};
-            cuuint32_t rbox[2] = {(cuuint32_t)(bn / 2 / 16) * 4 * K, (cuuint32_t)(TC_BK / 16)};
+            cuuint32_t rbox[2] = {(cuuint32_t)((ts ? 128 : bn / 2) / 16) * 4 * K, (cuuint32_t)(ts ? TS_ROWS : TC_BK / 16)};
             r = enc(&rmap[i], CU_TENSOR_MAP_DATA_TYPE_UINT64, 2, const_cast<void*>(trellis[i]), rdims, rstrides, rbox, estr,
                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
             if (r != CUDA_SUCCESS) return exl3_fail(ctx, EXL3_ERR_CUDA, "exl3_gemm: cuTensorMapEncodeTiled failed for the trellis");
             // the fp16 output as [m][n]: an epilogue warp stores its 32 rows x 128 columns as two boxes of 64 columns
-            if (!c_fp32) {
+            if (!c_fp32 && !ts) {
                 cuuint64_t cdims[2] = {(cuuint64_t)n[i], (cuuint64_t)m};
                 cuuint64_t cstrides[1] = {(cuuint64_t)n[i] * 2};
                 cuuint32_t cbox[2] = {64u, 32u};
@@ -423,6 +452,24 @@ int gemm_tc_rows(exl3_ctx* ctx, cudaStream_t st, const half* A, int nseg, const 
     } else
         exl3_launch(ctx, gemm_prologue_plain_kernel, dim3(m, nseg), 256, 0, st, A, pa, k);
     if (!pre) ctx->launches++;
+    if (ts) {
+        GemmTsParams q;
+        memset(&q, 0, sizeof(q));
+        for (int i = 0; i < TC_MAX_SEG; ++i) { q.C[i] = p.C[i]; q.svh[i] = p.svh[i]; q.n[i] = p.n[i]; q.blk_end[i] = i < nseg ? p.blk_end[i] : blocks; }
+        q.m = m; q.k = k; q.c_fp32 = c_fp32; q.nb = (m + 15) & ~15;
+        q.sb = ts_b_bytes(K) / (q.nb * TS_UNIT_K * 2);
+        if (q.sb > TS_SB) q.sb = TS_SB;
+        q.counters = ctx->counters; q.status = ctx->status;
+        int grid = ts_split(ctx->num_sms, blocks, k / TS_UNIT_K, m, blocks <= ctx->n_counters, &q.aligned);
+        if (!q.aligned) {
+            q.partial = (float*)exl3_ws_take(ctx, &off, (size_t)grid * 2 * m * 128 * 4);
+            if (!q.partial) grid = ts_split(ctx->num_sms, blocks, k / TS_UNIT_K, m, false, &q.aligned);
+        }
+        cudaError_t e = gemm_ts_launch(K, cb, amap, rmap, q, grid, st);
+        ctx->launches++;
+        if (e != cudaSuccess) { cudaGetLastError(); return exl3_fail(ctx, EXL3_ERR_CUDA, cudaGetErrorString(e)); }
+        return EXL3_OK;
+    }
     p.status = ctx->status; p.m = m; p.k = k; p.c_fp32 = c_fp32;
     cudaError_t e = launch_tc_k(K, cb, ctx->use_pair != 0, bn, amap, rmap, cmap, p, blocks, st);
     ctx->launches++;
@@ -569,21 +616,17 @@ extern "C" int exl3_gemm(exl3_ctx* ctx, exl3_stream stream, const void* A, const
     const int NB = n / 128, NST = k / 128;
     EXL3_REQUIRE(NB <= ctx->n_counters, "exl3_gemm: n too large for the context's counters");
 
-    // tcgen05 kernel over 512-row blocks per CTA pair and 256-column slabs (with CTA pairs a last slab of 128 columns is
-    // allowed: its missing half reads zero-filled codes and is never stored) (the last block may be partial: its rows past m are
-    // zero-filled by TMA, and a block with at most 256 valid rows runs a single MMA per K step).  Measured on 5120 x 17408
-    // at 4 bpw: the tcgen05 kernel takes 47-52 us for any m <= 256 (its decoders set the pace), the mma.sync small-M
-    // kernel 54 us at m = 1, 73 us at m = 16 and 209 us at m = 64, so every row count goes to the former.  The small-M
-    // kernel serves exl3_gemm_noalloc, EXL3_B200_NO_TC, and n % 256 == 128 under EXL3_B200_NO_PAIR.
+    // Up to 16 rows the streaming decode kernel, up to 128 the kernel that keeps the weights in tensor memory (gemm_ts.cuh), above
+    // that the tcgen05 kernel over 512-row blocks per CTA pair and 256-column slabs (with CTA pairs a last slab of 128 columns is
+    // allowed: its missing half reads zero-filled codes and is never stored; the last row block may be partial: its rows past m
+    // are zero-filled by TMA, and a block with at most 256 valid rows runs a single MMA per K step).  The mma.sync small-M kernel
+    // (209 us at 64 rows of 5120 x 17408) serves exl3_gemm_noalloc, EXL3_B200_NO_TC, and n % 256 == 128 under EXL3_B200_NO_PAIR.
     if (m <= GD_MAX_M && ctx->use_decode) {
         const half* suh1 = (const half*)suh; const half* svh1 = (const half*)svh;
         return gemm_decode_rows(ctx, st, (const half*)A, 1, &trellis, &C, &suh1, &svh1, &n, m, k, K, c_fp32, cb);
     }
-    // (17..32 rows on a tensor with few column slabs and a long reduction dimension, 17408 x 5120, used to run as two
-    // 16-row passes of the streaming kernel: 100 us against 126 us on 256-column slabs.  With 128-column slabs the
-    // tcgen05 kernel takes 80 us, so every row count above 16 goes there.)
     int tc_rows = 0;
-    if (m > TC_MAX_SMALL_M && (n % TC_BN == 0 || ctx->use_pair) && ctx->use_tc) {
+    if (m > TC_MAX_SMALL_M && (n % TC_BN == 0 || ctx->use_pair || m <= TS_MAX_N) && ctx->use_tc) {
         tc_rows = m;
         const half* suh1 = (const half*)suh; const half* svh1 = (const half*)svh;
         int rc = gemm_tc_rows(ctx, st, (const half*)A, 1, &trellis, &C, &suh1, &svh1, &n, tc_rows, k, K, c_fp32, cb);

@@ -397,6 +397,28 @@ def test_gemm_tc_pair_equals_one_cta(ctx, ctx_one_cta, m):
     assert torch.equal(outs[0], outs[1])
 
 
+# 17 to 128 rows: edges of the 16-row steps of the accumulator, of the 64-row output tile and of the activation ring's depths;
+# whole blocks, blocks cut into equal parts (k = 5120 and 1664, whose 13 units do not divide evenly), and an even share of
+# all units (more blocks than half the SMs, long k)
+@pytest.mark.parametrize("m,k,n,K,cb,c_fp32", [
+    (17, 128, 128, 4, 1, False), (33, 1152, 640, 8, 0, False), (48, 1664, 384, 6, 1, True), (49, 1664, 1280, 7, 2, False),
+    (64, 5120, 1024, 3, 0, False), (65, 5120, 1024, 8, 1, True), (96, 640, 25600, 5, 1, False), (112, 5120, 256, 7, 1, False),
+    (127, 2048, 1152, 2, 2, True), (128, 1024, 3072, 6, 0, False), (128, 5120, 512, 8, 1, False), (40, 5120, 12800, 4, 1, False)])
+def test_gemm_weights_in_tensor_memory(ctx, ref, m, k, n, K, cb, c_fp32):
+    _gemm_case(ctx, ref, m, k, n, K, cb, c_fp32, 1500 + m + K)
+
+
+def test_gemm_without_room_for_partial_sums():
+    """a context whose scratch holds the activations but no partial sums runs whole blocks, with the same result up to the
+    order of fp32 sums"""
+    import exl3b200
+    c = exl3b200.Ctx(0, workspace_bytes=768 << 10)
+    try:
+        _gemm_case(c, None, 64, 5120, 1024, 4, 1, False, 1600)
+    finally:
+        c.close()
+
+
 # ------------------------------------------------------------------------------------------ dense fp16 GEMM (tcgen05)
 
 @pytest.mark.parametrize("m,k,n,c_fp32", [(1, 64, 8, False), (128, 128, 256, False), (129, 192, 264, True),
