@@ -30,7 +30,6 @@ extern "C" int exl3_ctx_create(int device, size_t workspace_bytes, exl3_ctx** ou
     ctx->fuse_transform = getenv("EXL3_B200_NO_FUSED_TRANSFORM") ? 0 : 1;
     ctx->stage_prof = 0; ctx->prof_ev = nullptr; ctx->prof_stage = nullptr; ctx->prof_ev_n = 0; ctx->stage_steps = 0;
     for (int i = 0; i < EXL3_STAGES; ++i) ctx->stage_ms[i] = 0.0;
-    ctx->use_decode = (getenv("EXL3_B200_NO_DECODE") || getenv("EXL3_B200_NO_TC")) ? 0 : 1;
     cudaDeviceProp prop;
     if (cudaGetDeviceProperties(&prop, device) != cudaSuccess) { delete ctx; cudaGetLastError(); return EXL3_ERR_CUDA; }
     if (prop.major != 10) {

@@ -5,6 +5,7 @@
 #include <stdint.h>
 #include <stdio.h>
 #include <string.h>
+#include <utility>
 #include "../../include/exl3_abi.h"
 
 #define EXL3_PAGE 256
@@ -27,7 +28,6 @@ struct exl3_ctx {
     uint64_t launches;
     int mma_attn;
     int use_tc;             // 1: tcgen05 GEMM for large M (default), 0: small-M kernel in passes (for A/B runs)
-    int use_decode;         // 1: the streaming decode kernel takes calls of up to 16 rows (default), 0: they go the way of larger row counts
     int use_pair;           // 1: the tcgen05 GEMM runs on CTA pairs (cta_group::2, default), 0: one CTA per tile
     // per-stage device times of exl3_step_forward (off by default): events recorded at the stage boundaries of a step that
     // is not being captured, read back at its end
@@ -58,6 +58,15 @@ __device__ __forceinline__ void pdl_enter()
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
+// The same for the first kernel of a call: the kernel behind it may read weights at once, so unless the work in front is known to
+// be this library's (early), it is let go only when that is complete.
+__device__ __forceinline__ void pdl_enter_first(int early)
+{
+    if (early) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (!early) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // Launch as a programmatic dependent of the previous kernel where the context says that there is one: the launch then
 // overlaps the tail of its predecessor.  A decode step of a small model is some fifteen kernels of 3 to 10 us per layer
 // (28 layers, hidden 1024, 8 rows: 2.79 -> 2.23 ms; verify step of 64 layers at 32 rows: 20.55 -> 20.11 ms).
@@ -77,6 +86,32 @@ static inline cudaError_t exl3_launch(exl3_ctx* ctx, void (*kern)(P...), dim3 gr
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr; cfg.numAttrs = exl3_chained(ctx) ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+}
+// The first kernel of a call, which begins with pdl_enter_first and takes its argument last: a programmatic dependent whatever is
+// in front of it, because it touches nothing and lets nothing go before that is complete.  Back to back, the set-up of its blocks
+// and the launch of the kernel behind it then overlap the tail of the call before (EXL3 GEMM at 4 bits, us: 5120 x 5120, 1 row
+// 17.1 -> 15.1, 5120 x 17408, 52 rows 33.1 -> 29.2).  Under stream capture, where the node in front need not be a kernel, a plain
+// launch outside of a chain.
+static inline int exl3_first_early(exl3_ctx* ctx, cudaStream_t st, bool* overlap)
+{
+    if (exl3_chained(ctx)) { *overlap = true; return 1; }
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    *overlap = cudaStreamIsCapturing(st, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone;
+    if (!*overlap) cudaGetLastError();
+    return 0;
+}
+template <typename... P, typename... A>
+static inline cudaError_t exl3_launch_first(exl3_ctx* ctx, void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args)
+{
+    bool overlap;
+    const int early = exl3_first_early(ctx, st, &overlap);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr; cfg.numAttrs = overlap ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kern, std::forward<A>(args)..., early);
 }
 // Marks the launches of a scope as a chain.
 struct exl3_chain_scope {
@@ -109,9 +144,7 @@ static inline bool aligned16(const void* p) { return (((uintptr_t)p) & 15) == 0;
 
 // Transformed activations of up to three EXL3 tensors that share an input, written by the kernel that produces the input
 // (norm, activation) instead of by the GEMM's own transform launch: where each tensor's copy goes and its sign vector.
-// frag_rows = 0: rows of a_had, for the tensor-core GEMM.  frag_rows = 8 or 16: the decode GEMM's fragment order in a_frag,
-// where row slots from `rows` on are zero-filled.
-struct exl3_pre_act { const half* suh[3]; half* a_had[3]; uint32_t* a_frag[3]; int nseg, rows, frag_rows; };
+struct exl3_pre_act { const half* suh[3]; half* a_had[3]; int nseg; };
 // gemm.cu: fills `pre` and returns true when exl3_gemm_fanout_pre can run these tensors on m rows of `dim` values (a tensor
 // whose k is not the producer's width keeps the separate launches: the buffers are sized by k, the producer fills rows of dim)
 bool exl3_pre_buffers(exl3_ctx* ctx, int count, const exl3_linear* const* w, int m, int dim, exl3_pre_act* pre);

@@ -180,16 +180,6 @@ __device__ __forceinline__ uint2 had128_signed_lane(half2 a, half2 b, const half
     return o;
 }
 
-// Four transformed values (k = 128 blk + 4 lane ..) of batch row `b` in the decode GEMM's fragment order: word
-// (set, kslot, r, lane' = 4 g + t, w) holds row 8 set + g at k = 64 kslot + 16 r + 2 t + (w & 1) + 8 (w >> 1), duplicated.
-__device__ __forceinline__ void store_frag(uint32_t* __restrict__ out, uint2 h, int b, int blk, int lane, int k)
-{
-    const int q = lane & 3, t0 = 2 * (q & 1), w0 = 2 * (q >> 1);
-    uint32_t* p = out + ((((size_t)(b >> 3) * (k / 64) + 2 * blk + (lane >> 4)) * 4 + ((lane >> 2) & 3)) * 32 + 4 * (b & 7) + t0) * 4 + w0;
-    *reinterpret_cast<uint2*>(p) = make_uint2((h.x & 0xffffu) * 0x10001u, (h.x >> 16) * 0x10001u);
-    *reinterpret_cast<uint2*>(p + 4) = make_uint2((h.y & 0xffffu) * 0x10001u, (h.y >> 16) * 0x10001u);
-}
-
 // rms_norm_kernel whose fp16 result goes straight through the input transform of the EXL3 tensors that read it (up to
 // three: q/k/v or gate/up, each with its own sign vector) instead of to memory: the norm's own output and the separate
 // transform launch drop out.  A warp's 32 float4 columns of one pass are one 128-block (dim % 128 == 0).
@@ -201,11 +191,6 @@ __global__ void __launch_bounds__(1024) rms_norm_had_kernel(const TI* __restrict
     __shared__ float sh[32];
     const int cols = dim >> 2, lane = threadIdx.x & 31;
     const size_t row = blockIdx.x;
-    if ((int)row >= pre.rows) {                                 // a row slot of the fragments without a row
-        for (int c = threadIdx.x; c < cols; c += blockDim.x)
-            for (int sgm = 0; sgm < pre.nseg; ++sgm) store_frag(pre.a_frag[sgm], make_uint2(0u, 0u), (int)row, c >> 5, lane, dim);
-        return;
-    }
     float4 v[8];
     float sum = 0.0f;
     #pragma unroll
@@ -249,8 +234,7 @@ __global__ void __launch_bounds__(1024) rms_norm_had_kernel(const TI* __restrict
             for (int sgm = 0; sgm < 3; ++sgm)
                 if (sgm < pre.nseg) {
                     const uint2 h = had128_signed_lane(a, b, pre.suh[sgm], c, lane);
-                    if (pre.frag_rows) store_frag(pre.a_frag[sgm], h, (int)row, c >> 5, lane, dim);
-                    else reinterpret_cast<uint2*>(pre.a_had[sgm] + row * dim)[c] = h;
+                    reinterpret_cast<uint2*>(pre.a_had[sgm] + row * dim)[c] = h;
                 }
         }
     }
@@ -370,22 +354,20 @@ __global__ void __launch_bounds__(256) silu_mul_tail_kernel(const half* x, const
 
 // silu_mul_kernel whose result goes straight through the input transform of the EXL3 tensor that reads it (down_proj):
 // one warp per 128-block of a row, lane = 4 consecutive elements.
-constexpr int SH_BLOCKS = 4;          // 128-blocks per warp: their loads are all in flight before the first is used
-// FRAG: one block per warp, and the result goes to a_frag in the decode GEMM's order; blocks past `valid` are zeros.
-template <bool FRAG>
+// U blocks per warp, whose loads are all in flight before the first is used: four where there are many, one where a block is a
+// few microseconds of latency.
+template <int U>
 __global__ void __launch_bounds__(256) silu_mul_had_kernel(const half* __restrict__ x, const half* __restrict__ y,
-                                                           const half* __restrict__ suh, half* __restrict__ a_had, uint32_t* __restrict__ a_frag,
-                                                           long long blocks, long long valid, int bpr)
+                                                           const half* __restrict__ suh, half* __restrict__ a_had, long long blocks, int bpr)
 {
     pdl_enter();
-    constexpr int U = FRAG ? 1 : SH_BLOCKS;
     const int lane = threadIdx.x & 31;
     const long long blk0 = ((long long)blockIdx.x * 8 + (threadIdx.x >> 5)) * U;
     if (blk0 >= blocks) return;
     uint2 xr[U], yr[U];
     #pragma unroll
     for (int u = 0; u < U; ++u) {
-        const long long blk = blk0 + u < valid ? blk0 + u : valid - 1;         // the tail repeats the last block
+        const long long blk = blk0 + u < blocks ? blk0 + u : blocks - 1;         // the tail repeats the last block
         xr[u] = reinterpret_cast<const uint2*>(x + blk * 128)[lane];
         yr[u] = reinterpret_cast<const uint2*>(y + blk * 128)[lane];
     }
@@ -402,12 +384,7 @@ __global__ void __launch_bounds__(256) silu_mul_had_kernel(const half* __restric
             z[j] = __hmul2(__hmul2(a, rr), b);
         }
         const int col = (int)(blk % bpr) * 32 + lane;           // uint2 index inside the sign vector
-        uint2 h = had128_signed_lane(z[0], z[1], suh, col, lane);
-        if constexpr (FRAG) {
-            if (blk >= valid) h = make_uint2(0u, 0u);
-            store_frag(a_frag, h, (int)(blk / bpr), (int)(blk % bpr), lane, bpr * 128);
-        } else
-            reinterpret_cast<uint2*>(a_had + blk * 128)[lane] = h;
+        reinterpret_cast<uint2*>(a_had + blk * 128)[lane] = had128_signed_lane(z[0], z[1], suh, col, lane);
     }
 }
 
@@ -641,15 +618,15 @@ int exl3_rms_norm_pre(exl3_ctx* ctx, exl3_stream stream, const void* x, int x_fp
     const int cols = dim / 4;
     int threads = cols <= 2048 ? 256 : 1024;
     if (cols < 256) threads = ((cols + 31) / 32) * 32;
+    if (rows < 128 && cols > 256) threads = cols < 1024 ? ((cols + 31) / 32) * 32 : 1024;       // few rows: a block or two per warp
     cudaStream_t st = (cudaStream_t)stream;
-    const int grid = pre->frag_rows ? pre->frag_rows : rows;
     const half* wp = (const half*)w;
     if (x_fp32) {
-        if (r) exl3_launch(ctx, rms_norm_had_kernel<float, true>, grid, threads, 0, st, (const float*)x, wp, r, eps, cbias, cscale, dim, *pre);
-        else   exl3_launch(ctx, rms_norm_had_kernel<float, false>, grid, threads, 0, st, (const float*)x, wp, r, eps, cbias, cscale, dim, *pre);
+        if (r) exl3_launch(ctx, rms_norm_had_kernel<float, true>, rows, threads, 0, st, (const float*)x, wp, r, eps, cbias, cscale, dim, *pre);
+        else   exl3_launch(ctx, rms_norm_had_kernel<float, false>, rows, threads, 0, st, (const float*)x, wp, r, eps, cbias, cscale, dim, *pre);
     } else {
-        if (r) exl3_launch(ctx, rms_norm_had_kernel<half, true>, grid, threads, 0, st, (const half*)x, wp, r, eps, cbias, cscale, dim, *pre);
-        else   exl3_launch(ctx, rms_norm_had_kernel<half, false>, grid, threads, 0, st, (const half*)x, wp, r, eps, cbias, cscale, dim, *pre);
+        if (r) exl3_launch(ctx, rms_norm_had_kernel<half, true>, rows, threads, 0, st, (const half*)x, wp, r, eps, cbias, cscale, dim, *pre);
+        else   exl3_launch(ctx, rms_norm_had_kernel<half, false>, rows, threads, 0, st, (const half*)x, wp, r, eps, cbias, cscale, dim, *pre);
     }
     ctx->launches++;
     return exl3_check_launch(ctx, "rms_norm (fused transform)");
@@ -661,15 +638,10 @@ int exl3_silu_mul_pre(exl3_ctx* ctx, exl3_stream stream, const void* x, const vo
     EXL3_REQUIRE(rows >= 0 && dim > 0 && dim % 128 == 0, "silu_mul (fused transform): dim % 128 == 0 required");
     EXL3_REQUIRE(aligned16(x) && aligned16(y), "silu_mul (fused transform): pointers must be 16-byte aligned");
     if (rows == 0) return EXL3_OK;
-    const long long valid = (long long)rows * (dim / 128);
+    const long long blocks = (long long)rows * (dim / 128);
     cudaStream_t st = (cudaStream_t)stream;
-    if (pre->frag_rows) {
-        const long long blocks = (long long)pre->frag_rows * (dim / 128);
-        exl3_launch(ctx, silu_mul_had_kernel<true>, (unsigned)((blocks + 7) / 8), 256, 0, st, (const half*)x, (const half*)y, pre->suh[0],
-                    nullptr, pre->a_frag[0], blocks, valid, dim / 128);
-    } else
-        exl3_launch(ctx, silu_mul_had_kernel<false>, (unsigned)((valid + 8 * SH_BLOCKS - 1) / (8 * SH_BLOCKS)), 256, 0, st, (const half*)x, (const half*)y,
-                    pre->suh[0], pre->a_had[0], nullptr, valid, valid, dim / 128);
+    if (rows < 128) exl3_launch(ctx, silu_mul_had_kernel<1>, (unsigned)((blocks + 7) / 8), 256, 0, st, (const half*)x, (const half*)y, pre->suh[0], pre->a_had[0], blocks, dim / 128);
+    else            exl3_launch(ctx, silu_mul_had_kernel<4>, (unsigned)((blocks + 31) / 32), 256, 0, st, (const half*)x, (const half*)y, pre->suh[0], pre->a_had[0], blocks, dim / 128);
     ctx->launches++;
     return exl3_check_launch(ctx, "silu_mul (fused transform)");
 }

@@ -127,17 +127,19 @@ cudaError_t launch_small_k(int K, int cb, int mt, GemmSmallParams& p, int sms, s
     }
 }
 
-// Input transform for the tensor-core path: plain fp16 A_had[row][k] (one CTA per row, as above without duplication).
+// Input transform for the tensor-core path: plain fp16 A_had[row][k] (one CTA per row and share of k, as above without
+// duplication).  Up to 16 rows, a warp per 128-block: with few blocks in flight the tensor-core form has nothing to gain, and the
+// bits are those of the kernels that write the transform themselves.
 struct ProloguePlainArgs { const half* suh[TC_MAX_SEG]; half* a_had[TC_MAX_SEG]; };
 
-__global__ void __launch_bounds__(256) gemm_prologue_plain_kernel(const half* __restrict__ A, const ProloguePlainArgs args, int k)
+__global__ void __launch_bounds__(256) gemm_prologue_plain_kernel(const half* __restrict__ A, const ProloguePlainArgs args, int k, int early)
 {
-    pdl_enter();
+    pdl_enter_first(early);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const size_t row = blockIdx.x;
     const half* __restrict__ suh = args.suh[blockIdx.y];
     half* __restrict__ a_had = args.a_had[blockIdx.y];
-    for (int blk = warp; blk < k / 128; blk += 8) {
+    for (int blk = blockIdx.z * 8 + warp; blk < k / 128; blk += 8 * gridDim.z) {
         uint2 raw = reinterpret_cast<const uint2*>(A + row * k + blk * 128)[lane];
         half2 a = *reinterpret_cast<half2*>(&raw.x), b = *reinterpret_cast<half2*>(&raw.y);
         if (suh) {
@@ -186,9 +188,9 @@ __device__ __forceinline__ uint32_t sign_pair(int i, int j0, int j1)
 constexpr int GP_PAIRS = 4;          // block pairs per warp: their loads are all in flight before the first is used
 
 __global__ void __launch_bounds__(256) gemm_prologue_mma_kernel(const half* __restrict__ A, const ProloguePlainArgs args, int k,
-                                                                long long pairs_total)
+                                                                long long pairs_total, int early)
 {
-    pdl_enter();
+    pdl_enter_first(early);
     __shared__ __align__(16) uint8_t stage[8][512];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, t = lane & 3;
@@ -360,18 +362,20 @@ cudaError_t launch_tc_k(int K, int cb, bool pair, int bn, const CUtensorMap* ama
 // 3072 columns whole, in 2, 3 parts 6.2, 6.2, 6.6).
 constexpr int TS_MIN_PART = 5;
 
-int ts_split(int sms, int blocks, int units, int m, bool may_share, int* whole)
+int ts_split(int sms, int blocks, int units, int m, bool may_share, int* whole, int* longest = nullptr)
 {
-    int grid = blocks < sms ? blocks : sms;
-    float best = (float)((blocks + sms - 1) / sms * units);
+    int grid = blocks < sms ? blocks : sms, part = (blocks + sms - 1) / sms * units;
+    float best = (float)part;
     *whole = 1;
-    if (!may_share) return grid;
-    for (int s = 2; s * blocks <= sms && s * TS_MIN_PART <= units; ++s) {
-        const float cost = (units + s - 1) / s + 1.2f + m / 160.0f + s * (0.25f + m / 170.0f);
-        if (cost < best) { best = cost; grid = s * blocks; *whole = 0; }
+    if (may_share) {
+        for (int s = 2; s * blocks <= sms && s * TS_MIN_PART <= units; ++s) {
+            const float cost = (units + s - 1) / s + 1.2f + m / 160.0f + s * (0.25f + m / 170.0f);
+            if (cost < best) { best = cost; grid = s * blocks; part = (units + s - 1) / s; *whole = 0; }
+        }
+        const long long total = (long long)blocks * units, even = (total + sms - 1) / sms;
+        if (total >= (long long)sms * TS_MIN_PART && even + 7.0f + m / 24.0f < best) { grid = sms; part = (int)even; *whole = 0; }
     }
-    const long long total = (long long)blocks * units;
-    if (total >= (long long)sms * TS_MIN_PART && (total + sms - 1) / sms + 7.0f + m / 24.0f < best) { grid = sms; *whole = 0; }
+    if (longest) *longest = part;
     return grid;
 }
 
@@ -399,20 +403,28 @@ int gemm_tc_rows(exl3_ctx* ctx, cudaStream_t st, const half* A, int nseg, const 
     // Up to 128 rows the weights go through tensor memory in 128-column blocks (gemm_ts.cuh): at 128 rows 5120 x 17408 takes 35 us
     // against 47, at more its accumulator does not fit.
     const bool ts = n128 && m <= TS_MAX_N;
+    int blocks128 = 0, whole, longest;
+    for (int i = 0; i < nseg; ++i) blocks128 += n[i] / 128;
+    int grid = ts_split(ctx->num_sms, blocks128, k / TS_UNIT_K, m, blocks128 <= ctx->n_counters, &whole, &longest);
+    // One row always, up to four where a CTA has few units, that kernel transforms the activations itself, which takes the launch
+    // in front of it off the call (us: 1 row, 5120 x 17408 27.2 -> 25.6, 17408 x 5120 33.0 -> 30.0, 1024 x 3072 13.5 -> 11.6; 4
+    // rows, 5120 x 1024 in 5 units 13.8 -> 11.8, but 5120 x 5120 in 14 units 15.2 -> 16.0 and 5120 x 17408 in 40 27.2 -> 30.5).
+    const bool few = ts && !pre && (m == 1 || (m <= TS_FEW && longest <= 10));
     const int bn = ts || (ctx->use_pair && n128 && m <= 2 * TC_BM && blocks256 * 4 <= ctx->num_sms) ? 128 : TC_BN;
     int blocks = 0;
     for (int i = 0; i < TC_MAX_SEG; ++i) {
         const int j = i < nseg ? i : nseg - 1;              // unused slots repeat the last tensor (never selected)
         if (i < nseg) {
-            pa.a_had[i] = (half*)exl3_ws_take(ctx, &off, (size_t)m * k * 2);
-            if (!pa.a_had[i]) return exl3_fail(ctx, EXL3_ERR_WORKSPACE, "exl3_gemm: context scratch too small for the activations");
+            pa.a_had[i] = few ? nullptr : (half*)exl3_ws_take(ctx, &off, (size_t)m * k * 2);
+            if (!few && !pa.a_had[i]) return exl3_fail(ctx, EXL3_ERR_WORKSPACE, "exl3_gemm: context scratch too small for the activations");
             pa.suh[i] = suh[i];
             blocks += (n[i] + bn - 1) / bn;                // a trailing 128-column half slab counts (CTA pairs only)
             cuuint64_t dims[2] = {(cuuint64_t)k, (cuuint64_t)m};
             cuuint64_t strides[1] = {(cuuint64_t)k * 2};
             cuuint32_t box[2] = {(cuuint32_t)TC_BK, ts ? (cuuint32_t)((m + 15) & ~15) : 128u};
             cuuint32_t estr[2] = {1, 1};
-            CUresult r = enc(&amap[i], CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, pa.a_had[i], dims, strides, box, estr,
+            CUresult r = CUDA_SUCCESS;
+            if (!few) r = enc(&amap[i], CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, pa.a_had[i], dims, strides, box, estr,
                              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
             if (r != CUDA_SUCCESS) return exl3_fail(ctx, EXL3_ERR_CUDA, "exl3_gemm: cuTensorMapEncodeTiled failed");
@@ -425,6 +437,7 @@ int gemm_tc_rows(exl3_ctx* ctx, cudaStream_t st, const half* A, int nseg, const 
                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
             if (r != CUDA_SUCCESS) return exl3_fail(ctx, EXL3_ERR_CUDA, "exl3_gemm: cuTensorMapEncodeTiled failed for the trellis");
+            if (few) amap[i] = rmap[i];                        // never dereferenced
             // the fp16 output as [m][n]: an epilogue warp stores its 32 rows x 128 columns as two boxes of 64 columns
             if (!c_fp32 && !ts) {
                 cuuint64_t cdims[2] = {(cuuint64_t)n[i], (cuuint64_t)m};
@@ -444,14 +457,14 @@ int gemm_tc_rows(exl3_ctx* ctx, cudaStream_t st, const half* A, int nseg, const 
     }
     bool all_signed = true;
     for (int i = 0; i < nseg; ++i) all_signed = all_signed && pa.suh[i] != nullptr;
-    if (pre) {
+    if (pre || few) {
         // nothing to launch
-    } else if (k % 256 == 0 && all_signed) {
+    } else if (k % 256 == 0 && all_signed && m > 16) {
         const long long pairs = (long long)m * (k / 256);
-        exl3_launch(ctx, gemm_prologue_mma_kernel, dim3((unsigned)((pairs + 8 * GP_PAIRS - 1) / (8 * GP_PAIRS)), nseg), 256, 0, st, A, pa, k, pairs);
+        exl3_launch_first(ctx, gemm_prologue_mma_kernel, dim3((unsigned)((pairs + 8 * GP_PAIRS - 1) / (8 * GP_PAIRS)), nseg), 256, 0, st, A, pa, k, pairs);
     } else
-        exl3_launch(ctx, gemm_prologue_plain_kernel, dim3(m, nseg), 256, 0, st, A, pa, k);
-    if (!pre) ctx->launches++;
+        exl3_launch_first(ctx, gemm_prologue_plain_kernel, dim3(m, nseg, m > 16 ? 1 : (k + 1023) / 1024), 256, 0, st, A, pa, k);
+    if (!pre && !few) ctx->launches++;
     if (ts) {
         GemmTsParams q;
         memset(&q, 0, sizeof(q));
@@ -460,137 +473,25 @@ int gemm_tc_rows(exl3_ctx* ctx, cudaStream_t st, const half* A, int nseg, const 
         q.sb = ts_b_bytes(K) / (q.nb * TS_UNIT_K * 2);
         if (q.sb > TS_SB) q.sb = TS_SB;
         q.counters = ctx->counters; q.status = ctx->status;
-        int grid = ts_split(ctx->num_sms, blocks, k / TS_UNIT_K, m, blocks <= ctx->n_counters, &q.aligned);
-        if (!q.aligned) {
+        q.early = 1;
+        bool overlap = true;
+        if (few) {
+            q.x = A;
+            for (int i = 0; i < TC_MAX_SEG; ++i) q.suh[i] = pa.suh[i];
+            q.early = exl3_first_early(ctx, st, &overlap);
+        }
+        q.aligned = whole;
+        if (!whole) {
             q.partial = (float*)exl3_ws_take(ctx, &off, (size_t)grid * 2 * m * 128 * 4);
             if (!q.partial) grid = ts_split(ctx->num_sms, blocks, k / TS_UNIT_K, m, false, &q.aligned);
         }
-        cudaError_t e = gemm_ts_launch(K, cb, amap, rmap, q, grid, st);
+        cudaError_t e = gemm_ts_launch(K, cb, amap, rmap, q, grid, overlap, st);
         ctx->launches++;
         if (e != cudaSuccess) { cudaGetLastError(); return exl3_fail(ctx, EXL3_ERR_CUDA, cudaGetErrorString(e)); }
         return EXL3_OK;
     }
     p.status = ctx->status; p.m = m; p.k = k; p.c_fp32 = c_fp32;
     cudaError_t e = launch_tc_k(K, cb, ctx->use_pair != 0, bn, amap, rmap, cmap, p, blocks, st);
-    ctx->launches++;
-    if (e != cudaSuccess) { cudaGetLastError(); return exl3_fail(ctx, EXL3_ERR_CUDA, cudaGetErrorString(e)); }
-    return EXL3_OK;
-}
-
-// ---- decode-regime kernel (1..16 rows)
-
-constexpr int GD_MAX_M = 16;
-
-template <int K, int CB, int MT>
-cudaError_t launch_decode(const CUtensorMap* rmap, const GemmDecodeParams& p, int grid, cudaStream_t st)
-{
-    constexpr int bytes = GdSmem<K, MT>::BYTES;
-    static bool configured[64] = {};
-    auto kern = gemm_decode_kernel<K, CB, MT>;
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev < 0 || dev >= 64 || !configured[dev]) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-        if (e != cudaSuccess) return e;
-        if (dev >= 0 && dev < 64) configured[dev] = true;
-    }
-    // launched as a programmatic dependent of the input transform that precedes it on the stream
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid); cfg.blockDim = dim3(GD_THREADS); cfg.dynamicSmemBytes = bytes; cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr; cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kern, rmap[0], rmap[1], rmap[2], p);
-}
-
-template <int K, int CB>
-cudaError_t launch_decode_mt(int mt, const CUtensorMap* rmap, const GemmDecodeParams& p, int grid, cudaStream_t st)
-{
-    return mt == 1 ? launch_decode<K, CB, 1>(rmap, p, grid, st) : launch_decode<K, CB, 2>(rmap, p, grid, st);
-}
-
-template <int K>
-cudaError_t launch_decode_cb(int cb, int mt, const CUtensorMap* rmap, const GemmDecodeParams& p, int grid, cudaStream_t st)
-{
-    if (cb == 0) return launch_decode_mt<K, 0>(mt, rmap, p, grid, st);
-    if (cb == 1) return launch_decode_mt<K, 1>(mt, rmap, p, grid, st);
-    return launch_decode_mt<K, 2>(mt, rmap, p, grid, st);
-}
-
-cudaError_t launch_decode_k(int K, int cb, int mt, const CUtensorMap* rmap, const GemmDecodeParams& p, int grid, cudaStream_t st)
-{
-    switch (K) {
-        case 1: return launch_decode_cb<1>(cb, mt, rmap, p, grid, st);
-        case 2: return launch_decode_cb<2>(cb, mt, rmap, p, grid, st);
-        case 3: return launch_decode_cb<3>(cb, mt, rmap, p, grid, st);
-        case 4: return launch_decode_cb<4>(cb, mt, rmap, p, grid, st);
-        case 5: return launch_decode_cb<5>(cb, mt, rmap, p, grid, st);
-        case 6: return launch_decode_cb<6>(cb, mt, rmap, p, grid, st);
-        case 7: return launch_decode_cb<7>(cb, mt, rmap, p, grid, st);
-        default: return launch_decode_cb<8>(cb, mt, rmap, p, grid, st);
-    }
-}
-
-// Decode path for m <= 16 rows and `nseg` weight tensors that share the activations, k, bits and codebook: one launch of
-// the input transforms (fragment order, one per tensor) and one of the streaming kernel over all their column blocks.
-int gemm_decode_rows(exl3_ctx* ctx, cudaStream_t st, const half* A, int nseg, const void* const* trellis, void* const* C,
-                     const half* const* suh, const half* const* svh, const int* n, int m, int k, int K, int c_fp32, int cb,
-                     bool pre = false)
-{
-    EncodeTiledFn enc = get_encode_tiled();
-    if (!enc) return exl3_fail(ctx, EXL3_ERR_CUDA, "exl3_gemm: cuTensorMapEncodeTiled is not available from this driver");
-    const int mt = m <= 8 ? 1 : 2;
-    size_t off = 0;
-    GemmDecodePrologueArgs pa;
-    CUtensorMap rmap[GD_MAX_SEG];
-    GemmDecodeParams p;
-    memset(&p, 0, sizeof(p));
-    int blocks = 0;
-    for (int i = 0; i < GD_MAX_SEG; ++i) {
-        const int j = i < nseg ? i : nseg - 1;              // unused slots repeat the last tensor (never selected)
-        if (i < nseg) {
-            pa.a_frag[i] = (uint32_t*)exl3_ws_take(ctx, &off, (size_t)mt * k * 32);
-            pa.rowsum[i] = (float*)exl3_ws_take(ctx, &off, (size_t)GD_PRO_SPLIT * mt * 8 * 4);
-            if (!pa.a_frag[i] || !pa.rowsum[i]) return exl3_fail(ctx, EXL3_ERR_WORKSPACE, "exl3_gemm: context scratch too small for the activations");
-            pa.suh[i] = suh[i];
-            blocks += n[i] / 128;
-            cuuint64_t rdims[2] = {(cuuint64_t)(n[i] / 16) * 4 * K, (cuuint64_t)(k / 16)};
-            cuuint64_t rstrides[1] = {(cuuint64_t)(n[i] / 16) * 32 * K};
-            cuuint32_t rbox[2] = {(cuuint32_t)2 * GD_SLOT_TILES * 4 * K, (cuuint32_t)GD_SLOT_ROWS};      // 8 tiles x 4 tile rows
-            cuuint32_t estr[2] = {1, 1};
-            CUresult r = enc(&rmap[i], CU_TENSOR_MAP_DATA_TYPE_UINT64, 2, const_cast<void*>(trellis[i]), rdims, rstrides, rbox, estr,
-                             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-            if (r != CUDA_SUCCESS) return exl3_fail(ctx, EXL3_ERR_CUDA, "exl3_gemm: cuTensorMapEncodeTiled failed for the trellis");
-        } else {
-            pa.a_frag[i] = pa.a_frag[j]; pa.rowsum[i] = pa.rowsum[j]; pa.suh[i] = pa.suh[j]; rmap[i] = rmap[j];
-        }
-        p.a_frag[i] = (const uint4*)pa.a_frag[i]; p.rowsum[i] = pa.rowsum[i];
-        p.C[i] = C[j]; p.svh[i] = svh[j]; p.n[i] = n[j];
-        p.blk_end[i] = i < nseg ? blocks : 0x7fffffff;
-    }
-    p.blk_end[GD_MAX_SEG - 1] = blocks;                     // the kernel reads the total from the last entry
-    for (int i = nseg; i < GD_MAX_SEG - 1; ++i) p.blk_end[i] = blocks;
-    if (blocks > ctx->n_counters) return exl3_fail(ctx, EXL3_ERR_INVALID, "exl3_gemm: n too large for the context's counters");
-    // Split of the (column block, 512-k chunk) units over the CTAs: whole blocks per CTA when that costs at most one unit
-    // more on the longest CTA than an even share of all units (no block is then shared between CTAs: no partial sums, no
-    // arrival counters, and the block finish at the end of the CTA is local), an even share (stream-K) otherwise.
-    const int KC = (k + GD_UNIT_K - 1) / GD_UNIT_K;
-    const long long total = (long long)blocks * KC;
-    const int sms = ctx->num_sms;
-    const long long units_aligned = (long long)((blocks + sms - 1) / sms) * KC, units_even = (total + sms - 1) / sms;
-    p.aligned = units_aligned <= units_even + 1 ? 1 : 0;
-    const int grid = p.aligned ? (blocks < sms ? blocks : sms) : (int)(total < sms ? total : sms);
-    p.partial = (float*)exl3_ws_take(ctx, &off, (size_t)grid * 2 * m * 128 * 4);
-    if (!p.partial) return exl3_fail(ctx, EXL3_ERR_WORKSPACE, "exl3_gemm: context scratch too small for the partial sums");
-    p.counters = ctx->counters; p.status = ctx->status; p.m = m; p.k = k; p.c_fp32 = c_fp32;
-    p.rowsum_parts = GD_PRO_SPLIT;
-    if (!pre) {
-        exl3_launch(ctx, gemm_decode_prologue_kernel, dim3(8 * mt, nseg, GD_PRO_SPLIT), 256, 0, st, A, pa, m, k);
-        ctx->launches++;
-    }
-    cudaError_t e = launch_decode_k(K, cb, mt, rmap, p, grid, st);
     ctx->launches++;
     if (e != cudaSuccess) { cudaGetLastError(); return exl3_fail(ctx, EXL3_ERR_CUDA, cudaGetErrorString(e)); }
     return EXL3_OK;
@@ -616,15 +517,10 @@ extern "C" int exl3_gemm(exl3_ctx* ctx, exl3_stream stream, const void* A, const
     const int NB = n / 128, NST = k / 128;
     EXL3_REQUIRE(NB <= ctx->n_counters, "exl3_gemm: n too large for the context's counters");
 
-    // Up to 16 rows the streaming decode kernel, up to 128 the kernel that keeps the weights in tensor memory (gemm_ts.cuh), above
-    // that the tcgen05 kernel over 512-row blocks per CTA pair and 256-column slabs (with CTA pairs a last slab of 128 columns is
+    // Up to 128 rows the kernel that keeps the weights in tensor memory (gemm_ts.cuh), above that the tcgen05 kernel over 512-row blocks per CTA pair and 256-column slabs (with CTA pairs a last slab of 128 columns is
     // allowed: its missing half reads zero-filled codes and is never stored; the last row block may be partial: its rows past m
     // are zero-filled by TMA, and a block with at most 256 valid rows runs a single MMA per K step).  The mma.sync small-M kernel
     // (209 us at 64 rows of 5120 x 17408) serves exl3_gemm_noalloc, EXL3_B200_NO_TC, and n % 256 == 128 under EXL3_B200_NO_PAIR.
-    if (m <= GD_MAX_M && ctx->use_decode) {
-        const half* suh1 = (const half*)suh; const half* svh1 = (const half*)svh;
-        return gemm_decode_rows(ctx, st, (const half*)A, 1, &trellis, &C, &suh1, &svh1, &n, m, k, K, c_fp32, cb);
-    }
     int tc_rows = 0;
     if (m > TC_MAX_SMALL_M && (n % TC_BN == 0 || ctx->use_pair || m <= TS_MAX_N) && ctx->use_tc) {
         tc_rows = m;
@@ -670,11 +566,6 @@ extern "C" int exl3_gemm_fanout(exl3_ctx* ctx, exl3_stream stream, const void* A
                w[i]->k % 128 == 0 && w[i]->K >= 1 && w[i]->K <= 8 && aligned16(w[i]->trellis) && aligned16(C[i]) &&
                aligned16(w[i]->suh) && aligned16(w[i]->svh) && (w[i]->suh != nullptr) == (w[0]->suh != nullptr);
     }
-    if (count > 1 && same && m <= GD_MAX_M && ctx->use_decode && aligned16(A)) {
-        const void* tr[GD_MAX_SEG]; const half* suh[GD_MAX_SEG]; const half* svh[GD_MAX_SEG]; int n[GD_MAX_SEG];
-        for (int i = 0; i < count; ++i) { tr[i] = w[i]->trellis; suh[i] = (const half*)w[i]->suh; svh[i] = (const half*)w[i]->svh; n[i] = w[i]->n; }
-        return gemm_decode_rows(ctx, (cudaStream_t)stream, (const half*)A, count, tr, C, suh, svh, n, m, w[0]->k, w[0]->K, c_fp32, w[0]->cb);
-    }
     if (count > 1 && same && m > TC_MAX_SMALL_M && ctx->use_tc && aligned16(A)) {
         const void* tr[TC_MAX_SEG]; const half* suh[TC_MAX_SEG]; const half* svh[TC_MAX_SEG]; int n[TC_MAX_SEG];
         for (int i = 0; i < count; ++i) { tr[i] = w[i]->trellis; suh[i] = (const half*)w[i]->suh; svh[i] = (const half*)w[i]->svh; n[i] = w[i]->n; }
@@ -692,25 +583,12 @@ extern "C" int exl3_gemm_fanout(exl3_ctx* ctx, exl3_stream stream, const void* A
 // are the ones gemm_tc_rows carves from the start of the context scratch, so the two calls agree on them by construction.
 static bool tc_pre_applies(exl3_ctx* ctx, int count, const exl3_linear* const* w, int m)
 {
-    if (!ctx || !w || count < 1 || count > TC_MAX_SEG || m <= GD_MAX_M || !ctx->use_tc) return false;
+    if (!ctx || !w || count < 1 || count > TC_MAX_SEG || m < 1 || !ctx->use_tc) return false;
     for (int i = 0; i < count; ++i) {
         if (!w[i] || !w[i]->trellis || !w[i]->suh) return false;
         if (w[i]->k != w[0]->k || w[i]->K != w[0]->K || w[i]->cb != w[0]->cb) return false;
-        if (w[i]->k % 128 != 0 || w[i]->n % 128 != 0 || !(w[i]->n % TC_BN == 0 || (ctx->use_pair && count == 1))) return false;
-        if (w[i]->K < 1 || w[i]->K > 8 || !aligned16(w[i]->trellis) || !aligned16(w[i]->suh) || !aligned16(w[i]->svh)) return false;
-    }
-    return true;
-}
-
-// The same for the decode GEMM (gemm_decode_rows).  Codebook 2 also needs the row sums of the transformed activations, which
-// the producers do not form; it keeps the separate transform.
-static bool decode_pre_applies(exl3_ctx* ctx, int count, const exl3_linear* const* w, int m)
-{
-    if (!ctx || !w || count < 1 || count > GD_MAX_SEG || m < 1 || m > GD_MAX_M || !ctx->use_decode) return false;
-    for (int i = 0; i < count; ++i) {
-        if (!w[i] || !w[i]->trellis || !w[i]->suh || w[i]->cb == 2) return false;
-        if (w[i]->k != w[0]->k || w[i]->K != w[0]->K || w[i]->cb != w[0]->cb) return false;
-        if (w[i]->k % 128 != 0 || w[i]->n % (count > 1 ? TC_BN : 128) != 0) return false;
+        if (m <= 16 && w[i]->cb == 2) return false;          // few rows of codebook 2 keep their transform launches
+        if (w[i]->k % 128 != 0 || w[i]->n % 128 != 0 || !(w[i]->n % TC_BN == 0 || (ctx->use_pair && count == 1) || m <= TS_MAX_N)) return false;
         if (w[i]->K < 1 || w[i]->K > 8 || !aligned16(w[i]->trellis) || !aligned16(w[i]->suh) || !aligned16(w[i]->svh)) return false;
     }
     return true;
@@ -720,19 +598,7 @@ bool exl3_pre_buffers(exl3_ctx* ctx, int count, const exl3_linear* const* w, int
 {
     size_t off = 0;
     if (!w || count < 1 || !w[0] || w[0]->k != dim) return false;
-    pre->nseg = count; pre->rows = m; pre->frag_rows = 0;
-    for (int i = 0; i < 3; ++i) pre->a_frag[i] = nullptr;
-    if (decode_pre_applies(ctx, count, w, m)) {
-        const int mt = m <= 8 ? 1 : 2;
-        pre->frag_rows = 8 * mt;
-        for (int i = 0; i < 3; ++i) { pre->suh[i] = nullptr; pre->a_had[i] = nullptr; }
-        for (int i = 0; i < count; ++i) {
-            pre->a_frag[i] = (uint32_t*)exl3_ws_take(ctx, &off, (size_t)mt * w[0]->k * 32);
-            if (!exl3_ws_take(ctx, &off, (size_t)GD_PRO_SPLIT * mt * 8 * 4) || !pre->a_frag[i]) return false;
-            pre->suh[i] = (const half*)w[i]->suh;
-        }
-        return true;
-    }
+    pre->nseg = count;
     if (!tc_pre_applies(ctx, count, w, m)) return false;
     for (int i = 0; i < 3; ++i) { pre->suh[i] = nullptr; pre->a_had[i] = nullptr; }
     for (int i = 0; i < count; ++i) {
@@ -745,14 +611,12 @@ bool exl3_pre_buffers(exl3_ctx* ctx, int count, const exl3_linear* const* w, int
 
 int exl3_gemm_fanout_pre(exl3_ctx* ctx, exl3_stream stream, int count, const exl3_linear* const* w, void* const* C, int m, int c_fp32)
 {
-    const bool decode = decode_pre_applies(ctx, count, w, m);
-    EXL3_REQUIRE((decode || tc_pre_applies(ctx, count, w, m)) && C, "exl3_gemm (activations transformed by the producer): not applicable to these tensors");
+    EXL3_REQUIRE(tc_pre_applies(ctx, count, w, m) && C, "exl3_gemm (activations transformed by the producer): not applicable to these tensors");
     const void* tr[TC_MAX_SEG]; const half* suh[TC_MAX_SEG]; const half* svh[TC_MAX_SEG]; int n[TC_MAX_SEG];
     for (int i = 0; i < count; ++i) {
         EXL3_REQUIRE(C[i] && aligned16(C[i]), "exl3_gemm: bad output pointer");
         tr[i] = w[i]->trellis; suh[i] = (const half*)w[i]->suh; svh[i] = (const half*)w[i]->svh; n[i] = w[i]->n;
     }
-    if (decode) return gemm_decode_rows(ctx, (cudaStream_t)stream, nullptr, count, tr, C, suh, svh, n, m, w[0]->k, w[0]->K, c_fp32, w[0]->cb, true);
     return gemm_tc_rows(ctx, (cudaStream_t)stream, nullptr, count, tr, C, suh, svh, n, m, w[0]->k, w[0]->K, c_fp32, w[0]->cb, true);
 }
 
@@ -870,10 +734,3 @@ extern "C" int exl3_gemm_noalloc_poll_status(exl3_stream stream)
     cudaStreamSynchronize(st);
     return EXL3_ERR_DEVICE_WAIT;
 }
-
-#ifdef GD_TRACE
-extern "C" EXL3_API int exl3_debug_gd_trace(unsigned long long* host_out)
-{
-    return cudaMemcpyFromSymbol(host_out, exl3::g_gd_trace, sizeof(unsigned long long) * 148 * 16 * 8) == cudaSuccess ? 0 : -1;
-}
-#endif

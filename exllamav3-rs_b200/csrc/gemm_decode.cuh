@@ -1,8 +1,8 @@
-// EXL3 GEMM for the decode regime (1..16 rows): the weight stream sets the time, so the kernel is built around the cost
-// of turning trellis codes into multiplier operands, one warp-instruction at a time.
+// EXL3 GEMM over tables of tensors (exl3_mgemm), up to 16 rows per product: the weight stream sets the time, so the kernel is
+// built around the cost of turning trellis codes into multiplier operands, one warp-instruction at a time.
 //
-// Function computed (reference: kernels/quant/exl3_gemm_kernel.cuh:14-50, exl3_gemm_inner.cuh:456-480; the reference's
-// own small-m kernel is kernels/quant/exl3_gemv_kernel.cuh:138-402):
+// Function computed (reference: kernels/quant/exl3_gemm_kernel.cuh:88-314, exl3_gemm_inner.cuh:456-480; the reference's
+// own small-m kernel is kernels/quant/exl3_gemv_kernel.cuh:138-402), per slot:
 //   C = H128( fp16(H128(A o suh)/sqrt128) . W ) / sqrt128 o svh
 //
 // Layout of the work.  A CTA has 16 warps = 8 k-slices x 2 column halves.  Its unit of work is (128-column block,
@@ -15,9 +15,9 @@
 // order (deterministic), and the finisher applies the output Hadamard and svh.
 //
 // The two warps of a k-slice share a ring of slots; one warp of a fifth warpgroup is the producer for all eight rings
-// (setmaxnreg moves that group's registers to the decoders): lane l of it keeps k-slice l's ring full (one TMA box of 4
-// tile rows x 8 tiles of codes per slot and, for up to 8 rows, one bulk copy of the slot's activations in MMA fragment
-// order, written by gemm_decode_prologue_kernel), signalled through one "full" and one "empty" mbarrier per slot.  A
+// (setmaxnreg moves that group's registers to the decoders): lane l of it keeps k-slice l's ring full (the codes of 4
+// tile rows x 8 tiles per slot and, for up to 8 rows, one bulk copy of the slot's activations in MMA fragment
+// order, written by gemm_decode_prologue_multi_kernel), signalled through one "full" and one "empty" mbarrier per slot.  A
 // decoder's main loop is: wait, decode and multiply its 16 tiles, release - no CTA-wide barrier and no address arithmetic.
 //
 // Multiplier mapping.  The 16x16 tile is stored in mma.m16n8k16 B-fragment order; read as the A operand of the
@@ -35,28 +35,12 @@
 
 namespace exl3 {
 
-#ifdef GD_TRACE
-// timeline of one launch (debug builds only): per CTA and warp [start, first data, loop end, end] in nanoseconds
-__device__ unsigned long long g_gd_trace[148 * 16 * 8];
-__device__ __forceinline__ unsigned long long gd_now() { unsigned long long t; asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t)); return t; }
-#define GD_STAMP(slot) do { if (lane == 0 && warp < 16 && blockIdx.x < 148) g_gd_trace[(blockIdx.x * 16 + warp) * 8 + (slot)] = gd_now(); } while (0)
-#define GD_ACC(slot, v) do { if (lane == 0 && warp < 16 && blockIdx.x < 148) g_gd_trace[(blockIdx.x * 16 + warp) * 8 + (slot)] += (v); } while (0)
-#define GD_T0() const unsigned long long gd_t0_ = gd_now()
-#define GD_DT() (gd_now() - gd_t0_)
-#else
-#define GD_STAMP(slot) do { } while (0)
-#define GD_ACC(slot, v) do { } while (0)
-#define GD_T0() do { } while (0)
-#define GD_DT() 0
-#endif
-
 constexpr int GD_WARPS = 16;                 // decoder warps
 constexpr int GD_THREADS = (GD_WARPS + 4) * 32;            // + the producer's warpgroup (one of its four warps works)
 constexpr int GD_KSL = 8;                    // k-slices of a CTA unit
-constexpr int GD_SLOT_ROWS = 4;              // tile rows per TMA box = one k-slice (64 k)
+constexpr int GD_SLOT_ROWS = 4;              // tile rows per slot = one k-slice (64 k)
 constexpr int GD_UNIT_K = GD_KSL * GD_SLOT_ROWS * 16;      // k extent of a unit: 512
-constexpr int GD_SLOT_TILES = 4;             // tiles per row of a box (one column half)
-constexpr int GD_MAX_SEG = 3;
+constexpr int GD_SLOT_TILES = 4;             // tiles per row of a column half
 constexpr int GD_RSTRIDE = 132;              // floats per row of the reduction tiles
 constexpr float GD_R128 = 0.088388347648f;
 constexpr float GD_MUL1_KINV = 0.00676727294921875f;
@@ -80,28 +64,23 @@ template <int K, int MT> struct GdSmem {
     static constexpr int BYTES = OFF_BAR + 2 * GD_KSL * DEPTH * 8 + 128;           // + slack to align the base to 128 bytes
 };
 
+// `slots` products over tensors picked from device-resident tables.  Slot j uses tensor indices[j] (j itself when indices is
+// NULL; a negative entry leaves the slot untouched), reads its own activations, writes C + j * c_slot_stride, scaled by weights[j]
+// when given.  All tensors have n columns; the column blocks of slot j are blocks [j * n/128, (j + 1) * n/128).
 struct GemmDecodeParams {
-    const uint4* a_frag[GD_MAX_SEG];   // [MT][k/64][4][32] uint4: activations in B-fragment order, duplicated halves
-    const float* rowsum[GD_MAX_SEG];   // [rowsum_parts][8*MT] partial sums over k of the transformed activations (codebook 2 only)
-    int rowsum_parts;                  // k ranges the input transform was split into (their sums are added in order)
-    void* C[GD_MAX_SEG];               // [m][n] fp16 or fp32
-    const half* svh[GD_MAX_SEG];       // [n] or NULL
-    int n[GD_MAX_SEG];
-    int blk_end[GD_MAX_SEG];           // running count of 128-column blocks
-    float* partial;                    // [grid][2][m][128] fp32: a CTA's first and last column block when shared
-    int* counters;                     // [column blocks] arrival counters, zero on entry and on exit
-    int* status;
-    int m, k, c_fp32;
-    int aligned;                       // 1: every CTA owns whole column blocks (no block is shared), 0: stream-K over units
-    // Table mode (the kernel's MULTI form, exl3_mgemm): `slots` products over tensors picked from device-resident tables.
-    // Slot j uses tensor indices[j] (j itself when indices is NULL; a negative entry leaves the slot untouched), reads
-    // the activations a_frag[0] + j * slot stride and writes C[0] + j * m * n, scaled by weights[j] when given.  All
-    // tensors have n[0] columns; the column blocks of slot j are blocks [j * n/128, (j + 1) * n/128).
+    const uint4* a_frag;               // [slots][MT][k/64][4][32] uint4: activations in B-fragment order, duplicated halves
+    const float* rowsum;               // [slots][8*MT] sums over k of the transformed activations (codebook 2 only)
+    void* C;                           // [slots][m][n] fp16 or fp32
     const uint32_t* const* trellis_tab;
     const half* const* svh_tab;
     const int64_t* indices;
     const half* weights;
-    int slots;
+    float* partial;                    // [grid][2][m][128] fp32: a CTA's first and last column block when shared
+    int* counters;                     // [column blocks] arrival counters, zero on entry and on exit
+    int* status;
+    int m, k, n, c_fp32;
+    int blocks;                        // column blocks of all slots
+    int aligned;                       // 1: every CTA owns whole column blocks (no block is shared), 0: stream-K over units
     long long c_slot_stride;           // elements between the outputs of consecutive slots
 };
 
@@ -152,17 +131,12 @@ __device__ __forceinline__ void gd_slot(const uint32_t* __restrict__ sb, int ch,
     }
 }
 
-// Activations in fragment order.  One CTA per (batch row slot b, tensor): row b < m is transformed as in
+// Activations in fragment order.  One CTA per (batch row slot b, product slot): row b < m is transformed as in
 // kernels/quant/hadamard_inner.cuh:93-147 (fp16 pre-scale multiply, fp32 butterflies, one fp16 rounding); slots past m
 // are zero-filled.  Word (set, kslot, r, lane = 4 g + t, w) holds the value of batch row 8 set + g at
 // k = 64 kslot + 16 r + 2 t + (w & 1) + 8 (w >> 1), duplicated into both halves.
-struct GemmDecodePrologueArgs { const half* suh[GD_MAX_SEG]; uint32_t* a_frag[GD_MAX_SEG]; float* rowsum[GD_MAX_SEG]; };
-
-// one CTA: batch-row slot b of one tensor's activations
-constexpr int GD_PRO_SPLIT = 4;      // CTAs along k per row slot in the input transform of the single-tensor paths
-
 __device__ __forceinline__ void gd_prologue_row(const half* __restrict__ Arow, const half* __restrict__ suh, uint32_t* __restrict__ out,
-                                                float* __restrict__ rowsum, int b, bool valid, int k, int part_idx = 0, int parts = 1)
+                                                float* __restrict__ rowsum, int b, bool valid, int k)
 {
     __shared__ float sh[8];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -170,9 +144,7 @@ __device__ __forceinline__ void gd_prologue_row(const half* __restrict__ Arow, c
     const int q = lane & 3;                                  // position of the lane's 4 values inside a 16-k tile row
     const int t0 = 2 * (q & 1), w0 = 2 * (q >> 1);
     float part = 0.0f;
-    const int per = (k / 128 + parts - 1) / parts;             // 128-blocks of this CTA's k range
-    const int blk_end = min(k / 128, (part_idx + 1) * per);
-    for (int blk = part_idx * per + warp; blk < blk_end; blk += 8) {
+    for (int blk = warp; blk < k / 128; blk += 8) {
         uint32_t h0 = 0, h1 = 0, h2 = 0, h3 = 0;
         if (valid) {
             uint2 raw = reinterpret_cast<const uint2*>(Arow + blk * 128)[lane];
@@ -214,19 +186,11 @@ __device__ __forceinline__ void gd_prologue_row(const half* __restrict__ Arow, c
     if (threadIdx.x == 0) {
         float s = 0.0f;
         for (int w = 0; w < 8; ++w) s += sh[w];
-        rowsum[(size_t)part_idx * gridDim.x + b] = s;
+        rowsum[b] = s;
     }
 }
 
-static __global__ void __launch_bounds__(256) gemm_decode_prologue_kernel(const half* __restrict__ A, const GemmDecodePrologueArgs args,
-                                                                   int m, int k)
-{
-    pdl_enter();
-    const int b = blockIdx.x, seg = blockIdx.y;
-    gd_prologue_row(A + (size_t)b * k, args.suh[seg], args.a_frag[seg], args.rowsum[seg], b, b < m, k, blockIdx.z, gridDim.z);
-}
-
-// Table mode: grid (row slots, product slots).  Slot j transforms rows of A[j] (or of A[0] when a_slot_stride is 0) with
+// grid (row slots, product slots).  Slot j transforms rows of A[j] (or of A[0] when a_slot_stride is 0) with
 // the sign vector of the tensor it uses; an unused slot (negative index) gets zeros.
 static __global__ void __launch_bounds__(256) gemm_decode_prologue_multi_kernel(const half* __restrict__ A, size_t a_slot_stride,
                                                                          const half* const* __restrict__ suh_tab,
@@ -285,18 +249,14 @@ __device__ __forceinline__ void gd_store_row(float4 v, int lane, float rowsum, c
 }
 
 // grid = CTAs of the split (at most one per SM), 20 warps (16 decoders, the producer and its three idle warpgroup mates), GdSmem<K, MT>::BYTES of dynamic shared memory.
-// rmap*: the trellis of each tensor as a matrix of 64-bit words [k/16][n/16 * 4K], box 4 rows x 4 tiles.
 //
 // Leaving a column block does not stop the CTA: every decoder drops its accumulators into the reduction tile and goes on
 // with the next block; the one that arrives last adds the 8 k-slices, exchanges partial sums with the neighbouring CTAs
 // where the block is shared, transforms and stores, and then hands the tile back (an mbarrier the other warps test before
 // their next drop, several units later).  While that warp waits on the arrival counter of the exchange, the other warps
 // of its scheduler use its issue slots.
-template <int K, int CB, int MT, bool MULTI = false>
-__global__ void __launch_bounds__(GD_THREADS, 1) gemm_decode_kernel(const __grid_constant__ CUtensorMap rmap0,
-                                                                   const __grid_constant__ CUtensorMap rmap1,
-                                                                   const __grid_constant__ CUtensorMap rmap2,
-                                                                   const GemmDecodeParams p)
+template <int K, int CB, int MT>
+__global__ void __launch_bounds__(GD_THREADS, 1) gemm_decode_kernel(const GemmDecodeParams p)
 {
     using SM = GdSmem<K, MT>;
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -310,7 +270,7 @@ __global__ void __launch_bounds__(GD_THREADS, 1) gemm_decode_kernel(const __grid
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int KC = (p.k + GD_UNIT_K - 1) / GD_UNIT_K;                  // k chunks per column block
-    const int blocks = p.blk_end[GD_MAX_SEG - 1];
+    const int blocks = p.blocks;
     const long long total = (long long)blocks * KC;
     const long long G = gridDim.x;
     // this CTA's contiguous range of units (column-block-major): whole blocks, or an even share of all units
@@ -319,23 +279,13 @@ __global__ void __launch_bounds__(GD_THREADS, 1) gemm_decode_kernel(const __grid
     const int nunits = (int)(u1 - u0);
     const int mrows = p.m;
     const int nbg0 = (int)(u0 / KC), kc0 = (int)(u0 - (long long)nbg0 * KC);
-    const int bpm = p.n[0] >> 7;                                       // column blocks per tensor (table mode)
-    auto seg_of = [&](int nbg) -> int {
-        if constexpr (MULTI) return nbg / bpm;
-        else return (nbg >= p.blk_end[0]) + (nbg >= p.blk_end[1]);
-    };
-    auto col0_of = [&](int nbg, int seg) -> int {
-        if constexpr (MULTI) return (nbg - seg * bpm) * 128;
-        else return (nbg - (seg == 0 ? 0 : (seg == 1 ? p.blk_end[0] : p.blk_end[1]))) * 128;
-    };
-    // table mode: the tensor a slot uses, or -1
+    const int bpm = p.n >> 7;                                          // column blocks per tensor
+    auto seg_of = [&](int nbg) -> int { return nbg / bpm; };
+    auto col0_of = [&](int nbg, int seg) -> int { return (nbg - seg * bpm) * 128; };
+    // the tensor a slot uses, or -1
     auto mat_of = [&](int seg) -> int { return p.indices ? (int)p.indices[seg] : seg; };
-    const size_t afrag_slot = (size_t)MT * (p.k / 64) * GD_SLOT_ROWS * 32;        // uint4 per slot of activations (table mode)
+    const size_t afrag_slot = (size_t)MT * (p.k / 64) * GD_SLOT_ROWS * 32;        // uint4 per slot of activations
 
-    GD_STAMP(0);
-#ifdef GD_TRACE
-    if (lane == 0 && warp < 16 && blockIdx.x < 148) { for (int q = 4; q < 7; ++q) g_gd_trace[(blockIdx.x * 16 + warp) * 8 + q] = 0; }
-#endif
     if (tid == 0) {
         for (int i = 0; i < GD_KSL * SM::DEPTH; ++i) { mbar_init(&full_bars[i], 1); mbar_init(&empty_bars[i], 2); }
         mbar_init(&s_red_free, 1);
@@ -372,29 +322,23 @@ __global__ void __launch_bounds__(GD_THREADS, 1) gemm_decode_kernel(const __grid
             if (go) {
                 const uint32_t bar = fb + 8u * slot;
                 const int seg = seg_of(nbg);
-                const int mat = MULTI ? mat_of(seg) : 0;
+                const int mat = mat_of(seg);
                 if (kc * GD_UNIT_K + ks * (GD_SLOT_ROWS * 16) < p.k && mat >= 0) {
                     const uint32_t dst = ring + slot * SM::SLOT_BYTES;
                     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"((uint32_t)SM::SLOT_BYTES) : "memory");
-                    if constexpr (MULTI) {
-                        // the tensor comes out of a device table: four row copies of 8 tiles each instead of one tiled box
-                        const uint32_t* src = p.trellis_tab[mat] +
-                            ((size_t)(kc * (GD_UNIT_K / 16) + ks * GD_SLOT_ROWS) * (p.n[0] >> 4) + (col0_of(nbg, seg) >> 4)) * 8 * K;
-                        #pragma unroll
-                        for (int r = 0; r < GD_SLOT_ROWS; ++r)
-                            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                                         ::"r"(dst + (uint32_t)(r * (SM::CODE_BYTES / GD_SLOT_ROWS))), "l"(src + (size_t)r * (p.n[0] >> 4) * 8 * K),
-                                           "r"((uint32_t)(SM::CODE_BYTES / GD_SLOT_ROWS)), "r"(bar) : "memory");
-                    } else {
-                        const CUtensorMap* rmap = seg == 0 ? &rmap0 : (seg == 1 ? &rmap1 : &rmap2);
-                        gd_tma_load_2d(dst, rmap, (col0_of(nbg, seg) >> 4) * 4 * K, kc * (GD_UNIT_K / 16) + ks * GD_SLOT_ROWS, bar);
-                    }
+                    // the tensor comes out of a device table: no tensor map, but a copy of 8 tiles for each of the four rows
+                    const uint32_t* src = p.trellis_tab[mat] +
+                        ((size_t)(kc * (GD_UNIT_K / 16) + ks * GD_SLOT_ROWS) * (p.n >> 4) + (col0_of(nbg, seg) >> 4)) * 8 * K;
+                    #pragma unroll
+                    for (int r = 0; r < GD_SLOT_ROWS; ++r)
+                        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                                     ::"r"(dst + (uint32_t)(r * (SM::CODE_BYTES / GD_SLOT_ROWS))), "l"(src + (size_t)r * (p.n >> 4) * 8 * K),
+                                       "r"((uint32_t)(SM::CODE_BYTES / GD_SLOT_ROWS)), "r"(bar) : "memory");
                     if constexpr (SM::ACT_BYTES > 0) {
                         // The launch may overlap the tail of the kernel that writes the activations (programmatic dependent
                         // launch): the codes above do not depend on it, the activations do.
                         if (!waited) { pdl_wait(); waited = true; }
-                        const uint4* afr = MULTI ? p.a_frag[0] + (size_t)seg * afrag_slot
-                                                 : (seg == 0 ? p.a_frag[0] : (seg == 1 ? p.a_frag[1] : p.a_frag[2]));
+                        const uint4* afr = p.a_frag + (size_t)seg * afrag_slot;
                         asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                                      ::"r"(dst + (uint32_t)SM::CODE_BYTES), "l"(afr + (size_t)(kc * GD_KSL + ks) * kslot_stride),
                                        "r"((uint32_t)SM::ACT_BYTES), "r"(bar) : "memory");
@@ -437,14 +381,13 @@ __global__ void __launch_bounds__(GD_THREADS, 1) gemm_decode_kernel(const __grid
         #pragma unroll 1
         for (int i = 0; i < nunits; ++i) {
             if (++kc == KC) { kc = 0; ++nbg; }
-            const bool active = kc * GD_UNIT_K + ks * (GD_SLOT_ROWS * 16) < p.k && (!MULTI || mat_of(seg_of(nbg)) >= 0);
+            const bool active = kc * GD_UNIT_K + ks * (GD_SLOT_ROWS * 16) < p.k && mat_of(seg_of(nbg)) >= 0;
             if (!failed) {
                 uint4 af[MT][GD_SLOT_ROWS];
                 if (SM::ACT_BYTES == 0 && active) {
                     // batch rows 8 set + g, k = 64 kslot + 16 r + {2t, 2t+1, 2t+8, 2t+9}
                     const int seg = seg_of(nbg);
-                    const uint4* afr = MULTI ? p.a_frag[0] + (size_t)seg * afrag_slot
-                                             : (seg == 0 ? p.a_frag[0] : (seg == 1 ? p.a_frag[1] : p.a_frag[2]));
+                    const uint4* afr = p.a_frag + (size_t)seg * afrag_slot;
                     const int kslot = kc * GD_KSL + ks;
                     #pragma unroll
                     for (int s = 0; s < MT; ++s)
@@ -452,10 +395,7 @@ __global__ void __launch_bounds__(GD_THREADS, 1) gemm_decode_kernel(const __grid
                         for (int r = 0; r < GD_SLOT_ROWS; ++r)
                             af[s][r] = __ldg(afr + (((size_t)s * (p.k / 64) + kslot) * 4 + r) * 32 + lane);
                 }
-                GD_T0();
                 const bool ok = mbar_wait_sleep_warp(&full[slot], par);
-                if (i > 0) GD_ACC(4, GD_DT());
-                if (i == 0) GD_STAMP(1);
                 if (ok) {
                     if (active) gd_slot<K, CB, MT>(reinterpret_cast<const uint32_t*>(ring + slot * SM::SLOT_BYTES), ch, lane, lane_prev, af, acc);
                     __syncwarp();
@@ -465,7 +405,6 @@ __global__ void __launch_bounds__(GD_THREADS, 1) gemm_decode_kernel(const __grid
             }
 
             const bool block_done = kc == KC - 1 || i == nunits - 1;
-            if (i == nunits - 1) GD_STAMP(2);
             if (!block_done) continue;
 
             // ---- the CTA leaves column block nbg.  The reduction tile is free again once the warp that finished the
@@ -491,31 +430,17 @@ __global__ void __launch_bounds__(GD_THREADS, 1) gemm_decode_kernel(const __grid
             if (!last) continue;
 
             // ---- this warp arrived last: it finishes the block on its own
-            GD_T0();
             if (lane == 0) s_drops = 0;
             __threadfence_block();
             const int seg = seg_of(nbg);
             const int n0 = col0_of(nbg, seg);
-            const half* svh = seg == 0 ? p.svh[0] : (seg == 1 ? p.svh[1] : p.svh[2]);
-            void* Cout = seg == 0 ? p.C[0] : (seg == 1 ? p.C[1] : p.C[2]);
-            int n = seg == 0 ? p.n[0] : (seg == 1 ? p.n[1] : p.n[2]);
-            const float* rsum = seg == 0 ? p.rowsum[0] : (seg == 1 ? p.rowsum[1] : p.rowsum[2]);
-            float r128 = GD_R128;
-            bool store = true;
-            if constexpr (MULTI) {
-                const int mat = mat_of(seg);
-                store = mat >= 0;                         // an unused slot's rows of C are left as they are
-                n = p.n[0];
-                svh = store ? p.svh_tab[mat] : nullptr;
-                Cout = p.c_fp32 ? (void*)((float*)p.C[0] + (size_t)seg * p.c_slot_stride) : (void*)((half*)p.C[0] + (size_t)seg * p.c_slot_stride);
-                rsum = p.rowsum[0] + (size_t)seg * SM::ROWS;
-                if (p.weights) r128 *= __half2float(p.weights[seg]);
-            }
-            auto rs_of = [&](int row) -> float {
-                float a = 0.f;
-                for (int z = 0; z < p.rowsum_parts; ++z) a += rsum[(size_t)z * SM::ROWS + row];
-                return a;
-            };
+            const int mat = mat_of(seg);
+            const bool store = mat >= 0;                  // an unused slot's rows of C are left as they are
+            const int n = p.n;
+            const half* svh = store ? p.svh_tab[mat] : nullptr;
+            void* Cout = p.c_fp32 ? (void*)((float*)p.C + (size_t)seg * p.c_slot_stride) : (void*)((half*)p.C + (size_t)seg * p.c_slot_stride);
+            const float* rsum = p.rowsum + (size_t)seg * SM::ROWS;
+            const float r128 = p.weights ? GD_R128 * __half2float(p.weights[seg]) : GD_R128;
             // sum of the 8 k-slices of one row, in slice order; lane = 4 consecutive columns
             auto row_sum = [&](int row) -> float4 {
                 float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -536,7 +461,7 @@ __global__ void __launch_bounds__(GD_THREADS, 1) gemm_decode_kernel(const __grid
             const int ncontrib = c_last - c_first + 1;
             if (ncontrib == 1) {
                 for (int row = 0; row < mrows && store; ++row)
-                    gd_store_row<CB>(row_sum(row), lane, CB == 2 ? rs_of(row) : 0.f, svh, Cout, (size_t)row * n + n0 + lane * 4, n0, p.c_fp32, r128);
+                    gd_store_row<CB>(row_sum(row), lane, CB == 2 ? rsum[row] : 0.f, svh, Cout, (size_t)row * n + n0 + lane * 4, n0, p.c_fp32, r128);
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&s_red_free);
             } else {
@@ -579,13 +504,11 @@ __global__ void __launch_bounds__(GD_THREADS, 1) gemm_decode_kernel(const __grid
                         #pragma unroll
                         for (int r = 0; r < 8; ++r)
                             if (row0 + r < mrows && store)
-                                gd_store_row<CB>(a[r], lane, CB == 2 ? rs_of(row0 + r) : 0.f, svh, Cout, (size_t)(row0 + r) * n + n0 + lane * 4, n0, p.c_fp32, r128);
+                                gd_store_row<CB>(a[r], lane, CB == 2 ? rsum[row0 + r] : 0.f, svh, Cout, (size_t)(row0 + r) * n + n0 + lane * 4, n0, p.c_fp32, r128);
                     }
                 }
             }
-            GD_ACC(5, GD_DT());
         }
-        GD_STAMP(3);
     }
     // A wait that ran out ends the CTA's work; the status word tells the host.  (Copies still in flight belong to slots
     // whose barrier nobody waits on any more; they were requested at most a ring's depth ahead and land within microseconds,

@@ -1,4 +1,4 @@
-// EXL3 GEMM for medium row counts (verify batches, many users, the ragged end of a prefill): the decoded weights are the
+// EXL3 GEMM up to 128 rows (decoding, verify batches, many users, the ragged end of a prefill): the decoded weights are the
 // tensor core's A operand and never leave the SM's tensor memory.
 //
 // What bounds it: turning codes into fp16 weights, 43 warp instructions per 16 x 16 tile and 47 cycles per scheduler with
@@ -18,6 +18,10 @@
 // Whole calls, us, tcgen05 kernel of gemm_tc.cuh -> this one: 5120 x 17408 at 4 bits 45.5 -> 32.8 (32 rows), 45.6 -> 33.1 (52),
 // 47.4 -> 35.1 (128); 52 rows at 3 and 8 bits 49.1 -> 36.0, 46.6 -> 34.9; 17408 x 5120 80.3 -> 34.6 (32 rows), 85.6 -> 41.3
 // (128); 5120 x 5120 30.9 -> 17.3 and 31.1 -> 22.9; 5120 x 151936, 52 rows, 359 -> 183.
+// Up to 16 rows it replaces a kernel that streamed raw codes through mma.sync (50 cycles per tile and scheduler up to 8 rows, more
+// than twice that above), us: 5120 x 17408 at 4 bits 27.9 -> 25.6 (1 row), 29.3 -> 27.4 (8), 39.2 -> 27.4 (16); 17408 x 5120 at 3
+// bits 37.2 -> 29.8, 39.9 -> 32.0, 58.5 -> 32.5; 5120 x 5120 18.8 -> 15.1, 21.0 -> 15.3, 33.2 -> 15.4.  The weights being rounded
+// to fp16 here, as the format has them, the error against 64 bits falls from 4.2e-4 to 3.6e-4.
 //
 // Work: units of (128-column block, 128 k), column-block-major, in contiguous ranges per CTA (ts_split in gemm.cu); partial sums
 // of a block that several CTAs share are added in owner order by the last one to arrive (deterministic).  Roles: warps 0..15
@@ -43,6 +47,7 @@ constexpr int TS_SB = 6;                            // most slots of the activat
 // phase's parity for its own.
 constexpr int TS_SR = 8;
 constexpr uint32_t TS_POLLS = 1u << 24, TS_NS = 100;   // a wait gives up after about two seconds
+constexpr int TS_FEW = 4;                           // most rows that the kernel transforms itself
 constexpr int TS_T_ROWS = 64, TS_TSTRIDE = 132;     // output tile: rows at a time, floats per row
 
 // the activation ring takes what the codes leave of a CTA's 227 KB, 96 KB at most
@@ -78,10 +83,14 @@ struct GemmTsParams {
     int nb;                            // m rounded up to 16
     int sb;                            // slots of the activation ring
     int aligned;                       // 1: every CTA owns whole column blocks
+    // few rows: the activations as they come, [m][k] fp16 with a sign vector per tensor; the kernel transforms them itself
+    const half* x;
+    const half* suh[TC_MAX_SEG];
+    int early;                         // 0: nothing of global memory is touched before the kernels in front are complete
 };
 
 // gemm_ts.cu
-cudaError_t gemm_ts_launch(int K, int cb, const CUtensorMap* amap, const CUtensorMap* rmap, const GemmTsParams& p, int grid, cudaStream_t st);
+cudaError_t gemm_ts_launch(int K, int cb, const CUtensorMap* amap, const CUtensorMap* rmap, const GemmTsParams& p, int grid, bool overlap, cudaStream_t st);
 
 __device__ __forceinline__ void ts_mma(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate)
 {
@@ -214,6 +223,37 @@ __device__ __forceinline__ void ts_finish_partials(const GemmTsParams& p, const 
     }
 }
 
+// 128-point Hadamard transform of (x o signs) for 128 values of R rows, lane = 4 consecutive ones (arithmetic of gd_prologue_row)
+template <int R>
+__device__ __forceinline__ void ts_transform(uint2 (&x)[R], uint2 sg, int lane)
+{
+    float v[R][4];
+    #pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const half2 a = __hmul2(*reinterpret_cast<const half2*>(&x[r].x), *reinterpret_cast<const half2*>(&sg.x));
+        const half2 b = __hmul2(*reinterpret_cast<const half2*>(&x[r].y), *reinterpret_cast<const half2*>(&sg.y));
+        const float s0 = __low2float(a) + __high2float(a), d0 = __low2float(a) - __high2float(a);
+        const float s1 = __low2float(b) + __high2float(b), d1 = __low2float(b) - __high2float(b);
+        v[r][0] = s0 + s1; v[r][1] = d0 + d1; v[r][2] = s0 - s1; v[r][3] = d0 - d1;
+    }
+    #pragma unroll
+    for (int i = 1; i < 32; i <<= 1) {
+        const bool up = lane & i;
+        #pragma unroll
+        for (int r = 0; r < R; ++r)
+            #pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const float o = __shfl_xor_sync(0xffffffffu, v[r][e], i);
+                v[r][e] = (up ? -v[r][e] : v[r][e]) + o;
+            }
+    }
+    #pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const half2 p = __floats2half2_rn(v[r][0] * TC_R128, v[r][1] * TC_R128), q = __floats2half2_rn(v[r][2] * TC_R128, v[r][3] * TC_R128);
+        x[r] = make_uint2(*reinterpret_cast<const uint32_t*>(&p), *reinterpret_cast<const uint32_t*>(&q));
+    }
+}
+
 // Warp-uniform bounded wait with a short way through when the phase is complete already: one poll and one vote.
 __device__ __forceinline__ bool ts_wait(uint64_t* bar, uint32_t parity)
 {
@@ -226,7 +266,53 @@ __device__ __forceinline__ bool ts_wait(uint64_t* bar, uint32_t parity)
     return ok;
 }
 
-// the same for one thread
+// Activations of up to R rows, units odd, odd + 2, ... of the CTA: (x o signs), 128-point transform, rows of 128 bytes with the
+// 16-byte chunks XORed with row & 7 in slot u % SW; the rows past m stay zero.  False when a wait ran out.
+template <int R>
+__device__ __forceinline__ bool ts_few_rows(const GemmTsParams& p, uint8_t* ring, uint64_t* done, uint64_t* w_full, int nbg, int ks, int KS, int nst, int odd, int lane)
+{
+    for (int i = lane; i < 3 * 256; i += 32)
+        *reinterpret_cast<uint4*>(ring + (2 * (i >> 8) + odd) * 4096 + (i & 255) * 16) = make_uint4(0u, 0u, 0u, 0u);
+    __syncwarp();
+    pdl_wait();
+    ks += odd;
+    int sw = odd;
+    uint32_t par = 1;
+    uint2 x[R], sg = make_uint2(0u, 0u);
+    bool sign = false;
+    auto fetch = [&]() {
+        while (ks >= KS) { ks -= KS; ++nbg; }
+        const int seg = (nbg >= p.blk_end[0]) + (nbg >= p.blk_end[1]);
+        const half* suh = seg == 0 ? p.suh[0] : (seg == 1 ? p.suh[1] : p.suh[2]);
+        sign = suh != nullptr;
+        if (sign) sg = reinterpret_cast<const uint2*>(suh + ks * TS_UNIT_K)[lane];
+        #pragma unroll
+        for (int r = 0; r < R; ++r)                                   // (rows past m repeat the last one and are not written)
+            x[r] = reinterpret_cast<const uint2*>(p.x + (size_t)(r < p.m ? r : p.m - 1) * p.k + ks * TS_UNIT_K)[lane];
+    };
+    if (odd < nst) fetch();
+    for (int s = odd; s < nst; s += 2) {
+        uint2 h[R];
+        #pragma unroll
+        for (int r = 0; r < R; ++r) h[r] = x[r];
+        if (sign) ts_transform<R>(h, sg, lane);
+        ks += 2;
+        if (s + 2 < nst) fetch();                                      // the next unit's, under the wait
+        if (!ts_wait(&done[sw], par)) return false;
+        uint8_t* dst = ring + sw * 4096 + (lane >> 4) * 2048 + (lane & 1) * 8;
+        #pragma unroll
+        for (int r = 0; r < R; ++r)
+            if (r < p.m) *reinterpret_cast<uint2*>(dst + r * 128 + ((((lane & 15) >> 1) ^ r) << 4)) = h[r];
+        fence_proxy_async();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&w_full[sw]);
+        __syncwarp();
+        sw += 2; if (sw >= TS_SW) { sw -= TS_SW; par ^= 1; }
+    }
+    return true;
+}
+
+// the same wait for one thread
 __device__ __forceinline__ bool ts_wait1(uint32_t bar, uint32_t parity)
 {
     uint32_t ok;
@@ -267,7 +353,7 @@ __global__ void __launch_bounds__(TS_THREADS, 1) gemm_ts_kernel(const __grid_con
     __shared__ uint32_t s_tmem;
     __shared__ int s_failed, s_fin, s_last;
 
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (p.early) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int KS = p.k / TS_UNIT_K;                                    // units per column block
     const int blocks = p.blk_end[TC_MAX_SEG - 1];
@@ -295,11 +381,17 @@ __global__ void __launch_bounds__(TS_THREADS, 1) gemm_ts_kernel(const __grid_con
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    if (!p.early) pdl_enter_first(0);
     const uint32_t tmem = s_tmem;
     bool failed = false;
     int issued = 0;                                                    // copies requested by a producer
 
-    if (warp == TS_SERVICE) {
+    if (p.x && (warp == TS_SERVICE + 1 || warp == TS_SERVICE + 3)) {
+        // ===== few rows: two warps take units in turn, transform their activations and write them where the TMA would
+        const int odd = warp == TS_SERVICE + 3;
+        failed = !(p.m == 1 ? ts_few_rows<1>(p, smem + SM::OFF_B, done, w_full, nbg0, ks0, KS, nst, odd, lane)
+                            : ts_few_rows<TS_FEW>(p, smem + SM::OFF_B, done, w_full, nbg0, ks0, KS, nst, odd, lane));
+    } else if (warp == TS_SERVICE) {
         // ===== codes: one box of 8 tile rows x 8 tiles per unit
         if (lane == 0) {
             const uint32_t bars = smem_u32(r_full), ring = smem_u32(smem + SM::OFF_RAW);

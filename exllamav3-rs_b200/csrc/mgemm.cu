@@ -3,7 +3,7 @@
 // csrc/exl3_shim.cpp:57-75).  The routing never touches the host: one launch covers every slot, a slot whose index is
 // negative is skipped, and with `weights` the slots of each token are scaled and summed into that token's row.
 //
-// Built on the streaming decode kernel in its table form: slot j is a run of column blocks whose codes come from
+// Built on the streaming decode kernel (gemm_decode.cuh): slot j is a run of column blocks whose codes come from
 // trellis_tab[indices[j]] by plain bulk copies (the tensor is not known on the host, so there is no tensor map), whose
 // activations were transformed with that tensor's input sign vector, and whose output goes to C[j].
 #include "gemm_decode.cuh"
@@ -17,7 +17,7 @@ cudaError_t launch_multi(const GemmDecodeParams& p, int grid, cudaStream_t st)
 {
     constexpr int bytes = GdSmem<K, MT>::BYTES;
     static bool configured[64] = {};
-    auto kern = gemm_decode_kernel<K, CB, MT, true>;
+    auto kern = gemm_decode_kernel<K, CB, MT>;
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64 || !configured[dev]) {
@@ -31,9 +31,7 @@ cudaError_t launch_multi(const GemmDecodeParams& p, int grid, cudaStream_t st)
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr; cfg.numAttrs = 1;
-    CUtensorMap none;
-    memset(&none, 0, sizeof(none));
-    return cudaLaunchKernelEx(&cfg, kern, none, none, none, p);
+    return cudaLaunchKernelEx(&cfg, kern, p);
 }
 
 template <int K, int CB>
@@ -130,13 +128,12 @@ extern "C" int exl3_mgemm(exl3_ctx* ctx, exl3_stream stream, const void* A, cons
         gemm_decode_prologue_multi_kernel<<<dim3(8 * mt, bszm), 256, 0, st>>>(a0, bszm_in == 1 ? 0 : (size_t)m * k, (const half* const*)suh,
                                                                              indices, a_frag, rowsum, 8 * mt, rows, k);
         ctx->launches++;
-        p.a_frag[0] = (const uint4*)a_frag; p.rowsum[0] = rowsum; p.rowsum_parts = 1;
-        p.C[0] = c_fp32 ? (void*)((float*)C + (size_t)r0 * n) : (void*)((half*)C + (size_t)r0 * n);
-        p.n[0] = p.n[1] = p.n[2] = n;
-        p.blk_end[0] = p.blk_end[1] = p.blk_end[2] = blocks;
+        p.a_frag = (const uint4*)a_frag; p.rowsum = rowsum;
+        p.C = c_fp32 ? (void*)((float*)C + (size_t)r0 * n) : (void*)((half*)C + (size_t)r0 * n);
+        p.n = n; p.blocks = blocks;
         p.counters = ctx->counters; p.status = ctx->status; p.m = rows; p.k = k; p.c_fp32 = c_fp32;
         p.trellis_tab = (const uint32_t* const*)trellis; p.svh_tab = (const half* const*)svh;
-        p.indices = indices; p.weights = (const half*)weights; p.slots = bszm; p.c_slot_stride = (long long)m * n;
+        p.indices = indices; p.weights = (const half*)weights; p.c_slot_stride = (long long)m * n;
         cudaError_t e = launch_multi_k(K, cb, mt, p, grid, st);
         ctx->launches++;
         if (e != cudaSuccess) { cudaGetLastError(); return exl3_fail(ctx, EXL3_ERR_CUDA, cudaGetErrorString(e)); }

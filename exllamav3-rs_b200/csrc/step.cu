@@ -201,21 +201,18 @@ static int step_forward_impl(exl3_ctx* ctx, exl3_stream stream, const exl3_model
     STAGE(0);                           // descriptors and embedding
     exl3_chain_scope chain(ctx);        // from here on every launch follows one of this library
     const half* pending = nullptr;      // output of the previous block's MLP, added to the residual by the next norm
-    // Who transforms the activations, a launch of its own or their producer.  Norms, from 128 rows on: 85.3 against 84.6 ms at
-    // 1052 rows of the 27B-class shard, but 22.5 against 22.7 ms at 32, where one CTA per row leaves a row's three transforms
-    // to 32 CTAs.  Up to 16 rows, where every kernel of a layer is a few microseconds of latency, the launches that drop out
-    // count: the activation, which has a warp per 128-block, always writes the transform (16 layers, 8 rows: hidden 1024 1154
-    // against 1132 us, 2048 1394 against 1368, 5120 2650 against 2587); the norms where a warp of a row's CTA has one block,
-    // which is up to hidden 1024 (within 2 % either way at 512 and 1024).  From the second block on the transforms of a
-    // block follow one another in a warp (hidden 1536 1260 against 1317 us, 2048 1368 against 1462, 5120 1329 against 1484
-    // at 8 layers).
+    // Who transforms the activations, a launch of its own or their producer.  From 128 rows on the producers (85.3 against 84.6 ms
+    // at 1052 rows of the 27B-class shard).  Below, where a kernel is a few microseconds of latency, they write the transforms too,
+    // with up to a warp per 128-block of a row (six layers of hidden 5120, 16 of 1024, us: 32 rows 1236 -> 1176 and 1308 -> 1210,
+    // 64 rows 1377 -> 1324 and 1559 -> 1450, 120 rows 1611 -> 1563 and 2088 -> 2015); up to 16 rows the activation always, the
+    // norms up to hidden 1024 (at 5120 within 2 % either way).
     const bool few = rows <= 16;
-    const bool fuse_pre = ctx->fuse_transform != 0 && (rows >= 128 || (few && hidden <= 1024));
-    const bool fuse_act = ctx->fuse_transform != 0 && (rows >= 128 || few);
+    const bool fuse_pre = ctx->fuse_transform != 0 && (!few || hidden <= 1024);
+    const bool fuse_act = ctx->fuse_transform != 0;
     for (int l = 0; l < m->n_layers; ++l) {
         const exl3_layer& L = m->layers[l];
         {
-            // with enough rows for the tensor-core GEMM the norm writes the transformed activations of q/k/v itself
+            // the norm writes the transformed activations of q/k/v itself
             const exl3_linear* w[3] = {&L.q_proj, &L.k_proj, &L.v_proj};
             void* out[3] = {s.q, s.k, s.v};
             exl3_pre_act pre;

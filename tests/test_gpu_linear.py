@@ -408,6 +408,27 @@ def test_gemm_weights_in_tensor_memory(ctx, ref, m, k, n, K, cb, c_fp32):
     _gemm_case(ctx, ref, m, k, n, K, cb, c_fp32, 1500 + m + K)
 
 
+# up to four rows, where the kernel transforms its activations itself: one row at every length, two to four where a CTA has few
+# units; odd and even unit counts, one unit, several blocks per CTA; with and without sign vectors
+@pytest.mark.parametrize("signed", [True, False])
+@pytest.mark.parametrize("m,k,n,K,cb", [(1, 128, 128, 4, 1), (1, 1152, 384, 3, 0), (1, 128, 25600, 2, 2), (1, 5120, 1024, 8, 1),
+                                        (2, 128, 1280, 4, 2), (3, 1408, 256, 5, 1), (4, 1280, 640, 7, 0), (4, 256, 25600, 6, 1)])
+def test_gemm_transforms_few_rows_itself(ctx, m, k, n, K, cb, signed):
+    from oracle import oracle as O
+    torch = _torch()
+    r = H.rng(1700 + m + k)
+    A = r.standard_normal((m, k)).astype(np.float16)
+    tr = H.rand_trellis(r, k, n, K)
+    suh, svh = (H.rand_signs(r, k), H.rand_signs(r, n)) if signed else (None, None)
+    out = torch.full((m, n), float("nan"), dtype=torch.float32, device="cuda")
+    n0 = ctx.launch_count()
+    ctx.exl3_gemm(H.to_dev(A), H.to_dev(tr), out, None if suh is None else H.to_dev(suh), None,
+                  None if svh is None else H.to_dev(svh), mcg=cb == 1, mul1=cb == 2)
+    assert ctx.launch_count() - n0 == 1
+    ctx.poll_status()
+    assert H.gemm_mismatch(out.cpu().numpy(), O.exl3_gemm(A, tr, suh, svh, K, cb, c_fp32=True), GEMM_TOL, False) <= 1.0
+
+
 def test_gemm_without_room_for_partial_sums():
     """a context whose scratch holds the activations but no partial sums runs whole blocks, with the same result up to the
     order of fp32 sums"""
