@@ -169,6 +169,29 @@ def test_argmax(ctx, ref, fp32):
         assert np.array_equal(got, ids2.cpu().numpy().reshape(-1))
 
 
+# one CTA and a cluster per row: the largest value at the borders of the parts, ties across them, a limit below the row's width,
+# rows without any finite value, NaN
+@pytest.mark.parametrize("n,limit", [(1, 0), (1023, 0), (8191, 0), (8192, 0), (8193, 0), (20001, 9001), (65536, 0)])
+def test_argmax_parts(ctx, n, limit):
+    torch = _torch()
+    r = H.rng(53 + n)
+    m = limit or n
+    per = -(-m // 8)
+    lg = r.standard_normal((7, n)).astype(np.float32)
+    lg[0, m - 1] = 9.0
+    lg[1, [0, m - 1]] = 9.0
+    lg[2, min(per, m - 1)] = lg[2, min(2 * per - 1, m - 1)] = 9.0
+    lg[3, :] = -np.inf
+    lg[4, :] = np.nan
+    lg[5, ::2] = np.nan
+    lg[6, m:] = 20.0
+    d = H.to_dev(lg)
+    ids = torch.full((7,), -1, dtype=torch.int64, device="cuda")
+    ctx.argmax_sample(d, ids, max_logit=limit)
+    want = np.argmax(np.where(np.isnan(lg[:, :m]), -np.inf, lg[:, :m]), axis=1)
+    assert np.array_equal(ids.cpu().numpy(), want)
+
+
 def test_embed(ctx):
     from oracle import oracle as O
     torch = _torch()
