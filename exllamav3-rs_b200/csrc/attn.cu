@@ -178,7 +178,17 @@ __global__ void __launch_bounds__(256) attn_combine_kernel(const AttnParams p, i
         b = lo;
     } else b = row / p.q_len;
     const int splits = p.seq_splits[b];
-    if (splits <= 1) return;                                   // the attention kernel wrote the final value itself
+    half* op = p.o + ((size_t)row * p.nq + head) * D + lane * (D / 32);
+    // the input transform of the projection behind the attention: a head is one 128-block of its k
+    auto transform = [&](uint2 v) {
+        const uint2 sg = reinterpret_cast<const uint2*>(p.had_suh)[head * 32 + lane];
+        reinterpret_cast<uint2*>(p.had_out)[((size_t)row * p.nq + head) * 32 + lane] =
+            had128_signed_lane(*reinterpret_cast<const half2*>(&v.x), *reinterpret_cast<const half2*>(&v.y), sg, lane);
+    };
+    if (splits <= 1) {                                         // the attention kernel wrote the final value itself
+        if (p.had_out) transform(*reinterpret_cast<const uint2*>(op));
+        return;
+    }
     const int row_base = p.cu_q ? p.cu_q[b] : b * p.q_len;
     const int G = p.nq / p.nkv, kvh = head / G;
     const int packed = (row - row_base) * G + (head - kvh * G);
@@ -220,9 +230,9 @@ __global__ void __launch_bounds__(256) attn_combine_kernel(const AttnParams p, i
     #pragma unroll
     for (int o = 16; o > 0; o >>= 1) ll += __shfl_xor_sync(0xffffffffu, ll, o);
     const float inv = ll > 0.f ? 1.0f / ll : 0.f;
-    half* op = p.o + ((size_t)row * p.nq + head) * D + lane * (D / 32);
-    #pragma unroll
-    for (int e = 0; e < D / 32; e += 2) *reinterpret_cast<uint32_t*>(op + e) = pack_h2(acc[e] * inv, acc[e + 1] * inv);
+    const uint2 v = make_uint2(pack_h2(acc[0] * inv, acc[1] * inv), pack_h2(acc[2] * inv, acc[3] * inv));
+    *reinterpret_cast<uint2*>(op) = v;
+    if (p.had_out) transform(v);
 }
 
 template <int D, int WM, int WN, int QB>
@@ -487,8 +497,21 @@ int attn_impl(exl3_ctx* ctx, cudaStream_t st, AttnParams p, int total_rows, int 
     // (Sending the decode rows of a ragged fp16 batch through the tcgen05 kernel as well, as items of 128 rows with 5 in
     // use, was measured on the benchmark step: the attention stage takes the same 28.0 ms of the step's 83.)
     const int dec_rows = qdec_kernel_applies(p, quant) ? 48 : 16;
-    if (max_rows <= dec_rows) return attn_pass(ctx, st, p, total_rows, max_rows, 0, dec_rows, true, quant, &off);
-    if (!p.cu_q) return attn_pass(ctx, st, p, total_rows, max_rows, 0, 1 << 30, false, quant, &off);
+    // (The transform behind the attention is left to its own launch where two passes share the rows, and where the scratch does
+    // not hold it beside the partials; attn_pass refuses before it launches anything.)
+    if (max_rows <= dec_rows || !p.cu_q) {
+        const bool dec = max_rows <= dec_rows;
+        if (ctx->had_out) {
+            p.had_suh = ctx->had_suh; p.had_out = ctx->had_out;
+            off = ctx->had_bytes;
+            const int rc = attn_pass(ctx, st, p, total_rows, max_rows, 0, dec ? dec_rows : 1 << 30, dec, quant, &off);
+            ctx->had_done = rc == EXL3_OK;
+            if (rc != EXL3_ERR_WORKSPACE) return rc;
+            p.had_suh = nullptr; p.had_out = nullptr;
+            off = 0;
+        }
+        return attn_pass(ctx, st, p, total_rows, max_rows, 0, dec ? dec_rows : 1 << 30, dec, quant, &off);
+    }
     // Ragged batch with both classes: the decode-class pass (bound by HBM) is issued on the context's second stream and
     // the long-class pass (bound by the tensor core and the MUFU) on the caller's; they touch disjoint sequences and
     // output rows, and each has its own scratch.  Fork and join by events, which also works while the caller's stream

@@ -42,6 +42,10 @@ struct exl3_ctx {
     size_t plan_slot_bytes;
     int plan_keep;
     int plan_valid[2];
+    // Set for one attention call of a step: where the input transform of o_proj's activations goes and its signs.  The combine
+    // kernel, which has a head's 128 values in a warp, writes it (had_done says that it does); had_bytes of the scratch in front
+    // of the attention's own are taken by it.
+    const half* had_suh; half* had_out; size_t had_bytes; int had_done;
     // Programmatic dependent launches (exl3_launch): set while the work in front of a launch on its stream is known to be a
     // kernel of this library - inside a step, and after the first launch of a call of several - and broken for one launch
     // where a stream forks or joins.
@@ -65,6 +69,30 @@ __device__ __forceinline__ void pdl_enter_first(int early)
     if (early) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
     if (!early) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+// 128-point Hadamard transform of (x o signs) for a block whose elements 4 * lane + j are a, b of lane `lane`; `signs` holds the
+// lane's four.  Same arithmetic as the GEMM's input transform of few rows: fp16 product, fp32 butterflies, one fp16 rounding.
+__device__ __forceinline__ uint2 had128_signed_lane(half2 a, half2 b, uint2 signs, int lane)
+{
+    a = __hmul2(a, *reinterpret_cast<const half2*>(&signs.x));
+    b = __hmul2(b, *reinterpret_cast<const half2*>(&signs.y));
+    float v0 = __low2float(a), v1 = __high2float(a), v2 = __low2float(b), v3 = __high2float(b);
+    const float s0 = v0 + v1, d0 = v0 - v1, s1 = v2 + v3, d1 = v2 - v3;
+    v0 = s0 + s1; v1 = d0 + d1; v2 = s0 - s1; v3 = d0 - d1;
+    #pragma unroll
+    for (int i = 1; i < 32; i <<= 1) {
+        const float p0 = __shfl_xor_sync(0xffffffffu, v0, i), p1 = __shfl_xor_sync(0xffffffffu, v1, i);
+        const float p2 = __shfl_xor_sync(0xffffffffu, v2, i), p3 = __shfl_xor_sync(0xffffffffu, v3, i);
+        const bool up = lane & i;
+        v0 = (up ? -v0 : v0) + p0; v1 = (up ? -v1 : v1) + p1;
+        v2 = (up ? -v2 : v2) + p2; v3 = (up ? -v3 : v3) + p3;
+    }
+    constexpr float R128 = 0.088388347648f;
+    a = __floats2half2_rn(v0 * R128, v1 * R128);
+    b = __floats2half2_rn(v2 * R128, v3 * R128);
+    uint2 o; o.x = *reinterpret_cast<uint32_t*>(&a); o.y = *reinterpret_cast<uint32_t*>(&b);
+    return o;
 }
 
 // Launch as a programmatic dependent of the previous kernel where the context says that there is one: the launch then

@@ -155,31 +155,6 @@ __global__ void __launch_bounds__(1024) rms_norm_kernel(const TI* __restrict__ x
     }
 }
 
-// 128-point Hadamard transform of a block whose element 4 * lane + j sits in v[j] of lane `lane`, after the fp16 sign
-// multiply: same arithmetic as the large-M GEMM's input transform (fp16 product, fp32 butterflies, one fp16 rounding).
-__device__ __forceinline__ uint2 had128_signed_lane(half2 a, half2 b, const half* __restrict__ suh, int col, int lane)
-{
-    const uint2 sr = reinterpret_cast<const uint2*>(suh)[col];
-    a = __hmul2(a, *reinterpret_cast<const half2*>(&sr.x));
-    b = __hmul2(b, *reinterpret_cast<const half2*>(&sr.y));
-    float v0 = __low2float(a), v1 = __high2float(a), v2 = __low2float(b), v3 = __high2float(b);
-    const float s0 = v0 + v1, d0 = v0 - v1, s1 = v2 + v3, d1 = v2 - v3;
-    v0 = s0 + s1; v1 = d0 + d1; v2 = s0 - s1; v3 = d0 - d1;
-    #pragma unroll
-    for (int i = 1; i < 32; i <<= 1) {
-        const float p0 = __shfl_xor_sync(0xffffffffu, v0, i), p1 = __shfl_xor_sync(0xffffffffu, v1, i);
-        const float p2 = __shfl_xor_sync(0xffffffffu, v2, i), p3 = __shfl_xor_sync(0xffffffffu, v3, i);
-        const bool up = lane & i;
-        v0 = (up ? -v0 : v0) + p0; v1 = (up ? -v1 : v1) + p1;
-        v2 = (up ? -v2 : v2) + p2; v3 = (up ? -v3 : v3) + p3;
-    }
-    constexpr float R128 = 0.088388347648f;
-    a = __floats2half2_rn(v0 * R128, v1 * R128);
-    b = __floats2half2_rn(v2 * R128, v3 * R128);
-    uint2 o; o.x = *reinterpret_cast<uint32_t*>(&a); o.y = *reinterpret_cast<uint32_t*>(&b);
-    return o;
-}
-
 // rms_norm_kernel whose fp16 result goes straight through the input transform of the EXL3 tensors that read it (up to
 // three: q/k/v or gate/up, each with its own sign vector) instead of to memory: the norm's own output and the separate
 // transform launch drop out.  A warp's 32 float4 columns of one pass are one 128-block (dim % 128 == 0).
@@ -233,7 +208,7 @@ __global__ void __launch_bounds__(1024) rms_norm_had_kernel(const TI* __restrict
             #pragma unroll
             for (int sgm = 0; sgm < 3; ++sgm)
                 if (sgm < pre.nseg) {
-                    const uint2 h = had128_signed_lane(a, b, pre.suh[sgm], c, lane);
+                    const uint2 h = had128_signed_lane(a, b, reinterpret_cast<const uint2*>(pre.suh[sgm])[c], lane);
                     reinterpret_cast<uint2*>(pre.a_had[sgm] + row * dim)[c] = h;
                 }
         }
@@ -384,7 +359,7 @@ __global__ void __launch_bounds__(256) silu_mul_had_kernel(const half* __restric
             z[j] = __hmul2(__hmul2(a, rr), b);
         }
         const int col = (int)(blk % bpr) * 32 + lane;           // uint2 index inside the sign vector
-        reinterpret_cast<uint2*>(a_had + blk * 128)[lane] = had128_signed_lane(z[0], z[1], suh, col, lane);
+        reinterpret_cast<uint2*>(a_had + blk * 128)[lane] = had128_signed_lane(z[0], z[1], reinterpret_cast<const uint2*>(suh)[col], lane);
     }
 }
 

@@ -229,6 +229,19 @@ static int step_forward_impl(exl3_ctx* ctx, exl3_stream stream, const exl3_model
         STAGE(1);                       // attention norm + q/k/v
         STEP_TRY(exl3_rope(ctx, stream, s.q, nullptr, s.k, nullptr, m->inv_freq, m->n_freq, 0, nullptr, s.row_pos, L.q_norm, L.k_norm,
                            m->norm_eps, 0.f, m->rope_mode, m->attn_factor, 1, rows, m->nq, m->nkv, m->hd));
+        // the attention's combine kernel writes o_proj's transformed activations where it can (16 layers of hidden 5120 at 32 rows,
+        // together with the shorter argmax, 3400 -> 3301 us; 28 layers of 1024 at 8 rows 1839 -> 1756)
+        const exl3_linear* wo[1] = {&L.o_proj};
+        exl3_pre_act opre;
+        struct HadScope {
+            exl3_ctx* c;
+            explicit HadScope(exl3_ctx* ctx_) : c(ctx_) { c->had_done = 0; }
+            ~HadScope() { c->had_out = nullptr; c->had_suh = nullptr; c->had_bytes = 0; }
+        } had(ctx);
+        if (exl3_pre_buffers(ctx, 1, wo, rows, m->nq * m->hd, &opre)) {
+            ctx->had_suh = opre.suh[0]; ctx->had_out = opre.a_had[0];
+            ctx->had_bytes = (size_t)rows * L.o_proj.k * 2;
+        }
         if (m->kv_bits == 0)
             STEP_TRY(exl3_bighead_attn_paged(ctx, stream, s.q, s.k, s.v, L.k_cache, L.v_cache, b->block_table,
                                              b->cache_seqlens, s.cu_q, s.attn_o, bsz, b->max_q_len, rows, m->nq, m->nkv,
@@ -239,7 +252,11 @@ static int step_forward_impl(exl3_ctx* ctx, exl3_stream stream, const exl3_model
                                                m->nkv, m->hd, m->pages, b->pages_per_seq, m->kv_bits, m->kv_bits, 256, 1,
                                                0.f, 0.f));
         STAGE(2);                       // rope, KV write, attention
-        STEP_TRY(linear(ctx, stream, L.o_proj, s.attn_o, s.proj, rows, 0));
+        if (ctx->had_done) {
+            void* out[1] = {s.proj};
+            STEP_TRY(exl3_gemm_fanout_pre(ctx, stream, 1, wo, out, rows, 0));
+        } else
+            STEP_TRY(linear(ctx, stream, L.o_proj, s.attn_o, s.proj, rows, 0));
         STAGE(3);                       // o_proj
         {
             const exl3_linear* w[2] = {&L.gate_proj, &L.up_proj};

@@ -60,6 +60,18 @@ def test_decode_step_matches_oracle(ctx, kv_bits, K, cb):
     assert np.array_equal(dsl.cpu().numpy(), ctx_lens + 1)
 
 
+@pytest.mark.parametrize("q_len,ctx_lens,kv_bits", [(1, [3, 255, 2900, 700, 5000], 0), (1, [90], 4), (7, [40, 3000, 1000], 4), (20, [600, 0, 2000], 0)])
+def test_step_with_transform_behind_attention(ctx, q_len, ctx_lens, kv_bits):
+    """o_proj's activations are transformed by the kernel that merges the split attention: sequences of one split and of several
+    in one batch, decode rows, verify rows and chunks, against the oracle."""
+    from oracle import oracle_model
+    model, nm, ids, q_lens, ctx_lens, bt = _setup(kv_bits, 4, 1, [q_len] * len(ctx_lens), ctx_lens, 800 + q_len)
+    _, logits = model.step(ctx, H.to_dev(ids), H.to_dev(q_lens), H.to_dev(ctx_lens), H.to_dev(bt), q_len, want_logits=True)
+    ctx.poll_status()
+    _, wlog = oracle_model.step(nm, ids, q_lens, ctx_lens, bt)
+    assert H.rel_rms_err(logits.cpu().numpy(), wlog) < (2e-2 if kv_bits else 1e-2)
+
+
 def test_ragged_step_equals_sequence_by_sequence(ctx):
     """A packed ragged step (decode + verify + prefill chunk) gives the same tokens as one call per sequence."""
     from oracle import oracle_model
