@@ -43,7 +43,7 @@ extern "C" int exl3_ctx_create(int device, size_t workspace_bytes, exl3_ctx** ou
     ctx->plan_slot_bytes = (size_t)1 << 20;
     ctx->plan_keep = 0; ctx->plan_valid[0] = ctx->plan_valid[1] = 0;
     ctx->chain = ctx->chain_break = 0;
-    ctx->had_suh = nullptr; ctx->had_out = nullptr; ctx->had_bytes = 0; ctx->had_done = 0;
+    ctx->had_suh = nullptr; ctx->had_out = nullptr; ctx->had_bytes = 0; ctx->had_done = 0; ctx->kv_appended = 0;
     bool ok = cudaMalloc(&ctx->ws, ctx->ws_bytes) == cudaSuccess &&
               cudaMalloc(&ctx->counters, ctx->n_counters * sizeof(int)) == cudaSuccess &&
               cudaMalloc(&ctx->status, 64) == cudaSuccess &&

@@ -558,7 +558,7 @@ extern "C" int exl3_bighead_attn_paged(exl3_ctx* ctx, exl3_stream stream, const 
     EXL3_REQUIRE(k_cache && v_cache && aligned16(k_cache) && aligned16(v_cache), "attention: bad cache pointers");
     if (bsz == 0 || q_len == 0) return EXL3_OK;
     const int append = cu_q ? q_len : kv_append;
-    if (append > 0) {
+    if (append > 0 && !ctx->kv_appended) {
         EXL3_REQUIRE(k && v, "attention: kv_append > 0 needs k and v");
         rc = exl3_paged_kv_cache_update(ctx, stream, k, v, k_cache, v_cache, block_table, cache_seqlens, cu_q, bsz, append,
                                         nkv, hd, pages, pages_per_seq);
@@ -591,7 +591,7 @@ extern "C" int exl3_bighead_attn_paged_q(exl3_ctx* ctx, exl3_stream stream, cons
     if (compand_a > 0.0f) return exl3_fail(ctx, EXL3_ERR_UNSUPPORTED, "attention: compand_a > 0 is not supported");
     if (bsz == 0 || q_len == 0) return EXL3_OK;
     const int append = cu_q ? q_len : kv_append;
-    if (append > 0) {
+    if (append > 0 && !ctx->kv_appended) {
         EXL3_REQUIRE(k && v, "attention: kv_append > 0 needs k and v");
         rc = exl3_quant_cache_paged(ctx, stream, k, qk, sk, v, qv, sv, cache_seqlens, block_table, cu_q, bsz, append,
                                     nkv * hd, pages, pages_per_seq, k_bits, v_bits, EXL3_PAGE, 0.0f, 1);

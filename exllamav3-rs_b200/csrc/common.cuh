@@ -46,6 +46,7 @@ struct exl3_ctx {
     // kernel, which has a head's 128 values in a warp, writes it (had_done says that it does); had_bytes of the scratch in front
     // of the attention's own are taken by it.
     const half* had_suh; half* had_out; size_t had_bytes; int had_done;
+    int kv_appended;        // set for one attention call of a step whose new keys and values are in the pools already
     // Programmatic dependent launches (exl3_launch): set while the work in front of a launch on its stream is known to be a
     // kernel of this library - inside a step, and after the first launch of a call of several - and broken for one launch
     // where a stream forks or joins.
@@ -178,6 +179,13 @@ struct exl3_pre_act { const half* suh[3]; half* a_had[3]; int nseg; };
 bool exl3_pre_buffers(exl3_ctx* ctx, int count, const exl3_linear* const* w, int m, int dim, exl3_pre_act* pre);
 int exl3_gemm_fanout_pre(exl3_ctx* ctx, exl3_stream stream, int count, const exl3_linear* const* w, void* const* C, int m, int c_fp32);
 // elementwise.cu
+// Where a step's new keys and values go: pools of one layer (kc and vc in fp16, or codes and scales) and every row's token slot
+// (page * 256 + offset, -1: none).
+struct exl3_kv_dst { const half* v; half* kc; half* vc; uint32_t* qk; half* sk; uint32_t* qv; half* sv; const int32_t* slot; int bits; };
+// exl3_rope for head_dim 128 whose keys go to the pool instead of back to k, together with v
+int exl3_rope_append(exl3_ctx* ctx, exl3_stream stream, void* q, const void* k, const float* inv_freq, int n_freq, const int32_t* row_pos,
+                     const void* q_norm, const void* k_norm, float norm_eps, int rope_mode, float attn_factor, int rows, int nq, int nk,
+                     const exl3_kv_dst* dst);
 int exl3_rms_norm_pre(exl3_ctx* ctx, exl3_stream stream, const void* x, int x_fp32, const void* w, float* r, float eps,
                       float cbias, float cscale, int rows, int dim, const exl3_pre_act* pre);
 int exl3_silu_mul_pre(exl3_ctx* ctx, exl3_stream stream, const void* x, const void* y, int rows, int dim, const exl3_pre_act* pre);

@@ -1,6 +1,7 @@
 // Memory-bound row ops of the decode step: Hadamard-128, RMSNorm (+ fused residual add), RoPE (+ fused per-head
 // RMSNorm), SiLU*mul, add, argmax, embedding gather.  Each op states the reference kernel whose arithmetic it follows.
 #include "common.cuh"
+#include "kvquant.cuh"
 
 namespace {
 
@@ -219,13 +220,16 @@ __global__ void __launch_bounds__(1024) rms_norm_had_kernel(const TI* __restrict
 // One warp per (row, head); lane holds elements lane + 32*i.  Arithmetic follows kernels/rope.cu:55-255: optional
 // RMSNorm (value rounded to fp16, weight + bias in fp16, fp16 product), then the rotation in fp32 with __sinf/__cosf of
 // inv_freq[t] * float(pos), rounded to fp16.
-template <int EPL>   // elements per lane = hd / 32
+// APPEND: keys leave through shared memory for the pool, with the row's values, instead of going back to out_k, so that a step needs
+// no append of its own behind it (us: 28 layers of hidden 1024, 8 rows 1744 -> 1722; 16 of 5120, 32 rows over 4-bit pools 3307 ->
+// 3252; 16 of 1024, 24 rows over 4-bit pools 1152 -> 1130).
+template <int EPL, bool APPEND>   // elements per lane = hd / 32
 __global__ void __launch_bounds__(256) rope_kernel(const half* q, const half* k, half* out_q, half* out_k,
                                                    const float* __restrict__ inv_freq, int n_freq, uint32_t position,
                                                    const int32_t* __restrict__ positions,
                                                    const int32_t* __restrict__ row_pos, const half* __restrict__ q_norm,
                                                    const half* __restrict__ k_norm, float norm_eps, float norm_cbias,
-                                                   int rope_mode, float attn_factor, int rows, int seq, int nq, int nk)
+                                                   int rope_mode, float attn_factor, int rows, int seq, int nq, int nk, const exl3_kv_dst dst)
 {
     pdl_enter();
     constexpr int HD = EPL * 32;
@@ -290,6 +294,28 @@ __global__ void __launch_bounds__(256) rope_kernel(const half* q, const half* k,
                 float sn = __sinf(ang) * attn_factor, cs = __cosf(ang) * attn_factor;
                 x[i] = (e & 1) ? __float2half_rn(mine * cs + other * sn) : __float2half_rn(mine * cs - other * sn);
             }
+        }
+    }
+    if constexpr (APPEND) {
+        static_assert(EPL == 4, "a lane of the append holds four consecutive values");
+        if (h >= nq) {
+            __shared__ __align__(16) half s_k[8][HD];
+            half* sk = s_k[threadIdx.x >> 5];
+            #pragma unroll
+            for (int i = 0; i < EPL; ++i) sk[lane + 32 * i] = x[i];
+            __syncwarp();
+            const int slot = dst.slot[row];
+            if (slot < 0) return;
+            const size_t head = (size_t)slot * nk + (h - nq);
+            const half* v = dst.v + ((size_t)row * nk + (h - nq)) * HD;
+            if (dst.bits == 0) {
+                reinterpret_cast<uint2*>(dst.kc + head * HD)[lane] = reinterpret_cast<const uint2*>(sk)[lane];
+                reinterpret_cast<uint2*>(dst.vc + head * HD)[lane] = reinterpret_cast<const uint2*>(v)[lane];
+            } else {
+                exl3::quant_x4(sk, dst.qk + head * 4 * dst.bits, dst.sk + head * 4, 4, dst.bits);
+                exl3::quant_x4(v, dst.qv + head * 4 * dst.bits, dst.sv + head * 4, 4, dst.bits);
+            }
+            return;
         }
     }
     #pragma unroll
@@ -536,13 +562,31 @@ extern "C" int exl3_rope(exl3_ctx* ctx, exl3_stream stream, void* q, void* out_q
     cudaStream_t st = (cudaStream_t)stream;
     const int nk_eff = k ? nk : 0;
 #define ROPE_LAUNCH(E)                                                                                                 \
-    exl3_launch(ctx, rope_kernel<E>, grid, 256, 0, st, (const half*)q, (const half*)k, (half*)(out_q ? out_q : q), (half*)(out_k ? out_k : k), inv_freq, n_freq, position, positions, row_pos, \
+    exl3_launch(ctx, rope_kernel<E, false>, grid, 256, 0, st, (const half*)q, (const half*)k, (half*)(out_q ? out_q : q), (half*)(out_k ? out_k : k), inv_freq, n_freq, position, positions, row_pos, \
                                          (const half*)q_norm, (const half*)k_norm, norm_eps, norm_constant_bias,       \
-                                         rope_mode, attn_factor, rows, seq, nq, nk_eff)
+                                         rope_mode, attn_factor, rows, seq, nq, nk_eff, exl3_kv_dst{})
     if (hd == 64) ROPE_LAUNCH(2); else if (hd == 128) ROPE_LAUNCH(4); else ROPE_LAUNCH(8);
 #undef ROPE_LAUNCH
     ctx->launches++;
     return exl3_check_launch(ctx, "rope");
+}
+
+int exl3_rope_append(exl3_ctx* ctx, exl3_stream stream, void* q, const void* k, const float* inv_freq, int n_freq, const int32_t* row_pos,
+                     const void* q_norm, const void* k_norm, float norm_eps, int rope_mode, float attn_factor, int rows, int nq, int nk,
+                     const exl3_kv_dst* dst)
+{
+    EXL3_REQUIRE(ctx && q && k && inv_freq && row_pos && dst && dst->slot, "rope (append): null argument");
+    EXL3_REQUIRE(n_freq > 0 && 2 * n_freq <= 128, "rope: 2*n_freq must be <= head_dim");
+    if (rope_mode == EXL3_ROPE_NEOX && n_freq % 32 != 0)
+        return exl3_fail(ctx, EXL3_ERR_UNSUPPORTED, "rope: NEOX mode needs n_freq % 32 == 0");
+    if (rope_mode != EXL3_ROPE_NEOX && rope_mode != EXL3_ROPE_GPTJ && rope_mode != EXL3_ROPE_NONE)
+        return exl3_fail(ctx, EXL3_ERR_INVALID, "rope: unknown rope_mode");
+    const long long warps = (long long)rows * (nq + nk);
+    exl3_launch(ctx, rope_kernel<4, true>, (unsigned)((warps + 7) / 8), 256, 0, (cudaStream_t)stream, (const half*)q, (const half*)k, (half*)q, (half*)nullptr,
+                inv_freq, n_freq, 0u, (const int32_t*)nullptr, row_pos, (const half*)q_norm, (const half*)k_norm, norm_eps, 0.f, rope_mode, attn_factor,
+                rows, 1, nq, nk, *dst);
+    ctx->launches++;
+    return exl3_check_launch(ctx, "rope (append)");
 }
 
 extern "C" int exl3_silu_mul(exl3_ctx* ctx, exl3_stream stream, const void* x, const void* y, void* z,

@@ -10,7 +10,8 @@ namespace {
 __global__ void __launch_bounds__(1024) build_desc_kernel(const int32_t* __restrict__ q_lens,
                                                           const int32_t* __restrict__ seqlens, int bsz, int rows,
                                                           int32_t* __restrict__ cu_q, int32_t* __restrict__ row_pos,
-                                                          int32_t* __restrict__ last_row)
+                                                          int32_t* __restrict__ last_row, const int32_t* __restrict__ block_table,
+                                                          int pps, int pages, int32_t* __restrict__ row_slot)
 {
     __shared__ int s_scan[1024];
     __shared__ int s_carry;
@@ -33,7 +34,14 @@ __global__ void __launch_bounds__(1024) build_desc_kernel(const int32_t* __restr
             cu_q[b + 1] = end;
             last_row[b] = (ql > 0 && end <= rows) ? end - 1 : -1;
             const int start = end - ql, pos0 = seqlens[b];
-            for (int i = 0; i < ql && start + i < rows; ++i) row_pos[start + i] = pos0 + i;
+            for (int i = 0; i < ql && start + i < rows; ++i) {
+                const int pos = pos0 + i;
+                row_pos[start + i] = pos;
+                if (row_slot) {                                       // token slot of the row in a layer's pool
+                    const int page = (pos >> 8) < pps ? block_table[(size_t)b * pps + (pos >> 8)] : -1;
+                    row_slot[start + i] = page >= 0 && page < pages ? page * EXL3_PAGE + (pos & 255) : -1;
+                }
+            }
         }
         __syncthreads();
         if (tid == 1023) s_carry += s_scan[1023];
@@ -59,7 +67,7 @@ __global__ void __launch_bounds__(256) gather_rows_kernel(const uint4* __restric
 }
 
 struct Scratch {
-    int32_t *cu_q, *row_pos, *last_row;
+    int32_t *cu_q, *row_pos, *last_row, *row_slot;
     float *resid, *resid_last;
     half *a_in, *q, *k, *v, *attn_o, *proj, *gate, *up, *act, *pend_last, *y_last;
     float* logits;
@@ -79,6 +87,7 @@ size_t carve(const exl3_model* m, int max_rows, int max_bsz, int head_rows, uint
     t.cu_q = (int32_t*)take((B + 1) * 4);
     t.row_pos = (int32_t*)take(R * 4);
     t.last_row = (int32_t*)take(B * 4);
+    t.row_slot = (int32_t*)take(R * 4);
     t.resid = (float*)take(R * m->hidden * 4);
     t.resid_last = (float*)take(B * m->hidden * 4);
     t.a_in = (half*)take(R * m->hidden * 2);
@@ -116,7 +125,7 @@ extern "C" int exl3_step_build_descriptors(exl3_ctx* ctx, exl3_stream stream, co
 {
     EXL3_REQUIRE(ctx && q_lens && cache_seqlens && cu_q && row_pos && last_row, "step_build_descriptors: null argument");
     EXL3_REQUIRE(bsz > 0 && rows >= 0, "step_build_descriptors: bad shape");
-    build_desc_kernel<<<1, 1024, 0, (cudaStream_t)stream>>>(q_lens, cache_seqlens, bsz, rows, cu_q, row_pos, last_row);
+    build_desc_kernel<<<1, 1024, 0, (cudaStream_t)stream>>>(q_lens, cache_seqlens, bsz, rows, cu_q, row_pos, last_row, nullptr, 0, 0, nullptr);
     ctx->launches++;
     return exl3_check_launch(ctx, "step_build_descriptors");
 }
@@ -195,7 +204,10 @@ static int step_forward_impl(exl3_ctx* ctx, exl3_stream stream, const exl3_model
     cudaStream_t st = (cudaStream_t)stream;
     const int rows = b->rows, bsz = b->bsz, hidden = m->hidden;
 
-    STEP_TRY(exl3_step_build_descriptors(ctx, stream, b->q_lens, b->cache_seqlens, bsz, rows, s.cu_q, s.row_pos, s.last_row));
+    build_desc_kernel<<<1, 1024, 0, st>>>(b->q_lens, b->cache_seqlens, bsz, rows, s.cu_q, s.row_pos, s.last_row, b->block_table,
+                                          b->pages_per_seq, m->pages, s.row_slot);
+    ctx->launches++;
+    STEP_TRY(exl3_check_launch(ctx, "step_build_descriptors"));
     STEP_TRY(exl3_embed(ctx, stream, b->ids, m->embed, s.resid, rows, hidden, m->vocab));
 
     STAGE(0);                           // descriptors and embedding
@@ -209,6 +221,13 @@ static int step_forward_impl(exl3_ctx* ctx, exl3_stream stream, const exl3_model
     const bool few = rows <= 16;
     const bool fuse_pre = ctx->fuse_transform != 0 && (!few || hidden <= 1024);
     const bool fuse_act = ctx->fuse_transform != 0;
+    // Keys and values go to the pools from the rotation's kernel, unless the separate append would refuse the call (or the attention,
+    // other head sizes) or the pool's slots do not fit 31 bits.
+    bool append = m->hd == 128 && m->nq > 0 && m->nkv > 0 && m->pages < (1 << 23) && bsz <= 65535 && b->max_q_len <= 65535;
+    for (int l = 0; l < m->n_layers; ++l) {
+        const exl3_layer& L = m->layers[l];
+        append = append && (m->kv_bits == 0 ? L.k_cache && L.v_cache && aligned16(L.k_cache) && aligned16(L.v_cache) : L.qk && L.sk && L.qv && L.sv);
+    }
     for (int l = 0; l < m->n_layers; ++l) {
         const exl3_layer& L = m->layers[l];
         {
@@ -227,17 +246,22 @@ static int step_forward_impl(exl3_ctx* ctx, exl3_stream stream, const exl3_model
             }
         }
         STAGE(1);                       // attention norm + q/k/v
-        STEP_TRY(exl3_rope(ctx, stream, s.q, nullptr, s.k, nullptr, m->inv_freq, m->n_freq, 0, nullptr, s.row_pos, L.q_norm, L.k_norm,
-                           m->norm_eps, 0.f, m->rope_mode, m->attn_factor, 1, rows, m->nq, m->nkv, m->hd));
+        if (append) {
+            exl3_kv_dst dst = {s.v, (half*)L.k_cache, (half*)L.v_cache, (uint32_t*)L.qk, (half*)L.sk, (uint32_t*)L.qv, (half*)L.sv, s.row_slot, m->kv_bits};
+            STEP_TRY(exl3_rope_append(ctx, stream, s.q, s.k, m->inv_freq, m->n_freq, s.row_pos, L.q_norm, L.k_norm, m->norm_eps, m->rope_mode,
+                                      m->attn_factor, rows, m->nq, m->nkv, &dst));
+        } else
+            STEP_TRY(exl3_rope(ctx, stream, s.q, nullptr, s.k, nullptr, m->inv_freq, m->n_freq, 0, nullptr, s.row_pos, L.q_norm, L.k_norm,
+                               m->norm_eps, 0.f, m->rope_mode, m->attn_factor, 1, rows, m->nq, m->nkv, m->hd));
         // the attention's combine kernel writes o_proj's transformed activations where it can (16 layers of hidden 5120 at 32 rows,
         // together with the shorter argmax, 3400 -> 3301 us; 28 layers of 1024 at 8 rows 1839 -> 1756)
         const exl3_linear* wo[1] = {&L.o_proj};
         exl3_pre_act opre;
         struct HadScope {
             exl3_ctx* c;
-            explicit HadScope(exl3_ctx* ctx_) : c(ctx_) { c->had_done = 0; }
-            ~HadScope() { c->had_out = nullptr; c->had_suh = nullptr; c->had_bytes = 0; }
-        } had(ctx);
+            HadScope(exl3_ctx* ctx_, bool appended) : c(ctx_) { c->had_done = 0; c->kv_appended = appended; }
+            ~HadScope() { c->had_out = nullptr; c->had_suh = nullptr; c->had_bytes = 0; c->kv_appended = 0; }
+        } had(ctx, append);
         if (exl3_pre_buffers(ctx, 1, wo, rows, m->nq * m->hd, &opre)) {
             ctx->had_suh = opre.suh[0]; ctx->had_out = opre.a_had[0];
             ctx->had_bytes = (size_t)rows * L.o_proj.k * 2;

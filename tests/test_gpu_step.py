@@ -72,6 +72,45 @@ def test_step_with_transform_behind_attention(ctx, q_len, ctx_lens, kv_bits):
     assert H.rel_rms_err(logits.cpu().numpy(), wlog) < (2e-2 if kv_bits else 1e-2)
 
 
+@pytest.mark.parametrize("kv_bits", [0, 3, 4, 6, 8])
+def test_step_writes_its_keys_and_values(ctx, kv_bits):
+    """The rotation's kernel writes the new rows of the pools: first and last offset of a page, rows over a page border, and no
+    other slot.  Against the same layer's keys and values through the separate operators."""
+    import torch
+    q_lens, ctx_lens = [1, 5, 1, 3], [0, 254, 255, 511]
+    model, nm, ids, q_lens, ctx_lens, bt = _setup(kv_bits, 4, 1, q_lens, ctx_lens, 900 + kv_bits, n_layers=1)
+    L = model.layers[0]
+    names = ["k_cache", "v_cache"] if kv_bits == 0 else ["qk", "sk", "qv", "sv"]
+    for x in names:
+        L[x].copy_(torch.randint(-100, 100, L[x].shape, device="cuda").to(L[x].dtype))
+    before = [L[x].clone() for x in names]
+    d_q, d_c, d_bt = H.to_dev(q_lens), H.to_dev(ctx_lens), H.to_dev(bt)
+    model.step(ctx, H.to_dev(ids), d_q, d_c, d_bt, 5)
+    ctx.poll_status()
+    got = [L[x].clone() for x in names]
+    slots = [int(bt[b, p >> 8]) * 256 + (p & 255) for b in range(4) for p in range(ctx_lens[b], ctx_lens[b] + q_lens[b])]
+    mask = torch.ones(got[0].shape[0] * 256, dtype=torch.bool, device="cuda")
+    mask[slots] = False
+    for g, w in zip(got, before):
+        g, w = g.flatten(0, 1).flatten(1), w.flatten(0, 1).flatten(1)
+        assert torch.equal(g[mask], w[mask])
+        assert not torch.equal(g[~mask], w[~mask])
+    # the same rows one sequence at a time (other rows per call, the same arithmetic per row up to the order of fp32 sums)
+    for x, w in zip(names, before):
+        L[x].copy_(w)
+    at = 0
+    for b in range(4):
+        model.step(ctx, H.to_dev(ids[at:at + q_lens[b]]), H.to_dev(q_lens[b:b + 1]), H.to_dev(ctx_lens[b:b + 1]), H.to_dev(bt[b:b + 1]), int(q_lens[b]))
+        at += q_lens[b]
+    ctx.poll_status()
+    for x, g in zip(names, got):
+        w = L[x]
+        if g.dtype == torch.float16:
+            assert H.rel_rms_err(g.flatten(0, 1)[slots].float().cpu().numpy(), w.flatten(0, 1)[slots].float().cpu().numpy()) < 1e-2
+        else:
+            assert (g.flatten(0, 1)[slots] == w.flatten(0, 1)[slots]).float().mean() > 0.9
+
+
 def test_ragged_step_equals_sequence_by_sequence(ctx):
     """A packed ragged step (decode + verify + prefill chunk) gives the same tokens as one call per sequence."""
     from oracle import oracle_model
