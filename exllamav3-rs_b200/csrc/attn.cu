@@ -161,8 +161,10 @@ __global__ void __launch_bounds__(1024) attn_plan_kernel(const int32_t* __restri
 }
 
 // Merges the split-KV partials of one output row (b, query, head); one warp per row, lane = D/32 dims.
-template <int D>
-__global__ void __launch_bounds__(256) attn_combine_kernel(const AttnParams p, int rows_per_cta, int total_rows)
+// HAD: also writes the 128-point transform of (output o signs).  (A form of its own: with the test at run time in every call 24
+// sequences over 8-bit pools took 67.3 us instead of 65.4.)
+template <int D, bool HAD>
+__global__ void __launch_bounds__(256) attn_combine_kernel(const AttnParams p, int rows_per_cta, int total_rows, const half* had_suh, half* had_out)
 {
     pdl_enter();
     const int lane = threadIdx.x & 31;
@@ -178,15 +180,14 @@ __global__ void __launch_bounds__(256) attn_combine_kernel(const AttnParams p, i
         b = lo;
     } else b = row / p.q_len;
     const int splits = p.seq_splits[b];
-    half* op = p.o + ((size_t)row * p.nq + head) * D + lane * (D / 32);
     // the input transform of the projection behind the attention: a head is one 128-block of its k
     auto transform = [&](uint2 v) {
-        const uint2 sg = reinterpret_cast<const uint2*>(p.had_suh)[head * 32 + lane];
-        reinterpret_cast<uint2*>(p.had_out)[((size_t)row * p.nq + head) * 32 + lane] =
+        const uint2 sg = reinterpret_cast<const uint2*>(had_suh)[head * 32 + lane];
+        reinterpret_cast<uint2*>(had_out)[((size_t)row * p.nq + head) * 32 + lane] =
             had128_signed_lane(*reinterpret_cast<const half2*>(&v.x), *reinterpret_cast<const half2*>(&v.y), sg, lane);
     };
     if (splits <= 1) {                                         // the attention kernel wrote the final value itself
-        if (p.had_out) transform(*reinterpret_cast<const uint2*>(op));
+        if constexpr (HAD) transform(*reinterpret_cast<const uint2*>(p.o + ((size_t)row * p.nq + head) * D + lane * (D / 32)));
         return;
     }
     const int row_base = p.cu_q ? p.cu_q[b] : b * p.q_len;
@@ -230,9 +231,10 @@ __global__ void __launch_bounds__(256) attn_combine_kernel(const AttnParams p, i
     #pragma unroll
     for (int o = 16; o > 0; o >>= 1) ll += __shfl_xor_sync(0xffffffffu, ll, o);
     const float inv = ll > 0.f ? 1.0f / ll : 0.f;
-    const uint2 v = make_uint2(pack_h2(acc[0] * inv, acc[1] * inv), pack_h2(acc[2] * inv, acc[3] * inv));
-    *reinterpret_cast<uint2*>(op) = v;
-    if (p.had_out) transform(v);
+    half* op = p.o + ((size_t)row * p.nq + head) * D + lane * (D / 32);
+    #pragma unroll
+    for (int e = 0; e < D / 32; e += 2) *reinterpret_cast<uint32_t*>(op + e) = pack_h2(acc[e] * inv, acc[e + 1] * inv);
+    if constexpr (HAD) transform(make_uint2(pack_h2(acc[0] * inv, acc[1] * inv), pack_h2(acc[2] * inv, acc[3] * inv)));
 }
 
 template <int D, int WM, int WN, int QB>
@@ -370,7 +372,7 @@ bool qdec_kernel_applies(const AttnParams& p, bool quant);
 
 // One pass = plan + attention + combine over the sequences whose packed row count lies in (rows_lo, rows_hi].
 int attn_pass(exl3_ctx* ctx, cudaStream_t st, AttnParams p, int total_rows, int max_rows, int rows_lo, int rows_hi,
-              bool decode_shape, bool quant, size_t* ws_off)
+              bool decode_shape, bool quant, size_t* ws_off, bool had = false)
 {
     const int D = 128;
     const int G = p.nq / p.nkv;
@@ -464,7 +466,8 @@ int attn_pass(exl3_ctx* ctx, cudaStream_t st, AttnParams p, int total_rows, int 
     ctx->launches++;
     if (e != cudaSuccess) { cudaGetLastError(); return exl3_fail(ctx, EXL3_ERR_CUDA, cudaGetErrorString(e)); }
     const long long warps = (long long)total_rows * p.nq;
-    exl3_launch(ctx, attn_combine_kernel<128>, (unsigned)((warps + 7) / 8), 256, 0, st, p, rows_per_cta, total_rows);
+    if (had) exl3_launch(ctx, attn_combine_kernel<128, true>, (unsigned)((warps + 7) / 8), 256, 0, st, p, rows_per_cta, total_rows, ctx->had_suh, ctx->had_out);
+    else     exl3_launch(ctx, attn_combine_kernel<128, false>, (unsigned)((warps + 7) / 8), 256, 0, st, p, rows_per_cta, total_rows, (const half*)nullptr, (half*)nullptr);
     ctx->launches++;
     return exl3_check_launch(ctx, "attention");
 }
@@ -502,12 +505,10 @@ int attn_impl(exl3_ctx* ctx, cudaStream_t st, AttnParams p, int total_rows, int 
     if (max_rows <= dec_rows || !p.cu_q) {
         const bool dec = max_rows <= dec_rows;
         if (ctx->had_out) {
-            p.had_suh = ctx->had_suh; p.had_out = ctx->had_out;
             off = ctx->had_bytes;
-            const int rc = attn_pass(ctx, st, p, total_rows, max_rows, 0, dec ? dec_rows : 1 << 30, dec, quant, &off);
+            const int rc = attn_pass(ctx, st, p, total_rows, max_rows, 0, dec ? dec_rows : 1 << 30, dec, quant, &off, true);
             ctx->had_done = rc == EXL3_OK;
             if (rc != EXL3_ERR_WORKSPACE) return rc;
-            p.had_suh = nullptr; p.had_out = nullptr;
             off = 0;
         }
         return attn_pass(ctx, st, p, total_rows, max_rows, 0, dec ? dec_rows : 1 << 30, dec, quant, &off);

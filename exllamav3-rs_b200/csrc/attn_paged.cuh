@@ -44,7 +44,6 @@ struct AttnParams {
     int bsz, q_len, kv_append, nq, nkv, pps, pages, causal, k_bits, v_bits;
     int contig_kv;                 // > 0: kc/vc are plain [bsz, contig_kv, nkv, D] tensors, no block table (mma.sync fp16 kernel only)
     float scale_log2;              // sm_scale * log2(e)
-    const half* had_suh; half* had_out;        // combine kernel: also write the 128-point transform of (output o signs), or NULL
 };
 
 __device__ __forceinline__ void cp_async16(void* dst, const void* src)
