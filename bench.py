@@ -302,7 +302,7 @@ def gemm_alg_bytes(m, k, n, K):
 
 # DRAM bytes of one gemm_tc_kernel launch at M = 1052 on 5120 x 17408, 4 bpw (dram__bytes_read.sum + dram__bytes_write.sum of
 # one ncu capture); the figure belongs to the commit named with it and is not re-measured by the run
-NCU_TRAFFIC_TC_M1052 = {"bytes": 63079680 + 12018944, "source": "ncu capture of gemm_tc_kernel<4,1,2,256> at M=1052 (summary under profiles/)"}
+NCU_TRAFFIC_TC_M1052 = {"bytes": None, "source": "no capture of this shape (1024 rows and the last 28 are two launches)"}
 
 
 def run_ours(args):

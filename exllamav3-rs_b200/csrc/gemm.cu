@@ -379,17 +379,36 @@ int ts_split(int sms, int blocks, int units, int m, bool may_share, int* whole, 
     return grid;
 }
 
+// Rows behind the last whole 512-row block that go to gemm_ts_kernel instead of being a block of their own, which costs its
+// decoders 0.65 of a whole one however few rows it has: worth it where those blocks do not fit beside the last wave of whole ones,
+// or where the rest then runs on 128-column slabs.  Items of 512 rows x 256 columns take 12.1 us per 1000 k.  Kept -> apart, us, 4
+// bits: 5120 x 17408, 540 rows 113 -> 99, 1052 rows 183 -> 165; 17408 x 5120, 640 rows 196 -> 154; 5120 x 7168, 1100 rows 90 -> 89;
+// four layers of a mixed batch of 1052 rows 4076 -> 3949; but 5120 x 5120, 600 rows 63.3 -> 65.6, which the constants leave alone.
+int tc_tail(const exl3_ctx* ctx, int slabs, int blocks128, int m, int k)
+{
+    const int tail = m % (2 * TC_BM), slots = ctx->num_sms / 2;
+    if (!ctx->use_pair || m < 2 * TC_BM || tail == 0 || tail > TS_MAX_N) return 0;
+    const int rows = m - tail, full = slabs * (rows / (2 * TC_BM)), r = full % slots;
+    const int left = slabs - (r ? slots - r : 0);
+    const float item = k * 0.0121f, waves = (float)((full + slots - 1) / slots);
+    const float unit = rows <= 2 * TC_BM && slabs * 4 <= ctx->num_sms ? 0.65f : 1.0f;
+    int whole, longest;
+    ts_split(ctx->num_sms, blocks128, k / TS_UNIT_K, tail, blocks128 <= ctx->n_counters, &whole, &longest);
+    const float keep = item * (waves + (left > 0 ? 0.65f * ((left + slots - 1) / slots) : 0.0f));
+    return item * waves * unit + 14.0f + 0.57f * longest < keep ? tail : 0;
+}
+
 // Tensor-core path for rows [0, m) and `nseg` weight tensors that share the activations, k, bits and codebook:
 // one launch of the input transforms (each tensor has its own suh) and one of the tcgen05 kernel.
 // With `pre` the transformed activations are already in place (written into the buffers exl3_pre_buffers named, by the
-// kernel that produced the input), and the transform launch is skipped.
+// kernel that produced the input), and the transform launch is skipped; with `given` they are there, and the scratch is free from
+// off on.
 int gemm_tc_rows(exl3_ctx* ctx, cudaStream_t st, const half* A, int nseg, const void* const* trellis, void* const* C,
                  const half* const* suh, const half* const* svh, const int* n, int m, int k, int K, int c_fp32, int cb,
-                 bool pre = false)
+                 bool pre = false, half* const* given = nullptr, size_t off = 0)
 {
     EncodeTiledFn enc = get_encode_tiled();
     if (!enc) return exl3_fail(ctx, EXL3_ERR_CUDA, "exl3_gemm: cuTensorMapEncodeTiled is not available from this driver");
-    size_t off = 0;
     ProloguePlainArgs pa;
     CUtensorMap amap[TC_MAX_SEG], rmap[TC_MAX_SEG], cmap[TC_MAX_SEG];
     GemmTcParams p;
@@ -410,16 +429,17 @@ int gemm_tc_rows(exl3_ctx* ctx, cudaStream_t st, const half* A, int nseg, const 
     // in front of it off the call (us: 1 row, 5120 x 17408 27.2 -> 25.6, 17408 x 5120 33.0 -> 30.0, 1024 x 3072 13.5 -> 11.6; 4
     // rows, 5120 x 1024 in 5 units 13.8 -> 11.8, but 5120 x 5120 in 14 units 15.2 -> 16.0 and 5120 x 17408 in 40 27.2 -> 30.5).
     const bool few = ts && !pre && (m == 1 || (m <= TS_FEW && longest <= 10));
-    const int bn = ts || (ctx->use_pair && n128 && m <= 2 * TC_BM && blocks256 * 4 <= ctx->num_sms) ? 128 : TC_BN;
+    const int tail = !ts && n128 ? tc_tail(ctx, blocks256, blocks128, m, k) : 0, mm = m - tail;
+    const int bn = ts || (ctx->use_pair && n128 && mm <= 2 * TC_BM && blocks256 * 4 <= ctx->num_sms) ? 128 : TC_BN;
     int blocks = 0;
     for (int i = 0; i < TC_MAX_SEG; ++i) {
         const int j = i < nseg ? i : nseg - 1;              // unused slots repeat the last tensor (never selected)
         if (i < nseg) {
-            pa.a_had[i] = few ? nullptr : (half*)exl3_ws_take(ctx, &off, (size_t)m * k * 2);
+            pa.a_had[i] = given ? given[i] : few ? nullptr : (half*)exl3_ws_take(ctx, &off, (size_t)m * k * 2);
             if (!few && !pa.a_had[i]) return exl3_fail(ctx, EXL3_ERR_WORKSPACE, "exl3_gemm: context scratch too small for the activations");
             pa.suh[i] = suh[i];
             blocks += (n[i] + bn - 1) / bn;                // a trailing 128-column half slab counts (CTA pairs only)
-            cuuint64_t dims[2] = {(cuuint64_t)k, (cuuint64_t)m};
+            cuuint64_t dims[2] = {(cuuint64_t)k, (cuuint64_t)mm};
             cuuint64_t strides[1] = {(cuuint64_t)k * 2};
             cuuint32_t box[2] = {(cuuint32_t)TC_BK, ts ? (cuuint32_t)((m + 15) & ~15) : 128u};
             cuuint32_t estr[2] = {1, 1};
@@ -440,7 +460,7 @@ int gemm_tc_rows(exl3_ctx* ctx, cudaStream_t st, const half* A, int nseg, const 
             if (few) amap[i] = rmap[i];                        // never dereferenced
             // the fp16 output as [m][n]: an epilogue warp stores its 32 rows x 128 columns as two boxes of 64 columns
             if (!c_fp32 && !ts) {
-                cuuint64_t cdims[2] = {(cuuint64_t)n[i], (cuuint64_t)m};
+                cuuint64_t cdims[2] = {(cuuint64_t)n[i], (cuuint64_t)mm};
                 cuuint64_t cstrides[1] = {(cuuint64_t)n[i] * 2};
                 cuuint32_t cbox[2] = {64u, 32u};
                 r = enc(&cmap[i], CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, C[i], cdims, cstrides, cbox, estr,
@@ -490,10 +510,19 @@ int gemm_tc_rows(exl3_ctx* ctx, cudaStream_t st, const half* A, int nseg, const 
         if (e != cudaSuccess) { cudaGetLastError(); return exl3_fail(ctx, EXL3_ERR_CUDA, cudaGetErrorString(e)); }
         return EXL3_OK;
     }
-    p.status = ctx->status; p.m = m; p.k = k; p.c_fp32 = c_fp32;
+    p.status = ctx->status; p.m = mm; p.k = k; p.c_fp32 = c_fp32;
     cudaError_t e = launch_tc_k(K, cb, ctx->use_pair != 0, bn, amap, rmap, cmap, p, blocks, st);
     ctx->launches++;
     if (e != cudaSuccess) { cudaGetLastError(); return exl3_fail(ctx, EXL3_ERR_CUDA, cudaGetErrorString(e)); }
+    if (tail) {
+        half* at[TC_MAX_SEG];
+        void* Ct[TC_MAX_SEG];
+        for (int i = 0; i < nseg; ++i) {
+            at[i] = pa.a_had[i] + (size_t)mm * k;
+            Ct[i] = c_fp32 ? (void*)((float*)C[i] + (size_t)mm * n[i]) : (void*)((half*)C[i] + (size_t)mm * n[i]);
+        }
+        return gemm_tc_rows(ctx, st, nullptr, nseg, trellis, Ct, suh, svh, n, tail, k, K, c_fp32, cb, true, at, off);
+    }
     return EXL3_OK;
 }
 

@@ -336,6 +336,16 @@ def test_gemm_tc_step_shape(ctx, ctx_small_only):
     _tc_case(ctx, ctx_small_only, None, 1052, 5120, 17408, 4, 1, False, 1200)
 
 
+@pytest.mark.parametrize("m,k,n,K,c_fp32", [(513, 5120, 17408, 4, True), (576, 5120, 17280, 3, False), (640, 5120, 17408, 8, False),
+                                            (1025, 5120, 17408, 4, False), (600, 17408, 5120, 5, False)])
+def test_gemm_tc_last_rows_apart(ctx, ctx_small_only, m, k, n, K, c_fp32):
+    """up to 128 rows behind the last block of 512 as a second launch with the weights in tensor memory: one row, 64, 88 and 128, two
+    blocks in front, 128-column slabs in front"""
+    n0 = ctx.launch_count()
+    _tc_case(ctx, ctx_small_only, None, m, k, n, K, 1, c_fp32, 1800 + m)
+    assert ctx.launch_count() - n0 == 3                     # transform, whole blocks, last rows
+
+
 @pytest.mark.parametrize("m,ns,K,c_fp32", [(200, (512, 256, 256), 4, False), (1052, (1024, 256, 256), 4, False),
                                             (300, (768, 768), 3, True), (40, (512, 256), 4, False), (5, (512, 256, 256), 4, False), (16, (768, 768), 5, True),
                                             (1, (5120, 1024, 1024), 4, False),
