@@ -178,6 +178,7 @@ __global__ void __launch_bounds__(256) attn_combine_kernel(const AttnParams p, i
         int lo = 0, hi = p.bsz - 1;
         while (lo < hi) { int mid = (lo + hi + 1) >> 1; if (p.cu_q[mid] <= row) lo = mid; else hi = mid - 1; }
         b = lo;
+        if (row >= p.cu_q[b + 1]) return;                      // rows behind the last sequence have no partials
     } else b = row / p.q_len;
     const int splits = p.seq_splits[b];
     // the input transform of the projection behind the attention: a head is one 128-block of its k

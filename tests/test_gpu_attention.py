@@ -163,6 +163,41 @@ def test_attention_non_causal_and_no_append(ctx):
     assert _close(o.cpu().numpy(), want, TOL_FP16) <= 1.0
 
 
+@pytest.mark.parametrize("bits,q_lens,ctx_lens", [(0, [1, 1, 1], [40, 3000, 5000]), (0, [20, 3], [100, 4000]), (0, [1, 0, 30], [700, 64, 3000]),
+                                                  (4, [1, 2], [300, 6000]), (8, [5, 1], [10, 4000]), (6, [1, 1], [50, 3000])])
+def test_attention_rows_behind_the_last_sequence(ctx, bits, q_lens, ctx_lens):
+    """A ragged call whose packed tensor has more rows than the sequences (cu_q on the device may shrink under a captured call): the
+    surplus rows of the output stay as they are, although the last sequence has several splits, and the others' bits do too."""
+    torch = _torch()
+    r = H.rng(1900 + bits + len(q_lens))
+    nq, nkv, extra = 40, 8, 37
+    rows = sum(q_lens)
+    bt, pages = H.make_paged(r, len(q_lens), [c + q for c, q in zip(ctx_lens, q_lens)], nkv, 128)
+    g = torch.Generator(device="cuda").manual_seed(bits)
+    half = lambda *s: torch.randn(*s, device="cuda", generator=g).to(torch.float16) * 0.5  # noqa: E731
+    q, k, v = half(rows + extra, nq, 128), half(rows + extra, nkv, 128), half(rows + extra, nkv, 128)
+    if bits == 0:
+        pools = [half(pages, 256, nkv, 128) for _ in range(2)]
+    else:
+        pools = [t for _ in range(2) for t in (torch.randint(-2 ** 31, 2 ** 31 - 1, (pages, 256, nkv * 4 * bits), dtype=torch.int32, device="cuda", generator=g),
+                                               half(pages, 256, nkv * 4).abs() * 0.1)]
+    cu = H.to_dev(np.concatenate([[0], np.cumsum(q_lens)]).astype(np.int32))
+    sl, d_bt = H.to_dev(np.asarray(ctx_lens, np.int32)), H.to_dev(bt)
+    got = []
+    for n in (rows, rows + extra):
+        p = [t.clone() for t in pools]
+        o = torch.full((n, nq, 128), 7.0, dtype=torch.float16, device="cuda")
+        if bits == 0:
+            ctx.bighead_attn_paged(q[:n], k[:n], v[:n], p[0], p[1], d_bt, sl, o, cu_q=cu, max_q_len=max(q_lens))
+        else:
+            ctx.bighead_attn_paged_q(q[:n], k[:n], v[:n], p[0], p[1], p[2], p[3], d_bt, sl, o, nkv, cu_q=cu, max_q_len=max(q_lens))
+        ctx.poll_status()
+        got.append((o, p))
+    assert (got[1][0][rows:] == 7.0).all()
+    assert torch.isfinite(got[0][0]).all() and torch.equal(got[0][0], got[1][0][:rows])
+    assert all(torch.equal(a, b) for a, b in zip(got[0][1], got[1][1]))
+
+
 def test_attention_ragged_equals_per_sequence(ctx):
     """One ragged call over mixed decode / verify / prefill-chunk sequences == the rectangular calls one by one."""
     from oracle import oracle as O
