@@ -11,7 +11,7 @@ __global__ void __launch_bounds__(1024) build_desc_kernel(const int32_t* __restr
                                                           const int32_t* __restrict__ seqlens, int bsz, int rows,
                                                           int32_t* __restrict__ cu_q, int32_t* __restrict__ row_pos,
                                                           int32_t* __restrict__ last_row, const int32_t* __restrict__ block_table,
-                                                          int pps, int pages, int32_t* __restrict__ row_slot)
+                                                          int pps, int pages, int max_q, int32_t* __restrict__ row_slot)
 {
     __shared__ int s_scan[1024];
     __shared__ int s_carry;
@@ -38,7 +38,7 @@ __global__ void __launch_bounds__(1024) build_desc_kernel(const int32_t* __restr
                 const int pos = pos0 + i;
                 row_pos[start + i] = pos;
                 if (row_slot) {                                       // token slot of the row in a layer's pool
-                    const int page = (pos >> 8) < pps ? block_table[(size_t)b * pps + (pos >> 8)] : -1;
+                    const int page = i < max_q && (pos >> 8) < pps ? block_table[(size_t)b * pps + (pos >> 8)] : -1;
                     row_slot[start + i] = page >= 0 && page < pages ? page * EXL3_PAGE + (pos & 255) : -1;
                 }
             }
@@ -46,6 +46,12 @@ __global__ void __launch_bounds__(1024) build_desc_kernel(const int32_t* __restr
         __syncthreads();
         if (tid == 1023) s_carry += s_scan[1023];
         __syncthreads();
+    }
+    // rows behind the last sequence (q_lens can shrink under a captured step): the scratch holds an earlier step's slots there, or
+    // whatever was in it, and these rows' keys and values go nowhere
+    for (int i = s_carry + tid; i < rows; i += 1024) {
+        row_pos[i] = 0;
+        if (row_slot) row_slot[i] = -1;
     }
 }
 
@@ -125,7 +131,7 @@ extern "C" int exl3_step_build_descriptors(exl3_ctx* ctx, exl3_stream stream, co
 {
     EXL3_REQUIRE(ctx && q_lens && cache_seqlens && cu_q && row_pos && last_row, "step_build_descriptors: null argument");
     EXL3_REQUIRE(bsz > 0 && rows >= 0, "step_build_descriptors: bad shape");
-    build_desc_kernel<<<1, 1024, 0, (cudaStream_t)stream>>>(q_lens, cache_seqlens, bsz, rows, cu_q, row_pos, last_row, nullptr, 0, 0, nullptr);
+    build_desc_kernel<<<1, 1024, 0, (cudaStream_t)stream>>>(q_lens, cache_seqlens, bsz, rows, cu_q, row_pos, last_row, nullptr, 0, 0, 0, nullptr);
     ctx->launches++;
     return exl3_check_launch(ctx, "step_build_descriptors");
 }
@@ -205,7 +211,7 @@ static int step_forward_impl(exl3_ctx* ctx, exl3_stream stream, const exl3_model
     const int rows = b->rows, bsz = b->bsz, hidden = m->hidden;
 
     build_desc_kernel<<<1, 1024, 0, st>>>(b->q_lens, b->cache_seqlens, bsz, rows, s.cu_q, s.row_pos, s.last_row, b->block_table,
-                                          b->pages_per_seq, m->pages, s.row_slot);
+                                          b->pages_per_seq, m->pages, b->max_q_len, s.row_slot);
     ctx->launches++;
     STEP_TRY(exl3_check_launch(ctx, "step_build_descriptors"));
     STEP_TRY(exl3_embed(ctx, stream, b->ids, m->embed, s.resid, rows, hidden, m->vocab));

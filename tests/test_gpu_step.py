@@ -111,6 +111,76 @@ def test_step_writes_its_keys_and_values(ctx, kv_bits):
             assert (g.flatten(0, 1)[slots] == w.flatten(0, 1)[slots]).float().mean() > 0.9
 
 
+def _pools(model):
+    names = ["k_cache", "v_cache"] if model.cfg["kv_bits"] == 0 else ["qk", "sk", "qv", "sv"]
+    return [L[x] for L in model.layers for x in names]
+
+
+def _untouched(model, before, bt, ctx_lens, q_lens):
+    """every token slot of every plane but the sequences' new ones is what it was, and those are not"""
+    import torch
+    slots = [int(bt[b, p >> 8]) * 256 + (p & 255) for b in range(len(q_lens)) for p in range(ctx_lens[b], ctx_lens[b] + q_lens[b])]
+    mask = torch.ones(before[0].shape[0] * 256, dtype=torch.bool, device="cuda")
+    mask[slots] = False
+    for g, w in zip(_pools(model), before):
+        g, w = g.flatten(0, 1).flatten(1), w.flatten(0, 1).flatten(1)
+        assert torch.equal(g[mask], w[mask])
+        assert not torch.equal(g[~mask], w[~mask])
+
+
+# (the scratch is filled with slots that exist, so that a row that took one of them would show and not fault)
+@pytest.mark.parametrize("kv_bits", [0, 4, 6, 8])
+@pytest.mark.parametrize("q_lens,extra", [([1, 0, 1, 2], 3), ([1, 30, 0], 100), ([1] * 7, 9)])
+def test_rows_behind_the_last_sequence_write_no_slot(ctx, kv_bits, q_lens, extra):
+    """A step with more packed rows than q_lens counts: the surplus rows' keys and values go nowhere, and the sequences' logits are
+    those of the step without them (other rows per call: up to the order of fp32 sums)."""
+    import torch
+    r = H.rng(1000 + kv_bits + extra)
+    ctx_lens = r.integers(200, 1500, len(q_lens))
+    model, _, ids, q_lens, ctx_lens, bt = _setup(kv_bits, 4, 1, q_lens, ctx_lens, 1100 + kv_bits + extra)
+    before = [t.clone() for t in _pools(model)]
+    args = (H.to_dev(q_lens), H.to_dev(ctx_lens), H.to_dev(bt), int(q_lens.max()))
+    _, want = model.step(ctx, H.to_dev(ids), *args, want_logits=True)
+    for t, w in zip(_pools(model), before):
+        t.copy_(w)
+    more = np.concatenate([ids, np.arange(extra)])
+    model.step(ctx, H.to_dev(more), *args)                  # sizes the scratch
+    for t, w in zip(_pools(model), before):
+        t.copy_(w)
+    model._scratch.view(torch.int32).fill_(300)
+    _, got = model.step(ctx, H.to_dev(more), *args, want_logits=True)
+    ctx.poll_status()
+    _untouched(model, before, bt, ctx_lens, q_lens)
+    live = np.asarray(q_lens) > 0
+    assert H.rel_rms_err(got.cpu().numpy()[live], want.cpu().numpy()[live]) < (2e-2 if kv_bits else 5e-3)
+
+
+@pytest.mark.parametrize("kv_bits", [0, 4])
+def test_replayed_step_after_a_sequence_retired(ctx, kv_bits):
+    """A captured step whose last sequence retires (its q_len on the device drops to 0) while another goes on: the replay has a
+    row that belongs to nobody, whose slot of the replay before must not be written again."""
+    import torch
+    import exl3b200
+    model, _, ids, q_lens, ctx_lens, bt = _setup(kv_bits, 4, 1, [1, 1, 1], [300, 700, 40], 1200 + kv_bits)
+    d_ids, d_q, d_c, d_bt = H.to_dev(ids), H.to_dev(q_lens), H.to_dev(ctx_lens), H.to_dev(bt)
+    tokens = torch.empty(3, dtype=torch.int64, device="cuda")
+    model.step(ctx, d_ids, d_q, d_c, d_bt, 1, tokens_out=tokens)
+    g = exl3b200.CudaGraph(ctx)
+    g.capture_begin()
+    model.step(ctx, d_ids, d_q, d_c, d_bt, 1, stream=g.side_stream(), tokens_out=tokens, advance=True)
+    g.capture_end()
+    torch.cuda.synchronize()
+    g.replay()
+    assert exl3b200.lib().exl3_sync_side_stream(ctx.handle) == 0
+    d_q.copy_(torch.tensor([1, 1, 0], dtype=torch.int32))
+    before = [t.clone() for t in _pools(model)]
+    torch.cuda.synchronize()
+    g.replay()
+    assert exl3b200.lib().exl3_sync_side_stream(ctx.handle) == 0
+    ctx.poll_status()
+    _untouched(model, before, bt, ctx_lens + 1, np.array([1, 1, 0]))
+
+
 def test_ragged_step_equals_sequence_by_sequence(ctx):
     """A packed ragged step (decode + verify + prefill chunk) gives the same tokens as one call per sequence."""
     from oracle import oracle_model
