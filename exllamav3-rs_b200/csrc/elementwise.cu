@@ -439,6 +439,7 @@ __global__ void __launch_bounds__(1024) argmax_kernel(const T* __restrict__ logi
         warp_best();
         if (lane == 0) s_best = make_int2(__float_as_int(best), bi);
     }
+    __syncwarp();                                             // the aligned barriers are for whole warps
     if (parts > 1) {
         asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
         if (part == 0 && warp == 0) {
