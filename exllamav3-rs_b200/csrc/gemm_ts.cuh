@@ -484,8 +484,8 @@ __global__ void __launch_bounds__(TS_THREADS, 1) gemm_ts_kernel(const __grid_con
         uint32_t par_r = 0, par_w = 1;
         #pragma unroll 1
         for (int s = grp; s < nst; s += 4) {
+            if (!waited && s >= TS_SW) { pdl_wait(); waited = true; }      // in front of the waits, which then count from here
             if (!ts_wait(&r_full[sr], par_r)) { failed = true; break; }
-            if (!waited && s >= TS_SW) { pdl_wait(); waited = true; }
             if (!ts_wait(&done[sw], par_w)) { failed = true; break; }      // at once in the first round
             tc_fence_after();
             const uint32_t* raw = reinterpret_cast<const uint32_t*>(smem + SM::OFF_RAW + sr * SM::RAW) + 2 * q * 8 * K;
