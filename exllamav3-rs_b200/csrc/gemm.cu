@@ -367,7 +367,8 @@ int ts_split(int sms, int blocks, int units, int m, bool may_share, int* whole, 
     int grid = blocks < sms ? blocks : sms, part = (blocks + sms - 1) / sms * units;
     float best = (float)part;
     *whole = 1;
-    if (may_share) {
+    // the kernel finds the owners of a block with 32-bit products of units and CTAs
+    if (may_share && (unsigned long long)blocks * units * (sms + 1) <= 0xffffffffull) {
         for (int s = 2; s * blocks <= sms && s * TS_MIN_PART <= units; ++s) {
             const float cost = (units + s - 1) / s + 1.2f + m / 160.0f + s * (0.25f + m / 170.0f);
             if (cost < best) { best = cost; grid = s * blocks; part = (units + s - 1) / s; *whole = 0; }

@@ -15,6 +15,13 @@
 // (5120 x 17408, 4 bits, 52 rows, kernel alone: 43 us; 128-k units 33; lean producer loops and one elected issuer thread 29;
 // epilogue warps of their own 26.5).  The loop runs at 55 cycles per tile and scheduler.
 //
+// A call behind other kernels also waits for its own instructions, every role for its own, at about 0.4 us per KB that it comes to
+// first.  So what a CTA runs once is kept short: levels of a transform in a loop, a sign as the factor of an fma, 32-bit indices
+// (64-bit divisions are subroutines).  Against everything unrolled, us, with four other instantiations run in front of each call:
+// 5120 x 17408 at 4 bits, 1, 8 and 52 rows 22.9 -> 20.2, 25.0 -> 21.8, 27.5 -> 25.2; back to back 25.5 -> 25.4, 27.5 -> 27.2, 29.1
+// both; steps of 28 layers of hidden 1024 with 8 rows 1706 -> 1625, six of 5120 with 8 rows 1125 -> 1098.  The decoders' tiles stay
+// unrolled: half of them in a loop gives a cold call another 2 us and takes 0.3 us of every warm one.
+//
 // Whole calls, us, tcgen05 kernel of gemm_tc.cuh -> this one: 5120 x 17408 at 4 bits 45.5 -> 32.8 (32 rows), 45.6 -> 33.1 (52),
 // 47.4 -> 35.1 (128); 52 rows at 3 and 8 bits 49.1 -> 36.0, 46.6 -> 34.9; 17408 x 5120 80.3 -> 34.6 (32 rows), 85.6 -> 41.3
 // (128); 5120 x 5120 30.9 -> 17.3 and 31.1 -> 22.9; 5120 x 151936, 52 rows, 359 -> 183.
@@ -115,7 +122,8 @@ __device__ __forceinline__ void ts_ld16(uint32_t taddr, float (&v)[16])
 }
 
 // Output transform of four rows of a 128-column block held by a warp (lane = 4 consecutive columns): 128-point Hadamard,
-// signs, store.  Four at a time, because a row's five shuffle levels are one chain.
+// signs, store.  Four at a time, because a row's five shuffle levels are one chain; the levels are a loop, which a cold call
+// reaches sooner (see above).
 __device__ __forceinline__ void ts_store_rows(float4 (&a)[4], int row, int m, int lane, bool transform, uint2 sv, void* Cout, int n, int n0, int c_fp32)
 {
     const half2 s0 = *reinterpret_cast<const half2*>(&sv.x), s1 = *reinterpret_cast<const half2*>(&sv.y);
@@ -125,15 +133,15 @@ __device__ __forceinline__ void ts_store_rows(float4 (&a)[4], int row, int m, in
             const float p = a[i].x + a[i].y, d = a[i].x - a[i].y, q = a[i].z + a[i].w, e = a[i].z - a[i].w;
             a[i].x = p + q; a[i].y = d + e; a[i].z = p - q; a[i].w = d - e;
         }
-        #pragma unroll
+        #pragma unroll 1
         for (int o = 1; o < 32; o <<= 1) {
-            const bool up = lane & o;
+            const float sg = lane & o ? -1.0f : 1.0f;
             #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 const float p0 = __shfl_xor_sync(0xffffffffu, a[i].x, o), p1 = __shfl_xor_sync(0xffffffffu, a[i].y, o);
                 const float p2 = __shfl_xor_sync(0xffffffffu, a[i].z, o), p3 = __shfl_xor_sync(0xffffffffu, a[i].w, o);
-                a[i].x = (up ? -a[i].x : a[i].x) + p0; a[i].y = (up ? -a[i].y : a[i].y) + p1;
-                a[i].z = (up ? -a[i].z : a[i].z) + p2; a[i].w = (up ? -a[i].w : a[i].w) + p3;
+                a[i].x = fmaf(a[i].x, sg, p0); a[i].y = fmaf(a[i].y, sg, p1);
+                a[i].z = fmaf(a[i].z, sg, p2); a[i].w = fmaf(a[i].w, sg, p3);
             }
         }
     }
@@ -161,7 +169,7 @@ struct TsBlock {
     int n, n0, c_first, c_last, first1;
     __device__ __forceinline__ bool split() const { return c_first != c_last; }
 };
-__device__ __forceinline__ TsBlock ts_block(const GemmTsParams& p, int nbg, int KS, long long total, long long G, int lane)
+__device__ __forceinline__ TsBlock ts_block(const GemmTsParams& p, int nbg, int KS, unsigned total, unsigned G, int lane)
 {
     TsBlock b;
     const int seg = (nbg >= p.blk_end[0]) + (nbg >= p.blk_end[1]);
@@ -172,8 +180,8 @@ __device__ __forceinline__ TsBlock ts_block(const GemmTsParams& p, int nbg, int 
     b.sv = b.svh ? *reinterpret_cast<const uint2*>(b.svh + b.n0 + lane * 4) : make_uint2(0u, 0u);
     b.c_first = b.c_last = b.first1 = 0;
     if (!p.aligned) {
-        const long long first = (long long)nbg * KS;
-        auto owner = [&](long long u) -> int { return (int)(((u + 1) * G + total - 1) / total - 1); };
+        const unsigned first = (unsigned)nbg * KS;
+        auto owner = [&](unsigned u) -> int { return (int)(((u + 1) * G + total - 1) / total - 1); };
         b.c_first = owner(first); b.c_last = owner(first + KS - 1);
         // slot 0 of a CTA holds the partial sums of the block its range begins in, slot 1 of the one it ends in; only the first of
         // a block's owners can have begun in an earlier block
@@ -236,15 +244,15 @@ __device__ __forceinline__ void ts_transform(uint2 (&x)[R], uint2 sg, int lane)
         const float s1 = __low2float(b) + __high2float(b), d1 = __low2float(b) - __high2float(b);
         v[r][0] = s0 + s1; v[r][1] = d0 + d1; v[r][2] = s0 - s1; v[r][3] = d0 - d1;
     }
-    #pragma unroll
+    #pragma unroll (R == 1 ? 5 : 1)
     for (int i = 1; i < 32; i <<= 1) {
-        const bool up = lane & i;
+        const float sgn = lane & i ? -1.0f : 1.0f;
         #pragma unroll
         for (int r = 0; r < R; ++r)
             #pragma unroll
             for (int e = 0; e < 4; ++e) {
                 const float o = __shfl_xor_sync(0xffffffffu, v[r][e], i);
-                v[r][e] = (up ? -v[r][e] : v[r][e]) + o;
+                v[r][e] = fmaf(v[r][e], sgn, o);
             }
     }
     #pragma unroll
@@ -357,11 +365,11 @@ __global__ void __launch_bounds__(TS_THREADS, 1) gemm_ts_kernel(const __grid_con
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int KS = p.k / TS_UNIT_K;                                    // units per column block
     const int blocks = p.blk_end[TC_MAX_SEG - 1];
-    const long long total = (long long)blocks * KS, G = gridDim.x;
-    const long long u0 = p.aligned ? (long long)(blocks * (long long)blockIdx.x / G) * KS : total * blockIdx.x / G;
-    const long long u1 = p.aligned ? (long long)(blocks * (long long)(blockIdx.x + 1) / G) * KS : total * (blockIdx.x + 1) / G;
+    const unsigned total = (unsigned)blocks * KS, G = gridDim.x;
+    const unsigned u0 = p.aligned ? (unsigned)(blocks * (unsigned)blockIdx.x / G) * KS : total * blockIdx.x / G;
+    const unsigned u1 = p.aligned ? (unsigned)(blocks * (unsigned)(blockIdx.x + 1) / G) * KS : total * (blockIdx.x + 1) / G;
     const int nst = (int)(u1 - u0);
-    const int nbg0 = (int)(u0 / KS), ks0 = (int)(u0 - (long long)nbg0 * KS);
+    const int nbg0 = (int)(u0 / KS), ks0 = (int)(u0 - (unsigned)nbg0 * KS);
     auto seg_of = [&](int nbg) -> int { return (nbg >= p.blk_end[0]) + (nbg >= p.blk_end[1]); };
     auto col0_of = [&](int nbg, int seg) -> int { return (nbg - (seg == 0 ? 0 : (seg == 1 ? p.blk_end[0] : p.blk_end[1]))) * 128; };
 
