@@ -268,7 +268,7 @@ static int step_forward_impl(exl3_ctx* ctx, exl3_stream stream, const exl3_model
             HadScope(exl3_ctx* ctx_, bool appended) : c(ctx_) { c->had_done = 0; c->kv_appended = appended; }
             ~HadScope() { c->had_out = nullptr; c->had_suh = nullptr; c->had_bytes = 0; c->kv_appended = 0; }
         } had(ctx, append);
-        if (exl3_pre_buffers(ctx, 1, wo, rows, m->nq * m->hd, &opre)) {
+        if (ctx->fuse_transform && exl3_pre_buffers(ctx, 1, wo, rows, m->nq * m->hd, &opre)) {
             ctx->had_suh = opre.suh[0]; ctx->had_out = opre.a_had[0];
             ctx->had_bytes = (size_t)rows * L.o_proj.k * 2;
         }

@@ -24,6 +24,11 @@ def _setup(kv_bits, K, cb, q_lens, ctx_lens, seed, n_layers=2, vocab=2048):
     return model, oracle_model.model_to_numpy(model), ids, q_lens, ctx_lens, bt
 
 
+def _pools(model):
+    names = ["k_cache", "v_cache"] if model.cfg["kv_bits"] == 0 else ["qk", "sk", "qv", "sv"]
+    return [L[x] for L in model.layers for x in names]
+
+
 def test_build_descriptors(ctx):
     import torch
     from exl3b200 import lib
@@ -60,14 +65,33 @@ def test_decode_step_matches_oracle(ctx, kv_bits, K, cb):
     assert np.array_equal(dsl.cpu().numpy(), ctx_lens + 1)
 
 
-@pytest.mark.parametrize("q_len,ctx_lens,kv_bits", [(1, [3, 255, 2900, 700, 5000], 0), (1, [90], 4), (7, [40, 3000, 1000], 4), (20, [600, 0, 2000], 0)])
+@pytest.mark.parametrize("q_len,ctx_lens,kv_bits", [(1, [3, 255, 2900, 700, 5000], 0), (1, [90], 4), (7, [40, 3000, 1000], 4), (5, [2000, 10, 0], 8), (20, [600, 0, 2000], 0)])
 def test_step_with_transform_behind_attention(ctx, q_len, ctx_lens, kv_bits):
     """o_proj's activations are transformed by the kernel that merges the split attention: sequences of one split and of several
-    in one batch, decode rows, verify rows and chunks, against the oracle."""
+    in one batch, decode rows, verify rows and chunks, against the oracle, and against a context that transforms them in a launch of
+    its own: the same bits up to 16 rows (above, that launch sums in another order)."""
+    import os
+    import torch
+    from exl3b200 import Ctx
     from oracle import oracle_model
     model, nm, ids, q_lens, ctx_lens, bt = _setup(kv_bits, 4, 1, [q_len] * len(ctx_lens), ctx_lens, 800 + q_len)
-    _, logits = model.step(ctx, H.to_dev(ids), H.to_dev(q_lens), H.to_dev(ctx_lens), H.to_dev(bt), q_len, want_logits=True)
+    before = [t.clone() for t in _pools(model)]
+    args = (H.to_dev(ids), H.to_dev(q_lens), H.to_dev(ctx_lens), H.to_dev(bt), q_len)
+    os.environ["EXL3_B200_NO_FUSED_TRANSFORM"] = "1"
+    try:
+        plain = Ctx(0)
+    finally:
+        del os.environ["EXL3_B200_NO_FUSED_TRANSFORM"]
+    _, separate = model.step(plain, *args, want_logits=True)
+    plain.poll_status()
+    for t, w in zip(_pools(model), before):
+        t.copy_(w)
+    _, logits = model.step(ctx, *args, want_logits=True)
     ctx.poll_status()
+    if len(ids) <= 16:
+        assert torch.equal(logits, separate)
+    else:
+        assert H.rel_rms_err(logits.cpu().numpy(), separate.cpu().numpy()) < (2e-2 if kv_bits else 5e-3)
     _, wlog = oracle_model.step(nm, ids, q_lens, ctx_lens, bt)
     assert H.rel_rms_err(logits.cpu().numpy(), wlog) < (2e-2 if kv_bits else 1e-2)
 
@@ -109,11 +133,6 @@ def test_step_writes_its_keys_and_values(ctx, kv_bits):
             assert H.rel_rms_err(g.flatten(0, 1)[slots].float().cpu().numpy(), w.flatten(0, 1)[slots].float().cpu().numpy()) < 1e-2
         else:
             assert (g.flatten(0, 1)[slots] == w.flatten(0, 1)[slots]).float().mean() > 0.9
-
-
-def _pools(model):
-    names = ["k_cache", "v_cache"] if model.cfg["kv_bits"] == 0 else ["qk", "sk", "qv", "sv"]
-    return [L[x] for L in model.layers for x in names]
 
 
 def _untouched(model, before, bt, ctx_lens, q_lens):
@@ -348,14 +367,16 @@ def test_multi_step_greedy_generation_with_page_allocator(ctx, kv_bits):
 
 @pytest.mark.parametrize("rows,cb", [(1, 1), (7, 0), (8, 1), (9, 1), (16, 0), (9, 2)])
 def test_decode_step_with_fused_transforms_is_bit_identical(ctx, rows, cb):
-    """Up to 16 rows the norms and the activation write the decode GEMM's operand themselves (codebook 2 keeps the separate
-    transform).  They do the same operations in the same order, so the results are the same bits, with one and with two
-    groups of eight rows."""
+    """Up to 16 rows the norms, the attention's merge kernel and the activation write the next GEMM's operand themselves (codebook 2
+    keeps the separate transform).  They do the same operations in the same order, so the results are the same bits.  Sequences
+    of one split of the attention and of several."""
     import os
     import torch
     from exl3b200 import Ctx
     r = H.rng(300 + rows)
-    model, _, ids, q_lens, ctx_lens, bt = _setup(0, 4, cb, [1] * rows, r.integers(3, 400, rows), 70 + rows)
+    lens = r.integers(3, 400, rows)
+    lens[-1] = 3000
+    model, _, ids, q_lens, ctx_lens, bt = _setup(0, 4, cb, [1] * rows, lens, 70 + rows)
     os.environ["EXL3_B200_NO_FUSED_TRANSFORM"] = "1"
     try:
         plain = Ctx(0)
@@ -372,10 +393,10 @@ def test_decode_step_with_fused_transforms_is_bit_identical(ctx, rows, cb):
     assert torch.isfinite(got[0]).all() and torch.equal(got[0], got[1])
 
 
-@pytest.mark.parametrize("hidden,cb,fewer", [(1024, 1, 3), (1024, 2, 0), (1152, 1, 1), (2048, 0, 1), (2176, 1, 1)])
+@pytest.mark.parametrize("hidden,cb,fewer", [(1024, 1, 4), (1024, 2, 0), (1152, 1, 2), (2048, 0, 2), (2176, 1, 2)])
 def test_decode_step_fused_launches(ctx, hidden, cb, fewer):
-    """Which transforms drop out of a step of few rows: q/k/v, gate/up and down_proj up to hidden 1024, above it down_proj's,
-    none in codebook 2; the results are the same bits either way."""
+    """Which transforms drop out of a step of few rows: q/k/v, o_proj, gate/up and down_proj up to hidden 1024, above it o_proj's
+    and down_proj's, none in codebook 2; the results are the same bits either way."""
     import os
     import torch
     from exl3b200 import Ctx
