@@ -227,9 +227,10 @@ static int step_forward_impl(exl3_ctx* ctx, exl3_stream stream, const exl3_model
     const bool few = rows <= 16;
     const bool fuse_pre = ctx->fuse_transform != 0 && (!few || hidden <= 1024);
     const bool fuse_act = ctx->fuse_transform != 0;
-    // Keys and values go to the pools from the rotation's kernel, unless the separate append would refuse the call (or the attention,
-    // other head sizes) or the pool's slots do not fit 31 bits.
-    bool append = m->hd == 128 && m->nq > 0 && m->nkv > 0 && m->pages < (1 << 23) && bsz <= 65535 && b->max_q_len <= 65535;
+    // Keys and values go to the pools from the rotation's kernel, unless the separate append or the attention would refuse the call
+    // (they do so before anything is written) or the pool's slots do not fit 31 bits.
+    bool append = m->hd == 128 && m->nq > 0 && m->nkv > 0 && m->nkv <= 65535 && m->nq % m->nkv == 0 && m->nq / m->nkv <= 16 &&
+                  m->pages < (1 << 23) && bsz <= 65535 && b->max_q_len <= 65535;
     for (int l = 0; l < m->n_layers; ++l) {
         const exl3_layer& L = m->layers[l];
         append = append && (m->kv_bits == 0 ? L.k_cache && L.v_cache && aligned16(L.k_cache) && aligned16(L.v_cache) : L.qk && L.sk && L.qv && L.sv);

@@ -175,6 +175,23 @@ def test_rows_behind_the_last_sequence_write_no_slot(ctx, kv_bits, q_lens, extra
 
 
 @pytest.mark.parametrize("kv_bits", [0, 4])
+@pytest.mark.parametrize("nq,nkv", [(12, 8), (17, 1)])
+def test_refused_step_leaves_the_pools(ctx, kv_bits, nq, nkv):
+    """Head counts that the attention refuses: the step fails before a key or a value is written."""
+    import torch
+    import exl3b200
+    from exl3b200.step import SyntheticModel
+    model = SyntheticModel(1, 1024, nq, nkv, 128, 1024, 512, K=4, cb=1, pages=4, kv_bits=kv_bits, seed=nq)
+    before = [t.clone() for t in _pools(model)]
+    i32 = lambda *v: torch.tensor(v, dtype=torch.int32, device="cuda")  # noqa: E731
+    with pytest.raises(exl3b200.Exl3Error):
+        model.step(ctx, torch.tensor([5, 6, 7], device="cuda"), i32(1, 2), i32(10, 20), i32(0, 1).view(2, 1), 2)
+    torch.cuda.synchronize()
+    ctx.poll_status()
+    assert all(torch.equal(t, w) for t, w in zip(_pools(model), before))
+
+
+@pytest.mark.parametrize("kv_bits", [0, 4])
 def test_replayed_step_after_a_sequence_retired(ctx, kv_bits):
     """A captured step whose last sequence retires (its q_len on the device drops to 0) while another goes on: the replay has a
     row that belongs to nobody, whose slot of the replay before must not be written again."""
