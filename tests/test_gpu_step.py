@@ -47,6 +47,26 @@ def test_build_descriptors(ctx):
     assert np.array_equal(last.cpu().numpy(), [0, 8, -1, 264, 265])
 
 
+@pytest.mark.parametrize("bsz,longest,extra", [(1, 2500, 0), (3, 700, 5), (33, 64, 0), (600, 3, 2000), (1024, 9, 1), (1500, 4, 0)])
+def test_build_descriptors_of_many_rows(ctx, bsz, longest, extra):
+    """one sequence longer than the kernel's block, group sizes from a whole block to one thread, more sequences than threads, empty
+    sequences, and rows that belong to none"""
+    import torch
+    from exl3b200 import lib
+    r = H.rng(bsz)
+    q_lens = r.integers(0, longest + 1, bsz).astype(np.int32)
+    q_lens[0] = longest
+    seqlens = r.integers(0, 5000, bsz).astype(np.int32)
+    rows = int(q_lens.sum()) + extra
+    cu, pos, last = (torch.full((n,), -7, dtype=torch.int32, device="cuda") for n in (bsz + 1, rows, bsz))
+    dq, dsl = H.to_dev(q_lens), H.to_dev(seqlens)
+    assert lib().exl3_step_build_descriptors(ctx.handle, ctx.stream(), H.ptr(dq), H.ptr(dsl), bsz, rows, H.ptr(cu), H.ptr(pos), H.ptr(last)) == 0
+    wcu = np.concatenate([[0], np.cumsum(q_lens)])
+    assert np.array_equal(cu.cpu().numpy(), wcu)
+    assert np.array_equal(pos.cpu().numpy(), np.concatenate([seqlens[b] + np.arange(q_lens[b]) for b in range(bsz)] + [np.zeros(extra)]))
+    assert np.array_equal(last.cpu().numpy(), np.where(q_lens > 0, wcu[1:] - 1, -1))
+
+
 @pytest.mark.parametrize("kv_bits,K,cb", [(0, 8, 0), (0, 4, 1), (4, 4, 2)])
 def test_decode_step_matches_oracle(ctx, kv_bits, K, cb):
     """Op-level reference workload: 8 decode sequences with contexts in [64, 1024] on a 0.6B-shaped layer stack."""
