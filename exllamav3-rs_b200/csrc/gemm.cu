@@ -362,7 +362,7 @@ cudaError_t launch_tc_k(int K, int cb, bool pair, int bn, const CUtensorMap* ama
 // 3072 columns whole, in 2, 3 parts 6.2, 6.2, 6.6).
 constexpr int TS_MIN_PART = 5;
 
-int ts_split(int sms, int blocks, int units, int m, bool may_share, int* whole, int* longest = nullptr)
+int ts_split(int sms, int blocks, int units, int m, bool may_share, int* whole, int* longest = nullptr, float* cost = nullptr)
 {
     int grid = blocks < sms ? blocks : sms, part = (blocks + sms - 1) / sms * units;
     float best = (float)part;
@@ -370,33 +370,38 @@ int ts_split(int sms, int blocks, int units, int m, bool may_share, int* whole, 
     // the kernel finds the owners of a block with 32-bit products of units and CTAs
     if (may_share && (unsigned long long)blocks * units * (sms + 1) <= 0xffffffffull) {
         for (int s = 2; s * blocks <= sms && s * TS_MIN_PART <= units; ++s) {
-            const float cost = (units + s - 1) / s + 1.2f + m / 160.0f + s * (0.25f + m / 170.0f);
-            if (cost < best) { best = cost; grid = s * blocks; part = (units + s - 1) / s; *whole = 0; }
+            const float c = (units + s - 1) / s + 1.2f + m / 160.0f + s * (0.25f + m / 170.0f);
+            if (c < best) { best = c; grid = s * blocks; part = (units + s - 1) / s; *whole = 0; }
         }
         const long long total = (long long)blocks * units, even = (total + sms - 1) / sms;
-        if (total >= (long long)sms * TS_MIN_PART && even + 7.0f + m / 24.0f < best) { grid = sms; part = (int)even; *whole = 0; }
+        if (total >= (long long)sms * TS_MIN_PART && even + 7.0f + m / 24.0f < best) { best = even + 7.0f + m / 24.0f; grid = sms; part = (int)even; *whole = 0; }
     }
     if (longest) *longest = part;
+    if (cost) *cost = best;
     return grid;
 }
 
-// Rows behind the last whole 512-row block that go to gemm_ts_kernel instead of being a block of their own, which costs its
-// decoders 0.65 of a whole one however few rows it has: worth it where those blocks do not fit beside the last wave of whole ones,
-// or where the rest then runs on 128-column slabs.  Items of 512 rows x 256 columns take 12.1 us per 1000 k.  Kept -> apart, us, 4
-// bits: 5120 x 17408, 540 rows 113 -> 99, 1052 rows 183 -> 165; 17408 x 5120, 640 rows 196 -> 154; 5120 x 7168, 1100 rows 90 -> 89;
-// four layers of a mixed batch of 1052 rows 4076 -> 3949; but 5120 x 5120, 600 rows 63.3 -> 65.6, which the constants leave alone.
+// Rows behind the last whole 512-row block that go to gemm_ts_kernel instead of being a block of their own, whose decoders work as
+// for a whole one however few rows it has: worth it where those blocks do not fit beside the last wave of whole ones, or where the
+// rest then runs on 128-column slabs.  Items of 512 rows x 256 columns take 12.1 us per 1000 k, a wave of short ones 0.4 to 0.52 of
+// that, by how far it fills the chip, the rows apart 5 us and 0.55 per unit (ts_split).  Fitted at 1296 sizes, each with the rows kept
+// and apart (24 shapes of 1024 to 17408 k and 1024 to 34816 columns, 2 to 8 bits, 513 to 2176 rows); at none of them is the choice
+// behind by more than the runs differ.  Kept -> apart, us, 4 bits: 5120 x 17408, 540 rows 122 -> 107, 1052 rows 200 -> 184; 17408 x
+// 5120, 640 rows 188 -> 145; 5120 x 5120, 540 rows 61 -> 51; 2048 x 6144, 1564 rows 55 -> 48; but 4096 x 14336, 1052 rows 141 -> 145
+// and 5120 x 13824, 1144 rows 172 -> 178, which stay whole.
 int tc_tail(const exl3_ctx* ctx, int slabs, int blocks128, int m, int k)
 {
     const int tail = m % (2 * TC_BM), slots = ctx->num_sms / 2;
     if (!ctx->use_pair || m < 2 * TC_BM || tail == 0 || tail > TS_MAX_N) return 0;
     const int rows = m - tail, full = slabs * (rows / (2 * TC_BM)), r = full % slots;
-    const int left = slabs - (r ? slots - r : 0);
+    const int left = slabs - (r ? slots - r : 0);           // short items that the last wave has no slot for
     const float item = k * 0.0121f, waves = (float)((full + slots - 1) / slots);
     const float unit = rows <= 2 * TC_BM && slabs * 4 <= ctx->num_sms ? 0.65f : 1.0f;
-    int whole, longest;
-    ts_split(ctx->num_sms, blocks128, k / TS_UNIT_K, tail, blocks128 <= ctx->n_counters, &whole, &longest);
-    const float keep = item * (waves + (left > 0 ? 0.65f * ((left + slots - 1) / slots) : 0.0f));
-    return item * waves * unit + 14.0f + 0.57f * longest < keep ? tail : 0;
+    const float wave = left <= 0 ? 0.0f : left <= slots ? 0.4f + 0.12f * left / slots : 0.52f * ((left + slots - 1) / slots);
+    int whole;
+    float units;
+    ts_split(ctx->num_sms, blocks128, k / TS_UNIT_K, tail, blocks128 <= ctx->n_counters, &whole, nullptr, &units);
+    return item * waves * unit + 5.0f + 0.55f * units < item * (waves + wave) ? tail : 0;
 }
 
 // Tensor-core path for rows [0, m) and `nseg` weight tensors that share the activations, k, bits and codebook:

@@ -337,10 +337,11 @@ def test_gemm_tc_step_shape(ctx, ctx_small_only):
 
 
 @pytest.mark.parametrize("m,k,n,K,c_fp32", [(513, 5120, 17408, 4, True), (576, 5120, 17280, 3, False), (640, 5120, 17408, 8, False),
-                                            (1025, 5120, 17408, 4, False), (600, 17408, 5120, 5, False)])
+                                            (1025, 5120, 17408, 4, False), (600, 17408, 5120, 5, False),
+                                            (540, 5120, 5120, 4, False), (1564, 2048, 6144, 6, True)])
 def test_gemm_tc_last_rows_apart(ctx, ctx_small_only, m, k, n, K, c_fp32):
-    """up to 128 rows behind the last block of 512 as a second launch with the weights in tensor memory: one row, 64, 88 and 128, two
-    blocks in front, 128-column slabs in front"""
+    """up to 128 rows behind the last block of 512 as a second launch with the weights in tensor memory: one row, 28, 64, 88 and 128,
+    two and three blocks in front, 128-column slabs in front"""
     n0 = ctx.launch_count()
     _tc_case(ctx, ctx_small_only, None, m, k, n, K, 1, c_fp32, 1800 + m)
     assert ctx.launch_count() - n0 == 3                     # transform, whole blocks, last rows
