@@ -29,6 +29,18 @@ def _pools(model):
     return [L[x] for L in model.layers for x in names]
 
 
+def _untouched(model, before, bt, ctx_lens, q_lens):
+    """every token slot of every plane but the sequences' new ones is what it was, and those are not"""
+    import torch
+    slots = [int(bt[b, p >> 8]) * 256 + (p & 255) for b in range(len(q_lens)) for p in range(ctx_lens[b], ctx_lens[b] + q_lens[b])]
+    mask = torch.ones(before[0].shape[0] * 256, dtype=torch.bool, device="cuda")
+    mask[slots] = False
+    for g, w in zip(_pools(model), before):
+        g, w = g.flatten(0, 1).flatten(1), w.flatten(0, 1).flatten(1)
+        assert torch.equal(g[mask], w[mask])
+        assert not torch.equal(g[~mask], w[~mask])
+
+
 def test_build_descriptors(ctx):
     import torch
     from exl3b200 import lib
@@ -117,54 +129,50 @@ def test_step_with_transform_behind_attention(ctx, q_len, ctx_lens, kv_bits):
 
 
 @pytest.mark.parametrize("kv_bits", [0, 3, 4, 6, 8])
-def test_step_writes_its_keys_and_values(ctx, kv_bits):
-    """The rotation's kernel writes the new rows of the pools: first and last offset of a page, rows over a page border, and no
-    other slot.  Against the same layer's keys and values through the separate operators."""
+@pytest.mark.parametrize("q_lens,ctx_lens,rope_mode", [([1, 5, 1, 3], [0, 254, 255, 511], 2), ([600, 1, 33], [200, 0, 250], 2), ([2, 9], [300, 100], 1)])
+def test_step_writes_its_keys_and_values(ctx, kv_bits, q_lens, ctx_lens, rope_mode):
+    """The rotation's kernel writes the new rows of the pools: first and last offset of a page, rows over page borders, a chunk of
+    several pages, and no other slot.  Byte for byte what embedding, norm, projections, rotation and append leave there as operators of
+    their own, in a context whose step launches norm and projections separately; up to 16 rows the fused ones give the same bits."""
+    import os
     import torch
-    q_lens, ctx_lens = [1, 5, 1, 3], [0, 254, 255, 511]
-    model, nm, ids, q_lens, ctx_lens, bt = _setup(kv_bits, 4, 1, q_lens, ctx_lens, 900 + kv_bits, n_layers=1)
-    L = model.layers[0]
-    names = ["k_cache", "v_cache"] if kv_bits == 0 else ["qk", "sk", "qv", "sv"]
-    for x in names:
-        L[x].copy_(torch.randint(-100, 100, L[x].shape, device="cuda").to(L[x].dtype))
-    before = [L[x].clone() for x in names]
-    d_q, d_c, d_bt = H.to_dev(q_lens), H.to_dev(ctx_lens), H.to_dev(bt)
-    model.step(ctx, H.to_dev(ids), d_q, d_c, d_bt, 5)
-    ctx.poll_status()
-    got = [L[x].clone() for x in names]
-    slots = [int(bt[b, p >> 8]) * 256 + (p & 255) for b in range(4) for p in range(ctx_lens[b], ctx_lens[b] + q_lens[b])]
-    mask = torch.ones(got[0].shape[0] * 256, dtype=torch.bool, device="cuda")
-    mask[slots] = False
-    for g, w in zip(got, before):
-        g, w = g.flatten(0, 1).flatten(1), w.flatten(0, 1).flatten(1)
-        assert torch.equal(g[mask], w[mask])
-        assert not torch.equal(g[~mask], w[~mask])
-    # the same rows one sequence at a time (other rows per call, the same arithmetic per row up to the order of fp32 sums)
-    for x, w in zip(names, before):
-        L[x].copy_(w)
-    at = 0
-    for b in range(4):
-        model.step(ctx, H.to_dev(ids[at:at + q_lens[b]]), H.to_dev(q_lens[b:b + 1]), H.to_dev(ctx_lens[b:b + 1]), H.to_dev(bt[b:b + 1]), int(q_lens[b]))
-        at += q_lens[b]
-    ctx.poll_status()
-    for x, g in zip(names, got):
-        w = L[x]
-        if g.dtype == torch.float16:
-            assert H.rel_rms_err(g.flatten(0, 1)[slots].float().cpu().numpy(), w.flatten(0, 1)[slots].float().cpu().numpy()) < 1e-2
-        else:
-            assert (g.flatten(0, 1)[slots] == w.flatten(0, 1)[slots]).float().mean() > 0.9
-
-
-def _untouched(model, before, bt, ctx_lens, q_lens):
-    """every token slot of every plane but the sequences' new ones is what it was, and those are not"""
-    import torch
-    slots = [int(bt[b, p >> 8]) * 256 + (p & 255) for b in range(len(q_lens)) for p in range(ctx_lens[b], ctx_lens[b] + q_lens[b])]
-    mask = torch.ones(before[0].shape[0] * 256, dtype=torch.bool, device="cuda")
-    mask[slots] = False
-    for g, w in zip(_pools(model), before):
-        g, w = g.flatten(0, 1).flatten(1), w.flatten(0, 1).flatten(1)
-        assert torch.equal(g[mask], w[mask])
-        assert not torch.equal(g[~mask], w[~mask])
+    from exl3b200 import Ctx
+    model, _, ids, q_lens, ctx_lens, bt = _setup(kv_bits, 4, 1, q_lens, ctx_lens, 900 + kv_bits, n_layers=1)
+    model.struct.rope_mode = rope_mode
+    L, rows = model.layers[0], len(ids)
+    for t in _pools(model):
+        t.copy_(torch.randint(-100, 100, t.shape, device="cuda").to(t.dtype))
+    before = [t.clone() for t in _pools(model)]
+    os.environ["EXL3_B200_NO_FUSED_TRANSFORM"] = "1"
+    try:
+        plain = Ctx(0)
+    finally:
+        del os.environ["EXL3_B200_NO_FUSED_TRANSFORM"]
+    d_ids, d_q, d_c, d_bt = H.to_dev(ids), H.to_dev(q_lens), H.to_dev(ctx_lens), H.to_dev(bt)
+    got = []
+    for c in (plain, ctx):
+        for t, w in zip(_pools(model), before):
+            t.copy_(w)
+        model.step(c, d_ids, d_q, d_c, d_bt, int(q_lens.max()))
+        c.poll_status()
+        _untouched(model, before, bt, ctx_lens, q_lens)
+        got.append([t.clone() for t in _pools(model)])
+    half = lambda *shape: torch.empty(*shape, dtype=torch.float16, device="cuda")  # noqa: E731
+    x, a, q, k, v = torch.empty(rows, 1024, device="cuda"), half(rows, 1024), half(rows, 2048), half(rows, 1024), half(rows, 1024)
+    plain.embed(d_ids, model.embed, x)
+    plain.rms_norm(x, L["attn_norm"], a, 1e-6)
+    plain.gemm_fanout(a, [(w.trellis, w.suh, w.svh, w.cb) for w in (L["q_proj"], L["k_proj"], L["v_proj"])], [q, k, v])
+    row_pos = H.to_dev(np.concatenate([c + np.arange(n) for c, n in zip(ctx_lens, q_lens)]).astype(np.int32))
+    plain.rope(q.view(1, rows, 16, 128), k.view(1, rows, 8, 128), model.inv_freq, q_norm=L["q_norm"], k_norm=L["k_norm"], rope_mode=rope_mode, row_pos=row_pos)
+    cu = H.to_dev(np.concatenate([[0], np.cumsum(q_lens)]).astype(np.int32))
+    want = before
+    if kv_bits == 0:
+        plain.paged_kv_cache_update(k.view(rows, 8, 128), v.view(rows, 8, 128), want[0], want[1], d_bt, d_c, cu_q=cu)
+    else:
+        plain.quant_cache_paged(k, want[0], want[1], v, want[2], want[3], d_c, d_bt, cu_q=cu)
+    plain.poll_status()
+    for which in ([0, 1] if rows <= 16 else [0]):
+        assert all(torch.equal(g, w) for g, w in zip(got[which], want))
 
 
 # (the scratch is filled with slots that exist, so that a row that took one of them would show and not fault)
