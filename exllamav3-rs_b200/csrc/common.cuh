@@ -119,7 +119,7 @@ static inline cudaError_t exl3_launch(exl3_ctx* ctx, void (*kern)(P...), dim3 gr
 // The first kernel of a call, which begins with pdl_enter_first and takes its argument last: a programmatic dependent whatever is
 // in front of it, because it touches nothing and lets nothing go before that is complete.  Back to back, the set-up of its blocks
 // and the launch of the kernel behind it then overlap the tail of the call before (EXL3 GEMM at 4 bits, us: 5120 x 5120, 1 row
-// 17.1 -> 15.1, 5120 x 17408, 52 rows 33.1 -> 29.2).  Under stream capture, where the node in front need not be a kernel, a plain
+// 17.1 -> 15.1, 5120 x 17408, 52 rows 33.1 -> 29.2).  A call that is waited for before the next has none of this.  Under stream capture, where the node in front need not be a kernel, a plain
 // launch outside of a chain.
 static inline int exl3_first_early(exl3_ctx* ctx, cudaStream_t st, bool* overlap)
 {
