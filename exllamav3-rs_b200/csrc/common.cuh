@@ -119,13 +119,21 @@ static inline cudaError_t exl3_launch(exl3_ctx* ctx, void (*kern)(P...), dim3 gr
 // The first kernel of a call, which begins with pdl_enter_first and takes its argument last: a programmatic dependent whatever is
 // in front of it, because it touches nothing and lets nothing go before that is complete.  Back to back, the set-up of its blocks
 // and the launch of the kernel behind it then overlap the tail of the call before (EXL3 GEMM at 4 bits, us: 5120 x 5120, 1 row
-// 17.1 -> 15.1, 5120 x 17408, 52 rows 33.1 -> 29.2).  A call that is waited for before the next has none of this.  Under stream capture, where the node in front need not be a kernel, a plain
-// launch outside of a chain.
+// 17.1 -> 15.1, 5120 x 17408, 52 rows 33.1 -> 29.2).  A call that is waited for before the next has none of this.  Under stream
+// capture the node in front has to be a kernel for it, and the only one (replayed, against a plain launch there, us: 1024 x 3072 at 8
+// bits, 1 and 8 rows 9.1 -> 8.1 and 10.1 -> 9.5; 5120 x 17408 at 4 bits, 1 and 52 rows 26.7 -> 25.7 and 31.1 -> 29.0).
 static inline int exl3_first_early(exl3_ctx* ctx, cudaStream_t st, bool* overlap)
 {
     if (exl3_chained(ctx)) { *overlap = true; return 1; }
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     *overlap = cudaStreamIsCapturing(st, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone;
+    if (cs == cudaStreamCaptureStatusActive) {
+        const cudaGraphNode_t* deps = nullptr;
+        size_t n = 0;
+        cudaGraphNodeType type = cudaGraphNodeTypeEmpty;
+        *overlap = cudaStreamGetCaptureInfo_v2(st, &cs, nullptr, nullptr, &deps, &n) == cudaSuccess && n == 1 &&
+                   cudaGraphNodeGetType(deps[0], &type) == cudaSuccess && type == cudaGraphNodeTypeKernel;
+    }
     if (!*overlap) cudaGetLastError();
     return 0;
 }
