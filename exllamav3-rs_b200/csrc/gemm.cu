@@ -409,7 +409,12 @@ int gemm_tc_rows(exl3_ctx* ctx, cudaStream_t st, const half* A, int nseg, const 
     for (int i = 0; i < nseg; ++i) { blocks256 += (n[i] + TC_BN - 1) / TC_BN; n128 = n128 && n[i] % 128 == 0; }
     // Up to 128 rows the weights go through tensor memory in 128-column blocks (gemm_ts.cuh): at 128 rows 5120 x 17408 takes 35 us
     // against 47, at more its accumulator does not fit.
-    const bool ts = n128 && m <= TS_MAX_N;
+    // From 81 rows on a short k leaves a CTA of it little but the read-out of its accumulator: up to k = 1024 the 128-column slabs of
+    // the other kernel are ahead where they have an SM each (replayed back to back at 4 bits, us, that one against this: 1024 x 3072, 72
+    // rows 11.1 and 10.8, 88 rows 11.1 and 11.5, 128 rows 11.3 and 12.4, at 8 bits 11.3 and 13.3; 512 x 6144, 128 rows 9.2 and 10.4;
+    // but 1024 x 12800 16.2 and 13.9, 1536 x 6144 14.7 and 14.8, 2048 x 3072 15.2 and 14.4).
+    const bool slabs128 = ctx->use_pair && n128 && blocks256 * 4 <= ctx->num_sms;
+    const bool ts = n128 && m <= TS_MAX_N && !(slabs128 && k <= 1024 && m > 80 && !given);
     int blocks128 = 0, whole, longest;
     for (int i = 0; i < nseg; ++i) blocks128 += n[i] / 128;
     int grid = ts_split(ctx->num_sms, blocks128, k / TS_UNIT_K, m, blocks128 <= ctx->n_counters, &whole, &longest);
@@ -418,7 +423,7 @@ int gemm_tc_rows(exl3_ctx* ctx, cudaStream_t st, const half* A, int nseg, const 
     // rows, 5120 x 1024 in 5 units 13.8 -> 11.8, but 5120 x 5120 in 14 units 15.2 -> 16.0 and 5120 x 17408 in 40 27.2 -> 30.5).
     const bool few = ts && !pre && (m == 1 || (m <= TS_FEW && longest <= 10));
     const int tail = !ts && n128 ? tc_tail(ctx, blocks256, blocks128, m, k) : 0, mm = m - tail;
-    const int bn = ts || (ctx->use_pair && n128 && mm <= 2 * TC_BM && blocks256 * 4 <= ctx->num_sms) ? 128 : TC_BN;
+    const int bn = ts || (slabs128 && mm <= 2 * TC_BM) ? 128 : TC_BN;
     int blocks = 0;
     for (int i = 0; i < TC_MAX_SEG; ++i) {
         const int j = i < nseg ? i : nseg - 1;              // unused slots repeat the last tensor (never selected)

@@ -414,6 +414,7 @@ def test_gemm_tc_pair_equals_one_cta(ctx, ctx_one_cta, m):
 @pytest.mark.parametrize("m,k,n,K,cb,c_fp32", [
     (17, 128, 128, 4, 1, False), (33, 1152, 640, 8, 0, False), (48, 1664, 384, 6, 1, True), (49, 1664, 1280, 7, 2, False),
     (64, 5120, 1024, 3, 0, False), (65, 5120, 1024, 8, 1, True), (96, 640, 25600, 5, 1, False), (112, 5120, 256, 7, 1, False),
+    (80, 1024, 3072, 8, 1, False), (81, 1024, 3072, 8, 1, False), (128, 512, 9472, 5, 0, True), (100, 1024, 9600, 3, 2, False),   # both sides of the rule for a short k
     (127, 2048, 1152, 2, 2, True), (128, 1024, 3072, 6, 0, False), (128, 5120, 512, 8, 1, False), (40, 5120, 12800, 4, 1, False)])
 def test_gemm_weights_in_tensor_memory(ctx, ref, m, k, n, K, cb, c_fp32):
     _gemm_case(ctx, ref, m, k, n, K, cb, c_fp32, 1500 + m + K)

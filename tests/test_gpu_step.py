@@ -468,6 +468,36 @@ def test_decode_step_fused_launches(ctx, hidden, cb, fewer):
     assert launches[1] - launches[0] == fewer * layers
 
 
+@pytest.mark.parametrize("rows", [80, 81, 128])
+def test_fused_step_of_a_short_k_with_half_slabs(ctx, rows):
+    """From 81 rows on a short k runs on 128-column slabs of the other GEMM, here for two fused tensors with an odd number of
+    128-column blocks each: within the bar of fused against separate transforms."""
+    import os
+    import torch
+    from exl3b200 import Ctx
+    from exl3b200.step import SyntheticModel
+    r = H.rng(1300 + rows)
+    ctx_lens = np.array([40], np.int32)
+    bt, pages = H.make_paged(r, 1, ctx_lens + rows, 4, 128)
+    model = SyntheticModel(2, 1024, 8, 4, 128, 1152, 512, K=5, cb=1, pages=pages, seed=rows)
+    model.fill_kv()
+    before = [t.clone() for t in _pools(model)]
+    args = (H.to_dev(r.integers(0, 512, rows)), H.to_dev(np.array([rows], np.int32)), H.to_dev(ctx_lens), H.to_dev(bt), rows)
+    os.environ["EXL3_B200_NO_FUSED_TRANSFORM"] = "1"
+    try:
+        plain = Ctx(0)
+    finally:
+        del os.environ["EXL3_B200_NO_FUSED_TRANSFORM"]
+    logits = []
+    for c in (ctx, plain):
+        for t, w in zip(_pools(model), before):
+            t.copy_(w)
+        logits.append(model.step(c, *args, want_logits=True, all_rows=True)[1].cpu())
+        c.poll_status()
+    assert torch.isfinite(logits[0]).all()
+    assert H.rel_rms_err(logits[0].numpy(), logits[1].numpy()) < 5e-3
+
+
 @pytest.mark.parametrize("kv_bits", [4, 8])
 def test_ragged_step_over_quantised_pools(ctx, kv_bits):
     """Decode rows, verify rows and a prefill chunk in one step over quantised pools: the two attention passes of every layer
