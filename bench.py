@@ -300,9 +300,10 @@ def gemm_alg_bytes(m, k, n, K):
     return k * n * K / 8 + 2 * (k + n) + 2 * m * k + 2 * m * n
 
 
-# DRAM bytes of one gemm_tc_kernel launch at M = 1052 on 5120 x 17408, 4 bpw (dram__bytes_read.sum + dram__bytes_write.sum of
-# one ncu capture); the figure belongs to the commit named with it and is not re-measured by the run
-NCU_TRAFFIC_TC_M1052 = {"bytes": None, "source": "no capture of this shape (1024 rows and the last 28 are two launches)"}
+# DRAM bytes of the two GEMM launches of one call at M = 1052 on 5120 x 17408, 4 bpw (dram__bytes_read.sum + dram__bytes_write.sum of
+# gemm_tc_kernel over 1024 rows and gemm_ts_kernel over 28, one ncu capture; not re-measured by the run)
+NCU_TRAFFIC_M1052 = {"bytes": 58847232 + 5451008 + 44969728 + 14080,
+                     "source": "ncu capture of gemm_tc_kernel<4,1,2,256> and gemm_ts_kernel<4,1> at M=1052 (summary under profiles/)"}
 
 
 def run_ours(args):
@@ -432,7 +433,8 @@ def run_ours(args):
             ach = flops / t_op / 1e12
             roof = {"bound": "tensor", "kernel": "exl3_gemm (gate_proj 5120x17408, M=%d)" % rows, "achieved": ach,
                     "peak": tf_peak, "unit": "TFLOP/s", "frac": ach / tf_peak,
-                    "traffic": NCU_TRAFFIC_TC_M1052["bytes"], "traffic_source": NCU_TRAFFIC_TC_M1052["source"],
+                    "traffic": NCU_TRAFFIC_M1052["bytes"] if rows == 1052 else None,
+                    "traffic_source": NCU_TRAFFIC_M1052["source"] if rows == 1052 else "no capture of this shape",
                     "algorithmic_bytes": gemm_alg_bytes(rows, k, n, K), "peak_source": which, "launches_per_op": launches_op,
                     "op_ms": t_op * 1e3, "step_hbm_gbs": step_hbm, "step_hbm_frac": step_hbm / hbm_peak}
         else:
