@@ -1,6 +1,6 @@
 // exl3_bighead_attn_paged / exl3_bighead_attn_paged_q: planning, launch and split-KV combine.
 #include <algorithm>
-#include "attn_paged.cuh"
+#include "attn_front.cuh"
 #include "attn_tc.cuh"
 #include "attn_tc2.cuh"
 #include "attn_qdec.cuh"
@@ -8,157 +8,6 @@
 namespace {
 
 using namespace exl3;
-
-// Inclusive scan over the 1024 threads of the block: three barriers instead of the twenty of a scan through shared memory
-// (the list is built in one block in front of the attention kernel, so its latency is the call's).
-__device__ __forceinline__ int plan_scan(int v, int* s_warp)
-{
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) { const int u = __shfl_up_sync(0xffffffffu, v, o); if (lane >= o) v += u; }
-    if (lane == 31) s_warp[warp] = v;
-    __syncthreads();
-    if (warp == 0) {
-        int w = s_warp[lane];
-        #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) { const int u = __shfl_up_sync(0xffffffffu, w, o); if (lane >= o) w += u; }
-        s_warp[lane] = w;
-    }
-    __syncthreads();
-    if (warp > 0) v += s_warp[warp - 1];
-    __syncthreads();
-    return v;
-}
-
-// Builds the split-KV work list from the REAL sequence lengths (one CTA; bsz is small next to the KV walk).
-// Each sequence gets ceil(total_k / chunk) splits per row block, with chunk sized so that the list has about
-// `target_items` entries; the reference sizes its splits from the padded block-table width instead
-// (kernels/attention.cu:1805), which launches empty CTAs for the short sequences of a ragged batch.
-// Only sequences whose packed row count ql*G lies in (rows_lo, rows_hi] get work items; the others are left to another pass.
-__global__ void __launch_bounds__(1024) attn_plan_kernel(const int32_t* __restrict__ seqlens,
-                                                         const int32_t* __restrict__ cu_q, int bsz, int q_len,
-                                                         int kv_append, int G, int rows_per_cta, int rows_lo, int rows_hi, int chunk_mult, int target_items,
-                                                         int max_items, AttnPlan* plan, AttnItem* items, int* seq_base,
-                                                         int* seq_splits, int* order, int causal, int slots, int* status)
-{
-    pdl_enter();
-    __shared__ long long s_total;
-    __shared__ int s_scan[1024];
-    __shared__ int s_cursor[1024];
-    __shared__ int s_warp[32];
-    __shared__ int s_carry, s_chunk;
-    const int tid = threadIdx.x;
-    if (tid == 0) { s_total = 0; s_carry = 0; }
-    __syncthreads();
-    long long local = 0;
-    for (int b = tid; b < bsz; b += 1024) {
-        const int ql = cu_q ? cu_q[b + 1] - cu_q[b] : q_len;
-        const int tk = (seqlens ? seqlens[b] : 0) + (cu_q ? ql : kv_append);
-        const int pr = ql * G;
-        const int rb = (pr > rows_lo && pr <= rows_hi) ? (pr + rows_per_cta - 1) / rows_per_cta : 0;
-        local += (long long)tk * rb;
-    }
-    atomicAdd((unsigned long long*)&s_total, (unsigned long long)local);
-    __syncthreads();
-    // Keys per split: total work / target_items.  slots > 0 (kernels whose CTAs are whole items, target_items = two per CTA
-    // slot): one item per slot instead when that already gives two or more items per slot, because every row block and
-    // every sequence rounds its split count up.  Then the longest-first order balances the slots and fewer items save the
-    // fixed cost of a CTA and the partials (four 256-row chunks: 125 us at one item per slot, 135 at two, 150 at three; 32
-    // x 8 verify rows: 125 against 133 us), while a batch of few long items (one 256-row chunk over 32768 keys: 20 items
-    // on 18 slots) keeps the finer split.
-    auto chunk_for = [&](long long t) {
-        long long c = (s_total + t - 1) / t;
-        c = (c + chunk_mult - 1) / chunk_mult * chunk_mult;       // splits start on a key-tile boundary of the kernel
-        if (c < 256) c = 256;
-        if (c > (1 << 30)) c = 1 << 30;
-        return (int)c;
-    };
-    if (slots <= 0) {
-        if (tid == 0) s_chunk = chunk_for(target_items);
-        __syncthreads();
-    } else {
-        __shared__ long long s_count;
-        const int c1 = chunk_for(slots);
-        if (tid == 0) s_count = 0;
-        __syncthreads();
-        long long cnt = 0;
-        for (int b = tid; b < bsz; b += 1024) {
-            const int ql = cu_q ? cu_q[b + 1] - cu_q[b] : q_len;
-            const int tk = (seqlens ? seqlens[b] : 0) + (cu_q ? ql : kv_append);
-            const int pr = ql * G;
-            const int rb = (pr > rows_lo && pr <= rows_hi) ? (pr + rows_per_cta - 1) / rows_per_cta : 0;
-            cnt += (long long)rb * (tk > 0 ? (tk + c1 - 1) / c1 : 1);
-        }
-        atomicAdd((unsigned long long*)&s_count, (unsigned long long)cnt);
-        __syncthreads();
-        if (tid == 0) s_chunk = s_count >= 2LL * slots ? c1 : chunk_for(target_items);
-        __syncthreads();
-    }
-    const int chunk = s_chunk;
-    for (int b0 = 0; b0 < bsz; b0 += 1024) {
-        const int b = b0 + tid;
-        int ql = 0, tk = 0, rb = 0, sp = 0;
-        if (b < bsz) {
-            ql = cu_q ? cu_q[b + 1] - cu_q[b] : q_len;
-            tk = (seqlens ? seqlens[b] : 0) + (cu_q ? ql : kv_append);
-            const int pr = ql * G;
-            rb = (pr > rows_lo && pr <= rows_hi) ? (pr + rows_per_cta - 1) / rows_per_cta : 0;
-            sp = (rb > 0 && tk > 0) ? (tk + chunk - 1) / chunk : 1;
-        }
-        const int cnt = rb * sp;
-        const int incl = plan_scan(cnt, s_warp);
-        const int base = s_carry + incl - cnt;
-        if (b < bsz) {
-            seq_base[b] = base;
-            seq_splits[b] = sp;
-            for (int j = 0; j < cnt && base + j < max_items; ++j) {
-                AttnItem it; it.b = b; it.rb = j / sp; it.split = j % sp; it.pad = 0;
-                items[base + j] = it;
-            }
-        }
-        __syncthreads();
-        if (tid == 1023) s_carry += incl;
-        __syncthreads();
-    }
-    // Launch order: longest items first (counting sort by key tiles, most first).  Items differ in length - last splits,
-    // causal cuts, short sequences - and a long one started late leaves the other SMs idle at the end of the kernel
-    // (four 256-row chunks: a quarter of the SM time).
-    const int n_items = s_carry < max_items ? s_carry : max_items;
-    s_scan[tid] = 0; s_cursor[tid] = 0;
-    __syncthreads();
-    for (int i = tid; i < n_items; i += 1024) {
-        const AttnItem it = items[i];
-        const int ql = cu_q ? cu_q[it.b + 1] - cu_q[it.b] : q_len;
-        const int tk = (seqlens ? seqlens[it.b] : 0) + (cu_q ? ql : kv_append);
-        const int i_last = min(ql - 1, (it.rb * rows_per_cta + rows_per_cta - 1) / G);
-        const int vis = causal > 0 ? min(tk, tk - ql + i_last + 1) : tk;
-        const int k_begin = it.split * chunk;
-        const int k_end = min(min(k_begin + chunk, tk), vis);
-        int key = k_end > k_begin ? (k_end - k_begin + chunk_mult - 1) / chunk_mult : 0;
-        key = causal >= 0 ? 1023 - min(key, 1023) : 0;          // bin 0 = longest (causal < 0: A/B switch, plan order kept)
-        items[i].pad = key;
-        atomicAdd(&s_scan[key], 1);
-    }
-    __syncthreads();
-    {
-        const int cnt = s_scan[tid];
-        const int excl = plan_scan(cnt, s_warp) - cnt;
-        s_scan[tid] = excl;                                    // first position of bin tid
-        __syncthreads();
-    }
-    for (int i = tid; i < n_items; i += 1024) {
-        const int key = items[i].pad;
-        order[causal < 0 ? i : s_scan[key] + atomicAdd(&s_cursor[key], 1)] = i;
-    }
-    if (tid == 0) {
-        plan->n_items = n_items;
-        plan->next = 0;
-        plan->chunk = chunk;
-        // the host sizes the list from bounds on the batch; a list that does not fit would silently drop work, so it is
-        // reported through the status word like a device-side wait that ran out
-        if (s_carry > max_items) atomicExch(status, 3);
-    }
-}
 
 // Merges the split-KV partials of one output row (b, query, head); one warp per row, lane = D/32 dims.
 // HAD: also writes the 128-point transform of (output o signs).  (A form of its own: with the test at run time in every call 24
@@ -328,10 +177,9 @@ cudaError_t launch_attn_tc2(exl3_ctx* ctx, const AttnParams& p, int max_items, c
         if (e != cudaSuccess) return e;
         if (dev >= 0 && dev < 64) configured[dev] = true;
     }
-    (void)ctx;
-    if (tune_h == 4) attn_tc2_kernel<4><<<dim3((unsigned)max_items * p.nkv), a2_threads(4), A2_SMEM, st>>>(maps[0], maps[1], p);
-    else attn_tc2_kernel<2><<<dim3((unsigned)max_items * p.nkv), a2_threads(2), A2_SMEM, st>>>(maps[0], maps[1], p);
-    return cudaPeekAtLastError();
+    const dim3 grid((unsigned)max_items * p.nkv);
+    return tune_h == 4 ? exl3_launch(ctx, attn_tc2_kernel<4>, grid, a2_threads(4), A2_SMEM, st, maps[0], maps[1], p)
+                       : exl3_launch(ctx, attn_tc2_kernel<2>, grid, a2_threads(2), A2_SMEM, st, maps[0], maps[1], p);
 }
 
 // decode-class kernel over 4-bit and 8-bit pools: tensor maps over the code planes ([tokens][nkv * 4 * bits] words, copied in
@@ -373,7 +221,7 @@ bool qdec_kernel_applies(const AttnParams& p, bool quant);
 
 // One pass = plan + attention + combine over the sequences whose packed row count lies in (rows_lo, rows_hi].
 int attn_pass(exl3_ctx* ctx, cudaStream_t st, AttnParams p, int total_rows, int max_rows, int rows_lo, int rows_hi,
-              bool decode_shape, bool quant, size_t* ws_off, bool had = false)
+              bool decode_shape, bool quant, size_t* ws_off, const AttnAppendArgs* append, bool had = false)
 {
     const int D = 128;
     const int G = p.nq / p.nkv;
@@ -420,37 +268,38 @@ int attn_pass(exl3_ctx* ctx, cudaStream_t st, AttnParams p, int total_rows, int 
     // The work list depends on the batch's lengths, not on the layer: inside exl3_step_forward it is built by the first
     // layer's call into the context's slot for this class and reused by the other layers.
     const int cls = decode_shape ? 0 : 1;
-    const size_t list_bytes = 256 + (((size_t)max_items * sizeof(AttnItem) + 255) & ~(size_t)255) + 2 * (((size_t)p.bsz * 4 + 255) & ~(size_t)255) +
-                              (((size_t)max_items * 4 + 255) & ~(size_t)255);
+    const size_t list_bytes = 256 + (((size_t)max_items * sizeof(AttnItem) + 255) & ~(size_t)255) + 2 * (((size_t)p.bsz * 4 + 255) & ~(size_t)255);
     const bool keep = ctx->plan_keep && list_bytes <= ctx->plan_slot_bytes;
     size_t off = *ws_off;                                // scratch of an earlier pass that may still be running
-    AttnPlan* plan; AttnItem* items; int* seq_base; int* seq_splits; int* order;
+    AttnPlan* plan; AttnItem* items; int* seq_base; int* seq_splits;
     if (keep) {
         uint8_t* slot = ctx->plan_slots + cls * ctx->plan_slot_bytes;
         plan = (AttnPlan*)slot;
         items = (AttnItem*)(slot + 256);
         seq_base = (int*)(slot + 256 + (((size_t)max_items * sizeof(AttnItem) + 255) & ~(size_t)255));
         seq_splits = (int*)((uint8_t*)seq_base + (((size_t)p.bsz * 4 + 255) & ~(size_t)255));
-        order = (int*)((uint8_t*)seq_splits + (((size_t)p.bsz * 4 + 255) & ~(size_t)255));
     } else {
         plan = (AttnPlan*)exl3_ws_take(ctx, &off, sizeof(AttnPlan));
         items = (AttnItem*)exl3_ws_take(ctx, &off, (size_t)max_items * sizeof(AttnItem));
         seq_base = (int*)exl3_ws_take(ctx, &off, (size_t)p.bsz * 4);
         seq_splits = (int*)exl3_ws_take(ctx, &off, (size_t)p.bsz * 4);
-        order = (int*)exl3_ws_take(ctx, &off, (size_t)max_items * 4);
     }
     float* partial = (float*)exl3_ws_take(ctx, &off, (size_t)max_items * p.nkv * rows_per_cta * (D + 2) * 4);
-    if (!plan || !items || !seq_base || !seq_splits || !order || !partial)
+    if (!plan || !items || !seq_base || !seq_splits || !partial)
         return exl3_fail(ctx, EXL3_ERR_WORKSPACE, "attention: context scratch too small for the split-KV partials");
-    p.plan = plan; p.items = items; p.seq_base = seq_base; p.seq_splits = seq_splits; p.order = order; p.partial = partial;
+    p.plan = plan; p.items = items; p.seq_base = seq_base; p.seq_splits = seq_splits; p.partial = partial;
     p.status = ctx->status;
     *ws_off = off;
 
     static const bool no_lpt = getenv("EXL3_TUNE_NO_LPT") != nullptr;
     if (!(keep && ctx->plan_valid[cls])) {
-        exl3_launch(ctx, attn_plan_kernel, 1, 1024, 0, st, p.seqlens, p.cu_q, p.bsz, p.q_len, p.kv_append, G, rows_per_cta, rows_lo, rows_hi,
-                                              use_tc ? ATC_TN : AT_TK, target_items, max_items, plan, items, seq_base, seq_splits, order, no_lpt ? -1 : (p.causal ? 1 : 0),
-                                              (use_tc && !tc_items) ? grid_x : 0, ctx->status);
+        const AttnPlanArgs a = {p.seqlens, p.cu_q, plan, items, seq_base, seq_splits, ctx->status, p.bsz, p.q_len, p.kv_append, G, rows_per_cta, rows_lo, rows_hi,
+                                use_tc ? ATC_TN : AT_TK, target_items, max_items, no_lpt ? -1 : (p.causal ? 1 : 0), (use_tc && !tc_items) ? grid_x : 0};
+        if (append) {
+            const long long warps = (long long)append->rows * (append->k_bits ? append->nkv : 1);
+            exl3_launch_first(ctx, attn_front_kernel, 1 + (unsigned)((warps + AP_THREADS / 32 - 1) / (AP_THREADS / 32)), AP_THREADS, 0, st, a, *append);
+        } else
+            exl3_launch(ctx, attn_plan_kernel, 1, AP_THREADS, 0, st, a);
         ctx->launches++;
         if (keep) ctx->plan_valid[cls] = 1;
     }
@@ -484,7 +333,16 @@ bool qdec_kernel_applies(const AttnParams& p, bool quant)
            aligned16(p.sk) && aligned16(p.sv);
 }
 
-int attn_impl(exl3_ctx* ctx, cudaStream_t st, AttnParams p, int total_rows, int max_q_len, bool quant)
+// Appends a call's keys and values ahead of the attention, as the public operators do.
+int attn_append(exl3_ctx* ctx, cudaStream_t st, const AttnAppendArgs& a)
+{
+    return a.k_bits ? exl3_quant_cache_paged(ctx, st, a.k, a.qk, a.sk, a.v, a.qv, a.sv, a.seqlens, a.block_table, a.cu_q, a.bsz, a.seq, a.nkv * 128, a.pages, a.pps,
+                                             a.k_bits, a.v_bits, EXL3_PAGE, 0.0f, 1)
+                    : exl3_paged_kv_cache_update(ctx, st, a.k, a.v, a.kc, a.vc, a.block_table, a.seqlens, a.cu_q, a.bsz, a.seq, a.nkv, 128, a.pages, a.pps);
+}
+
+// `append`: the call's keys and values, which go to the pools in front of the attention, or NULL
+int attn_impl(exl3_ctx* ctx, cudaStream_t st, AttnParams p, int total_rows, int max_q_len, bool quant, const AttnAppendArgs* append)
 {
     const int G = p.nq / p.nkv;
     const int max_rows = max_q_len * G;
@@ -505,14 +363,32 @@ int attn_impl(exl3_ctx* ctx, cudaStream_t st, AttnParams p, int total_rows, int 
     // not hold it beside the partials; attn_pass refuses before it launches anything.)
     if (max_rows <= dec_rows || !p.cu_q) {
         const bool dec = max_rows <= dec_rows;
+        // The list and the append are one launch unless the list is another layer's already.
+        const bool one = append && !ctx->plan_keep;
+        exl3_chain_scope chain(ctx, append && !one);
+        if (append && !one) {
+            const int rc = attn_append(ctx, st, *append);
+            if (rc != EXL3_OK) return rc;
+        }
+        int rc = EXL3_ERR_WORKSPACE;
         if (ctx->had_out) {
             off = ctx->had_bytes;
-            const int rc = attn_pass(ctx, st, p, total_rows, max_rows, 0, dec ? dec_rows : 1 << 30, dec, quant, &off, true);
+            rc = attn_pass(ctx, st, p, total_rows, max_rows, 0, dec ? dec_rows : 1 << 30, dec, quant, &off, one ? append : nullptr, true);
             ctx->had_done = rc == EXL3_OK;
-            if (rc != EXL3_ERR_WORKSPACE) return rc;
             off = 0;
         }
-        return attn_pass(ctx, st, p, total_rows, max_rows, 0, dec ? dec_rows : 1 << 30, dec, quant, &off);
+        if (rc == EXL3_ERR_WORKSPACE) rc = attn_pass(ctx, st, p, total_rows, max_rows, 0, dec ? dec_rows : 1 << 30, dec, quant, &off, one ? append : nullptr);
+        if (rc == EXL3_ERR_WORKSPACE && one) {             // refused before anything was launched; the keys and values are appended all the same
+            const int rc2 = attn_append(ctx, st, *append);
+            if (rc2 != EXL3_OK) return rc2;
+            return exl3_fail(ctx, rc, "attention: context scratch too small for the split-KV partials");
+        }
+        return rc;
+    }
+    exl3_chain_scope chain(ctx, append != nullptr);
+    if (append) {
+        const int rc = attn_append(ctx, st, *append);
+        if (rc != EXL3_OK) return rc;
     }
     // Ragged batch with both classes: the decode-class pass (bound by HBM) is issued on the context's second stream and
     // the long-class pass (bound by the tensor core and the MUFU) on the caller's; they touch disjoint sequences and
@@ -523,9 +399,9 @@ int attn_impl(exl3_ctx* ctx, cudaStream_t st, AttnParams p, int total_rows, int 
     if (cudaEventRecord(ctx->ev_fork, st) != cudaSuccess || cudaStreamWaitEvent(ctx->aux_stream, ctx->ev_fork, 0) != cudaSuccess)
         return exl3_fail(ctx, EXL3_ERR_CUDA, "attention: stream fork failed");
     ctx->chain_break = 1;
-    int rc = attn_pass(ctx, ctx->aux_stream, p, total_rows, dec_rows, 0, dec_rows, true, quant, &off);
+    int rc = attn_pass(ctx, ctx->aux_stream, p, total_rows, dec_rows, 0, dec_rows, true, quant, &off, nullptr);
     ctx->chain_break = 1;
-    int rc2 = rc == EXL3_OK ? attn_pass(ctx, st, p, total_rows, max_rows, dec_rows, 1 << 30, false, quant, &off) : rc;
+    int rc2 = rc == EXL3_OK ? attn_pass(ctx, st, p, total_rows, max_rows, dec_rows, 1 << 30, false, quant, &off, nullptr) : rc;
     ctx->chain_break = 1;
     // always join, also after an error, so that a capture in progress stays well-formed
     if (cudaEventRecord(ctx->ev_join, ctx->aux_stream) != cudaSuccess || cudaStreamWaitEvent(st, ctx->ev_join, 0) != cudaSuccess)
@@ -560,13 +436,13 @@ extern "C" int exl3_bighead_attn_paged(exl3_ctx* ctx, exl3_stream stream, const 
     EXL3_REQUIRE(k_cache && v_cache && aligned16(k_cache) && aligned16(v_cache), "attention: bad cache pointers");
     if (bsz == 0 || q_len == 0) return EXL3_OK;
     const int append = cu_q ? q_len : kv_append;
-    if (append > 0 && !ctx->kv_appended) {
+    const bool write = append > 0 && !ctx->kv_appended;
+    if (write) {
         EXL3_REQUIRE(k && v, "attention: kv_append > 0 needs k and v");
-        rc = exl3_paged_kv_cache_update(ctx, stream, k, v, k_cache, v_cache, block_table, cache_seqlens, cu_q, bsz, append,
-                                        nkv, hd, pages, pages_per_seq);
-        if (rc) return rc;
+        EXL3_REQUIRE(aligned16(k) && aligned16(v), "paged_kv_cache_update: pointers must be 16-byte aligned");
+        EXL3_REQUIRE(bsz <= 65535 && append <= 65535, "paged_kv_cache_update: bsz and seq must be <= 65535");
     }
-    exl3_chain_scope chain(ctx, append > 0);
+    exl3_chain_scope chain(ctx, append > 0 && !write);
     AttnParams p;
     memset(&p, 0, sizeof(p));
     p.q = (const half*)q; p.o = (half*)o; p.kc = (const half*)k_cache; p.vc = (const half*)v_cache;
@@ -575,7 +451,9 @@ extern "C" int exl3_bighead_attn_paged(exl3_ctx* ctx, exl3_stream stream, const 
     p.causal = causal;
     p.scale_log2 = (sm_scale == 0.0f ? rsqrtf((float)hd) : sm_scale) * 1.4426950408889634f;
     const int total_rows = cu_q ? kv_append : bsz * q_len;
-    return attn_impl(ctx, (cudaStream_t)stream, p, total_rows, q_len, false);
+    const AttnAppendArgs a = {(const half*)k, (const half*)v, (half*)k_cache, (half*)v_cache, nullptr, nullptr, nullptr, nullptr, block_table, cache_seqlens, cu_q,
+                              bsz, append, cu_q ? kv_append : bsz * append, nkv, pages, pages_per_seq, 0, 0};
+    return attn_impl(ctx, (cudaStream_t)stream, p, total_rows, q_len, false, write ? &a : nullptr);
 }
 
 extern "C" int exl3_bighead_attn_paged_q(exl3_ctx* ctx, exl3_stream stream, const void* q, const void* k,
@@ -593,13 +471,12 @@ extern "C" int exl3_bighead_attn_paged_q(exl3_ctx* ctx, exl3_stream stream, cons
     if (compand_a > 0.0f) return exl3_fail(ctx, EXL3_ERR_UNSUPPORTED, "attention: compand_a > 0 is not supported");
     if (bsz == 0 || q_len == 0) return EXL3_OK;
     const int append = cu_q ? q_len : kv_append;
-    if (append > 0 && !ctx->kv_appended) {
+    const bool write = append > 0 && !ctx->kv_appended;
+    if (write) {
         EXL3_REQUIRE(k && v, "attention: kv_append > 0 needs k and v");
-        rc = exl3_quant_cache_paged(ctx, stream, k, qk, sk, v, qv, sv, cache_seqlens, block_table, cu_q, bsz, append,
-                                    nkv * hd, pages, pages_per_seq, k_bits, v_bits, EXL3_PAGE, 0.0f, 1);
-        if (rc) return rc;
+        EXL3_REQUIRE(bsz <= 65535 && append <= 65535, "quant_cache_paged: bad shape");
     }
-    exl3_chain_scope chain(ctx, append > 0);
+    exl3_chain_scope chain(ctx, append > 0 && !write);
     AttnParams p;
     memset(&p, 0, sizeof(p));
     p.q = (const half*)q; p.o = (half*)o;
@@ -609,7 +486,9 @@ extern "C" int exl3_bighead_attn_paged_q(exl3_ctx* ctx, exl3_stream stream, cons
     p.causal = causal; p.k_bits = k_bits; p.v_bits = v_bits;
     p.scale_log2 = (sm_scale == 0.0f ? rsqrtf((float)hd) : sm_scale) * 1.4426950408889634f;
     const int total_rows = cu_q ? kv_append : bsz * q_len;
-    return attn_impl(ctx, (cudaStream_t)stream, p, total_rows, q_len, true);
+    const AttnAppendArgs a = {(const half*)k, (const half*)v, nullptr, nullptr, (uint32_t*)qk, (half*)sk, (uint32_t*)qv, (half*)sv, block_table, cache_seqlens, cu_q,
+                              bsz, append, cu_q ? kv_append : bsz * append, nkv, pages, pages_per_seq, k_bits, v_bits};
+    return attn_impl(ctx, (cudaStream_t)stream, p, total_rows, q_len, true, write ? &a : nullptr);
 }
 
 // Attention over plain tensors: q, o [bsz, q_len, nq, hd], k, v [bsz, kv_len, nkv, hd], no cache and no block table
@@ -641,7 +520,7 @@ extern "C" int exl3_bighead_attn(exl3_ctx* ctx, exl3_stream stream, const void* 
     // the work lists kept across the layers of a step belong to the paged batch: plan afresh
     const int keep = ctx->plan_keep;
     ctx->plan_keep = 0;
-    const int rc = attn_impl(ctx, (cudaStream_t)stream, p, bsz * q_len, q_len, false);
+    const int rc = attn_impl(ctx, (cudaStream_t)stream, p, bsz * q_len, q_len, false, nullptr);
     ctx->plan_keep = keep;
     return rc;
 }

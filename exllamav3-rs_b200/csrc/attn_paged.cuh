@@ -16,7 +16,12 @@ constexpr int AT_TK = 64;          // keys per shared-memory tile
 constexpr int AT_THREADS = 128;    // 4 warps
 constexpr int AT_STAGES = 2;        // K/V tile stages per CTA (3 stages leave room for 2 CTAs per SM instead of 3: measured 10 % slower)
 
-struct AttnItem { int b, rb, split, pad; };
+// One entry of the work list, with all that a kernel needs to begin: looked up one after the other (item, sequence, lengths, splits)
+// these were four dependent loads in front of every unit.
+struct __align__(16) AttnItem {
+    int b, rb, split, idx;             // sequence, row block, KV split; idx: number in plan order, which places its partial sums
+    int row_base, ql, total_k, splits;
+};
 
 struct AttnPlan {          // device-resident, written by attn_plan_kernel
     int n_items;
@@ -35,9 +40,8 @@ struct AttnParams {
     const int32_t* seqlens;        // [bsz]  tokens in the cache BEFORE this step's append (NULL: none, all keys are "appended")
     const int32_t* cu_q;           // [bsz+1] or NULL (then rows of sequence b = [b*q_len, (b+1)*q_len))
     const AttnPlan* plan;
-    const AttnItem* items;
-    const int* order;              // [n_items] item indices, longest first: the order in which CTAs / work units take them
-    const int* seq_base;           // [bsz] first item of sequence b
+    const AttnItem* items;         // [n_items] longest first: the order in which CTAs / work units take them
+    const int* seq_base;           // [bsz] first item (in plan order) of sequence b
     const int* seq_splits;         // [bsz]
     float* partial;                // [n_items][nkv][ROWS][D+2]
     int* status;                   // context status word (bounded waits)
@@ -129,13 +133,9 @@ __global__ void __launch_bounds__(AT_THREADS, (QB == 4 && WN == 4) ? AT_Q4_DECOD
         __syncthreads();
         const int unit = s_unit;
         if (unit >= n_units) break;
-        const int item_idx = p.order[unit / p.nkv], kvh = unit % p.nkv;
-        const AttnItem item = p.items[item_idx];
-        const int b = item.b;
-        const int row_base = p.cu_q ? p.cu_q[b] : b * p.q_len;
-        const int ql = p.cu_q ? p.cu_q[b + 1] - row_base : p.q_len;
-        const int total_k = (p.seqlens ? p.seqlens[b] : 0) + (p.cu_q ? ql : p.kv_append);
-        const int splits = p.seq_splits[b];
+        const AttnItem item = p.items[unit / p.nkv];
+        const int item_idx = item.idx, kvh = unit % p.nkv;
+        const int b = item.b, row_base = item.row_base, ql = item.ql, total_k = item.total_k, splits = item.splits;
         const int r0 = item.rb * ROWS;                       // first packed (query, head) row of this CTA
         // keys this row block can see at all (causal, bottom-right aligned)
         const int i_last = min(ql - 1, (r0 + ROWS - 1) / G);

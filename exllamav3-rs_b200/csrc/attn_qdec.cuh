@@ -201,13 +201,9 @@ attn_qdec_kernel(const __grid_constant__ CUtensorMap map_qk, const __grid_consta
         __syncthreads();
         const int unit = s_unit;
         if (unit >= n_units) break;
-        const int item_idx = p.order[unit / p.nkv], kvh = unit % p.nkv;
-        const AttnItem item = p.items[item_idx];
-        const int b = item.b;
-        const int row_base = p.cu_q ? p.cu_q[b] : b * p.q_len;
-        const int ql = p.cu_q ? p.cu_q[b + 1] - row_base : p.q_len;
-        const int total_k = p.seqlens[b] + (p.cu_q ? ql : p.kv_append);
-        const int splits = p.seq_splits[b];
+        const AttnItem item = p.items[unit / p.nkv];
+        const int item_idx = item.idx, kvh = unit % p.nkv;
+        const int b = item.b, row_base = item.row_base, ql = item.ql, total_k = item.total_k, splits = item.splits;
         const int r0 = item.rb * ROWS;
         const int i_last = min(ql - 1, (r0 + ROWS - 1) / G);
         const int vis_max = p.causal ? min(total_k, total_k - ql + i_last + 1) : total_k;

@@ -128,7 +128,6 @@ __global__ void __launch_bounds__(ATC_THREADS, 1) attn_tc_kernel(const __grid_co
 {
     // grid max_items * nkv: the CTAs of one item are neighbours in launch order, items come longest first
     if ((int)(blockIdx.x / p.nkv) >= p.plan->n_items) return;
-    const int item_idx = p.order[blockIdx.x / p.nkv];
     extern __shared__ uint8_t smem_unaligned[];
     // aligned to 1024 bytes by an offset from the array, not through an integer, so that the compiler still knows the
     // pointer is in shared memory (32-bit addresses, ld/st.shared) instead of falling back to generic accesses
@@ -146,12 +145,8 @@ __global__ void __launch_bounds__(ATC_THREADS, 1) attn_tc_kernel(const __grid_co
     const int kvh = blockIdx.x % p.nkv;
     const int G = p.nq / p.nkv;
     const int chunk = p.plan->chunk;
-    const AttnItem item = p.items[item_idx];
-    const int b = item.b;
-    const int row_base = p.cu_q ? p.cu_q[b] : b * p.q_len;
-    const int ql = p.cu_q ? p.cu_q[b + 1] - row_base : p.q_len;
-    const int total_k = p.seqlens[b] + (p.cu_q ? ql : p.kv_append);
-    const int splits = p.seq_splits[b];
+    const AttnItem item = p.items[blockIdx.x / p.nkv];
+    const int item_idx = item.idx, b = item.b, row_base = item.row_base, ql = item.ql, total_k = item.total_k, splits = item.splits;
     const int r0 = item.rb * ATC_CTA_ROWS;
     const int i_last = min(ql - 1, (r0 + ATC_CTA_ROWS - 1) / G);
     const int vis_max = p.causal ? min(total_k, total_k - ql + i_last + 1) : total_k;

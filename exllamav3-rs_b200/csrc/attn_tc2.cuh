@@ -56,9 +56,9 @@ __global__ void __launch_bounds__(a2_threads(H), 1) attn_tc2_kernel(const __grid
     static_assert(H == 2 || H == 4, "two or four softmax threads per row");
     constexpr int NSW = 4 * H;                     // softmax warps; warp NSW = TMA producer, NSW + 1 = MMA issuer and TMEM owner
     constexpr int KPT = A2_TN / H;                 // keys of a tile, and columns of O, per softmax thread
+    pdl_wait();
     // grid max_items * nkv: the CTAs of one item are neighbours in launch order, items come longest first
     if ((int)(blockIdx.x / p.nkv) >= p.plan->n_items) return;
-    const int item_idx = p.order[blockIdx.x / p.nkv];
     extern __shared__ uint8_t smem_unaligned[];
     uint8_t* smem = smem_unaligned + ((1024u - (smem_u32(smem_unaligned) & 1023u)) & 1023u);
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + A2_OFF_BAR);
@@ -77,12 +77,8 @@ __global__ void __launch_bounds__(a2_threads(H), 1) attn_tc2_kernel(const __grid
     const int kvh = blockIdx.x % p.nkv;
     const int G = p.nq / p.nkv;
     const int chunk = p.plan->chunk;
-    const AttnItem item = p.items[item_idx];
-    const int b = item.b;
-    const int row_base = p.cu_q ? p.cu_q[b] : b * p.q_len;
-    const int ql = p.cu_q ? p.cu_q[b + 1] - row_base : p.q_len;
-    const int total_k = p.seqlens[b] + (p.cu_q ? ql : p.kv_append);
-    const int splits = p.seq_splits[b];
+    const AttnItem item = p.items[blockIdx.x / p.nkv];
+    const int item_idx = item.idx, b = item.b, row_base = item.row_base, ql = item.ql, total_k = item.total_k, splits = item.splits;
     const int r0 = item.rb * A2_ROWS;
     const int i_last = min(ql - 1, (r0 + A2_ROWS - 1) / G);
     const int vis_max = p.causal ? min(total_k, total_k - ql + i_last + 1) : total_k;
@@ -124,6 +120,8 @@ __global__ void __launch_bounds__(a2_threads(H), 1) attn_tc2_kernel(const __grid
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    // the merge kernel may be set up from here on (in front of the allocation its successors could take the tensor memory)
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const uint32_t tmem_base = *tmem_slot;
     bool failed = false;
 

@@ -23,9 +23,8 @@ __device__ __forceinline__ bool locate_row(const int32_t* cu_q, int b, int s, in
     return true;
 }
 
-// The two appends are the first kernels of an attention call (exl3_launch_first): back to back the set-up of their blocks overlaps the
-// merge of the call before (us: 24 sequences over 8-bit pools 65.2 -> 64.2, 64 over 4-bit ones 143.4 -> 142.1, 4 x 256 rows 137.9 ->
-// 136.4).
+// The appends as operators of their own, and in front of an attention call of two passes (one pass: attn_front.cuh).  Launched as
+// first kernels (exl3_launch_first): the set-up of their blocks overlaps what is in front.
 __global__ void __launch_bounds__(256) kv_append_kernel(const uint4* __restrict__ k, const uint4* __restrict__ v,
                                                         uint4* __restrict__ kc, uint4* __restrict__ vc,
                                                         const int32_t* __restrict__ block_table,

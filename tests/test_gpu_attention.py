@@ -531,3 +531,54 @@ def test_attention_quantised_ragged(ctx, bits):
     assert exl3b200.lib().exl3_sync_side_stream(ctx.handle) == 0
     ctx.poll_status()
     assert np.array_equal(o.cpu().numpy().view(np.uint16), got.view(np.uint16))
+
+
+@pytest.mark.parametrize("bits,nkv,q_lens,ragged", [(0, 3, [1] * 33, False), (0, 8, [5] * 2, False), (3, 5, [2] * 40, False), (0, 1, [1, 0, 9, 0, 0, 2] * 12 + [0], True),
+                                                    (6, 3, [0, 1, 4] * 30, True), (0, 2, [1] * 1100, False), (0, 2, [1, 3, 0] * 400, True)])
+def test_attention_appends_and_plans_in_one_launch(ctx, bits, nkv, q_lens, ragged):
+    """A call's keys and values reach the pools as through the separate operator, byte for byte, and its output is that of a call
+    over pools that hold them already: more sequences than one search step or one block takes, sequences without rows, odd head
+    counts.  Three sequences are held against the oracle."""
+    from oracle import oracle as O
+    torch = _torch()
+    r = H.rng(2100 + bits + len(q_lens))
+    nq, bsz = 2 * nkv, len(q_lens)
+    ctx_lens = r.integers(0, 600, bsz).astype(np.int32)
+    bt, pages = H.make_paged(r, bsz, ctx_lens + np.asarray(q_lens), nkv, 128)
+    g = torch.Generator(device="cuda").manual_seed(bits)
+    half = lambda *s: torch.randn(*s, device="cuda", generator=g).to(torch.float16) * 0.5  # noqa: E731
+    rows = sum(q_lens)
+    lead = (rows,) if ragged else (bsz, q_lens[0])
+    q, k, v = half(*lead, nq, 128), half(*lead, nkv, 128), half(*lead, nkv, 128)
+    if bits == 0:
+        pools = [half(pages, 256, nkv, 128) for _ in range(2)]
+    else:
+        pools = [t for _ in range(2) for t in (torch.randint(-2 ** 31, 2 ** 31 - 1, (pages, 256, nkv * 4 * bits), dtype=torch.int32, device="cuda", generator=g),
+                                               half(pages, 256, nkv * 4).abs() * 0.1)]
+    cu_h = np.concatenate([[0], np.cumsum(q_lens)]).astype(np.int32)
+    cu = H.to_dev(cu_h) if ragged else None
+    sl, d_bt, ql = H.to_dev(ctx_lens), H.to_dev(bt), max(q_lens)
+
+    def call(p, kk, vv, lens):
+        o = torch.full((*lead, nq, 128), float("nan"), dtype=torch.float16, device="cuda")
+        if bits == 0:
+            ctx.bighead_attn_paged(q, kk, vv, p[0], p[1], d_bt, lens, o, cu_q=cu, max_q_len=ql)
+        else:
+            ctx.bighead_attn_paged_q(q, kk, vv, p[0], p[1], p[2], p[3], d_bt, lens, o, nkv, cu_q=cu, max_q_len=ql)
+        ctx.poll_status()
+        return o
+
+    one, two = [t.clone() for t in pools], [t.clone() for t in pools]
+    o = call(one, k, v, sl)
+    if bits == 0:
+        ctx.paged_kv_cache_update(k, v, two[0], two[1], d_bt, sl, cu_q=cu)
+    else:
+        ctx.quant_cache_paged(k, two[0], two[1], v, two[2], two[3], sl, d_bt, seq_len=ql, cu_q=cu)
+    assert all(torch.equal(a, b) for a, b in zip(one, two))
+    assert torch.isfinite(o).all()
+    if not ragged:                                     # the list alone: nothing to append, the rows count as cached
+        assert torch.equal(o, call(two, None, None, sl + ql))
+    for b in [i for i in (0, bsz // 2, bsz - 1) if q_lens[i]] if bits == 0 else []:
+        part = [x[cu_h[b]:cu_h[b + 1]][None] if ragged else x[b:b + 1] for x in (q, o)]
+        want = O.attn_paged(part[0].cpu().numpy(), one[0].cpu().numpy(), one[1].cpu().numpy(), bt[b:b + 1], ctx_lens[b:b + 1])
+        assert _close(part[1].cpu().numpy(), want, TOL_FP16) <= 1.0
