@@ -4,6 +4,7 @@
 #include "attn_tc.cuh"
 #include "attn_tc2.cuh"
 #include "attn_qdec.cuh"
+#include "attn_qt.cuh"
 
 namespace {
 
@@ -182,21 +183,20 @@ cudaError_t launch_attn_tc2(exl3_ctx* ctx, const AttnParams& p, int max_items, c
                        : exl3_launch(ctx, attn_tc2_kernel<2>, grid, a2_threads(2), A2_SMEM, st, maps[0], maps[1], p);
 }
 
-// decode-class kernel over 4-bit and 8-bit pools: tensor maps over the code planes ([tokens][nkv * 4 * bits] words, copied in
+// kernels over 4-bit and 8-bit pools: tensor maps over the code planes ([tokens][nkv * 4 * bits] words, copied in
 // the swizzle of a head's 64 or 128 bytes) and the scale planes ([tokens][nkv * 4] halves, copied in 16-byte pairs of heads)
-template <int B, int NB>
-cudaError_t launch_attn_qdec(exl3_ctx* ctx, const AttnParams& p, dim3 grid, cudaStream_t st)
+template <int B>
+cudaError_t quant_maps(const AttnParams& p, int tile_keys, CUtensorMap (&maps)[4])
 {
     EncodeTiledFn enc = attn_encode_tiled();
     if (!enc) return cudaErrorNotSupported;
-    CUtensorMap maps[4];
     const void* planes[4] = {p.qk, p.qv, p.sk, p.sv};
     const cuuint64_t tokens = (cuuint64_t)p.pages * EXL3_PAGE;
     for (int i = 0; i < 4; ++i) {
         const bool codes = i < 2;
         cuuint64_t dims[2] = {(cuuint64_t)p.nkv * (codes ? 4 * B : 4), tokens};
         cuuint64_t strides[1] = {(cuuint64_t)p.nkv * (codes ? 16 * B : 8)};
-        cuuint32_t box[2] = {codes ? 4u * B : 8u, (cuuint32_t)QD_TK};
+        cuuint32_t box[2] = {codes ? 4u * B : 8u, (cuuint32_t)tile_keys};
         cuuint32_t estr[2] = {1, 1};
         if (enc(&maps[i], codes ? CU_TENSOR_MAP_DATA_TYPE_UINT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(planes[i]),
                 dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
@@ -204,27 +204,50 @@ cudaError_t launch_attn_qdec(exl3_ctx* ctx, const AttnParams& p, dim3 grid, cuda
                 CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
             return cudaErrorInvalidValue;
     }
-    constexpr int bytes = QdSmem<B, NB>::BYTES;
-    auto kern = attn_qdec_kernel<B, NB>;
-    static bool configured[64] = {};
+    return cudaSuccess;
+}
+
+// launch of a kernel over quantised pools with `bytes` of dynamic shared memory
+template <int B, typename Kern>
+cudaError_t launch_quant(exl3_ctx* ctx, Kern kern, bool (&configured)[64], int bytes, int threads, int tile_keys, const AttnParams& p, dim3 grid, cudaStream_t st)
+{
+    CUtensorMap maps[4];
+    cudaError_t e = quant_maps<B>(p, tile_keys, maps);
+    if (e != cudaSuccess) return e;
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64 || !configured[dev]) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
         if (e != cudaSuccess) return e;
         if (dev >= 0 && dev < 64) configured[dev] = true;
     }
-    return exl3_launch(ctx, kern, grid, QD_THREADS, bytes, st, maps[0], maps[1], maps[2], maps[3], p);
+    return exl3_launch(ctx, kern, grid, threads, bytes, st, maps[0], maps[1], maps[2], maps[3], p);
+}
+template <int B, int NB>
+cudaError_t launch_attn_qdec(exl3_ctx* ctx, const AttnParams& p, dim3 grid, cudaStream_t st)
+{
+    static bool configured[64] = {};
+    return launch_quant<B>(ctx, attn_qdec_kernel<B, NB>, configured, QdSmem<B, NB>::BYTES, QD_THREADS, QD_TK, p, grid, st);
+}
+template <int B>
+cudaError_t launch_attn_qt(exl3_ctx* ctx, const AttnParams& p, dim3 grid, cudaStream_t st)
+{
+    static bool configured[64] = {};
+    return launch_quant<B>(ctx, attn_qt_kernel<B>, configured, QtSmem<B>::BYTES, QT_THREADS, QT_TK, p, grid, st);
 }
 
 bool qdec_kernel_applies(const AttnParams& p, bool quant);
 
+// Which kernels a pass runs: those for few packed rows, those for more, or (4-bit and 8-bit pools) the tcgen05 kernel over codes.
+enum AttnClass { ATTN_FEW, ATTN_MANY, ATTN_CODES };
+
 // One pass = plan + attention + combine over the sequences whose packed row count lies in (rows_lo, rows_hi].
 int attn_pass(exl3_ctx* ctx, cudaStream_t st, AttnParams p, int total_rows, int max_rows, int rows_lo, int rows_hi,
-              bool decode_shape, bool quant, size_t* ws_off, const AttnAppendArgs* append, bool had = false)
+              AttnClass kind, bool quant, size_t* ws_off, const AttnAppendArgs* append, bool had = false)
 {
     const int D = 128;
     const int G = p.nq / p.nkv;
+    const bool decode_shape = kind == ATTN_FEW, use_qt = kind == ATTN_CODES;
     const bool q4 = quant && p.k_bits == 4 && p.v_bits == 4;       // the common cache format has its own, smaller staging
     // long class on fp16 pools: tcgen05 kernel (256-row items) unless the context was switched to the mma.sync kernels
     // (its row maximum is taken on the raw scores, which needs a positive scale)
@@ -237,12 +260,13 @@ int attn_pass(exl3_ctx* ctx, cudaStream_t st, AttnParams p, int total_rows, int 
     // wide = two heads, so the kv head count must be even and the planes 16-byte aligned).  Row blocks of 8 where no
     // sequence has more rows (a decode batch), else of 16, whose second half costs nothing where it is empty.
     const bool use_qdec = decode_shape && qdec_kernel_applies(p, quant);
-    const int rows_per_cta = decode_shape ? (use_qdec && max_rows <= 8 ? 8 : 16) : (use_tc ? (tc_256 ? ATC_CTA_ROWS : A2_ROWS) : 64);
+    const int rows_per_cta = use_qt ? QT_ROWS : decode_shape ? (use_qdec && max_rows <= 8 ? 8 : 16) : (use_tc ? (tc_256 ? ATC_CTA_ROWS : A2_ROWS) : 64);
     const int rb_max = (max_rows + rows_per_cta - 1) / rows_per_cta;
     // resident CTAs per SM over all kv heads: about 3 for the mma.sync kernels, 1 for the tcgen05 kernel (all of TMEM)
     // (rounded down: one CTA more than fits would run alone in a second wave after all the others have finished)
     int per_sm = 1;
-    if (use_qdec) per_sm = qd_ctas(p.k_bits, rows_per_cta / 8);
+    if (use_qt) per_sm = 2;
+    else if (use_qdec) per_sm = qd_ctas(p.k_bits, rows_per_cta / 8);
     else if (!use_tc) {
         // CTAs of the mma.sync kernel that fit on an SM (bounded by shared memory: stages x 34.8 KB for fp16 pools)
         const size_t smem = quant ? (q4 ? AttnSmem<128, 4>::BYTES : AttnSmem<128, 8>::BYTES) : AttnSmem<128, 0>::BYTES;
@@ -259,7 +283,7 @@ int attn_pass(exl3_ctx* ctx, cudaStream_t st, AttnParams p, int total_rows, int 
     // quantised pools, whose units start with the rotation of their queries (24 sequences, contexts 512 .. 16384, 40 / 8
     // heads, one and two items: 4 bits, 5 rows 68 and 72 us, 40 rows 188 and 193; 8 bits 68 and 75, 188 and 196).
     static const int dec_items = getenv("EXL3_TUNE_DEC_ITEMS") ? atoi(getenv("EXL3_TUNE_DEC_ITEMS")) : 0;
-    const int target_items = grid_x * (use_tc ? (tc_items ? tc_items : 2) : (dec_items ? dec_items : (use_qdec ? 1 : 2)));
+    const int target_items = grid_x * (use_tc ? (tc_items ? tc_items : 2) : (dec_items ? dec_items : (use_qdec || use_qt ? 1 : 2)));
     // items <= target + sum of row blocks (every (sequence, row block) rounds its split count up once); the row blocks are
     // bounded by bsz * rb_max and, usually much tighter for ragged batches, by total_rows * G / rows_per_cta + bsz
     const long long rb_sum = std::min((long long)p.bsz * rb_max, ((long long)total_rows * G + rows_per_cta - 1) / rows_per_cta + p.bsz);
@@ -294,7 +318,7 @@ int attn_pass(exl3_ctx* ctx, cudaStream_t st, AttnParams p, int total_rows, int 
     static const bool no_lpt = getenv("EXL3_TUNE_NO_LPT") != nullptr;
     if (!(keep && ctx->plan_valid[cls])) {
         const AttnPlanArgs a = {p.seqlens, p.cu_q, plan, items, seq_base, seq_splits, ctx->status, p.bsz, p.q_len, p.kv_append, G, rows_per_cta, rows_lo, rows_hi,
-                                use_tc ? ATC_TN : AT_TK, target_items, max_items, no_lpt ? -1 : (p.causal ? 1 : 0), (use_tc && !tc_items) ? grid_x : 0};
+                                use_tc ? ATC_TN : use_qt ? QT_TK : AT_TK, target_items, max_items, no_lpt ? -1 : (p.causal ? 1 : 0), (use_tc && !tc_items) ? grid_x : 0};
         if (append) {
             const long long warps = (long long)append->rows * (append->k_bits ? append->nkv : 1);
             exl3_launch_first(ctx, attn_front_kernel, 1 + (unsigned)((warps + AP_THREADS / 32 - 1) / (AP_THREADS / 32)), AP_THREADS, 0, st, a, *append);
@@ -307,6 +331,7 @@ int attn_pass(exl3_ctx* ctx, cudaStream_t st, AttnParams p, int total_rows, int 
     dim3 grid(grid_x, p.nkv);
     cudaError_t e;
     if (use_tc) e = tc_256 ? launch_attn_tc(ctx, p, max_items, st) : launch_attn_tc2(ctx, p, max_items, st);
+    else if (use_qt) e = q4 ? launch_attn_qt<4>(ctx, p, grid, st) : launch_attn_qt<8>(ctx, p, grid, st);
     else if (use_qdec)
         e = q4 ? (rows_per_cta == 8 ? launch_attn_qdec<4, 1>(ctx, p, grid, st) : launch_attn_qdec<4, 2>(ctx, p, grid, st))
                : (rows_per_cta == 8 ? launch_attn_qdec<8, 1>(ctx, p, grid, st) : launch_attn_qdec<8, 2>(ctx, p, grid, st));
@@ -346,7 +371,6 @@ int attn_impl(exl3_ctx* ctx, cudaStream_t st, AttnParams p, int total_rows, int 
 {
     const int G = p.nq / p.nkv;
     const int max_rows = max_q_len * G;
-    size_t off = 0;
     // Decode class = sequences with at most 16 packed rows.  Over 4-bit and 8-bit pools it also takes up to 48 rows
     // (speculative verify: 8 query rows x 5 heads) as row blocks of 16 that each walk the codes again: the kernel that
     // builds its operands from the codes is that much cheaper per key than the generic one.  Against the generic kernel, us,
@@ -359,34 +383,57 @@ int attn_impl(exl3_ctx* ctx, cudaStream_t st, AttnParams p, int total_rows, int 
     // (Sending the decode rows of a ragged fp16 batch through the tcgen05 kernel as well, as items of 128 rows with 5 in
     // use, was measured on the benchmark step: the attention stage takes the same 28.0 ms of the step's 83.)
     const int dec_rows = qdec_kernel_applies(p, quant) ? 48 : 16;
-    // (The transform behind the attention is left to its own launch where two passes share the rows, and where the scratch does
-    // not hold it beside the partials; attn_pass refuses before it launches anything.)
-    if (max_rows <= dec_rows || !p.cu_q) {
-        const bool dec = max_rows <= dec_rows;
-        // The list and the append are one launch unless the list is another layer's already.
-        const bool one = append && !ctx->plan_keep;
-        exl3_chain_scope chain(ctx, append && !one);
-        if (append && !one) {
-            const int rc = attn_append(ctx, st, *append);
-            if (rc != EXL3_OK) return rc;
-        }
+    // The tcgen05 kernel over codes unpacks them once for 40 rows; its blocks cost the same however few of those they hold, and a unit
+    // some 10 us before and behind its tiles.  So, us, the other kernels and it (40 / 8 heads unless said):
+    //  * sequences of 33 to 48 rows at 4 bits, where there is work for all SMs: 4 of 40 rows, contexts 1024 .. 32768, 64 -> 47; 32 of
+    //    them, 128 .. 4000, 77 -> 64; 12 of 35 rows, 512 .. 8192, 71 -> 55; but 4 of 40 rows, 256 .. 8000, 33 and 33, one over 4000
+    //    keys 26 to 33 and 30 to 33.  The pages of the block table bound the work from above.  At 8 bits, where the ring of codes
+    //    has one slot: 67 and 67.  Up to 32 rows two blocks of 16 of the other kernel are as good (24 of 25 rows 94 and 94).
+    //  * longer ones: 3 of 100 rows, 500 .. 4000, 4 bits 106 -> 98, 8 bits 140 -> 134; one of 128 over 4000 keys 102 -> 82, 124 ->
+    //    111; 16 / 8 heads 55 -> 42, 71 -> 54; behind at 8 bits with 1024 packed rows (110 and 120) and on 3 of 60 rows at 16 / 8
+    //    heads (41 and 46).
+    //  * a ragged batch of both kinds in one pass instead of two, unless it has many sequences of a row: 28 and 2 of 64 rows, 4 bits
+    //    112 -> 93, 8 bits 149 -> 139; 4 and one of 24 rows 45 -> 26; 64 and one of 50 rows 56 and 62, 63 and 82.
+    const bool codes = qdec_kernel_applies(p, quant), long_codes = codes && max_rows > dec_rows && (p.k_bits == 4 || max_rows <= 800);
+    const int n_long = max_q_len > 1 ? (int)std::max(0LL, ((long long)total_rows - p.bsz + max_q_len - 2) / (max_q_len - 1)) : 0;     // at least so many have more than a row
+    const bool codes_alone = long_codes ? !p.cu_q || p.bsz - n_long <= 40
+                                        : codes && p.k_bits == 4 && max_rows > 32 && max_rows <= dec_rows && (long long)p.bsz * p.pps >= 200;
+    // One pass.  (The transform behind the attention is left to its own launch where the scratch does not hold it beside the
+    // partials; attn_pass refuses before it launches anything.)  The list and the append are one launch unless the list is another
+    // layer's already.
+    const bool one = append && !ctx->plan_keep;
+    auto single = [&](AttnClass kind, int rows_hi) -> int {
         int rc = EXL3_ERR_WORKSPACE;
         if (ctx->had_out) {
-            off = ctx->had_bytes;
-            rc = attn_pass(ctx, st, p, total_rows, max_rows, 0, dec ? dec_rows : 1 << 30, dec, quant, &off, one ? append : nullptr, true);
+            size_t off = ctx->had_bytes;
+            rc = attn_pass(ctx, st, p, total_rows, max_rows, 0, rows_hi, kind, quant, &off, one ? append : nullptr, true);
             ctx->had_done = rc == EXL3_OK;
-            off = 0;
         }
-        if (rc == EXL3_ERR_WORKSPACE) rc = attn_pass(ctx, st, p, total_rows, max_rows, 0, dec ? dec_rows : 1 << 30, dec, quant, &off, one ? append : nullptr);
-        if (rc == EXL3_ERR_WORKSPACE && one) {             // refused before anything was launched; the keys and values are appended all the same
+        size_t off = 0;
+        if (rc == EXL3_ERR_WORKSPACE) rc = attn_pass(ctx, st, p, total_rows, max_rows, 0, rows_hi, kind, quant, &off, one ? append : nullptr);
+        return rc;
+    };
+    const bool general_single = max_rows <= dec_rows || !p.cu_q;
+    exl3_chain_scope chain(ctx, append && !(one && (codes_alone || general_single)));
+    if (append && !(one && (codes_alone || general_single))) {
+        const int rc = attn_append(ctx, st, *append);
+        if (rc != EXL3_OK) return rc;
+        append = nullptr;
+    }
+    if (codes_alone) {
+        const int rc = single(ATTN_CODES, 1 << 30);
+        if (rc != EXL3_ERR_WORKSPACE) return rc;
+    }
+    if (general_single) {
+        const int rc = single(max_rows <= dec_rows ? ATTN_FEW : ATTN_MANY, max_rows <= dec_rows ? dec_rows : 1 << 30);
+        if (rc == EXL3_ERR_WORKSPACE && append) {          // nothing has been launched; the keys and values are appended all the same
             const int rc2 = attn_append(ctx, st, *append);
             if (rc2 != EXL3_OK) return rc2;
             return exl3_fail(ctx, rc, "attention: context scratch too small for the split-KV partials");
         }
         return rc;
     }
-    exl3_chain_scope chain(ctx, append != nullptr);
-    if (append) {
+    if (append) {                                          // the codes' kernel alone has been refused
         const int rc = attn_append(ctx, st, *append);
         if (rc != EXL3_OK) return rc;
     }
@@ -399,9 +446,14 @@ int attn_impl(exl3_ctx* ctx, cudaStream_t st, AttnParams p, int total_rows, int 
     if (cudaEventRecord(ctx->ev_fork, st) != cudaSuccess || cudaStreamWaitEvent(ctx->aux_stream, ctx->ev_fork, 0) != cudaSuccess)
         return exl3_fail(ctx, EXL3_ERR_CUDA, "attention: stream fork failed");
     ctx->chain_break = 1;
-    int rc = attn_pass(ctx, ctx->aux_stream, p, total_rows, dec_rows, 0, dec_rows, true, quant, &off, nullptr);
+    size_t off = 0;
+    int rc = attn_pass(ctx, ctx->aux_stream, p, total_rows, dec_rows, 0, dec_rows, ATTN_FEW, quant, &off, nullptr);
     ctx->chain_break = 1;
-    int rc2 = rc == EXL3_OK ? attn_pass(ctx, st, p, total_rows, max_rows, dec_rows, 1 << 30, false, quant, &off, nullptr) : rc;
+    int rc2 = rc;
+    if (rc == EXL3_OK) {
+        rc2 = long_codes && !codes_alone ? attn_pass(ctx, st, p, total_rows, max_rows, dec_rows, 1 << 30, ATTN_CODES, quant, &off, nullptr) : EXL3_ERR_WORKSPACE;
+        if (rc2 == EXL3_ERR_WORKSPACE) rc2 = attn_pass(ctx, st, p, total_rows, max_rows, dec_rows, 1 << 30, ATTN_MANY, quant, &off, nullptr);
+    }
     ctx->chain_break = 1;
     // always join, also after an error, so that a capture in progress stays well-formed
     if (cudaEventRecord(ctx->ev_join, ctx->aux_stream) != cudaSuccess || cudaStreamWaitEvent(st, ctx->ev_join, 0) != cudaSuccess)

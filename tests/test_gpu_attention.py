@@ -582,3 +582,38 @@ def test_attention_appends_and_plans_in_one_launch(ctx, bits, nkv, q_lens, ragge
         part = [x[cu_h[b]:cu_h[b + 1]][None] if ragged else x[b:b + 1] for x in (q, o)]
         want = O.attn_paged(part[0].cpu().numpy(), one[0].cpu().numpy(), one[1].cpu().numpy(), bt[b:b + 1], ctx_lens[b:b + 1])
         assert _close(part[1].cpu().numpy(), want, TOL_FP16) <= 1.0
+
+
+@pytest.mark.parametrize("bits", [4, 8])
+@pytest.mark.parametrize("q_len,nq,nkv,v_mul", [(11, 24, 8, 1), (8, 40, 8, 1), (41, 2, 2, 1), (9, 40, 8, 2e4), (3, 32, 2, 1), (7, 14, 2, 1), (16, 10, 2, 2e4),
+                                               (81, 2, 2, 1), (24, 10, 2, 1), (50, 32, 2, 1)])
+def test_attention_over_codes_edges(ctx, bits, q_len, nq, nkv, v_mul):
+    """The tcgen05 kernel over 4- and 8-bit pools: 33 to 800 packed rows around its blocks of 40 and the 8, 16 and 24 rows that its
+    threads take, contexts around its tiles of 128 keys and the pages of 256, scales that are not numbers behind every sequence,
+    values whose product with a code leaves fp16; causal and not.  Bar: the repository's for quantised pools."""
+    from oracle import oracle as O
+    torch = _torch()
+    lens = [0, 1, 85, 126, 127, 128, 129, 255, 256, 257, 3000]
+    c = _make_case(8200 + bits + q_len, lens, q_len, nq, nkv)
+    c["block_table"] = np.pad(c["block_table"], ((0, 0), (0, 8)))          # a table wide enough for the kernel to be chosen
+    for x in ("v", "vc"):                              # deviation 1e4: a group's scale, its largest rotated value, is an fp16 number up to 6.5 of them
+        c[x] = (c[x].astype(np.float32) * v_mul).astype(np.float16)
+    pools = _quant_pools(c, bits)
+    assert all(np.isfinite(pools[i]).all() for i in (1, 3))
+    live = np.zeros((c["kc"].shape[0], 256), bool)
+    for b, n in enumerate(lens):
+        for pos in range(n + q_len):
+            live[c["block_table"][b, pos // 256], pos % 256] = True
+    for i in (1, 3):
+        pools[i][~live] = np.nan
+    for causal in (True, False):
+        o = torch.full(c["q"].shape, float("nan"), dtype=torch.float16, device="cuda")
+        ctx.bighead_attn_paged_q(H.to_dev(c["q"]), H.to_dev(c["k"]), H.to_dev(c["v"]), *_to_dev(pools), H.to_dev(c["block_table"]),
+                                 H.to_dev(c["seqlens"]), o, nkv, causal=causal)
+        ctx.poll_status()
+        got, now = o.cpu().numpy(), [x.copy() for x in pools]
+        O.quant_cache_paged(c["k"], now[0], now[1], c["v"], now[2], now[3], c["seqlens"], c["block_table"], bits, bits)
+        want = O.attn_paged(c["q"], None, None, c["block_table"], c["seqlens"], nkv=nkv, quant=(*now, bits), causal=causal)
+        assert np.isfinite(got).all()
+        for b in range(len(lens)):                     # each sequence against its own size
+            assert _close(got[b], want[b], TOL_QUANT) <= 1.0, lens[b]
