@@ -2,6 +2,7 @@
 // RMSNorm), SiLU*mul, add, argmax, embedding gather.  Each op states the reference kernel whose arithmetic it follows.
 #include "common.cuh"
 #include "kvquant.cuh"
+#include "had_mma.cuh"
 
 namespace {
 
@@ -216,6 +217,93 @@ __global__ void __launch_bounds__(1024) rms_norm_had_kernel(const TI* __restrict
     }
 }
 
+// The same for many rows, with the transforms on the tensor core (had_mma.cuh): a lane's twenty shuffles per 128-block and tensor are
+// what bound the kernel above (1052 rows of 5120, in a step, two and three tensors in turn: 27.0 us,
+// here 20.5; their 75 and 86 MB of loads and stores are 12).  A warp takes two pairs of blocks, whose loads are all in flight before the first is used.
+constexpr int RW_PAIRS = 2;
+template <typename TI, bool RES_IN>
+__global__ void __launch_bounds__(1024) rms_norm_had_wide_kernel(const TI* __restrict__ x, const half* __restrict__ w, float* __restrict__ r,
+                                                                 float eps, float cbias, float cscale, int dim, const exl3_pre_act pre)
+{
+    pdl_enter();
+    __shared__ float sh[32];
+    __shared__ __align__(16) uint8_t stage[32][512];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, pairs = dim >> 8;
+    const size_t row = (size_t)blockIdx.x * dim;
+    float v[RW_PAIRS][8];
+    float sum = 0.0f;
+    #pragma unroll
+    for (int u = 0; u < RW_PAIRS; ++u) {
+        const int pair = warp * RW_PAIRS + u;
+        if (pair >= pairs) break;                                  // warp-uniform
+        const size_t at = row + pair * 256 + lane * 8;
+        if constexpr (sizeof(TI) == 2) {
+            const uint4 raw = *reinterpret_cast<const uint4*>(x + at);
+            const half2* h = reinterpret_cast<const half2*>(&raw);
+            #pragma unroll
+            for (int e = 0; e < 4; ++e) { v[u][2 * e] = __low2float(h[e]); v[u][2 * e + 1] = __high2float(h[e]); }
+        } else {
+            #pragma unroll
+            for (int e = 0; e < 8; e += 4) *reinterpret_cast<float4*>(&v[u][e]) = *reinterpret_cast<const float4*>(x + at + e);
+        }
+    }
+    if constexpr (RES_IN) {
+        float4 q[RW_PAIRS][2];
+        #pragma unroll
+        for (int u = 0; u < RW_PAIRS; ++u)
+            if (warp * RW_PAIRS + u < pairs) {
+                const float4* src = reinterpret_cast<const float4*>(r + row + (warp * RW_PAIRS + u) * 256 + lane * 8);
+                q[u][0] = src[0]; q[u][1] = src[1];
+            }
+        #pragma unroll
+        for (int u = 0; u < RW_PAIRS; ++u)
+            if (warp * RW_PAIRS + u < pairs) {
+                float4* dst = reinterpret_cast<float4*>(r + row + (warp * RW_PAIRS + u) * 256 + lane * 8);
+                #pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    v[u][4 * e] += q[u][e].x; v[u][4 * e + 1] += q[u][e].y; v[u][4 * e + 2] += q[u][e].z; v[u][4 * e + 3] += q[u][e].w;
+                    dst[e] = make_float4(v[u][4 * e], v[u][4 * e + 1], v[u][4 * e + 2], v[u][4 * e + 3]);
+                }
+            }
+    }
+    #pragma unroll
+    for (int u = 0; u < RW_PAIRS; ++u)
+        if (warp * RW_PAIRS + u < pairs) {
+            #pragma unroll
+            for (int e = 0; e < 8; ++e) sum = fmaf(v[u][e], v[u][e], sum);
+        }
+    sum = block_sum(sum, sh);
+    const float rmf = rsqrtf(sum / (float)dim + eps) * cscale;
+    const exl3::HadMma had(lane);
+    #pragma unroll
+    for (int u = 0; u < RW_PAIRS; ++u) {
+        const int pair = warp * RW_PAIRS + u;
+        if (pair >= pairs) break;
+        const int col = pair * 256 + lane * 8;
+        uint4 h;
+        half2* hh = reinterpret_cast<half2*>(&h);
+        if (w) {
+            const uint4 raw = *reinterpret_cast<const uint4*>(w + col);
+            const half2* wh = reinterpret_cast<const half2*>(&raw);
+            #pragma unroll
+            for (int e = 0; e < 4; ++e)
+                hh[e] = __floats2half2_rn(v[u][2 * e] * (__low2float(wh[e]) + cbias) * rmf, v[u][2 * e + 1] * (__high2float(wh[e]) + cbias) * rmf);
+        } else {
+            #pragma unroll
+            for (int e = 0; e < 4; ++e) hh[e] = __floats2half2_rn(v[u][2 * e] * rmf, v[u][2 * e + 1] * rmf);
+        }
+        #pragma unroll
+        for (int sgm = 0; sgm < 3; ++sgm)
+            if (sgm < pre.nseg) {
+                uint2 o[2];
+                had(exl3::had_signed8(h, *reinterpret_cast<const uint4*>(pre.suh[sgm] + col)), stage[warp], lane, o);
+                half* dst = pre.a_had[sgm] + row + pair * 256 + exl3::HadMma::offset(lane);
+                *reinterpret_cast<uint2*>(dst) = o[0];
+                *reinterpret_cast<uint2*>(dst + 128) = o[1];
+            }
+    }
+}
+
 // ---------------------------------------------------------------------------------------------------- RoPE
 // One warp per (row, head); lane holds elements lane + 32*i.  Arithmetic follows kernels/rope.cu:55-255: optional
 // RMSNorm (value rounded to fp16, weight + bias in fp16, fp16 product), then the rotation in fp32 with __sinf/__cosf of
@@ -353,39 +441,59 @@ __global__ void __launch_bounds__(256) silu_mul_tail_kernel(const half* x, const
     z[i] = __hmul(__hmul(a, r), y[i]);
 }
 
-// silu_mul_kernel whose result goes straight through the input transform of the EXL3 tensor that reads it (down_proj):
-// one warp per 128-block of a row, lane = 4 consecutive elements.
-// U blocks per warp, whose loads are all in flight before the first is used: four where there are many, one where a block is a
-// few microseconds of latency.
-template <int U>
+// silu_mul_kernel whose result goes straight through the input transform of the EXL3 tensor that reads it (down_proj).
+__device__ __forceinline__ half2 silu_mul2(half2 a, half2 b)
+{
+    return __hmul2(__hmul2(a, h2rcp(__hadd2(__float2half2_rn(1.0f), h2exp(__hneg2(a))))), b);
+}
+// One warp per 128-block of a row, lane = 4 consecutive elements: few rows, and rows with an odd number of blocks.
 __global__ void __launch_bounds__(256) silu_mul_had_kernel(const half* __restrict__ x, const half* __restrict__ y,
                                                            const half* __restrict__ suh, half* __restrict__ a_had, long long blocks, int bpr)
 {
     pdl_enter();
     const int lane = threadIdx.x & 31;
-    const long long blk0 = ((long long)blockIdx.x * 8 + (threadIdx.x >> 5)) * U;
-    if (blk0 >= blocks) return;
-    uint2 xr[U], yr[U];
+    const long long blk = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (blk >= blocks) return;
+    const uint2 xr = reinterpret_cast<const uint2*>(x + blk * 128)[lane], yr = reinterpret_cast<const uint2*>(y + blk * 128)[lane];
+    half2 z[2];
     #pragma unroll
-    for (int u = 0; u < U; ++u) {
-        const long long blk = blk0 + u < blocks ? blk0 + u : blocks - 1;         // the tail repeats the last block
-        xr[u] = reinterpret_cast<const uint2*>(x + blk * 128)[lane];
-        yr[u] = reinterpret_cast<const uint2*>(y + blk * 128)[lane];
+    for (int j = 0; j < 2; ++j) z[j] = silu_mul2(*reinterpret_cast<const half2*>(&xr.x + j), *reinterpret_cast<const half2*>(&yr.x + j));
+    const int col = (int)(blk % bpr) * 32 + lane;               // uint2 index inside the sign vector
+    reinterpret_cast<uint2*>(a_had + blk * 128)[lane] = had128_signed_lane(z[0], z[1], reinterpret_cast<const uint2*>(suh)[col], lane);
+}
+// Many rows: pairs of blocks with the transform on the tensor core (had_mma.cuh), two per warp whose loads are all in flight before the
+// first is used (1052 rows of 17408, in a step: 31.4 us with four blocks per warp and shuffles, 24.3 here; 110 MB of loads and stores
+// are 17).
+constexpr int SW_PAIRS = 2;
+__global__ void __launch_bounds__(256) silu_mul_had_wide_kernel(const half* __restrict__ x, const half* __restrict__ y,
+                                                                const half* __restrict__ suh, half* __restrict__ a_had, long long pairs, int ppr)
+{
+    pdl_enter();
+    __shared__ __align__(16) uint8_t stage[8][512];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const long long pair0 = ((long long)blockIdx.x * 8 + warp) * SW_PAIRS;
+    if (pair0 >= pairs) return;
+    uint4 xr[SW_PAIRS], yr[SW_PAIRS];
+    #pragma unroll
+    for (int u = 0; u < SW_PAIRS; ++u) {
+        const long long pair = pair0 + u < pairs ? pair0 + u : pairs - 1;        // the tail repeats the last pair
+        xr[u] = reinterpret_cast<const uint4*>(x + pair * 256)[lane];
+        yr[u] = reinterpret_cast<const uint4*>(y + pair * 256)[lane];
     }
-    const half2 one = __float2half2_rn(1.0f);
+    const exl3::HadMma had(lane);
     #pragma unroll
-    for (int u = 0; u < U; ++u) {
-        const long long blk = blk0 + u;
-        if (blk >= blocks) break;                                                // warp-uniform
-        half2 z[2];
+    for (int u = 0; u < SW_PAIRS; ++u) {
+        const long long pair = pair0 + u;
+        if (pair >= pairs) break;                                                // warp-uniform
+        half2* a = reinterpret_cast<half2*>(&xr[u]);
+        const half2* b = reinterpret_cast<const half2*>(&yr[u]);
         #pragma unroll
-        for (int j = 0; j < 2; ++j) {
-            const half2 a = *reinterpret_cast<const half2*>(&xr[u].x + j), b = *reinterpret_cast<const half2*>(&yr[u].x + j);
-            const half2 rr = h2rcp(__hadd2(one, h2exp(__hneg2(a))));
-            z[j] = __hmul2(__hmul2(a, rr), b);
-        }
-        const int col = (int)(blk % bpr) * 32 + lane;           // uint2 index inside the sign vector
-        reinterpret_cast<uint2*>(a_had + blk * 128)[lane] = had128_signed_lane(z[0], z[1], reinterpret_cast<const uint2*>(suh)[col], lane);
+        for (int e = 0; e < 4; ++e) a[e] = silu_mul2(a[e], b[e]);
+        uint2 o[2];
+        had(exl3::had_signed8(xr[u], reinterpret_cast<const uint4*>(suh + (pair % ppr) * 256)[lane]), stage[warp], lane, o);
+        half* dst = a_had + pair * 256 + exl3::HadMma::offset(lane);
+        *reinterpret_cast<uint2*>(dst) = o[0];
+        *reinterpret_cast<uint2*>(dst + 128) = o[1];
     }
 }
 
@@ -667,17 +775,20 @@ int exl3_rms_norm_pre(exl3_ctx* ctx, exl3_stream stream, const void* x, int x_fp
     EXL3_REQUIRE(aligned16(x) && aligned16(w) && aligned16(r), "rms_norm (fused transform): pointers must be 16-byte aligned");
     if (rows == 0) return EXL3_OK;
     const int cols = dim / 4;
-    int threads = cols <= 2048 ? 256 : 1024;
-    if (cols < 256) threads = ((cols + 31) / 32) * 32;
-    if (rows < 128 && cols > 256) threads = cols < 1024 ? ((cols + 31) / 32) * 32 : 1024;       // few rows: a block or two per warp
     cudaStream_t st = (cudaStream_t)stream;
     const half* wp = (const half*)w;
-    if (x_fp32) {
-        if (r) exl3_launch(ctx, rms_norm_had_kernel<float, true>, rows, threads, 0, st, (const float*)x, wp, r, eps, cbias, cscale, dim, *pre);
-        else   exl3_launch(ctx, rms_norm_had_kernel<float, false>, rows, threads, 0, st, (const float*)x, wp, r, eps, cbias, cscale, dim, *pre);
-    } else {
-        if (r) exl3_launch(ctx, rms_norm_had_kernel<half, true>, rows, threads, 0, st, (const half*)x, wp, r, eps, cbias, cscale, dim, *pre);
-        else   exl3_launch(ctx, rms_norm_had_kernel<half, false>, rows, threads, 0, st, (const half*)x, wp, r, eps, cbias, cscale, dim, *pre);
+    auto launch = [&](auto half_res, auto half_plain, auto float_res, auto float_plain, int threads) {
+        if (x_fp32) exl3_launch(ctx, r ? float_res : float_plain, rows, threads, 0, st, (const float*)x, wp, r, eps, cbias, cscale, dim, *pre);
+        else        exl3_launch(ctx, r ? half_res : half_plain, rows, threads, 0, st, (const half*)x, wp, r, eps, cbias, cscale, dim, *pre);
+    };
+    if (rows >= 128 && dim % 256 == 0 && dim <= 32 * RW_PAIRS * 256)
+        launch(rms_norm_had_wide_kernel<half, true>, rms_norm_had_wide_kernel<half, false>, rms_norm_had_wide_kernel<float, true>, rms_norm_had_wide_kernel<float, false>,
+               (dim / 256 + RW_PAIRS - 1) / RW_PAIRS * 32);
+    else {
+        int threads = cols <= 2048 ? 256 : 1024;
+        if (cols < 256) threads = ((cols + 31) / 32) * 32;
+        if (rows < 128 && cols > 256) threads = cols < 1024 ? ((cols + 31) / 32) * 32 : 1024;       // few rows: a block or two per warp
+        launch(rms_norm_had_kernel<half, true>, rms_norm_had_kernel<half, false>, rms_norm_had_kernel<float, true>, rms_norm_had_kernel<float, false>, threads);
     }
     ctx->launches++;
     return exl3_check_launch(ctx, "rms_norm (fused transform)");
@@ -691,8 +802,10 @@ int exl3_silu_mul_pre(exl3_ctx* ctx, exl3_stream stream, const void* x, const vo
     if (rows == 0) return EXL3_OK;
     const long long blocks = (long long)rows * (dim / 128);
     cudaStream_t st = (cudaStream_t)stream;
-    if (rows < 128) exl3_launch(ctx, silu_mul_had_kernel<1>, (unsigned)((blocks + 7) / 8), 256, 0, st, (const half*)x, (const half*)y, pre->suh[0], pre->a_had[0], blocks, dim / 128);
-    else            exl3_launch(ctx, silu_mul_had_kernel<4>, (unsigned)((blocks + 31) / 32), 256, 0, st, (const half*)x, (const half*)y, pre->suh[0], pre->a_had[0], blocks, dim / 128);
+    if (rows >= 128 && dim % 256 == 0)
+        exl3_launch(ctx, silu_mul_had_wide_kernel, (unsigned)((blocks / 2 + 8 * SW_PAIRS - 1) / (8 * SW_PAIRS)), 256, 0, st, (const half*)x, (const half*)y, pre->suh[0], pre->a_had[0], blocks / 2, dim / 256);
+    else
+        exl3_launch(ctx, silu_mul_had_kernel, (unsigned)((blocks + 7) / 8), 256, 0, st, (const half*)x, (const half*)y, pre->suh[0], pre->a_had[0], blocks, dim / 128);
     ctx->launches++;
     return exl3_check_launch(ctx, "silu_mul (fused transform)");
 }
