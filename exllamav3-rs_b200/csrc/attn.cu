@@ -16,11 +16,14 @@ using namespace exl3;
 template <int D, bool HAD>
 __global__ void __launch_bounds__(256) attn_combine_kernel(const AttnParams p, int rows_per_cta, int total_rows, const half* had_suh, half* had_out)
 {
-    pdl_enter();
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int lane = threadIdx.x & 31;
+    const long long w = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
+    uint2 sg = make_uint2(0u, 0u);                             // signs do not depend on the kernels in front
+    if constexpr (HAD) sg = reinterpret_cast<const uint2*>(had_suh)[(int)(w % p.nq) * 32 + lane];
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     // the attention kernel in front has handed out all its units: the work list is ready for the next layer's
     if (blockIdx.x == 0 && threadIdx.x == 0) const_cast<AttnPlan*>(p.plan)->next = 0;
-    const long long w = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
     if (w >= (long long)total_rows * p.nq) return;
     const int row = (int)(w / p.nq), head = (int)(w % p.nq);
     int b;
@@ -33,7 +36,6 @@ __global__ void __launch_bounds__(256) attn_combine_kernel(const AttnParams p, i
     const int splits = p.seq_splits[b];
     // the input transform of the projection behind the attention: a head is one 128-block of its k
     auto transform = [&](uint2 v) {
-        const uint2 sg = reinterpret_cast<const uint2*>(had_suh)[head * 32 + lane];
         reinterpret_cast<uint2*>(had_out)[((size_t)row * p.nq + head) * 32 + lane] =
             had128_signed_lane(*reinterpret_cast<const half2*>(&v.x), *reinterpret_cast<const half2*>(&v.y), sg, lane);
     };

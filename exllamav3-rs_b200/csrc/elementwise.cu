@@ -160,18 +160,35 @@ __global__ void __launch_bounds__(1024) rms_norm_kernel(const TI* __restrict__ x
 // rms_norm_kernel whose fp16 result goes straight through the input transform of the EXL3 tensors that read it (up to
 // three: q/k/v or gate/up, each with its own sign vector) instead of to memory: the norm's own output and the separate
 // transform launch drop out.  A warp's 32 float4 columns of one pass are one 128-block (dim % 128 == 0).
-template <typename TI, bool RES_IN>
+// I: float4 columns per thread.  Up to two the norm's weights and the signs, which no kernel of a chain writes, are read ahead of the
+// wait for the kernels in front, where they take no time.  (With the same in the activation, the rotation and the attention's merge
+// kernel, us: 28 layers of hidden 1024, 8 rows 1618 -> 1473; 64 of 5120, 4 x 8 rows over 4-bit pools 10819 -> 10424.)
+template <typename TI, bool RES_IN, int I>
 __global__ void __launch_bounds__(1024) rms_norm_had_kernel(const TI* __restrict__ x, const half* __restrict__ w, float* __restrict__ r,
                                                             float eps, float cbias, float cscale, int dim, const exl3_pre_act pre)
 {
-    pdl_enter();
+    constexpr bool AHEAD = I <= 2;
     __shared__ float sh[32];
     const int cols = dim >> 2, lane = threadIdx.x & 31;
     const size_t row = blockIdx.x;
-    float4 v[8];
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    uint2 wr[AHEAD ? I : 1], sg[AHEAD ? I : 1][3];
+    auto weights = [&](int c, uint2& wv, uint2 (&sv)[3]) {
+        if (w) wv = reinterpret_cast<const uint2*>(w)[c];
+        #pragma unroll
+        for (int sgm = 0; sgm < 3; ++sgm)
+            if (sgm < pre.nseg) sv[sgm] = reinterpret_cast<const uint2*>(pre.suh[sgm])[c];
+    };
+    if constexpr (AHEAD) {
+        #pragma unroll
+        for (int i = 0; i < I; ++i)
+            if (threadIdx.x + i * blockDim.x < cols) weights(threadIdx.x + i * blockDim.x, wr[i], sg[i]);
+    }
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    float4 v[I];
     float sum = 0.0f;
     #pragma unroll
-    for (int i = 0; i < 8; ++i) {
+    for (int i = 0; i < I; ++i) {
         const int c = threadIdx.x + i * blockDim.x;
         if (c < cols) {
             float4 f;
@@ -194,12 +211,13 @@ __global__ void __launch_bounds__(1024) rms_norm_had_kernel(const TI* __restrict
     sum = block_sum(sum, sh);
     const float rmf = rsqrtf(sum / (float)dim + eps) * cscale;
     #pragma unroll
-    for (int i = 0; i < 8; ++i) {
+    for (int i = 0; i < I; ++i) {
         const int c = threadIdx.x + i * blockDim.x;
         if (c < cols) {                                         // warp-uniform: cols % 32 == 0
             float4 f = v[i];
+            if constexpr (!AHEAD) weights(c, wr[0], sg[0]);
+            uint2& raw = wr[AHEAD ? i : 0];
             if (w) {
-                uint2 raw = reinterpret_cast<const uint2*>(w)[c];
                 half2 a = *reinterpret_cast<half2*>(&raw.x), b = *reinterpret_cast<half2*>(&raw.y);
                 f.x = f.x * (__low2float(a) + cbias) * rmf;  f.y = f.y * (__high2float(a) + cbias) * rmf;
                 f.z = f.z * (__low2float(b) + cbias) * rmf;  f.w = f.w * (__high2float(b) + cbias) * rmf;
@@ -210,7 +228,7 @@ __global__ void __launch_bounds__(1024) rms_norm_had_kernel(const TI* __restrict
             #pragma unroll
             for (int sgm = 0; sgm < 3; ++sgm)
                 if (sgm < pre.nseg) {
-                    const uint2 h = had128_signed_lane(a, b, reinterpret_cast<const uint2*>(pre.suh[sgm])[c], lane);
+                    const uint2 h = had128_signed_lane(a, b, sg[AHEAD ? i : 0][sgm], lane);
                     reinterpret_cast<uint2*>(pre.a_had[sgm] + row * dim)[c] = h;
                 }
         }
@@ -319,7 +337,7 @@ __global__ void __launch_bounds__(256) rope_kernel(const half* q, const half* k,
                                                    const half* __restrict__ k_norm, float norm_eps, float norm_cbias,
                                                    int rope_mode, float attn_factor, int rows, int seq, int nq, int nk, const exl3_kv_dst dst)
 {
-    pdl_enter();
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     constexpr int HD = EPL * 32;
     const int lane = threadIdx.x & 31;
     const long long gw = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
@@ -329,6 +347,19 @@ __global__ void __launch_bounds__(256) rope_kernel(const half* q, const half* k,
     const half* p; half* po; const half* nw;
     if (h < nq) { p = q + ((size_t)row * nq + h) * HD; po = out_q + ((size_t)row * nq + h) * HD; nw = q_norm; }
     else        { p = k + ((size_t)row * nk + (h - nq)) * HD; po = out_k + ((size_t)row * nk + (h - nq)) * HD; nw = k_norm; }
+    // a step's norm weights and frequencies, which its kernels only read, are there before the kernels in front are complete
+    half nwr[EPL]; float fr[EPL / 2];
+    auto ahead = [&]() {
+        #pragma unroll
+        for (int i = 0; i < EPL; ++i) nwr[i] = nw ? nw[lane + 32 * i] : __float2half_rn(0.f);
+        #pragma unroll
+        for (int i = 0; i < EPL / 2; ++i) fr[i] = rope_mode == EXL3_ROPE_NEOX && lane + 32 * i < n_freq ? inv_freq[lane + 32 * i] : 0.f;
+    };
+    if constexpr (APPEND) ahead();
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if constexpr (!APPEND) ahead();
+    int slot = -1;
+    if constexpr (APPEND) slot = dst.slot[row];
     int pos;
     if (row_pos) pos = row_pos[row];
     else         pos = (row % seq) + (positions ? positions[row / seq] : (int)position);
@@ -347,7 +378,7 @@ __global__ void __launch_bounds__(256) rope_kernel(const half* q, const half* k,
         const half cb = __float2half_rn(norm_cbias);
         #pragma unroll
         for (int i = 0; i < EPL; ++i)
-            x[i] = __hmul(__hadd(nw[lane + 32 * i], cb), __float2half_rn(__half2float(x[i]) * rmf));
+            x[i] = __hmul(__hadd(nwr[i], cb), __float2half_rn(__half2float(x[i]) * rmf));
     }
 
     const float pf = __int2float_rn(pos);
@@ -357,8 +388,7 @@ __global__ void __launch_bounds__(256) rope_kernel(const half* q, const half* k,
         #pragma unroll
         for (int i = 0; i < EPL / 2; ++i) {
             if (i < off) {
-                const int t = lane + 32 * i;
-                float ang = inv_freq[t] * pf;
+                float ang = fr[i] * pf;
                 float sn = __sinf(ang) * attn_factor, cs = __cosf(ang) * attn_factor;
                 #pragma unroll
                 for (int j = 0; j < EPL; ++j) {
@@ -392,7 +422,6 @@ __global__ void __launch_bounds__(256) rope_kernel(const half* q, const half* k,
             #pragma unroll
             for (int i = 0; i < EPL; ++i) sk[lane + 32 * i] = x[i];
             __syncwarp();
-            const int slot = dst.slot[row];
             if (slot < 0) return;
             const size_t head = (size_t)slot * nk + (h - nq);
             const half* v = dst.v + ((size_t)row * nk + (h - nq)) * HD;
@@ -450,16 +479,18 @@ __device__ __forceinline__ half2 silu_mul2(half2 a, half2 b)
 __global__ void __launch_bounds__(256) silu_mul_had_kernel(const half* __restrict__ x, const half* __restrict__ y,
                                                            const half* __restrict__ suh, half* __restrict__ a_had, long long blocks, int bpr)
 {
-    pdl_enter();
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int lane = threadIdx.x & 31;
     const long long blk = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
     if (blk >= blocks) return;
+    const int col = (int)(blk % bpr) * 32 + lane;               // uint2 index inside the sign vector
+    const uint2 sg = reinterpret_cast<const uint2*>(suh)[col];  // signs do not depend on the kernels in front
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     const uint2 xr = reinterpret_cast<const uint2*>(x + blk * 128)[lane], yr = reinterpret_cast<const uint2*>(y + blk * 128)[lane];
     half2 z[2];
     #pragma unroll
     for (int j = 0; j < 2; ++j) z[j] = silu_mul2(*reinterpret_cast<const half2*>(&xr.x + j), *reinterpret_cast<const half2*>(&yr.x + j));
-    const int col = (int)(blk % bpr) * 32 + lane;               // uint2 index inside the sign vector
-    reinterpret_cast<uint2*>(a_had + blk * 128)[lane] = had128_signed_lane(z[0], z[1], reinterpret_cast<const uint2*>(suh)[col], lane);
+    reinterpret_cast<uint2*>(a_had + blk * 128)[lane] = had128_signed_lane(z[0], z[1], sg, lane);
 }
 // Many rows: pairs of blocks with the transform on the tensor core (had_mma.cuh), two per warp whose loads are all in flight before the
 // first is used (1052 rows of 17408, in a step: 31.4 us with four blocks per warp and shuffles, 24.3 here; 110 MB of loads and stores
@@ -788,7 +819,10 @@ int exl3_rms_norm_pre(exl3_ctx* ctx, exl3_stream stream, const void* x, int x_fp
         int threads = cols <= 2048 ? 256 : 1024;
         if (cols < 256) threads = ((cols + 31) / 32) * 32;
         if (rows < 128 && cols > 256) threads = cols < 1024 ? ((cols + 31) / 32) * 32 : 1024;       // few rows: a block or two per warp
-        launch(rms_norm_had_kernel<half, true>, rms_norm_had_kernel<half, false>, rms_norm_had_kernel<float, true>, rms_norm_had_kernel<float, false>, threads);
+        if (cols <= 2 * threads)
+            launch(rms_norm_had_kernel<half, true, 2>, rms_norm_had_kernel<half, false, 2>, rms_norm_had_kernel<float, true, 2>, rms_norm_had_kernel<float, false, 2>, threads);
+        else
+            launch(rms_norm_had_kernel<half, true, 8>, rms_norm_had_kernel<half, false, 8>, rms_norm_had_kernel<float, true, 8>, rms_norm_had_kernel<float, false, 8>, threads);
     }
     ctx->launches++;
     return exl3_check_launch(ctx, "rms_norm (fused transform)");
