@@ -416,12 +416,13 @@ int attn_impl(exl3_ctx* ctx, cudaStream_t st, AttnParams p, int total_rows, int 
         return rc;
     };
     const bool general_single = max_rows <= dec_rows || !p.cu_q;
-    exl3_chain_scope chain(ctx, append && !(one && (codes_alone || general_single)));
-    if (append && !(one && (codes_alone || general_single))) {
+    const bool apart = append && !(one && (codes_alone || general_single));
+    if (apart) {
         const int rc = attn_append(ctx, st, *append);
         if (rc != EXL3_OK) return rc;
         append = nullptr;
     }
+    exl3_chain_scope chain(ctx, apart);                    // (the append itself follows what the caller has in front)
     if (codes_alone) {
         const int rc = single(ATTN_CODES, 1 << 30);
         if (rc != EXL3_ERR_WORKSPACE) return rc;
