@@ -45,6 +45,7 @@ struct AttnParams {
     const int* seq_splits;         // [bsz]
     float* partial;                // [n_items][nkv][ROWS][D+2]
     int* status;                   // context status word (bounded waits)
+    const half* had_suh; half* had_out;        // cluster form: also the 128-point transform of (output o signs); NULL: none
     int bsz, q_len, kv_append, nq, nkv, pps, pages, causal, k_bits, v_bits;
     int contig_kv;                 // > 0: kc/vc are plain [bsz, contig_kv, nkv, D] tensors, no block table (mma.sync fp16 kernel only)
     float scale_log2;              // sm_scale * log2(e)
@@ -84,7 +85,7 @@ __device__ __forceinline__ uint32_t pack_h2(float a, float b)
 
 // Shared memory: per stage a K tile and a V tile [AT_TK][D+8] fp16; quantised pools (QB > 0: codes of at most QB bits)
 // stage the raw codes and scales instead and decode them into one pair of fp16 tiles.
-template <int D, int QB>
+template <int D, int QB, int STAGES = AT_STAGES>
 struct AttnSmem {
     static constexpr bool QUANT = QB > 0;
     static constexpr int ROWB = (D + 8) * 2;                       // bytes per key row (padding keeps ldmatrix conflict-free)
@@ -95,20 +96,50 @@ struct AttnSmem {
     static constexpr int RAW = AT_TK * RAW_ROW + 64;
     static constexpr int STAGE = QUANT ? 2 * RAW : 2 * TILE;      // QUANT stages the raw bytes; tiles are decoded in place below
     static constexpr int DECODED = QUANT ? 2 * TILE : 0;
-    static constexpr int PIPE = AT_STAGES * STAGE + DECODED;
+    static constexpr int PIPE = STAGES * STAGE + DECODED;
     static constexpr int MERGE = 4 * 16 * (D + 4) * 4;             // cross-warp merge / output staging, fp32
     static constexpr int BYTES = PIPE > MERGE ? PIPE : MERGE;
 };
+
+// ---- cluster form.  A batch that is small in every respect (attn_impl says when) is a few microseconds of latency: the work list, the
+// draw of a unit, the partial sums' way through memory and the merge kernel behind took longer than the keys.  There a cluster of CTAs
+// shares the keys of one sequence and kv head in equal parts and merges them through its shared memory.
+constexpr int AT_CL_STAGES = 3;
+__device__ __forceinline__ void at_cluster_sync() { asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ uint32_t at_peer(const void* p, int cta)
+{
+    uint32_t a;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(cta));
+    return a;
+}
+__device__ __forceinline__ float4 at_ld_peer4(uint32_t a)
+{
+    float4 v;
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a) : "memory");
+    return v;
+}
+__device__ __forceinline__ float2 at_ld_peer2(uint32_t a)
+{
+    float2 v;
+    asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a) : "memory");
+    return v;
+}
 
 // WM x WN = 4 warps: WM 16-row tiles, WN key slices of every tile.  (4,1): prefill/verify rows, (1,4): decode rows.
 #ifndef AT_Q4_DECODE_BLOCKS
 #define AT_Q4_DECODE_BLOCKS 4         // resident CTAs per SM the 4-bit decode-class kernel is compiled for (register cap)
 #endif
-template <int D, int WM, int WN, int QB>
-__global__ void __launch_bounds__(AT_THREADS, (QB == 4 && WN == 4) ? AT_Q4_DECODE_BLOCKS : 1) attn_paged_kernel(const AttnParams p)
+// CL: cluster form, grid (parts, nkv, bsz) in clusters of `parts`; else a persistent kernel over the work list.
+template <int D, int WM, int WN, int QB, bool CL = false>
+__global__ void __launch_bounds__(AT_THREADS, CL ? 2 : (QB == 4 && WN == 4) ? AT_Q4_DECODE_BLOCKS : 1) attn_paged_kernel(const AttnParams p)
 {
-    pdl_enter();
-    using SM = AttnSmem<D, QB>;
+    static_assert(!CL || (WM == 1 && D == 128), "a cluster shares one block of 16 rows");
+    // The cluster form waits for the kernels in front where it needs what they write, the queries and the new keys and values.  Lengths,
+    // block table and the pools' older tokens were there before its chain began.
+    if constexpr (CL) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    else pdl_enter();
+    constexpr int STAGES = CL ? AT_CL_STAGES : AT_STAGES;
+    using SM = AttnSmem<D, QB, STAGES>;
     constexpr bool QUANT = QB > 0;
     constexpr int ROWS = 16 * WM;
     constexpr int KEYS_W = AT_TK / WN;          // keys of a tile handled by one warp
@@ -121,20 +152,33 @@ __global__ void __launch_bounds__(AT_THREADS, (QB == 4 && WN == 4) ? AT_Q4_DECOD
     const int g = lane >> 2, t = lane & 3;
     const int wm = warp / WN, wn = warp % WN;
     const int G = p.nq / p.nkv;
-    const int n_items = p.plan->n_items, chunk = p.plan->chunk;
+    const int n_items = CL ? 0 : p.plan->n_items, plan_chunk = CL ? 0 : p.plan->chunk;
 
     // Work units = (item, kv head), handed out through a counter: items differ in length (last splits, causal cuts), and a
     // fixed assignment left a quarter of the SM time idle at the end of the kernel.
     __shared__ int s_unit;
     const int n_units = n_items * p.nkv;
     for (;;) {
-        __syncthreads();                                   // everyone is done with the previous unit (and with s_unit)
-        if (tid == 0) s_unit = atomicAdd(const_cast<int*>(&p.plan->next), 1);
-        __syncthreads();
-        const int unit = s_unit;
-        if (unit >= n_units) break;
-        const AttnItem item = p.items[unit / p.nkv];
-        const int item_idx = item.idx, kvh = unit % p.nkv;
+        AttnItem item;
+        int kvh, chunk = plan_chunk;
+        if constexpr (CL) {
+            const int b = blockIdx.z, parts = gridDim.x;
+            kvh = blockIdx.y;
+            item.b = b; item.rb = 0; item.split = blockIdx.x; item.idx = 0; item.splits = parts;
+            item.row_base = p.cu_q ? p.cu_q[b] : b * p.q_len;
+            item.ql = p.cu_q ? p.cu_q[b + 1] - item.row_base : p.q_len;
+            item.total_k = (p.seqlens ? p.seqlens[b] : 0) + (p.cu_q ? item.ql : p.kv_append);
+            if (item.ql <= 0) return;                          // the whole cluster
+            chunk = ((item.total_k + parts - 1) / parts + AT_TK - 1) / AT_TK * AT_TK;
+        } else {
+            __syncthreads();                                   // everyone is done with the previous unit (and with s_unit)
+            if (tid == 0) s_unit = atomicAdd(const_cast<int*>(&p.plan->next), 1);
+            __syncthreads();
+            const int unit = s_unit;
+            if (unit >= n_units) break;
+            item = p.items[unit / p.nkv]; kvh = unit % p.nkv;
+        }
+        const int item_idx = item.idx;
         const int b = item.b, row_base = item.row_base, ql = item.ql, total_k = item.total_k, splits = item.splits;
         const int r0 = item.rb * ROWS;                       // first packed (query, head) row of this CTA
         // keys this row block can see at all (causal, bottom-right aligned)
@@ -159,47 +203,6 @@ __global__ void __launch_bounds__(AT_THREADS, (QB == 4 && WN == 4) ? AT_Q4_DECOD
         int wlim = min(rvalid[0] ? lim[0] : 0x7fffffff, rvalid[1] ? lim[1] : 0x7fffffff);
         #pragma unroll
         for (int o = 16; o > 0; o >>= 1) wlim = min(wlim, __shfl_xor_sync(0xffffffffu, wlim, o));
-
-        // ---- Q fragments (A operand), straight from global memory
-        uint32_t qf[KSTEPS][4];
-        #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const int row = r0 + wm * 16 + g + 8 * h;
-            const int head = kvh * G + (row - qi[h] * G);
-            const half* qp = p.q + ((size_t)(row_base + qi[h]) * p.nq + head) * D;
-            #pragma unroll
-            for (int ks = 0; ks < KSTEPS; ++ks) {
-                qf[ks][h]     = rvalid[h] ? *reinterpret_cast<const uint32_t*>(qp + ks * 16 + 2 * t) : 0u;
-                qf[ks][h + 2] = rvalid[h] ? *reinterpret_cast<const uint32_t*>(qp + ks * 16 + 8 + 2 * t) : 0u;
-            }
-        }
-
-        if constexpr (QUANT) {
-            // Quantised pools hold codes of the rotated vectors H(k), H(v) (H = H32 / sqrt(32) per group of 32 dims).
-            // Instead of rotating every key and value back, the query is rotated once here (q . H(c) = H(q) . c) and the
-            // output row once at the end; the tiles below then hold the scaled codes as they are.
-            #pragma unroll
-            for (int gq = 0; gq < D / 32; ++gq) {
-                #pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    float v[4][2];
-                    #pragma unroll
-                    for (int b4 = 0; b4 < 4; ++b4) {
-                        const half2 x = *reinterpret_cast<const half2*>(&qf[2 * gq + (b4 >> 1)][h + 2 * (b4 & 1)]);
-                        v[b4][0] = __low2float(x); v[b4][1] = __high2float(x);
-                    }
-                    had32_quad(v, t);
-                    #pragma unroll
-                    for (int b4 = 0; b4 < 4; ++b4)
-                        qf[2 * gq + (b4 >> 1)][h + 2 * (b4 & 1)] = pack_h2(v[b4][0] * R32, v[b4][1] * R32);
-                }
-            }
-        }
-
-        float o_acc[DBLK][4];
-        #pragma unroll
-        for (int i = 0; i < DBLK; ++i) { o_acc[i][0] = o_acc[i][1] = o_acc[i][2] = o_acc[i][3] = 0.f; }
-        float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};
 
         const int n_tiles = k_end > k_begin ? (k_end - k_begin + AT_TK - 1) / AT_TK : 0;
 
@@ -249,23 +252,71 @@ __global__ void __launch_bounds__(AT_THREADS, (QB == 4 && WN == 4) ? AT_Q4_DECOD
             }
         };
 
+        bool waited = !CL;
+        const int old = CL && p.seqlens ? p.seqlens[b] : 0;
         #pragma unroll
-        for (int pre = 0; pre < AT_STAGES - 1; ++pre) {            // tiles 0 .. S-2 in flight before the loop
-            if (pre < n_tiles) load_tile(pre, pre);
+        for (int pre = 0; pre < STAGES - 1; ++pre) {               // tiles 0 .. S-2 in flight before the loop
+            if (pre < n_tiles) {
+                if (!waited && min(k_begin + (pre + 1) * AT_TK, k_end) > old) { asm volatile("griddepcontrol.wait;" ::: "memory"); waited = true; }
+                load_tile(pre, pre);
+            }
             cp_async_commit();
         }
+        if (!waited) asm volatile("griddepcontrol.wait;" ::: "memory");
+
+        // ---- Q fragments (A operand), straight from global memory
+        uint32_t qf[KSTEPS][4];
+        #pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int row = r0 + wm * 16 + g + 8 * h;
+            const int head = kvh * G + (row - qi[h] * G);
+            const half* qp = p.q + ((size_t)(row_base + qi[h]) * p.nq + head) * D;
+            #pragma unroll
+            for (int ks = 0; ks < KSTEPS; ++ks) {
+                qf[ks][h]     = rvalid[h] ? *reinterpret_cast<const uint32_t*>(qp + ks * 16 + 2 * t) : 0u;
+                qf[ks][h + 2] = rvalid[h] ? *reinterpret_cast<const uint32_t*>(qp + ks * 16 + 8 + 2 * t) : 0u;
+            }
+        }
+
+        if constexpr (QUANT) {
+            // Quantised pools hold codes of the rotated vectors H(k), H(v) (H = H32 / sqrt(32) per group of 32 dims).
+            // Instead of rotating every key and value back, the query is rotated once here (q . H(c) = H(q) . c) and the
+            // output row once at the end; the tiles below then hold the scaled codes as they are.
+            #pragma unroll
+            for (int gq = 0; gq < D / 32; ++gq) {
+                #pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    float v[4][2];
+                    #pragma unroll
+                    for (int b4 = 0; b4 < 4; ++b4) {
+                        const half2 x = *reinterpret_cast<const half2*>(&qf[2 * gq + (b4 >> 1)][h + 2 * (b4 & 1)]);
+                        v[b4][0] = __low2float(x); v[b4][1] = __high2float(x);
+                    }
+                    had32_quad(v, t);
+                    #pragma unroll
+                    for (int b4 = 0; b4 < 4; ++b4)
+                        qf[2 * gq + (b4 >> 1)][h + 2 * (b4 & 1)] = pack_h2(v[b4][0] * R32, v[b4][1] * R32);
+                }
+            }
+        }
+
+        float o_acc[DBLK][4];
+        #pragma unroll
+        for (int i = 0; i < DBLK; ++i) { o_acc[i][0] = o_acc[i][1] = o_acc[i][2] = o_acc[i][3] = 0.f; }
+        float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};
+
         int stage = 0;
         for (int tile = 0; tile < n_tiles; ++tile) {
-            const int ahead = tile + AT_STAGES - 1;
-            if (ahead < n_tiles) load_tile(ahead, (stage + AT_STAGES - 1) % AT_STAGES);
+            const int ahead = tile + STAGES - 1;
+            if (ahead < n_tiles) load_tile(ahead, (stage + STAGES - 1) % STAGES);
             cp_async_commit();
-            cp_async_wait<AT_STAGES - 1>();
+            cp_async_wait<STAGES - 1>();
             __syncthreads();
 
             const uint8_t* ktile; const uint8_t* vtile;
             if constexpr (QUANT) {
                 // scale the staged codes into fp16 tiles (rotated domain): one warp-op = 4 groups = the D=128 values of one key
-                uint8_t* dk = smem_raw + AT_STAGES * SM::STAGE;
+                uint8_t* dk = smem_raw + STAGES * SM::STAGE;
                 uint8_t* dv = dk + SM::TILE;
                 const uint8_t* raw = smem_raw + stage * SM::STAGE;
                 if (QB == 4) {
@@ -374,7 +425,7 @@ __global__ void __launch_bounds__(AT_THREADS, (QB == 4 && WN == 4) ? AT_Q4_DECOD
                 }
             }
             __syncthreads();      // the stage is refilled by the next iteration's loads
-            stage = stage + 1 == AT_STAGES ? 0 : stage + 1;
+            stage = stage + 1 == STAGES ? 0 : stage + 1;
         }
         cp_async_wait<0>();
         __syncthreads();
@@ -431,6 +482,13 @@ __global__ void __launch_bounds__(AT_THREADS, (QB == 4 && WN == 4) ? AT_Q4_DECOD
                 #pragma unroll
                 for (int e = 0; e < D / 32; ++e) acc[e] *= R32;
             }
+            if constexpr (CL) {
+                // this CTA's part of the row: behind the merge buffer, where the others read it
+                float* xs = ms + 4 * 16 * MS + lr * MS;
+                *reinterpret_cast<float4*>(xs + lane * 4) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+                if (lane == 0) *reinterpret_cast<float2*>(xs + D) = make_float2(mm, ll);
+                continue;
+            }
             const int qidx = row / G, head = kvh * G + (row - qidx * G);
             if (splits == 1) {
                 const float inv = ll > 0.f ? 1.0f / ll : 0.f;
@@ -444,6 +502,40 @@ __global__ void __launch_bounds__(AT_THREADS, (QB == 4 && WN == 4) ? AT_Q4_DECOD
                 for (int e = 0; e < D / 32; ++e) pp[lane * (D / 32) + e] = acc[e];
                 if (lane == 0) { pp[D] = mm; pp[D + 1] = ll; }
             }
+        }
+        if constexpr (CL) {
+            static_assert(2 * SM::MERGE <= SM::BYTES, "the parts stand behind the merge buffer");
+            at_cluster_sync();
+            // rows in turn over the cluster's CTAs and warps
+            for (int lr = item.split + splits * warp; lr < ql * G; lr += splits * 4) {
+                const float* xs = ms + 4 * 16 * MS + lr * MS;
+                float4 v[8]; float2 ml[8];
+                #pragma unroll
+                for (int c = 0; c < 8; ++c)
+                    if (c < splits) { const uint32_t a = at_peer(xs, c); v[c] = at_ld_peer4(a + lane * 16); ml[c] = at_ld_peer2(a + D * 4); }
+                float mm = -INFINITY, ll = 0.f;
+                #pragma unroll
+                for (int c = 0; c < 8; ++c)
+                    if (c < splits) mm = fmaxf(mm, ml[c].x);
+                float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+                #pragma unroll
+                for (int c = 0; c < 8; ++c)
+                    if (c < splits) {
+                        const float sc = ml[c].x == -INFINITY ? 0.f : exp2f(ml[c].x - mm);
+                        ll += ml[c].y * sc;
+                        acc.x += v[c].x * sc; acc.y += v[c].y * sc; acc.z += v[c].z * sc; acc.w += v[c].w * sc;
+                    }
+                const float inv = ll > 0.f ? 1.0f / ll : 0.f;
+                const int qidx = lr / G, head = kvh * G + (lr - qidx * G);
+                const uint2 o = make_uint2(pack_h2(acc.x * inv, acc.y * inv), pack_h2(acc.z * inv, acc.w * inv));
+                const size_t at = ((size_t)(row_base + qidx) * p.nq + head) * 32 + lane;
+                reinterpret_cast<uint2*>(p.o)[at] = o;
+                if (p.had_out)                                  // the input transform of the projection behind: a head is one 128-block of its k
+                    reinterpret_cast<uint2*>(p.had_out)[at] = had128_signed_lane(*reinterpret_cast<const half2*>(&o.x), *reinterpret_cast<const half2*>(&o.y),
+                                                                                 reinterpret_cast<const uint2*>(p.had_suh)[head * 32 + lane], lane);
+            }
+            at_cluster_sync();                                  // nobody leaves while its part is being read
+            return;
         }
         __syncthreads();
     }

@@ -617,3 +617,50 @@ def test_attention_over_codes_edges(ctx, bits, q_len, nq, nkv, v_mul):
         assert np.isfinite(got).all()
         for b in range(len(lens)):                     # each sequence against its own size
             assert _close(got[b], want[b], TOL_QUANT) <= 1.0, lens[b]
+
+
+@pytest.mark.parametrize("bits", [0, 6])
+@pytest.mark.parametrize("bsz,nq,nkv,q_len,ragged", [(2, 16, 8, 1, False), (8, 40, 8, 2, False), (11, 16, 8, 1, True), (4, 32, 2, 1, True), (30, 4, 4, 4, False)])
+def test_attention_of_a_small_batch_in_clusters(ctx, bits, bsz, nq, nkv, q_len, ragged):
+    """Two, four and eight CTAs that share a sequence's keys: contexts of no key, less than a key per part, around the tiles of 64 keys
+    and the parts' ends; new keys that fall into the tiles read ahead; sequences without rows; one to sixteen packed rows.  One launch
+    behind the append.  Bars: the repository's."""
+    from oracle import oracle as O
+    torch = _torch()
+    r = H.rng(2300 + bsz + bits)
+    parts = next(c for c in (8, 4, 2) if bsz * nkv * c <= 2 * torch.cuda.get_device_properties(0).multi_processor_count)
+    lens = [0, 1, 63, 64, 65, 127, 128, 129, 64 * parts - 1, 64 * parts, 64 * parts + 1, 250, 300, 511, 512 * parts - 260]
+    ctx_lens = np.array([lens[(3 * b + bsz) % len(lens)] if b else lens[-1] for b in range(bsz)], np.int32)
+    q_lens = np.array([(0 if b % 3 == 1 else 1 + b % 2) if ragged else q_len for b in range(bsz)], np.int32)
+    if ragged:
+        q_lens = np.minimum(q_lens, 16 * nkv // nq)
+    bt, pages = H.make_paged(r, bsz, ctx_lens + q_lens, nkv, 128)
+    cu = np.concatenate([[0], np.cumsum(q_lens)]).astype(np.int32)
+    lead = (int(cu[-1]),) if ragged else (bsz, q_len)
+    rnd = lambda *s: (0.5 * r.standard_normal(s)).astype(np.float16)  # noqa: E731
+    c = dict(q=rnd(*lead, nq, 128), k=rnd(*lead, nkv, 128), v=rnd(*lead, nkv, 128), kc=rnd(pages, 256, nkv, 128), vc=rnd(pages, 256, nkv, 128))
+    o = torch.full(c["q"].shape, float("nan"), dtype=torch.float16, device="cuda")
+    q, k, v, dbt, dsl = [H.to_dev(x) for x in (c["q"], c["k"], c["v"], bt, ctx_lens)]
+    dcu, ql = H.to_dev(cu) if ragged else None, int(q_lens.max())
+    n0 = ctx.launch_count()
+    if bits == 0:
+        ctx.bighead_attn_paged(q, k, v, H.to_dev(c["kc"]), H.to_dev(c["vc"]), dbt, dsl, o, cu_q=dcu, max_q_len=ql)
+    else:
+        pools = _quant_pools(c, bits)
+        ctx.bighead_attn_paged_q(q, k, v, *_to_dev(pools), dbt, dsl, o, nkv, cu_q=dcu, max_q_len=ql)
+    assert ctx.launch_count() - n0 == 2
+    ctx.poll_status()
+    got = o.cpu().numpy()
+    assert np.isfinite(got).all()
+    for b in range(bsz):
+        if q_lens[b] == 0:
+            continue
+        one = [x[cu[b]:cu[b + 1]][None] if ragged else x[b:b + 1] for x in (c["q"], c["k"], c["v"], got)]
+        if bits == 0:
+            kc, vc = c["kc"], c["vc"]
+            O.paged_kv_update(one[1], one[2], kc, vc, bt[b:b + 1], ctx_lens[b:b + 1])
+            want = O.attn_paged(one[0], kc, vc, bt[b:b + 1], ctx_lens[b:b + 1])
+        else:
+            O.quant_cache_paged(one[1], pools[0], pools[1], one[2], pools[2], pools[3], ctx_lens[b:b + 1], bt[b:b + 1], bits, bits)
+            want = O.attn_paged(one[0], None, None, bt[b:b + 1], ctx_lens[b:b + 1], nkv=nkv, quant=(*pools, bits))
+        assert _close(one[3], want, TOL_FP16 if bits == 0 else TOL_QUANT) <= 1.0, b
