@@ -61,6 +61,10 @@ def lib():
         L.exl3_ctx_launch_count.restype = C.c_uint64
         L.exl3_ctx_launch_count.argtypes = [C.c_void_p]
         L.exl3_cuda_free_mib.restype = C.c_int64
+        # the calls of a decode loop take plain integers for addresses: a c_void_p object per argument costs 0.2 us each
+        L.exl3_gemm.argtypes = [C.c_void_p] * 8 + [C.c_int] * 7
+        L.exl3_bighead_attn_paged.argtypes = [C.c_void_p] * 11 + [C.c_int] * 10 + [C.c_float]
+        L.exl3_bighead_attn_paged_q.argtypes = [C.c_void_p] * 13 + [C.c_int] * 12 + [C.c_float] * 2
         L.exl3_graph_new.restype = C.c_void_p
         L.exl3_graph_new.argtypes = [C.c_void_p]
         L.exl3_side_stream.restype = C.c_void_p
@@ -75,8 +79,18 @@ def _ptr(t):
     return C.c_void_p(0 if t is None else t.data_ptr())
 
 
+def _adr(t):
+    """address for a function whose argument types are declared"""
+    return None if t is None else t.data_ptr()
+
+
+def _raw_stream():
+    """handle of the current stream of the current device, without the objects of torch.cuda.current_stream (1.5 us)"""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+
+
 def _chk(t, dtype, name):
-    if t is None:
+    if t is None or (t.is_cuda and t.dtype is dtype and t.is_contiguous()):
         return
     if not t.is_cuda:
         raise Exl3Error(f"{name} must be a CUDA tensor")
@@ -113,11 +127,13 @@ class Ctx:
         return self._h
 
     def stream(self, stream=None):
+        return C.c_void_p(self._stream(stream))
+
+    @staticmethod
+    def _stream(stream):
         if stream is None:
-            return C.c_void_p(torch.cuda.current_stream().cuda_stream)
-        if isinstance(stream, int):
-            return C.c_void_p(stream)
-        return C.c_void_p(stream.cuda_stream)
+            return _raw_stream()
+        return stream if isinstance(stream, int) else stream.cuda_stream
 
     def check(self, rc, what):
         if rc != 0:
@@ -155,13 +171,14 @@ class Ctx:
         _chk(suh, torch.float16, "suh"); _chk(svh, torch.float16, "svh"); _chk(a_had, torch.float16, "a_had")
         k = a.shape[-1]
         m = a.numel() // k
-        n = trellis.shape[1] * 16
-        K = trellis.shape[2] // 16
-        if trellis.shape[0] * 16 != k or c.shape[-1] != n or c.numel() // n != m:
+        shape = trellis.shape
+        kt, n, words = shape[0], shape[1] * 16, shape[2]
+        if kt * 16 != k or c.shape[-1] != n or c.numel() != m * n:
             raise Exl3Error("exl3_gemm: shape mismatch")
-        rc = lib().exl3_gemm(self._h, self.stream(stream), _ptr(a), _ptr(trellis), _ptr(c), _ptr(suh), _ptr(a_had),
-                             _ptr(svh), m, k, n, K, int(c.dtype == torch.float32), int(mcg), int(mul1))
-        self.check(rc, "exl3_gemm")
+        rc = lib().exl3_gemm(self._h, self._stream(stream), a.data_ptr(), trellis.data_ptr(), c.data_ptr(), _adr(suh), _adr(a_had),
+                             _adr(svh), m, k, n, words // 16, c.dtype is torch.float32, bool(mcg), bool(mul1))
+        if rc:
+            self.check(rc, "exl3_gemm")
 
     def gemm_fanout(self, a, weights, outs, stream=None):
         """The same activations through up to three EXL3 tensors (the reference's back-to-back exl3_gemm calls for
@@ -399,10 +416,10 @@ class Ctx:
             q_len = max_q_len if max_q_len is not None else q.shape[0]
             kv_append = q.shape[0]          # ragged form: total packed rows
         nkv = k_cache.shape[2]
-        self.check(lib().exl3_bighead_attn_paged(self._h, self.stream(stream), _ptr(q), _ptr(k), _ptr(v), _ptr(k_cache),
-                                                 _ptr(v_cache), _ptr(block_table), _ptr(cache_seqlens), _ptr(cu_q),
-                                                 _ptr(o), bsz, q_len, kv_append, nq, nkv, hd, k_cache.shape[0], pps,
-                                                 kv_chunk_size, int(causal), C.c_float(sm_scale)), "bighead_attn_paged")
+        self.check(lib().exl3_bighead_attn_paged(self._h, self._stream(stream), _adr(q), _adr(k), _adr(v), _adr(k_cache),
+                                                 _adr(v_cache), _adr(block_table), _adr(cache_seqlens), _adr(cu_q),
+                                                 _adr(o), bsz, q_len, kv_append, nq, nkv, hd, k_cache.shape[0], pps,
+                                                 kv_chunk_size, int(causal), sm_scale), "bighead_attn_paged")
 
     def bighead_attn(self, q, k, v, o, causal=True, sm_scale=0.0, kv_chunk_size=256, stream=None):
         """src/ffi.rs:458-460: attention over plain tensors q, o [bsz,q_len,nq,hd], k, v [bsz,kv_len,nkv,hd]."""
@@ -432,11 +449,11 @@ class Ctx:
             q_len = max_q_len if max_q_len is not None else q.shape[0]
             kv_append = q.shape[0]          # ragged form: total packed rows
         groups = sk.shape[2]
-        self.check(lib().exl3_bighead_attn_paged_q(self._h, self.stream(stream), _ptr(q), _ptr(k), _ptr(v), _ptr(qk),
-                                                   _ptr(sk), _ptr(qv), _ptr(sv), _ptr(block_table), _ptr(cache_seqlens),
-                                                   _ptr(cu_q), _ptr(o), bsz, q_len, kv_append, nq, nkv, hd, qk.shape[0],
+        self.check(lib().exl3_bighead_attn_paged_q(self._h, self._stream(stream), _adr(q), _adr(k), _adr(v), _adr(qk),
+                                                   _adr(sk), _adr(qv), _adr(sv), _adr(block_table), _adr(cache_seqlens),
+                                                   _adr(cu_q), _adr(o), bsz, q_len, kv_append, nq, nkv, hd, qk.shape[0],
                                                    pps, qk.shape[2] // groups, qv.shape[2] // groups, kv_chunk_size,
-                                                   int(causal), C.c_float(sm_scale), C.c_float(compand_a)),
+                                                   int(causal), sm_scale, compand_a),
                    "bighead_attn_paged_q")
 
     def quant_cache_paged(self, k_in, k_out, k_out_scales, v_in, v_out, v_out_scales, cache_seqlens, block_table,
