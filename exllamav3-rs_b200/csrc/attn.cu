@@ -90,6 +90,99 @@ __global__ void __launch_bounds__(256) attn_combine_kernel(const AttnParams p, i
     if constexpr (HAD) transform(make_uint2(pack_h2(acc[0] * inv, acc[1] * inv), pack_h2(acc[2] * inv, acc[3] * inv)));
 }
 
+// The same for few rows, where the kernel is bounded by its chain of dependent loads.  The attention kernels let it go behind their own
+// wait, so a row's sequence, split count and place among the partials, which come from kernels in front of those, are found before the
+// wait; behind it the splits' maxima and sums and the first eight rows are requested together.  (us, together with the later release:
+// 24 sequences over 8-bit pools 58.2 -> 55.7, 4 x 8 rows over fp16 36.6 -> 31; as the last of a 27B-class verify layer, 32 rows and up to
+// 37 splits, 11.2 -> 5.0.)  Its 80 registers against 40 cost more than they give where there are many rows.
+template <int D, bool HAD>
+__global__ void __launch_bounds__(256) attn_combine_few_kernel(const AttnParams p, int rows_per_cta, int total_rows, const half* had_suh, half* had_out)
+{
+    static_assert(D == 128, "a lane covers 4 dims as two 8-byte loads");
+    constexpr int AHEAD = 8;                           // rows in flight per warp
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const int lane = threadIdx.x & 31;
+    const long long w = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
+    uint2 sg = make_uint2(0u, 0u);                             // signs do not depend on the kernels in front
+    int row = 0, head = 0, splits = 0;
+    const float* base = nullptr;
+    const size_t stride = (size_t)p.nkv * rows_per_cta * (D + 2);             // floats between consecutive splits
+    bool mine = w < (long long)total_rows * p.nq;
+    if (mine) {
+        row = (int)(w / p.nq); head = (int)(w % p.nq);
+        if constexpr (HAD) sg = reinterpret_cast<const uint2*>(had_suh)[head * 32 + lane];
+        int b, row_base;
+        if (p.cu_q) {                                          // binary search: cu_q[b] <= row < cu_q[b+1]
+            int lo = 0, hi = p.bsz - 1;
+            while (lo < hi) { int mid = (lo + hi + 1) >> 1; if (__ldcg(p.cu_q + mid) <= row) lo = mid; else hi = mid - 1; }
+            b = lo;
+            row_base = __ldcg(p.cu_q + b);
+            mine = row < __ldcg(p.cu_q + b + 1);                  // rows behind the last sequence have no partials
+        } else { b = row / p.q_len; row_base = b * p.q_len; }
+        splits = __ldcg(p.seq_splits + b);
+        const int G = p.nq / p.nkv, kvh = head / G;
+        const int packed = (row - row_base) * G + (head - kvh * G);
+        const int rb = packed / rows_per_cta, lr = packed - rb * rows_per_cta;
+        const int item0 = __ldcg(p.seq_base + b) + rb * splits;
+        base = p.partial + (((size_t)item0 * p.nkv + kvh) * rows_per_cta + lr) * (D + 2);
+    }
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    // the attention kernel in front has handed out all its units: the work list is ready for the next layer's
+    if (blockIdx.x == 0 && threadIdx.x == 0) const_cast<AttnPlan*>(p.plan)->next = 0;
+    if (!mine) return;
+    // the input transform of the projection behind the attention: a head is one 128-block of its k
+    auto transform = [&](uint2 v) {
+        reinterpret_cast<uint2*>(had_out)[((size_t)row * p.nq + head) * 32 + lane] =
+            had128_signed_lane(*reinterpret_cast<const half2*>(&v.x), *reinterpret_cast<const half2*>(&v.y), sg, lane);
+    };
+    if (splits <= 1) {                                         // the attention kernel wrote the final value itself
+        if constexpr (HAD) transform(*reinterpret_cast<const uint2*>(p.o + ((size_t)row * p.nq + head) * D + lane * (D / 32)));
+        return;
+    }
+    float2 v0[AHEAD], v1[AHEAD];
+    auto fetch = [&](int s0) {
+        #pragma unroll
+        for (int j = 0; j < AHEAD; ++j) {
+            v0[j] = v1[j] = make_float2(0.f, 0.f);
+            if (s0 + j < splits) {
+                const float* pp = base + (size_t)(s0 + j) * stride + lane * (D / 32);
+                v0[j] = *reinterpret_cast<const float2*>(pp); v1[j] = *reinterpret_cast<const float2*>(pp + 2);
+            }
+        }
+    };
+    auto max_sum = [&](int s) { return s < splits ? *reinterpret_cast<const float2*>(base + (size_t)s * stride + D) : make_float2(-INFINITY, 0.f); };
+    float2 ms = max_sum(lane);
+    fetch(0);
+    float mm = ms.x;
+    for (int s = lane + 32; s < splits; s += 32) mm = fmaxf(mm, max_sum(s).x);
+    #pragma unroll
+    for (int o = 16; o > 0; o >>= 1) mm = fmaxf(mm, __shfl_xor_sync(0xffffffffu, mm, o));
+    float acc[D / 32], ll = 0.f;
+    #pragma unroll
+    for (int e = 0; e < D / 32; ++e) acc[e] = 0.f;
+    for (int s0 = 0; s0 < splits; s0 += 32) {
+        if (s0 > 0) ms = max_sum(s0 + lane);
+        const float sc_l = ms.x == -INFINITY ? 0.f : exp2f(ms.x - mm);
+        ll += ms.y * sc_l;
+        const int cnt = min(32, splits - s0);
+        for (int j0 = 0; j0 < cnt; j0 += AHEAD) {
+            #pragma unroll
+            for (int j = 0; j < AHEAD; ++j) {           // rows behind the last split count as zeros
+                const float sc = __shfl_sync(0xffffffffu, sc_l, j0 + j);
+                acc[0] += v0[j].x * sc; acc[1] += v0[j].y * sc; acc[2] += v1[j].x * sc; acc[3] += v1[j].y * sc;
+            }
+            if (s0 + j0 + AHEAD < splits) fetch(s0 + j0 + AHEAD);
+        }
+    }
+    #pragma unroll
+    for (int o = 16; o > 0; o >>= 1) ll += __shfl_xor_sync(0xffffffffu, ll, o);
+    const float inv = ll > 0.f ? 1.0f / ll : 0.f;
+    half* op = p.o + ((size_t)row * p.nq + head) * D + lane * (D / 32);
+    #pragma unroll
+    for (int e = 0; e < D / 32; e += 2) *reinterpret_cast<uint32_t*>(op + e) = pack_h2(acc[e] * inv, acc[e + 1] * inv);
+    if constexpr (HAD) transform(make_uint2(pack_h2(acc[0] * inv, acc[1] * inv), pack_h2(acc[2] * inv, acc[3] * inv)));
+}
+
 template <int D, int WM, int WN, int QB>
 cudaError_t launch_attn(exl3_ctx* ctx, const AttnParams& p, dim3 grid, cudaStream_t st)
 {
@@ -368,8 +461,14 @@ int attn_pass(exl3_ctx* ctx, cudaStream_t st, AttnParams p, int total_rows, int 
     ctx->launches++;
     if (e != cudaSuccess) { cudaGetLastError(); return exl3_fail(ctx, EXL3_ERR_CUDA, cudaGetErrorString(e)); }
     const long long warps = (long long)total_rows * p.nq;
-    if (had) exl3_launch(ctx, attn_combine_kernel<128, true>, (unsigned)((warps + 7) / 8), 256, 0, st, p, rows_per_cta, total_rows, ctx->had_suh, ctx->had_out);
-    else     exl3_launch(ctx, attn_combine_kernel<128, false>, (unsigned)((warps + 7) / 8), 256, 0, st, p, rows_per_cta, total_rows, (const half*)nullptr, (half*)nullptr);
+    // The merge of few rows up to six blocks per SM (us, that of many and that of few: fp16, 24 rows of 40 heads 65.6 and 61.2, 4 x 32
+    // rows 48.0 and 43.2, 256 rows 451 and 452, a prefill chunk of 512 53.7 and 55.5; 4 bits, 64 rows 74.5 and 72.5, 256 rows 223.5
+    // and 225.1).
+    const bool few = (warps + 7) / 8 <= 6LL * ctx->num_sms;
+    auto merge = had ? (few ? attn_combine_few_kernel<128, true> : attn_combine_kernel<128, true>)
+                     : (few ? attn_combine_few_kernel<128, false> : attn_combine_kernel<128, false>);
+    exl3_launch(ctx, merge, (unsigned)((warps + 7) / 8), 256, 0, st, p, rows_per_cta, total_rows, had ? ctx->had_suh : (const half*)nullptr,
+                had ? ctx->had_out : (half*)nullptr);
     ctx->launches++;
     return exl3_check_launch(ctx, "attention");
 }

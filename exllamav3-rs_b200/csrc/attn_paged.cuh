@@ -137,7 +137,7 @@ __global__ void __launch_bounds__(AT_THREADS, CL ? 2 : (QB == 4 && WN == 4) ? AT
     // The cluster form waits for the kernels in front where it needs what they write, the queries and the new keys and values.  Lengths,
     // block table and the pools' older tokens were there before its chain began.
     if constexpr (CL) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    else pdl_enter();
+    else pdl_enter_late();
     constexpr int STAGES = CL ? AT_CL_STAGES : AT_STAGES;
     using SM = AttnSmem<D, QB, STAGES>;
     constexpr bool QUANT = QB > 0;

@@ -161,7 +161,7 @@ __global__ void __launch_bounds__(QD_THREADS, qd_ctas(B, NB))
 attn_qdec_kernel(const __grid_constant__ CUtensorMap map_qk, const __grid_constant__ CUtensorMap map_qv,
                  const __grid_constant__ CUtensorMap map_sk, const __grid_constant__ CUtensorMap map_sv, const AttnParams p)
 {
-    pdl_enter();
+    pdl_enter_late();
     using SM = QdSmem<B, NB>;
     constexpr int D = 128, ROWS = 8 * NB;
     extern __shared__ uint8_t qd_smem_unaligned[];

@@ -296,9 +296,10 @@ attn_qt_kernel(const __grid_constant__ CUtensorMap map_qk, const __grid_constant
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    // behind the allocation: a kernel let go before it could take the tensor memory that this one waits for
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    // behind the allocation: a kernel let go before it could take the tensor memory that this one waits for; and behind the wait, so
+    // that the merge kernel finds the work list complete
     pdl_wait();
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const uint32_t tmem = s_tmem;
     const int G = p.nq / p.nkv;
     volatile int* failed = &s_failed;

@@ -63,6 +63,13 @@ __device__ __forceinline__ void pdl_enter()
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
+// The same where the kernel behind reads, before its own wait, what the kernels in front of this one wrote.
+__device__ __forceinline__ void pdl_enter_late()
+{
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // The same for the first kernel of a call: the kernel behind it may read weights at once, so unless the work in front is known to
 // be this library's (early), it is let go only when that is complete.
 __device__ __forceinline__ void pdl_enter_first(int early)

@@ -664,3 +664,38 @@ def test_attention_of_a_small_batch_in_clusters(ctx, bits, bsz, nq, nkv, q_len, 
             O.quant_cache_paged(one[1], pools[0], pools[1], one[2], pools[2], pools[3], ctx_lens[b:b + 1], bt[b:b + 1], bits, bits)
             want = O.attn_paged(one[0], None, None, bt[b:b + 1], ctx_lens[b:b + 1], nkv=nkv, quant=(*pools, bits))
         assert _close(one[3], want, TOL_FP16 if bits == 0 else TOL_QUANT) <= 1.0, b
+
+
+@pytest.mark.parametrize("bits", [0, 4])
+@pytest.mark.parametrize("nq,nkv,q_len,totals", [(8, 2, 1, [100, 512, 2048, 2049, 8192, 8193, 16700, 300]), (32, 2, 16, [100, 512, 2048, 2100, 600] * 3)])
+def test_attention_merges_of_one_to_many_splits(ctx, bits, nq, nkv, q_len, totals):
+    """The merge of few rows behind 1, 2, 8, 9, 32, 33 and 66 splits of 256 keys, and, with 960 blocks of rows, that of many; rows behind
+    the last sequence keep what they hold.  Bars: the repository's."""
+    from oracle import oracle as O
+    r = H.rng(2400 + nq + bits)
+    bsz = len(totals)
+    ctx_lens = np.array(totals, np.int32) - q_len
+    bt, pages = H.make_paged(r, bsz, ctx_lens + q_len, nkv, 128)
+    cu = (q_len * np.arange(bsz + 1)).astype(np.int32)
+    rows = int(cu[-1])
+    rnd = lambda *s: (0.5 * r.standard_normal(s)).astype(np.float16)  # noqa: E731
+    c = dict(q=rnd(rows + 3, nq, 128), k=rnd(rows + 3, nkv, 128), v=rnd(rows + 3, nkv, 128), kc=rnd(pages, 256, nkv, 128), vc=rnd(pages, 256, nkv, 128))
+    o = H.to_dev(np.full(c["q"].shape, 7.0, np.float16))
+    q, k, v, dbt, dsl, dcu = [H.to_dev(x) for x in (c["q"], c["k"], c["v"], bt, ctx_lens, cu)]
+    if bits == 0:
+        ctx.bighead_attn_paged(q, k, v, H.to_dev(c["kc"]), H.to_dev(c["vc"]), dbt, dsl, o, cu_q=dcu, max_q_len=q_len)
+    else:
+        pools = _quant_pools(c, bits)
+        ctx.bighead_attn_paged_q(q, k, v, *_to_dev(pools), dbt, dsl, o, nkv, cu_q=dcu, max_q_len=q_len)
+    ctx.poll_status()
+    got = o.cpu().numpy()
+    assert (got[rows:] == 7.0).all()
+    for b in range(bsz):
+        one = [x[cu[b]:cu[b + 1]][None] for x in (c["q"], c["k"], c["v"], got)]
+        if bits == 0:
+            O.paged_kv_update(one[1], one[2], c["kc"], c["vc"], bt[b:b + 1], ctx_lens[b:b + 1])
+            want = O.attn_paged(one[0], c["kc"], c["vc"], bt[b:b + 1], ctx_lens[b:b + 1])
+        else:
+            O.quant_cache_paged(one[1], pools[0], pools[1], one[2], pools[2], pools[3], ctx_lens[b:b + 1], bt[b:b + 1], bits, bits)
+            want = O.attn_paged(one[0], None, None, bt[b:b + 1], ctx_lens[b:b + 1], nkv=nkv, quant=(*pools, bits))
+        assert _close(one[3], want, TOL_FP16 if bits == 0 else TOL_QUANT) <= 1.0, totals[b]
