@@ -165,9 +165,9 @@ __global__ void __launch_bounds__(AT_THREADS, CL ? 2 : (QB == 4 && WN == 4) ? AT
             const int b = blockIdx.z, parts = gridDim.x;
             kvh = blockIdx.y;
             item.b = b; item.rb = 0; item.split = blockIdx.x; item.idx = 0; item.splits = parts;
-            item.row_base = p.cu_q ? p.cu_q[b] : b * p.q_len;
-            item.ql = p.cu_q ? p.cu_q[b + 1] - item.row_base : p.q_len;
-            item.total_k = (p.seqlens ? p.seqlens[b] : 0) + (p.cu_q ? item.ql : p.kv_append);
+            item.row_base = p.cu_q ? __ldcg(p.cu_q + b) : b * p.q_len;      // (what is read ahead of the wait comes from L2)
+            item.ql = p.cu_q ? __ldcg(p.cu_q + b + 1) - item.row_base : p.q_len;
+            item.total_k = (p.seqlens ? __ldcg(p.seqlens + b) : 0) + (p.cu_q ? item.ql : p.kv_append);
             if (item.ql <= 0) return;                          // the whole cluster
             chunk = ((item.total_k + parts - 1) / parts + AT_TK - 1) / AT_TK * AT_TK;
         } else {
@@ -215,7 +215,7 @@ __global__ void __launch_bounds__(AT_THREADS, CL ? 2 : (QB == 4 && WN == 4) ? AT
                 // lookup per tile.  Thread layout: 16-byte chunk tid % 16 of keys tid / 16 + 8 i (D = 128: 16 chunks per
                 // key row).  Keys past the end of the split repeat the last valid key (masked later).
                 static_assert(D == 128, "loader assumes 16 chunks per key row");
-                const size_t tok0 = p.contig_kv ? (size_t)b * p.contig_kv + k0 : (size_t)bt[k0 >> 8] * EXL3_PAGE + (k0 & 255);
+                const size_t tok0 = p.contig_kv ? (size_t)b * p.contig_kv + k0 : (size_t)(CL ? __ldcg(bt + (k0 >> 8)) : bt[k0 >> 8]) * EXL3_PAGE + (k0 & 255);
                 const int kmax = k_end - 1 - k0;
                 const int ch = tid & 15, key0 = tid >> 4;
                 const size_t rstride = (size_t)p.nkv * D;
@@ -235,7 +235,7 @@ __global__ void __launch_bounds__(AT_THREADS, CL ? 2 : (QB == 4 && WN == 4) ? AT
                 // the other the V scales.
                 static_assert(D == 128, "loader assumes 4 groups per head");
                 const int groups = p.nkv * (D / 32);
-                const size_t tok0 = (size_t)bt[k0 >> 8] * EXL3_PAGE + (k0 & 255);
+                const size_t tok0 = (size_t)(CL ? __ldcg(bt + (k0 >> 8)) : bt[k0 >> 8]) * EXL3_PAGE + (k0 & 255);
                 const int key = tid >> 1, half_id = tid & 1;
                 const size_t tok = tok0 + min(key, k_end - 1 - k0);
                 const uint8_t* ksrc = reinterpret_cast<const uint8_t*>(p.qk + (tok * groups + kvh * 4) * p.k_bits);
@@ -253,7 +253,7 @@ __global__ void __launch_bounds__(AT_THREADS, CL ? 2 : (QB == 4 && WN == 4) ? AT
         };
 
         bool waited = !CL;
-        const int old = CL && p.seqlens ? p.seqlens[b] : 0;
+        const int old = CL && p.seqlens ? __ldcg(p.seqlens + b) : 0;
         #pragma unroll
         for (int pre = 0; pre < STAGES - 1; ++pre) {               // tiles 0 .. S-2 in flight before the loop
             if (pre < n_tiles) {

@@ -347,9 +347,14 @@ __global__ void __launch_bounds__(256) rope_kernel(const half* q, const half* k,
     const half* p; half* po; const half* nw;
     if (h < nq) { p = q + ((size_t)row * nq + h) * HD; po = out_q + ((size_t)row * nq + h) * HD; nw = q_norm; }
     else        { p = k + ((size_t)row * nk + (h - nq)) * HD; po = out_k + ((size_t)row * nk + (h - nq)) * HD; nw = k_norm; }
-    // a step's norm weights and frequencies, which its kernels only read, are there before the kernels in front are complete
+    // a step's norm weights and frequencies, which its kernels only read, and its rows' positions and slots, which are there before its
+    // chain begins, are read before the kernels in front are complete
     half nwr[EPL]; float fr[EPL / 2];
+    int pos = 0, slot = -1;
     auto ahead = [&]() {
+        if constexpr (APPEND) slot = __ldcg(dst.slot + row);
+        if (row_pos) pos = __ldcg(row_pos + row);
+        else         pos = (row % seq) + (positions ? positions[row / seq] : (int)position);
         #pragma unroll
         for (int i = 0; i < EPL; ++i) nwr[i] = nw ? nw[lane + 32 * i] : __float2half_rn(0.f);
         #pragma unroll
@@ -358,11 +363,6 @@ __global__ void __launch_bounds__(256) rope_kernel(const half* q, const half* k,
     if constexpr (APPEND) ahead();
     asm volatile("griddepcontrol.wait;" ::: "memory");
     if constexpr (!APPEND) ahead();
-    int slot = -1;
-    if constexpr (APPEND) slot = dst.slot[row];
-    int pos;
-    if (row_pos) pos = row_pos[row];
-    else         pos = (row % seq) + (positions ? positions[row / seq] : (int)position);
 
     half x[EPL];
     #pragma unroll
