@@ -812,7 +812,10 @@ int exl3_rms_norm_pre(exl3_ctx* ctx, exl3_stream stream, const void* x, int x_fp
         if (x_fp32) exl3_launch(ctx, r ? float_res : float_plain, rows, threads, 0, st, (const float*)x, wp, r, eps, cbias, cscale, dim, *pre);
         else        exl3_launch(ctx, r ? half_res : half_plain, rows, threads, 0, st, (const half*)x, wp, r, eps, cbias, cscale, dim, *pre);
     };
-    if (rows >= 128 && dim % 256 == 0 && dim <= 32 * RW_PAIRS * 256)
+    // Through the tensor core from 128 rows on where a row is long: a shorter one has too few warps then (steps of six layers, us, a block
+    // per warp and this: hidden 1024, 132 rows 712 and 742, 520 rows 814 and 843, 1052 rows 1357 and 1379; 2048, 132 rows 895 and 919, 520
+    // rows 1054 and 1075; 3072, 132 rows 1123 and 1117, 1052 rows 2523 and 2516; 4096, 192 rows 1642 and 1592; 5120, 256 rows 2138 and 2067).
+    if (rows >= 128 && dim > 2048 && dim % 256 == 0 && dim <= 32 * RW_PAIRS * 256)
         launch(rms_norm_had_wide_kernel<half, true>, rms_norm_had_wide_kernel<half, false>, rms_norm_had_wide_kernel<float, true>, rms_norm_had_wide_kernel<float, false>,
                (dim / 256 + RW_PAIRS - 1) / RW_PAIRS * 32);
     else {
@@ -836,7 +839,9 @@ int exl3_silu_mul_pre(exl3_ctx* ctx, exl3_stream stream, const void* x, const vo
     if (rows == 0) return EXL3_OK;
     const long long blocks = (long long)rows * (dim / 128);
     cudaStream_t st = (cudaStream_t)stream;
-    if (rows >= 128 && dim % 256 == 0)
+    // Through the tensor core from 256 rows on (the same steps, us, without and with it: 132 rows, hidden 1024 733 and 742, 5120 2071 and
+    // 2110; 192 rows 662 and 673, 1976 and 1980; 256 rows of 1024 716 and 717, of 2048 889 and 878; 1052 rows, 3072, 2542 and 2517).
+    if (rows >= 256 && dim % 256 == 0)
         exl3_launch(ctx, silu_mul_had_wide_kernel, (unsigned)((blocks / 2 + 8 * SW_PAIRS - 1) / (8 * SW_PAIRS)), 256, 0, st, (const half*)x, (const half*)y, pre->suh[0], pre->a_had[0], blocks / 2, dim / 256);
     else
         exl3_launch(ctx, silu_mul_had_kernel, (unsigned)((blocks + 7) / 8), 256, 0, st, (const half*)x, (const half*)y, pre->suh[0], pre->a_had[0], blocks, dim / 128);

@@ -572,18 +572,19 @@ def test_step_with_a_narrower_down_proj_keeps_separate_launches(ctx, rows):
         assert H.rel_rms_err(logits[0].numpy(), logits[1].numpy()) < 5e-3
 
 
-@pytest.mark.parametrize("hidden,inter", [(768, 1792), (1280, 512), (384, 640), (16384, 256)])
+@pytest.mark.parametrize("hidden,inter", [(768, 1792), (2304, 1792), (2560, 512), (384, 640), (16384, 256)])
 def test_transforms_of_many_rows_from_their_producers(ctx, hidden, inter):
-    """From 128 rows on norms and activation write the transforms through the tensor core, by pairs of 128-blocks: odd numbers of
-    pairs, a single pair, rows with an odd number of blocks (the shuffle versions), the widest row.  Against separate launches, whose
-    transforms are the same products (odd numbers of blocks: the same butterflies), every activation is the same number except for
-    the order in which a row's squares are summed: a few parts in 1e7 of the norm's factor, which moves single fp16 roundings.
+    """Of many rows norms (beyond 2048 wide) and activation write the transforms through the tensor core, by pairs of 128-blocks: odd
+    numbers of pairs, a single pair, short rows and rows with an odd number of blocks (the shuffle versions), the widest row.
+    Against separate launches, whose transforms are the same products (the shuffles of an even number of blocks sum in another order,
+    which moves single fp16 roundings), every activation is the same number except for the order in which a row's squares are summed:
+    a few parts in 1e7 of the norm's factor, which moves single fp16 roundings.
     Bar: the 5e-3 of the logits' RMS that such steps are held to above."""
     import os
     import exl3b200
     import torch
     from exl3b200.step import SyntheticModel
-    q_lens, ctx_lens = np.array([129, 1], np.int32), np.array([3, 40], np.int32)
+    q_lens, ctx_lens = np.array([258, 1], np.int32), np.array([3, 40], np.int32)
     bt, pages = H.make_paged(H.rng(hidden), 2, ctx_lens + q_lens, 2, 128)
     os.environ["EXL3_B200_NO_FUSED_TRANSFORM"] = "1"
     try:
@@ -592,10 +593,10 @@ def test_transforms_of_many_rows_from_their_producers(ctx, hidden, inter):
         del os.environ["EXL3_B200_NO_FUSED_TRANSFORM"]
     model = SyntheticModel(1, hidden, 2, 2, 128, inter, 512, K=4, cb=1, pages=pages, kv_bits=0, seed=hidden)
     model.fill_kv()
-    ids = torch.arange(130, device="cuda") % 512
+    ids = torch.arange(259, device="cuda") % 512
     got = []
     for c in (ctx, other):
-        _, logits = model.step(c, ids, H.to_dev(q_lens), H.to_dev(ctx_lens), H.to_dev(bt), 129, want_logits=True, all_rows=True)
+        _, logits = model.step(c, ids, H.to_dev(q_lens), H.to_dev(ctx_lens), H.to_dev(bt), 258, want_logits=True, all_rows=True)
         c.poll_status()
         got.append(logits.cpu().numpy())
     assert np.isfinite(got[0]).all()
