@@ -168,7 +168,9 @@ __global__ void __launch_bounds__(AT_THREADS, CL ? 2 : (QB == 4 && WN == 4) ? AT
             item.row_base = p.cu_q ? __ldcg(p.cu_q + b) : b * p.q_len;      // (what is read ahead of the wait comes from L2)
             item.ql = p.cu_q ? __ldcg(p.cu_q + b + 1) - item.row_base : p.q_len;
             item.total_k = (p.seqlens ? __ldcg(p.seqlens + b) : 0) + (p.cu_q ? item.ql : p.kv_append);
-            if (item.ql <= 0) return;                          // the whole cluster
+            // No rows, or more than the call declared: left out by the whole cluster, as by the work list.  (Behind the wait: a kernel
+            // none of whose blocks waited would be complete before those in front of it.)
+            if (item.ql <= 0 || item.ql > ROWS / G) { asm volatile("griddepcontrol.wait;" ::: "memory"); return; }
             chunk = ((item.total_k + parts - 1) / parts + AT_TK - 1) / AT_TK * AT_TK;
         } else {
             __syncthreads();                                   // everyone is done with the previous unit (and with s_unit)

@@ -699,3 +699,43 @@ def test_attention_merges_of_one_to_many_splits(ctx, bits, nq, nkv, q_len, total
             O.quant_cache_paged(one[1], pools[0], pools[1], one[2], pools[2], pools[3], ctx_lens[b:b + 1], bt[b:b + 1], bits, bits)
             want = O.attn_paged(one[0], None, None, bt[b:b + 1], ctx_lens[b:b + 1], nkv=nkv, quant=(*pools, bits))
         assert _close(one[3], want, TOL_FP16 if bits == 0 else TOL_QUANT) <= 1.0, totals[b]
+
+
+@pytest.mark.parametrize("bits", [0, 6])
+@pytest.mark.parametrize("q_lens,nq,nkv", [([1, 9, 2, 17, 0], 16, 8), ([1, 300, 2], 16, 8), ([2, 5, 1], 32, 8), ([0, 0, 0], 16, 8)])
+def test_sequences_longer_than_declared_are_left_out(ctx, bits, q_lens, nq, nkv):
+    """A small batch whose row counts on the device have outgrown the declared two (17 and more packed rows): those sequences' rows
+    keep what they hold and the others are right, as through a work list, which a block table too wide for clusters takes; a batch
+    without any rows."""
+    from oracle import oracle as O
+    r = H.rng(2500 + bits + len(q_lens))
+    bsz, q_lens = len(q_lens), np.array(q_lens, np.int32)
+    ctx_lens = np.array([70 + 41 * b for b in range(bsz)], np.int32)
+    bt, pages = H.make_paged(r, bsz, ctx_lens + q_lens, nkv, 128)
+    cu = np.concatenate([[0], np.cumsum(q_lens)]).astype(np.int32)
+    rows = max(int(cu[-1]), 1)
+    rnd = lambda *s: (0.5 * r.standard_normal(s)).astype(np.float16)  # noqa: E731
+    c = dict(q=rnd(rows, nq, 128), k=rnd(rows, nkv, 128), v=rnd(rows, nkv, 128), kc=rnd(pages, 256, nkv, 128), vc=rnd(pages, 256, nkv, 128))
+    pools = [c["kc"], c["vc"]] if bits == 0 else _quant_pools(c, bits)
+    q, k, v, dsl, dcu = [H.to_dev(x) for x in (c["q"], c["k"], c["v"], ctx_lens, cu)]
+    for table in (bt, np.pad(bt, ((0, 0), (0, 64)))):
+        o = H.to_dev(np.full(c["q"].shape, 7.0, np.float16))
+        if bits == 0:
+            ctx.bighead_attn_paged(q, k, v, *_to_dev(pools), H.to_dev(table), dsl, o, cu_q=dcu, max_q_len=2)
+        else:
+            ctx.bighead_attn_paged_q(q, k, v, *_to_dev(pools), H.to_dev(table), dsl, o, nkv, cu_q=dcu, max_q_len=2)
+        ctx.poll_status()
+        got = o.cpu().numpy()
+        for b in range(bsz):
+            if q_lens[b] * nq // nkv > 16:
+                assert (got[cu[b]:cu[b + 1]] == 7.0).all()
+            elif q_lens[b]:
+                one, now = [x[cu[b]:cu[b + 1]][None] for x in (c["q"], c["k"], c["v"], got)], [x.copy() for x in pools]
+                if bits == 0:
+                    O.paged_kv_update(one[1], one[2], *now, bt[b:b + 1], ctx_lens[b:b + 1])
+                    want = O.attn_paged(one[0], *now, bt[b:b + 1], ctx_lens[b:b + 1])
+                else:
+                    O.quant_cache_paged(one[1], now[0], now[1], one[2], now[2], now[3], ctx_lens[b:b + 1], bt[b:b + 1], bits, bits)
+                    want = O.attn_paged(one[0], None, None, bt[b:b + 1], ctx_lens[b:b + 1], nkv=nkv, quant=(*now, bits))
+                assert _close(one[3], want, TOL_FP16 if bits == 0 else TOL_QUANT) <= 1.0, b
+        assert (got[cu[-1]:] == 7.0).all()
