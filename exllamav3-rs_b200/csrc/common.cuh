@@ -79,12 +79,9 @@ __device__ __forceinline__ void pdl_enter_first(int early)
     if (!early) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
-// 128-point Hadamard transform of (x o signs) for a block whose elements 4 * lane + j are a, b of lane `lane`; `signs` holds the
-// lane's four.  Same arithmetic as the GEMM's input transform of few rows: fp16 product, fp32 butterflies, one fp16 rounding.
-__device__ __forceinline__ uint2 had128_signed_lane(half2 a, half2 b, uint2 signs, int lane)
+// 128-point Hadamard transform of a block whose elements 4 * lane + j are a, b of lane `lane`: fp32 butterflies, one fp16 rounding.
+__device__ __forceinline__ uint2 had128_lane(half2 a, half2 b, int lane)
 {
-    a = __hmul2(a, *reinterpret_cast<const half2*>(&signs.x));
-    b = __hmul2(b, *reinterpret_cast<const half2*>(&signs.y));
     float v0 = __low2float(a), v1 = __high2float(a), v2 = __low2float(b), v3 = __high2float(b);
     const float s0 = v0 + v1, d0 = v0 - v1, s1 = v2 + v3, d1 = v2 - v3;
     v0 = s0 + s1; v1 = d0 + d1; v2 = s0 - s1; v3 = d0 - d1;
@@ -101,6 +98,11 @@ __device__ __forceinline__ uint2 had128_signed_lane(half2 a, half2 b, uint2 sign
     b = __floats2half2_rn(v2 * R128, v3 * R128);
     uint2 o; o.x = *reinterpret_cast<uint32_t*>(&a); o.y = *reinterpret_cast<uint32_t*>(&b);
     return o;
+}
+// The same of (x o signs), `signs` holding the lane's four.  Same arithmetic as the GEMM's input transform of few rows: fp16 product first.
+__device__ __forceinline__ uint2 had128_signed_lane(half2 a, half2 b, uint2 signs, int lane)
+{
+    return had128_lane(__hmul2(a, *reinterpret_cast<const half2*>(&signs.x)), __hmul2(b, *reinterpret_cast<const half2*>(&signs.y)), lane);
 }
 
 // Launch as a programmatic dependent of the previous kernel where the context says that there is one: the launch then

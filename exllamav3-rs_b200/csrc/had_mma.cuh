@@ -1,15 +1,31 @@
 // 128-point Hadamard transform of two neighbouring blocks by a warp, with the butterflies on the tensor core.  H128 = H8 (x) H16 on
 // the index i = 16 a + b: X[a][b] of both blocks goes through shared memory into transposed MMA fragments (ldmatrix.trans),
-// D0 = (H8 (+) H8) X contracts over a with the sign matrix as the A operand, D0 - kept exact as an fp16 pair hi + lo - becomes the A
-// operand of the second product Y = D0 H16, whose columns are ordered so that a lane ends up with four consecutive outputs.
-// About a quarter of the instructions of the shuffle version (which needs 20 shuffles per 4 values); sums are formed in another
-// order than hadamard_inner.cuh:93-147 does, so single results may differ from the shuffle version's by one fp16 step where the
-// fp32 value sits on a rounding boundary.
+// D0 = (H8 (+) H8) X contracts over a with the sign matrix as the A operand, D0 - as an fp16 pair hi + lo, which keeps 22 of its bits -
+// becomes the A operand of the second product Y = D0 H16, whose columns are ordered so that a lane ends up with four consecutive
+// outputs.  About a quarter of the instructions of the shuffle version (which needs 20 shuffles per 4 values); sums are formed in
+// another order than hadamard_inner.cuh:93-147 does, so single results may differ from the shuffle version's by one fp16 step where
+// the fp32 value sits on a rounding boundary.
+// D0 is a sum of eight fp16 values and may leave fp16's range where the transform, which is 0.088 of such sums, does not.  A pair of
+// blocks with such a sum, or with an infinity or a NaN among its values, goes through the shuffles, whose fp32 sums hold every input.
+// (What the test costs, us without and with it: four layers of hidden 5120, 28 rows beside 4 x 256, 4334 and 4346; calls of 5120 x 17408
+// at 4 bits, 52 rows 28.7 and 28.8, 2048 rows 321 and 320.  Of D0's size, with the shuffles in line: 4248 and 4267, 28.8 and 29.1.)
 #pragma once
-#include <cuda_fp16.h>
-#include <stdint.h>
+#include "common.cuh"
 
 namespace exl3 {
+
+// the two blocks of 128 values in the warp's `stage` by shuffles; a call, because the code is seldom needed
+static __device__ __noinline__ uint4 had_shuffles(const uint8_t* stage, int lane)
+{
+    uint2 o[2];
+    #pragma unroll
+    for (int blk = 0; blk < 2; ++blk) {
+        const uint2 v = *reinterpret_cast<const uint2*>(stage + blk * 256 + lane * 8);
+        o[blk] = had128_lane(*reinterpret_cast<const half2*>(&v.x), *reinterpret_cast<const half2*>(&v.y), lane);
+    }
+    __syncwarp();
+    return make_uint4(o[0].x, o[0].y, o[1].x, o[1].y);
+}
 
 struct HadMma {
     uint32_t h8, hb[2][2];             // H8 (+) H8 as A of the first product, H16 with permuted columns as B of the second
@@ -79,6 +95,11 @@ struct HadMma {
             const half2 p = __floats2half2_rn(y[0][2 * blk] * r128, y[0][2 * blk + 1] * r128);
             const half2 q = __floats2half2_rn(y[1][2 * blk] * r128, y[1][2 * blk + 1] * r128);
             out[blk].x = *reinterpret_cast<const uint32_t*>(&p); out[blk].y = *reinterpret_cast<const uint32_t*>(&q);
+        }
+        // a hi beyond fp16 is a NaN in all sixteen outputs of its row, of which a lane has y[0][0] or y[0][2] (inf - inf in the products)
+        if (__any_sync(0xffffffffu, !(fabsf(y[0][0] + y[0][2]) < INFINITY))) {
+            const uint4 o = had_shuffles(stage, lane);
+            out[0] = make_uint2(o.x, o.y); out[1] = make_uint2(o.z, o.w);
         }
     }
     static __device__ __forceinline__ int offset(int lane) { return 16 * (lane >> 2) + 4 * (lane & 3); }

@@ -497,3 +497,35 @@ def test_gemm_tc_half_slab(ctx, ctx_small_only, m, n):
     """column counts with n % 256 == 128: the last slab has one valid 128-column half (decoded by one CTA of the pair, the
     other half reads zero-filled codes and is never stored)"""
     _tc_case(ctx, ctx_small_only, None, m, 1024, n, 4, 1, m == 200, 1600 + m + n, oracle=(m <= 200))
+
+
+@pytest.mark.parametrize("m", [17, 32, 300])
+def test_gemm_transform_holds_large_activations(ctx, m):
+    """Activations whose sums of eight leave fp16 (65 504) while the transform, 0.088 of such sums, does not: two values of 40 000
+    sixteen apart, eight of 60 000, eight of alternating 65 504, beside ordinary rows.  Against the oracle, and against calls of eight
+    rows, whose transforms are fp32 shuffles.  Rows with an infinity or a NaN are not finite in either and leave the others alone."""
+    from oracle import oracle as O
+    torch = _torch()
+    r = H.rng(1900 + m)
+    k, n, K, cb = 512, 384, 4, 1
+    A = r.standard_normal((m, k)).astype(np.float32)
+    tr, suh, svh = H.rand_trellis(r, k, n, K), H.rand_signs(r, k), (H.rand_signs(r, n) / 32).astype(np.float16)
+    A[0, [3, 19]] = 40000
+    A[1, 256 + 7:384:16] = 60000
+    A[m - 1, 2:128:16] = 65504 * (1 - 2 * (np.arange(8) & 1))
+    A[2, 130], A[5, 5] = np.inf, np.nan
+    A = (A * suh).astype(np.float16)                               # the signs multiply out: values as above
+    out = torch.empty((m, n), dtype=torch.float32, device="cuda")
+    part = torch.empty_like(out)
+    dA, dtr, dsuh, dsvh = [H.to_dev(x) for x in (A, tr, suh, svh)]
+    ctx.exl3_gemm(dA, dtr, out, dsuh, None, dsvh, mcg=True)
+    for i in range(0, m, 8):
+        ctx.exl3_gemm(dA[i:i + 8], dtr, part[i:i + 8], dsuh, None, dsvh, mcg=True)
+    ctx.poll_status()
+    got, part = out.cpu().numpy(), part.cpu().numpy()
+    fine = [i for i in range(m) if i not in (2, 5)]
+    assert np.isfinite(got[fine]).all()
+    assert not np.isfinite(got[[2, 5]]).all(axis=1).any()
+    want = O.exl3_gemm(A[fine], tr, suh, svh, K, cb, c_fp32=True)
+    for g, p, w in zip(got[fine], part[fine], want):               # each row against its own size
+        assert H.rel_rms_err(g, w) < GEMM_TOL and H.rel_rms_err(g, p) < GEMM_TOL

@@ -601,3 +601,45 @@ def test_transforms_of_many_rows_from_their_producers(ctx, hidden, inter):
         got.append(logits.cpu().numpy())
     assert np.isfinite(got[0]).all()
     assert H.rel_rms_err(got[0], got[1]) < 5e-3
+
+
+def test_activation_of_many_rows_holds_large_values(ctx):
+    """SiLU(gate) x up is bounded by nothing but fp16: eight columns of every block, sixteen apart, are given values up to its end, whose
+    sums leave it in some blocks.  From 256 rows on the transform goes through the tensor core, at 255 through shuffles: the same
+    rows are finite in both (an activation that is itself beyond fp16 makes its row infinite in either), and of the same values.
+    down_proj's weights are small ones of the codebook, whose products with such rows fp16 holds.
+    Bar: the 5e-3 of the logits' RMS that steps with another order of sums are held to above."""
+    import torch
+    from exl3b200.step import SyntheticModel
+    from oracle import oracle as O
+    r = H.rng(61)
+    bt, pages = H.make_paged(r, 1, np.array([1060], np.int32), 2, 128)
+    model = SyntheticModel(1, 512, 2, 2, 128, 1792, 512, K=8, cb=1, pages=pages, kv_bits=0, seed=61)
+    for name in ("gate_proj", "up_proj"):
+        svh = model.layers[0][name].svh
+        svh *= torch.where(torch.arange(1792, device="cuda") % 16 == 5, 80.0, 0.1).to(torch.float16)
+    # at 8 bits a state is two neighbouring bytes of a tile's ring, most significant first in words of 32 bits
+    small = (np.abs(O.codebook(1).astype(np.float32)) < 0.05).reshape(256, 256)
+    rings = []
+    while len(rings) < 16:
+        ring = [int(r.integers(0, 256))]
+        while len(ring) < 256 and small[ring[-1]].any():
+            ring.append(int(r.choice(np.flatnonzero(small[ring[-1]]))))
+        if len(ring) == 256 and small[ring[-1], ring[0]]:
+            rings.append(ring)
+    words = np.array(rings, np.uint8).reshape(16, 64, 4)[:, :, ::-1].copy().view(np.int16).reshape(16, 128)
+    down = model.layers[0]["down_proj"].trellis
+    trellis = words[r.integers(0, 16, down.shape[:2])]
+    assert np.abs(O.reconstruct(trellis[:2, :2], 8, 1).astype(np.float32)).max() < 0.05
+    down.copy_(torch.from_numpy(trellis))
+    ids = torch.from_numpy(r.integers(0, 512, 1052)).cuda()
+    got = {}
+    for rows in (255, 256, 1052):
+        q_lens = H.to_dev(np.array([rows], np.int32))
+        got[rows] = model.step(ctx, ids[:rows], q_lens, H.to_dev(np.zeros(1, np.int32)), H.to_dev(bt), rows, want_logits=True, all_rows=True)[1].cpu().numpy()[:255]
+        ctx.poll_status()
+    fine = np.isfinite(got[255]).all(axis=1)
+    assert fine.sum() > 200
+    for rows in (256, 1052):
+        assert np.array_equal(np.isfinite(got[rows]).all(axis=1), fine)
+        assert H.rel_rms_err(got[rows][fine], got[255][fine]) < 5e-3
