@@ -542,8 +542,12 @@ int attn_impl(exl3_ctx* ctx, cudaStream_t st, AttnParams p, int total_rows, int 
     const bool general_single = max_rows <= dec_rows || !p.cu_q;
     // A small batch in clusters (attn_paged.cuh): at most two CTAs per SM with as many parts per sequence and kv head as that allows, and
     // at most 512 keys per part, by the width of the block table: a longer sequence among short ones would hold up the others'
-    // SMs, which the work list shares out.  Us: step of 28 layers of hidden 1024, 8 sequences of up to 1024 tokens, 1470 -> 1312
-    // (attention per layer 13.7 -> 8.5; 10.3 without the reads ahead of the wait); 6-bit pools, 8 of up to 1024, 31.6 -> 24.2 a call.
+    // SMs, which the work list shares out.  Us, list and clusters: step of 28 layers of hidden 1024, 8 sequences of up to 1024 tokens,
+    // 1409 and 1332; calls of 16 / 8 heads over fp16 pools, replayed, 8 sequences of 1000 keys 15.8 and 13.7, of 2000 24.9 and 20.0, one
+    // of 2000 among seven of 64 14.4 and 13.6, but one of 4000 15.7 and 21.5; one of 4000 among three of 64 (eight parts) 15.7 and 13.9,
+    // among fifteen (two parts) 16.0 and 37.4; one sequence of 64 9.8 and 5.4, of 4000 15.2 and 13.0, of 8000 17.6 and 21.0.  Twice the
+    // parts, four CTAs per SM: 8 of 1000 17.6, 16 of 500 16.8 against 13.9 in two parts; 32 of 500 in two parts 23.4 and by the list 25.3,
+    // 32 of 250 16.5 and 15.3.
     int parts = 0;
     if (max_rows <= 16 && !codes && !p.contig_kv)
         for (int c = 8; c >= 2 && parts == 0; c >>= 1)

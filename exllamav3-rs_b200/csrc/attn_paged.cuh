@@ -112,6 +112,7 @@ __device__ __forceinline__ uint32_t at_peer(const void* p, int cta)
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(cta));
     return a;
 }
+__device__ __forceinline__ void at_prefetch(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 __device__ __forceinline__ float4 at_ld_peer4(uint32_t a)
 {
     float4 v;
@@ -134,8 +135,10 @@ template <int D, int WM, int WN, int QB, bool CL = false>
 __global__ void __launch_bounds__(AT_THREADS, CL ? 2 : (QB == 4 && WN == 4) ? AT_Q4_DECODE_BLOCKS : 1) attn_paged_kernel(const AttnParams p)
 {
     static_assert(!CL || (WM == 1 && D == 128), "a cluster shares one block of 16 rows");
-    // The cluster form waits for the kernels in front where it needs what they write, the queries and the new keys and values.  Lengths,
-    // block table and the pools' older tokens were there before its chain began.
+    // The cluster form reads lengths and block table, which were there before its chain began, ahead of its wait for the kernels in front,
+    // and requests the first tiles' lines into L2.  The pools themselves are read behind it: a token that is old to one sequence may be
+    // new to another one of the batch (two entries over one block table), and then the kernel in front is writing it.  (Read ahead of
+    // the wait, the step of 28 layers with 8 rows took 1306 us instead of 1329.)
     if constexpr (CL) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     else pdl_enter_late();
     constexpr int STAGES = CL ? AT_CL_STAGES : AT_STAGES;
@@ -254,17 +257,31 @@ __global__ void __launch_bounds__(AT_THREADS, CL ? 2 : (QB == 4 && WN == 4) ? AT
             }
         };
 
-        bool waited = !CL;
-        const int old = CL && p.seqlens ? __ldcg(p.seqlens + b) : 0;
+        if constexpr (CL) {
+            // ahead of the wait, the lines of the tiles that the loop below begins with: two threads per key, of K and of V
+            #pragma unroll
+            for (int pre = 0; pre < STAGES - 1; ++pre)
+                if (pre < n_tiles) {
+                    const int k0 = k_begin + pre * AT_TK, half_id = tid & 1;
+                    const size_t tok = (size_t)__ldcg(bt + (k0 >> 8)) * EXL3_PAGE + (k0 & 255) + min(tid >> 1, k_end - 1 - k0);
+                    if constexpr (!QUANT) {
+                        const size_t at = (tok * p.nkv + kvh) * D + half_id * 64;
+                        at_prefetch(p.kc + at); at_prefetch(p.vc + at);
+                    } else {
+                        const size_t group = tok * p.nkv * (D / 32) + kvh * 4;
+                        const int bits = half_id ? p.v_bits : p.k_bits;
+                        const uint32_t* codes = (half_id ? p.qv : p.qk) + group * bits;
+                        at_prefetch(codes); at_prefetch(codes + 4 * bits - 1);
+                        at_prefetch((half_id ? p.sv : p.sk) + group);
+                    }
+                }
+            asm volatile("griddepcontrol.wait;" ::: "memory");
+        }
         #pragma unroll
         for (int pre = 0; pre < STAGES - 1; ++pre) {               // tiles 0 .. S-2 in flight before the loop
-            if (pre < n_tiles) {
-                if (!waited && min(k_begin + (pre + 1) * AT_TK, k_end) > old) { asm volatile("griddepcontrol.wait;" ::: "memory"); waited = true; }
-                load_tile(pre, pre);
-            }
+            if (pre < n_tiles) load_tile(pre, pre);
             cp_async_commit();
         }
-        if (!waited) asm volatile("griddepcontrol.wait;" ::: "memory");
 
         // ---- Q fragments (A operand), straight from global memory
         uint32_t qf[KSTEPS][4];

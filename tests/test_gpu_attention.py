@@ -739,3 +739,60 @@ def test_sequences_longer_than_declared_are_left_out(ctx, bits, q_lens, nq, nkv)
                     want = O.attn_paged(one[0], None, None, bt[b:b + 1], ctx_lens[b:b + 1], nkv=nkv, quant=(*now, bits))
                 assert _close(one[3], want, TOL_FP16 if bits == 0 else TOL_QUANT) <= 1.0, b
         assert (got[cu[-1]:] == 7.0).all()
+
+
+@pytest.mark.parametrize("bits", [0, 6])
+def test_entries_over_one_block_table(ctx, bits):
+    """Two batch entries that are consecutive rows of one sequence: what the first appends is old to the second, and the call appends
+    before it attends.  A small batch (clusters), eager and twenty times back to back with the lengths moved on, and replayed from a
+    graph, each over pools that hold something else where the new rows go."""
+    import exl3b200
+    from oracle import oracle as O
+    torch = _torch()
+    r = H.rng(2600 + bits)
+    nq, nkv, n, calls = 16, 8, 4, 20
+    bt, pages = H.make_paged(r, 1, np.array([256 + 2 * n * calls]), nkv, 128)
+    bt = np.repeat(bt, 2, 0)
+    rnd = lambda *s: (0.5 * r.standard_normal(s)).astype(np.float16)  # noqa: E731
+    c = dict(kc=rnd(pages, 256, nkv, 128), vc=rnd(pages, 256, nkv, 128))
+    start = [c["kc"], c["vc"]] if bits == 0 else _quant_pools(c, bits)
+    q, k, v = rnd(calls, 2, n, nq, 128), rnd(calls, 2, n, nkv, 128), rnd(calls, 2, n, nkv, 128)
+    lens = np.array([[250 + 2 * n * i, 250 + 2 * n * i + n] for i in range(calls)], np.int32)
+    dq, dk, dv, dl, dbt = [H.to_dev(x) for x in (q, k, v, lens, bt)]
+    o = torch.full(q.shape, float("nan"), dtype=torch.float16, device="cuda")
+    dev = _to_dev(start)
+
+    def call(i, stream=None):
+        if bits == 0:
+            ctx.bighead_attn_paged(dq[i], dk[i], dv[i], *dev, dbt, dl[i], o[i], stream=stream)
+        else:
+            ctx.bighead_attn_paged_q(dq[i], dk[i], dv[i], *dev, dbt, dl[i], o[i], nkv, stream=stream)
+
+    n0 = ctx.launch_count()
+    for i in range(calls):
+        call(i)
+    assert ctx.launch_count() - n0 == 2 * calls
+    ctx.poll_status()
+    got = o.cpu().numpy()
+    now = [x.copy() for x in start]
+    for i in range(calls):
+        for e in range(2):
+            if bits == 0:
+                O.paged_kv_update(k[i, e:e + 1], v[i, e:e + 1], *now, bt[:1], lens[i, e:e + 1])
+            else:
+                O.quant_cache_paged(k[i, e:e + 1], now[0], now[1], v[i, e:e + 1], now[2], now[3], lens[i, e:e + 1], bt[:1], bits, bits)
+        want = O.attn_paged(q[i], *now, bt, lens[i]) if bits == 0 else O.attn_paged(q[i], None, None, bt, lens[i], nkv=nkv, quant=(*now, bits))
+        assert _close(got[i], want, TOL_FP16 if bits == 0 else TOL_QUANT) <= 1.0, i
+    for a, b in zip(dev, start):
+        a.copy_(H.to_dev(b))
+    o.fill_(float("nan"))
+    g = exl3b200.CudaGraph(ctx)
+    torch.cuda.synchronize()
+    g.capture_begin()
+    for i in range(calls):
+        call(i, g.side_stream())
+    g.capture_end()
+    g.replay()
+    assert exl3b200.lib().exl3_sync_side_stream(ctx.handle) == 0
+    ctx.poll_status()
+    assert np.array_equal(o.cpu().numpy().view(np.uint16), got.view(np.uint16))

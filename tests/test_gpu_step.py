@@ -643,3 +643,49 @@ def test_activation_of_many_rows_holds_large_values(ctx):
     for rows in (256, 1052):
         assert np.array_equal(np.isfinite(got[rows]).all(axis=1), fine)
         assert H.rel_rms_err(got[rows][fine], got[255][fine]) < 5e-3
+
+
+@pytest.mark.parametrize("kv_bits", [0, 6])
+@pytest.mark.parametrize("graph", [False, True])
+def test_steps_over_entries_of_one_sequence(ctx, kv_bits, graph):
+    """A step whose entries are consecutive rows of one sequence, twenty steps back to back: what an entry attends to as old, another's
+    rows of the same step have just written.  The small batch's clusters against the work list, which a wider block table takes: the
+    same but for the order of sums.  Bars on the relative 2-norm: fp16 roundings that fall the other way, some 24 of 2e-4 each way in
+    two layers, 1.4e-3, twice that; at 6 bits a key or value on the border of two codes may be stored as either, which at 4 bits is
+    1.4e-2 and at 8 bits 2.5e-3 of the logits (above): 6e-3 between them, twice that."""
+    import exl3b200
+    import torch
+    from exl3b200.step import SyntheticModel
+    steps, entries, n = 20, 3, 2
+    r = H.rng(62 + kv_bits)
+    bt, pages = H.make_paged(r, 1, np.array([100 + steps * entries * n]), 2, 128)
+    bt = np.repeat(bt, entries, 0)
+    q_lens = H.to_dev(np.full(entries, n, np.int32))
+    lens = H.to_dev(np.array([[100 + (i * entries + e) * n for e in range(entries)] for i in range(steps)], np.int32))
+    ids = H.to_dev(r.integers(0, 512, (steps, entries * n)))
+    got = []
+    for table in (bt, np.pad(bt, ((0, 0), (0, 64)))):
+        table = H.to_dev(table)
+        model = SyntheticModel(2, 512, 4, 2, 128, 512, 512, K=4, cb=1, pages=pages, kv_bits=kv_bits, seed=62)
+        model.fill_kv()
+        tokens = torch.empty(entries * n, dtype=torch.int64, device="cuda")
+        call = lambda stream=None: [model.step(ctx, ids[i], q_lens, lens[i], table, n, want_logits=True, stream=stream, tokens_out=tokens, all_rows=True)[1]  # noqa: E731
+                                    for i in range(steps)]
+        if graph:
+            model.step(ctx, ids[0], q_lens, lens[0], table, n, want_logits=True, tokens_out=tokens, all_rows=True)
+            model.fill_kv()
+            g = exl3b200.CudaGraph(ctx)
+            torch.cuda.synchronize()
+            g.capture_begin()
+            logits = call(g.side_stream())
+            g.capture_end()
+            g.replay()
+            assert exl3b200.lib().exl3_sync_side_stream(ctx.handle) == 0
+        else:
+            logits = call()
+        ctx.poll_status()
+        got.append(torch.stack(logits).cpu().numpy())
+    assert np.isfinite(got[0]).all()
+    err = [np.linalg.norm(a - b) / np.linalg.norm(b) for a, b in zip(*got)]
+    print(f"{kv_bits} bits: relative 2-norm up to {max(err):.2e}")
+    assert max(err) < (2.8e-3 if kv_bits == 0 else 1.2e-2)
