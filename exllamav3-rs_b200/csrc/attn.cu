@@ -358,6 +358,12 @@ cudaError_t launch_attn_qt(exl3_ctx* ctx, const AttnParams& p, dim3 grid, cudaSt
 
 bool qdec_kernel_applies(const AttnParams& p, bool quant);
 
+// at least so many sequences of a batch have more than one row
+int min_long(int total_rows, int bsz, int max_q_len)
+{
+    return max_q_len > 1 ? (int)std::max(0LL, ((long long)total_rows - bsz + max_q_len - 2) / (max_q_len - 1)) : 0;
+}
+
 // Which kernels a pass runs: those for few packed rows, those for more, or (4-bit and 8-bit pools) the tcgen05 kernel over codes.
 enum AttnClass { ATTN_FEW, ATTN_MANY, ATTN_CODES };
 
@@ -403,7 +409,12 @@ int attn_pass(exl3_ctx* ctx, cudaStream_t st, AttnParams p, int total_rows, int 
     // quantised pools, whose units start with the rotation of their queries (24 sequences, contexts 512 .. 16384, 40 / 8
     // heads, one and two items: 4 bits, 5 rows 68 and 72 us, 40 rows 188 and 193; 8 bits 68 and 75, 188 and 196).
     static const int dec_items = getenv("EXL3_TUNE_DEC_ITEMS") ? atoi(getenv("EXL3_TUNE_DEC_ITEMS")) : 0;
-    const int target_items = grid_x * (use_tc ? (tc_items ? tc_items : 2) : (dec_items ? dec_items : (use_qdec || use_qt ? 1 : 2)));
+    // The tcgen05 kernel over codes: one item per slot while its blocks are few, else two, which balance them (us, one and two: 4
+    // sequences of 65 rows, 512 .. 4096, 35 and 37, of 100, 512 .. 4096, 32 and 44, 1024 .. 32768 110 and 98, of 500 506 and 368; one of 250
+    // rows, 512 .. 4096, 25 and 35, of 500, 1024 .. 32768, 110 and 83; 16 of 250, 1024 .. 32768, 830 and 717).
+    const int n_long = min_long(total_rows, p.bsz, max_rows / G);
+    const bool qt_few = use_qt && 3LL * ((long long)n_long * rb_max + (rows_lo == 0 ? p.bsz - n_long : 0)) <= grid_x;
+    const int target_items = grid_x * (use_tc ? (tc_items ? tc_items : 2) : (dec_items ? dec_items : (use_qdec || qt_few ? 1 : 2)));
     // items <= target + sum of row blocks (every (sequence, row block) rounds its split count up once); the row blocks are
     // bounded by bsz * rb_max and, usually much tighter for ragged batches, by total_rows * G / rows_per_cta + bsz
     const long long rb_sum = std::min((long long)p.bsz * rb_max, ((long long)total_rows * G + rows_per_cta - 1) / rows_per_cta + p.bsz);
@@ -510,20 +521,30 @@ int attn_impl(exl3_ctx* ctx, cudaStream_t st, AttnParams p, int total_rows, int 
     // use, was measured on the benchmark step: the attention stage takes the same 28.0 ms of the step's 83.)
     const int dec_rows = qdec_kernel_applies(p, quant) ? 48 : 16;
     // The tcgen05 kernel over codes unpacks them once for 40 rows; its blocks cost the same however few of those they hold, and a unit
-    // some 10 us before and behind its tiles.  So, us, the other kernels and it (40 / 8 heads unless said):
-    //  * sequences of 33 to 48 rows at 4 bits, where there is work for all SMs: 4 of 40 rows, contexts 1024 .. 32768, 64 -> 47; 32 of
-    //    them, 128 .. 4000, 77 -> 64; 12 of 35 rows, 512 .. 8192, 71 -> 55; but 4 of 40 rows, 256 .. 8000, 33 and 33, one over 4000
-    //    keys 26 to 33 and 30 to 33.  The pages of the block table bound the work from above.  At 8 bits, where the ring of codes
-    //    has one slot: 67 and 67.  Up to 32 rows two blocks of 16 of the other kernel are as good (24 of 25 rows 94 and 94).
-    //  * longer ones: 3 of 100 rows, 500 .. 4000, 4 bits 106 -> 98, 8 bits 140 -> 134; one of 128 over 4000 keys 102 -> 82, 124 ->
-    //    111; 16 / 8 heads 55 -> 42, 71 -> 54; behind at 8 bits with 1024 packed rows (110 and 120) and on 3 of 60 rows at 16 / 8
-    //    heads (41 and 46).
-    //  * a ragged batch of both kinds in one pass instead of two, unless it has many sequences of a row: 28 and 2 of 64 rows, 4 bits
-    //    112 -> 93, 8 bits 149 -> 139; 4 and one of 24 rows 45 -> 26; 64 and one of 50 rows 56 and 62, 63 and 82.
-    const bool codes = qdec_kernel_applies(p, quant), long_codes = codes && max_rows > dec_rows && (p.k_bits == 4 || max_rows <= 800);
-    const int n_long = max_q_len > 1 ? (int)std::max(0LL, ((long long)total_rows - p.bsz + max_q_len - 2) / (max_q_len - 1)) : 0;     // at least so many have more than a row
-    const bool codes_alone = long_codes ? !p.cu_q || p.bsz - n_long <= 40
-                                        : codes && p.k_bits == 4 && max_rows > 32 && max_rows <= dec_rows && (long long)p.bsz * p.pps >= 200;
+    // some 10 us before and behind its tiles.  So, us, the other kernels and it (40 / 8 heads unless said, contexts spread evenly over
+    // the logarithm of a range, calls replayed):
+    //  * one block per sequence, 33 to 40 rows, at 4 bits, where the pages of the block table leave room for work for all SMs: 4 of 40
+    //    rows, 1024 .. 32768, 72 and 43; 12, 512 .. 4096, 50 and 41; 32, 128 .. 1024, 45 and 42; but 6, 128 .. 1024, 20.7 and 21.2, one,
+    //    128 .. 8192, 20 and 21.  Beside sequences of few rows, up to half as many: 8 of a row beside 16 of 40, 1024 .. 32768, 268 and
+    //    185, 512 .. 4096 69 and 62, 128 .. 1024 36 and 41; 8 beside 4, 128 .. 8192, 41 and 41, 128 .. 1024 21 and 23; 28 beside 4 51 and
+    //    70; 64 beside one 70 and 107; and with half the kv heads and so half the work 4 beside 12, 512 .. 4096, 32 and 38, 128 .. 8192 37
+    //    and 31.  Two blocks, 41 to 48 rows: 12 of 44, 128 .. 8192, 57 and 63, 32 of 48 with four kv heads 67 and 74.  At 8 bits, where the
+    //    ring of codes has one slot, 4 of 45, 1024 .. 32768, 82 and 117.
+    //  * more rows: 4 of 65 rows, 512 .. 4096, 43 and 35, of 120 47 and 33, of 500 124 and 109; 16 of 640, 1024 .. 32768, 1945 and 1531; at 8
+    //    bits 58 and 43, 63 and 42, 166 and 148, 3013 and 2361.  The other kernel's block has 64 rows: up to that many, 4 of 50, 512 .. 4096,
+    //    28 and 33, 16, 1024 .. 32768, 232 and 232, at 8 bits 334 and 361; one alone 26 and 20, 35 and 23, and of a ragged
+    //    batch, where the other kernel is a pass beside that of few rows, 8 of a row and 3 of 50 46 and 43, 58 and 52.  (8 bits with more
+    //    than 800 rows stay where they were.)
+    //  * a ragged batch of both kinds in one pass instead of two, as long as the short ones have few keys, by the width of the block table:
+    //    8 of a row and one of 100, two passes and one, 128 .. 1024 (5 pages) 25 and 20, 512 .. 4096 (17) 42 and 33, 1024 .. 32768 (129) 80 and
+    //    94; 32 and one 39 and 30, 63 and 64, 168 and 223; at 8 bits 29 and 23, 47 and 43, 89 and 142; 44 and 38, 71 and 96, 171 and 359.
+    const bool codes = qdec_kernel_applies(p, quant);
+    const int n_long = min_long(total_rows, p.bsz, max_q_len);
+    const long long table = (long long)p.bsz * p.pps;
+    const bool long_codes = codes && max_rows > dec_rows && (p.k_bits == 4 || max_rows <= 800) && (max_rows > 64 || p.cu_q || p.bsz == 1);
+    const bool codes_alone = long_codes ? (long long)(p.bsz - n_long) * p.pps <= (p.k_bits == 4 ? 300 : 200)
+                                        : codes && p.k_bits == 4 && max_rows > 32 && max_rows <= QT_ROWS && table >= 200 &&
+                                          (n_long >= p.bsz || (3 * n_long >= 2 * p.bsz && table * p.nkv >= 1600));
     // One pass.  (The transform behind the attention is left to its own launch where the scratch does not hold it beside the
     // partials; attn_pass refuses before it launches anything.)  The list and the append are one launch unless the list is another
     // layer's already.

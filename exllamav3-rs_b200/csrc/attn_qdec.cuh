@@ -1,7 +1,7 @@
 // Decode-class paged attention over 4-bit and 8-bit quantised KV pools (k_bits = v_bits, head_dim 128; one row block of a
 // work item holds 8 * NB packed (query, head) rows): the kernel behind exl3_bighead_attn_paged_q for decode and short
-// verify batches: up to 32 packed rows, and 33 to 48 at 8 bits or where a 4-bit batch is small (attn_impl in attn.cu has both sides;
-// else attn_qt.cuh).
+// verify batches: up to 48 packed rows, but for 33 to 40 at 4 bits where a batch has work for all SMs and few sequences of fewer rows
+// (attn_impl in attn.cu has both sides; else attn_qt.cuh).
 // Reference semantics: kernels/attention.cu:97-269,1716-1870 with the cache codec of
 // kernels/cache/q_cache_kernels.cuh:61-236 (a code c of a group of 32 rotated values stands for
 // (c - (2^(B-1) - 1/2)) * scale / 2^(B-1)).

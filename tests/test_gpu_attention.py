@@ -796,3 +796,42 @@ def test_entries_over_one_block_table(ctx, bits):
     assert exl3b200.lib().exl3_sync_side_stream(ctx.handle) == 0
     ctx.poll_status()
     assert np.array_equal(o.cpu().numpy().view(np.uint16), got.view(np.uint16))
+
+
+@pytest.mark.parametrize("bits,mix,pages_wide,launches", [
+    (4, [(12, 8), (4, 1), (2, 2)], 16, 3), (4, [(24, 7)], 0, 3), (4, [(4, 8), (8, 1)], 32, 3), (4, [(6, 9)], 64, 3),       # 33 to 48 rows: one block of 40, or blocks of 16
+    (4, [(3, 1), (1, 10)], 0, 3), (4, [(3, 1), (1, 10)], 128, 7), (8, [(12, 1), (2, 13)], 0, 3), (8, [(12, 1), (2, 13)], 32, 7),      # both kinds in one pass and in two
+    (4, [(3, 10)], 0, 3), (8, [(3, 13)], 0, 3), (4, [(1, 10)], 0, 3), (4, [(2, 0), (14, 13), (1, 3)], 0, 3)])      # blocks of 64 and of 40, one item per slot and two
+def test_attention_over_codes_of_mixed_batches(ctx, bits, mix, pages_wide, launches):
+    """The rules that say which kernel takes a batch over 4- or 8-bit pools, on both sides: by the rows of its sequences, how many are
+    short, and the block table's width.  Contexts around the tiles.  Bar: the repository's for quantised pools."""
+    from oracle import oracle as O
+    torch = _torch()
+    r = H.rng(2700 + bits + sum(n * x for n, x in mix))
+    nq, nkv = 40, 8
+    q_lens = np.array([x for n, x in mix for _ in range(n)], np.int32)
+    r.shuffle(q_lens)
+    bsz = len(q_lens)
+    ctx_lens = np.array([[0, 127, 128, 300, 515][b % 5] for b in range(bsz)], np.int32)
+    bt, pages = H.make_paged(r, bsz, ctx_lens + q_lens, nkv, 128)
+    bt = np.pad(bt, ((0, 0), (0, max(0, pages_wide - bt.shape[1]))))
+    cu = np.concatenate([[0], np.cumsum(q_lens)]).astype(np.int32)
+    rows = int(cu[-1])
+    rnd = lambda *s: (0.5 * r.standard_normal(s)).astype(np.float16)  # noqa: E731
+    c = dict(q=rnd(rows, nq, 128), k=rnd(rows, nkv, 128), v=rnd(rows, nkv, 128), kc=rnd(pages, 256, nkv, 128), vc=rnd(pages, 256, nkv, 128))
+    pools = _quant_pools(c, bits)
+    o = torch.full(c["q"].shape, float("nan"), dtype=torch.float16, device="cuda")
+    n0 = ctx.launch_count()
+    ctx.bighead_attn_paged_q(H.to_dev(c["q"]), H.to_dev(c["k"]), H.to_dev(c["v"]), *_to_dev(pools), H.to_dev(bt), H.to_dev(ctx_lens), o, nkv,
+                             cu_q=H.to_dev(cu), max_q_len=int(q_lens.max()))
+    assert ctx.launch_count() - n0 == launches
+    ctx.poll_status()
+    got = o.cpu().numpy()
+    for b in range(bsz):
+        if q_lens[b]:
+            O.quant_cache_paged(c["k"][None, cu[b]:cu[b + 1]], pools[0], pools[1], c["v"][None, cu[b]:cu[b + 1]], pools[2], pools[3], ctx_lens[b:b + 1], bt[b:b + 1], bits, bits)
+    want = O.attn_paged(c["q"], None, None, bt, ctx_lens, cu_q=cu, nkv=nkv, quant=(*pools, bits))
+    assert np.isfinite(got).all()
+    for b in range(bsz):
+        if q_lens[b]:
+            assert _close(got[cu[b]:cu[b + 1]], want[cu[b]:cu[b + 1]], TOL_QUANT) <= 1.0, b
