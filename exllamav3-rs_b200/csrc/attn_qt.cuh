@@ -61,6 +61,7 @@ template <int B> struct QtSmem {
     static constexpr int OFF_BAR = OFF_UNIT + 2 * 64;
     static constexpr int N_BARS = 2 * SLOTS + 4 + 5;       // ring full / empty, unit full / empty [2], k_ready, s_full, p_ready, pv_done, drain
     static constexpr int BYTES = OFF_BAR + N_BARS * 8 + 1024;
+    static_assert(BYTES + EXL3_TMEM_SMEM > EXL3_SM_SMEM, "not beside a GEMM that has yet to take tensor memory");
     static constexpr int OSTRIDE = 132;                    // floats per row of the output stage, in the value tile's place
     static_assert(NR * OSTRIDE * 4 <= VALUES && NR * 64 * 4 <= PROBS && SLOT % 512 == 0, "stage layout");
     // Tensor memory: codes 0..63, sums of the groups, output.  The sums of the last group take the place of the codes of the first

@@ -54,14 +54,30 @@ struct exl3_ctx {
     char err[256];
 };
 
-// Every kernel that exl3_launch starts begins with this: it lets the next kernel of the chain be set up on the SMs that fall
-// free, and waits until the kernels before it are complete and their writes visible.  Nothing of global memory is touched
-// before it (weights excepted, which no kernel of a chain writes).
+// Programmatic dependent launches.  Every kernel that exl3_launch starts waits (griddepcontrol.wait) until the kernels before it are
+// complete and their writes visible, and lets the next kernel of the chain be set up on the SMs that fall free
+// (griddepcontrol.launch_dependents).  Ahead of its wait a kernel may
+//  * read weights, sign vectors, norm weights and frequencies, which no kernel of a chain writes;
+//  * read what was complete before its chain began, which the chain's first kernel sees to: a step's lengths, block table, positions and
+//    slots (build_desc_kernel and the embedding are launched in full order), a call's lengths and block table (pdl_enter_first lets go
+//    only behind its own wait).  The pools are not among it: the chain's append writes them;
+//  * prefetch into L2 whatever it will read behind the wait;
+//  * read what a kernel further in front wrote, if the kernel directly in front lets go behind its own wait (pdl_enter_late): the
+//    merge of few rows reads the attention's work list;
+//  * take tensor memory, if no kernel in front that has yet to take its own can be on the same SM (EXL3_TMEM_SMEM).
+// At least one thread of every kernel waits, or the kernel would be complete before those in front of it.
+// This is the plain form: lets go at once and touches nothing ahead of the wait.
 __device__ __forceinline__ void pdl_enter()
 {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
+
+// Two kernels on one SM that both take tensor memory ahead of their waits, the one behind first, would wait for each other: the GEMMs let
+// their dependents go before they allocate, and the attention over codes allocates ahead of its wait (behind it, a verify step of 64
+// layers took 10064 us instead of 10013).  Shared memory keeps them apart: a GEMM that takes tensor memory has at least this much of an
+// SM's 228 KB, the attention over codes at least the rest.
+constexpr int EXL3_TMEM_SMEM = 120 * 1024, EXL3_SM_SMEM = 228 * 1024;
 
 // The same where the kernel behind reads, before its own wait, what the kernels in front of this one wrote.
 __device__ __forceinline__ void pdl_enter_late()

@@ -49,6 +49,7 @@ template <int K, int CTAS, int BN = 256> struct TcSmem {
     static constexpr int N_BARS = 4 * SA + 2 * SR + 2 * SB + 2;      // the A ring has 2 * SA slots for one-tile blocks
     static constexpr int OFF_TMEM = OFF_BAR + N_BARS * 8;
     static constexpr int BYTES = OFF_TMEM + 16 + 1024;      // + slack to align the base to 1024 bytes
+    static_assert(BYTES >= EXL3_TMEM_SMEM, "no other holder of tensor memory beside it");
 };
 
 // Up to TC_MAX_SEG weight tensors with the same k, bits and codebook share one launch (q/k/v or gate/up of a layer):

@@ -76,6 +76,7 @@ template <int K> struct TsSmem {
     static constexpr int N_BARS = 2 * SR + TS_SB + 2 * TS_SW + 7;
     static constexpr int OFF_BAR = OFF_T + TS_T_ROWS * TS_TSTRIDE * 4;
     static constexpr int BYTES = OFF_BAR + N_BARS * 8 + 1024;          // + slack to align the base to 1024 bytes
+    static_assert(BYTES >= EXL3_TMEM_SMEM, "no other holder of tensor memory beside it");
 };
 
 struct GemmTsParams {
