@@ -533,18 +533,21 @@ def test_attention_quantised_ragged(ctx, bits):
     assert np.array_equal(o.cpu().numpy().view(np.uint16), got.view(np.uint16))
 
 
-@pytest.mark.parametrize("bits,nkv,q_lens,ragged", [(0, 3, [1] * 33, False), (0, 8, [5] * 2, False), (3, 5, [2] * 40, False), (0, 1, [1, 0, 9, 0, 0, 2] * 12 + [0], True),
-                                                    (6, 3, [0, 1, 4] * 30, True), (0, 2, [1] * 1100, False), (0, 2, [1, 3, 0] * 400, True)])
+@pytest.mark.parametrize("bits,nkv,q_lens,ragged", [(0, 3, [1] * 33, False), (0, 8, [5] * 2, False), (3, 5, [2] * 40, False), (0, 1, [1, 0, 8, 0, 0, 2] * 12 + [0], True),
+                                                    (6, 3, [0, 1, 4] * 30, True), (0, 2, [1] * 1100, False), (0, 2, [1, 3, 0] * 400, True),
+                                                    (4, 2, [1] * 33, False), (8, 4, [5, 0, 1] * 20, True), (4, 2, [2] * 1100, False)])
 def test_attention_appends_and_plans_in_one_launch(ctx, bits, nkv, q_lens, ragged):
     """A call's keys and values reach the pools as through the separate operator, byte for byte, and its output is that of a call
     over pools that hold them already: more sequences than one search step or one block takes, sequences without rows, odd head
-    counts.  Three sequences are held against the oracle."""
+    counts.  The block table is too wide for clusters, which take no list: three launches with the append, as with the rows cached.  Three
+    sequences are held against the oracle."""
     from oracle import oracle as O
     torch = _torch()
     r = H.rng(2100 + bits + len(q_lens))
     nq, bsz = 2 * nkv, len(q_lens)
     ctx_lens = r.integers(0, 600, bsz).astype(np.int32)
     bt, pages = H.make_paged(r, bsz, ctx_lens + np.asarray(q_lens), nkv, 128)
+    bt = np.pad(bt, ((0, 0), (0, 17 - bt.shape[1])))
     g = torch.Generator(device="cuda").manual_seed(bits)
     half = lambda *s: torch.randn(*s, device="cuda", generator=g).to(torch.float16) * 0.5  # noqa: E731
     rows = sum(q_lens)
@@ -561,10 +564,12 @@ def test_attention_appends_and_plans_in_one_launch(ctx, bits, nkv, q_lens, ragge
 
     def call(p, kk, vv, lens):
         o = torch.full((*lead, nq, 128), float("nan"), dtype=torch.float16, device="cuda")
+        n0 = ctx.launch_count()
         if bits == 0:
             ctx.bighead_attn_paged(q, kk, vv, p[0], p[1], d_bt, lens, o, cu_q=cu, max_q_len=ql)
         else:
             ctx.bighead_attn_paged_q(q, kk, vv, p[0], p[1], p[2], p[3], d_bt, lens, o, nkv, cu_q=cu, max_q_len=ql)
+        assert ctx.launch_count() - n0 == 3
         ctx.poll_status()
         return o
 
