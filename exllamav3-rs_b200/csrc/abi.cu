@@ -41,7 +41,7 @@ extern "C" int exl3_ctx_create(int device, size_t workspace_bytes, exl3_ctx** ou
     ctx->ws_bytes = workspace_bytes ? workspace_bytes : ((size_t)512 << 20);
     ctx->n_counters = 1 << 16;
     ctx->plan_slot_bytes = (size_t)1 << 20;
-    ctx->plan_keep = 0; ctx->plan_valid[0] = ctx->plan_valid[1] = 0;
+    ctx->plan_keep = 0; ctx->plan_shape[0] = ctx->plan_shape[1] = 0;
     ctx->chain = ctx->chain_break = 0;
     ctx->had_suh = nullptr; ctx->had_out = nullptr; ctx->had_bytes = 0; ctx->had_done = 0; ctx->kv_appended = 0;
     bool ok = cudaMalloc(&ctx->ws, ctx->ws_bytes) == cudaSuccess &&

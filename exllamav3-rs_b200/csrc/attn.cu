@@ -447,16 +447,18 @@ int attn_pass(exl3_ctx* ctx, cudaStream_t st, AttnParams p, int total_rows, int 
     *ws_off = off;
 
     static const bool no_lpt = getenv("EXL3_TUNE_NO_LPT") != nullptr;
-    if (!(keep && ctx->plan_valid[cls])) {
+    const int chunk_mult = use_tc ? ATC_TN : use_qt ? QT_TK : AT_TK;
+    const unsigned long long shape = (unsigned long long)target_items << 36 | (unsigned long long)std::min(rows_hi, 255) << 28 | (unsigned long long)rows_lo << 20 | chunk_mult << 10 | rows_per_cta;
+    if (!(keep && ctx->plan_shape[cls] == shape)) {
         const AttnPlanArgs a = {p.seqlens, p.cu_q, plan, items, seq_base, seq_splits, ctx->status, p.bsz, p.q_len, p.kv_append, G, rows_per_cta, rows_lo, rows_hi,
-                                use_tc ? ATC_TN : use_qt ? QT_TK : AT_TK, target_items, max_items, no_lpt ? -1 : (p.causal ? 1 : 0), (use_tc && !tc_items) ? grid_x : 0};
+                                chunk_mult, target_items, max_items, no_lpt ? -1 : (p.causal ? 1 : 0), (use_tc && !tc_items) ? grid_x : 0};
         if (append) {
             const long long warps = (long long)append->rows * (append->k_bits ? append->nkv : 1);
             exl3_launch_first(ctx, attn_front_kernel, 1 + (unsigned)((warps + AP_THREADS / 32 - 1) / (AP_THREADS / 32)), AP_THREADS, 0, st, a, *append);
         } else
             exl3_launch(ctx, attn_plan_kernel, 1, AP_THREADS, 0, st, a);
         ctx->launches++;
-        if (keep) ctx->plan_valid[cls] = 1;
+        if (keep) ctx->plan_shape[cls] = shape;
     }
     exl3_chain_scope chain(ctx);
     dim3 grid(grid_x, p.nkv);

@@ -37,11 +37,12 @@ struct exl3_ctx {
     int fuse_transform;     // 1: in the step runner the norm / activation kernels write the next GEMM's transformed activations (default), 0: separate launches
     // Work lists of the attention kernels kept across the layers of one exl3_step_forward call (they depend on the batch's
     // lengths only, not on the layer): slot 0 = decode class, slot 1 = long class.  plan_keep is set for the duration of a
-    // step; outside of it every attention call builds its list anew.
+    // step; outside of it every attention call builds its list anew.  plan_shape says how a kept list cuts the batch (0: none is
+    // kept), because not every layer's pools need suit the same kernel.
     uint8_t* plan_slots;
     size_t plan_slot_bytes;
     int plan_keep;
-    int plan_valid[2];
+    unsigned long long plan_shape[2];
     // Set for one attention call of a step: where the input transform of o_proj's activations goes and its signs.  The combine
     // kernel, which has a head's 128 values in a warp, writes it (had_done says that it does); had_bytes of the scratch in front
     // of the attention's own are taken by it.

@@ -211,8 +211,8 @@ static int step_forward_impl(exl3_ctx* ctx, exl3_stream stream, const exl3_model
     // attention work lists are built by the first layer and kept for the others; the flag drops on every way out
     struct PlanKeep {
         exl3_ctx* c;
-        explicit PlanKeep(exl3_ctx* ctx_) : c(ctx_) { c->plan_keep = 1; c->plan_valid[0] = c->plan_valid[1] = 0; }
-        ~PlanKeep() { c->plan_keep = 0; c->plan_valid[0] = c->plan_valid[1] = 0; }
+        explicit PlanKeep(exl3_ctx* ctx_) : c(ctx_) { c->plan_keep = 1; c->plan_shape[0] = c->plan_shape[1] = 0; }
+        ~PlanKeep() { c->plan_keep = 0; c->plan_shape[0] = c->plan_shape[1] = 0; }
     } plan_keep(ctx);
     if (need > scratch_bytes) return exl3_fail(ctx, EXL3_ERR_WORKSPACE, "step_forward: scratch buffer too small");
     cudaStream_t st = (cudaStream_t)stream;
