@@ -697,6 +697,7 @@ extern "C" int exl3_bighead_attn_paged_q(exl3_ctx* ctx, exl3_stream stream, cons
     EXL3_REQUIRE(k_bits >= 2 && k_bits <= 8 && v_bits >= 2 && v_bits <= 8, "attention: bits must be 2..8");
     if (compand_a > 0.0f) return exl3_fail(ctx, EXL3_ERR_UNSUPPORTED, "attention: compand_a > 0 is not supported");
     if (bsz == 0 || q_len == 0) return EXL3_OK;
+    EXL3_REQUIRE(quant_planes_aligned(qk, sk, qv, sv), "attention: code planes must be 16-byte and scale planes 8-byte aligned");
     const int append = cu_q ? q_len : kv_append;
     const bool write = append > 0 && !ctx->kv_appended;
     if (write) {

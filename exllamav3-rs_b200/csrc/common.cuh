@@ -204,6 +204,11 @@ static inline int exl3_check_launch(exl3_ctx* ctx, const char* what)
 }
 
 static inline bool aligned16(const void* p) { return (((uintptr_t)p) & 15) == 0; }
+// what the attention's copies of a head's codes and scales need
+static inline bool quant_planes_aligned(const void* qk, const void* sk, const void* qv, const void* sv)
+{
+    return aligned16(qk) && aligned16(qv) && ((((uintptr_t)sk) | ((uintptr_t)sv)) & 7) == 0;
+}
 
 // Transformed activations of up to three EXL3 tensors that share an input, written by the kernel that produces the input
 // (norm, activation) instead of by the GEMM's own transform launch: where each tensor's copy goes and its sign vector.

@@ -241,7 +241,7 @@ static int step_forward_impl(exl3_ctx* ctx, exl3_stream stream, const exl3_model
                   m->pages < (1 << 23) && bsz <= 65535 && b->max_q_len <= 65535;
     for (int l = 0; l < m->n_layers; ++l) {
         const exl3_layer& L = m->layers[l];
-        append = append && (m->kv_bits == 0 ? L.k_cache && L.v_cache && aligned16(L.k_cache) && aligned16(L.v_cache) : L.qk && L.sk && L.qv && L.sv);
+        append = append && (m->kv_bits == 0 ? L.k_cache && L.v_cache && aligned16(L.k_cache) && aligned16(L.v_cache) : L.qk && L.sk && L.qv && L.sv && quant_planes_aligned(L.qk, L.sk, L.qv, L.sv));
     }
     for (int l = 0; l < m->n_layers; ++l) {
         const exl3_layer& L = m->layers[l];

@@ -188,7 +188,7 @@ EXL3_API int exl3_bighead_attn_paged(exl3_ctx* ctx, exl3_stream stream, const vo
 
 /* exl3_shim_bighead_attn_paged_q (src/ffi.rs:97-113, csrc/exl3_shim.cpp:122-129 -> kernels/attention.cu:2086-2290).
  * Same against the quantised pools: qk/qv [pages,256,groups*bits] int32, sk/sv [pages,256,groups] fp16,
- * groups = nkv*hd/32.  Fresh rows are quantised in first.  compand_a must be 0. */
+ * groups = nkv*hd/32; qk, qv on a 16-byte, sk, sv on an 8-byte boundary.  Fresh rows are quantised in first.  compand_a must be 0. */
 EXL3_API int exl3_bighead_attn_paged_q(exl3_ctx* ctx, exl3_stream stream, const void* q, const void* k, const void* v, void* qk,
                               void* sk, void* qv, void* sv, const int32_t* block_table, const int32_t* cache_seqlens,
                               const int32_t* cu_q, void* o, int bsz, int q_len, int kv_append, int nq, int nkv, int hd,

@@ -840,3 +840,21 @@ def test_attention_over_codes_of_mixed_batches(ctx, bits, mix, pages_wide, launc
     for b in range(bsz):
         if q_lens[b]:
             assert _close(got[cu[b]:cu[b + 1]], want[cu[b]:cu[b + 1]], TOL_QUANT) <= 1.0, b
+
+
+@pytest.mark.parametrize("plane", [0, 1, 2, 3])
+def test_quantised_planes_off_their_boundary_are_refused(ctx, plane):
+    """Codes are copied in 16 bytes and scales in 8: planes in between are an error on the host, and nothing is launched or written."""
+    import exl3b200
+    torch = _torch()
+    c = _make_case(2800, [40], 1, 4, 2)
+    dev = _to_dev(_quant_pools(c, 4))
+    flat = torch.cat([dev[plane].flatten(), dev[plane].flatten()[:8]])     # 4 bytes into a code plane, 2 into a scale plane
+    dev[plane] = flat[1:1 + dev[plane].numel()].view(dev[plane].shape)
+    before = [x.clone() for x in dev]
+    o = torch.full(c["q"].shape, 7.0, dtype=torch.float16, device="cuda")
+    n0 = ctx.launch_count()
+    with pytest.raises(exl3b200.Exl3Error, match="aligned"):
+        ctx.bighead_attn_paged_q(H.to_dev(c["q"]), H.to_dev(c["k"]), H.to_dev(c["v"]), *dev, H.to_dev(c["block_table"]), H.to_dev(c["seqlens"]), o, 2)
+    assert ctx.launch_count() == n0
+    assert (o == 7.0).all() and all(torch.equal(a.view(torch.uint8), b.view(torch.uint8)) for a, b in zip(dev, before))
