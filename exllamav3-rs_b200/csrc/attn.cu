@@ -476,8 +476,11 @@ int attn_pass(exl3_ctx* ctx, cudaStream_t st, AttnParams p, int total_rows, int 
     const long long warps = (long long)total_rows * p.nq;
     // The merge of few rows up to six blocks per SM (us, that of many and that of few: fp16, 24 rows of 40 heads 65.6 and 61.2, 4 x 32
     // rows 48.0 and 43.2, 256 rows 451 and 452, a prefill chunk of 512 53.7 and 55.5; 4 bits, 64 rows 74.5 and 72.5, 256 rows 223.5
-    // and 225.1).
-    const bool few = (warps + 7) / 8 <= 6LL * ctx->num_sms;
+    // and 225.1).  In a batch of two passes up to one: its blocks wait, with twice the registers, on SMs that the other pass could use
+    // (fp16, 40 heads, 8 of a row and one of 16, 120 blocks, 64.8 and 59.6; one of 40, 240, 24.9 and 23.2; 28 and one of 40, 340, 21.6 and
+    // 26.2; 64 and four of 16, 640, 28.4 and 42.0; 100 and one of 40 over 1000 .. 16000 keys 366 and 372).
+    const bool pair = rows_lo > 0 || st == ctx->aux_stream;
+    const bool few = (warps + 7) / 8 <= (pair ? 1LL : 6LL) * ctx->num_sms;
     auto merge = had ? (few ? attn_combine_few_kernel<128, true> : attn_combine_kernel<128, true>)
                      : (few ? attn_combine_few_kernel<128, false> : attn_combine_kernel<128, false>);
     exl3_launch(ctx, merge, (unsigned)((warps + 7) / 8), 256, 0, st, p, rows_per_cta, total_rows, had ? ctx->had_suh : (const half*)nullptr,
