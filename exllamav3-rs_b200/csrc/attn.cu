@@ -589,10 +589,22 @@ int attn_impl(exl3_ctx* ctx, cudaStream_t st, AttnParams p, int total_rows, int 
     // among fifteen (two parts) 16.0 and 37.4; one sequence of 64 9.8 and 5.4, of 4000 15.2 and 13.0, of 8000 17.6 and 21.0.  Twice the
     // parts, four CTAs per SM: 8 of 1000 17.6, 16 of 500 16.8 against 13.9 in two parts; 32 of 500 in two parts 23.4 and by the list 25.3,
     // 32 of 250 16.5 and 15.3.
+    // In a step, where the list is built once for all layers: us a layer of hidden 1024, 16 / 8 heads, list and clusters, 8 of 2000 keys 54.8
+    // and 51.1, 16 of 1000 54.9 and 50.9, one of 2000 among seven of 64 45.2 and 46.6; with fewer CTAs at most 448 keys per part, 4 of 2000 in
+    // four parts 45.2 and 48.3, one of 4000 in eight 45.1 and 47.5, of 3000 among three of 64 45.5 and 43.9; and clusters of eight only
+    // where they leave room, because one waits for eight places at a time: 32 of them (4 of 1000) 46.1, of four CTAs 42.7, list 45.0; 4 of
+    // 4000 in eight parts 63.5 and 55.2; 24 (3 of 3000) 46.0 and 46.2; 16 (2 of 2000) 41.8 and 44.4.
+    // Codes, whose tiles take longer, at most 320 keys per part there (6 bits: one of 2000 among seven of 64 63.4 and 73.2, 3 of 3000 in
+    // eight parts 60.5 and 68.6, 4 of 2000 62.5 and 80.4; but one of 1000 among seven 62.5 and 56.5; a call of its own, with its list, one of
+    // 2000 among seven 29.7 and 36.3, 36 before list and append were one launch).
     int parts = 0;
     if (max_rows <= 16 && !codes && !p.contig_kv)
-        for (int c = 8; c >= 2 && parts == 0; c >>= 1)
-            if ((long long)p.bsz * p.nkv * c <= 2LL * ctx->num_sms && (long long)p.pps * EXL3_PAGE <= 512LL * c) parts = c;
+        for (int c = 8; c >= 2 && parts == 0; c >>= 1) {
+            const long long ctas = (long long)p.bsz * p.nkv * c;
+            const bool full = 2 * ctas > 3LL * ctx->num_sms, step = ctx->plan_keep;
+            const int most = !step ? 512 : quant ? 320 : full ? 512 : 448;       // keys per part
+            if (ctas <= 2LL * ctx->num_sms && (long long)p.pps * EXL3_PAGE <= (long long)most * c && !(step && full && c == 8)) parts = c;
+        }
     if (parts) {
         if (append) {
             const int rc = attn_append(ctx, st, *append);

@@ -721,3 +721,28 @@ def test_step_whose_layers_take_different_attention_kernels(ctx, q_lens):
     assert launches[1] > launches[0] + 1                # the lists of layers two and three
     assert np.isfinite(logits[1]).all()
     assert np.linalg.norm(logits[1] - logits[0]) / np.linalg.norm(logits[0]) < 3.2e-2
+
+
+@pytest.mark.parametrize("kv_bits,lens,wide", [(0, [1500] * 4, 7), (0, [1500] * 4, 8), (0, [200] * 4, 1), (0, [2000] * 2, 14), (0, [2000] * 2, 15),
+                                               (6, [900, 40], 10), (6, [900, 40], 11)])
+def test_step_on_both_sides_of_the_cluster_rules(ctx, kv_bits, lens, wide):
+    """In a step, by the block table's width: clusters of four and of eight CTAs, and the work list on the other side (one launch more per
+    layer, and the list).  Against the table made far too wide.  Bars on the relative 2-norm as for steps over entries of one sequence."""
+    import torch
+    from exl3b200.step import SyntheticModel
+    r = H.rng(64 + len(lens))
+    ctx_lens = np.array(lens, np.int32)
+    bt, pages = H.make_paged(r, len(lens), ctx_lens + 1, 8, 128)
+    model = SyntheticModel(2, 512, 8, 8, 128, 512, 512, K=4, cb=1, pages=pages, kv_bits=kv_bits, seed=64)
+    ids, q_lens, sl = H.to_dev(r.integers(0, 512, len(lens))), H.to_dev(np.ones(len(lens), np.int32)), H.to_dev(ctx_lens)
+    logits, launches = [], []
+    for w in (wide, 64):
+        model.fill_kv()
+        n0 = ctx.launch_count()
+        logits.append(model.step(ctx, ids, q_lens, sl, H.to_dev(np.pad(bt, ((0, 0), (0, w - bt.shape[1])))), 1, want_logits=True)[1].cpu().numpy())
+        launches.append(ctx.launch_count() - n0)
+        ctx.poll_status()
+    clusters = {(4, 7): True, (4, 8): False, (4, 1): True, (2, 14): True, (2, 15): False, (2, 10): True, (2, 11): False}[len(lens), wide]
+    assert launches[1] - launches[0] == (3 if clusters else 0)
+    assert np.isfinite(logits[0]).all()
+    assert np.linalg.norm(logits[0] - logits[1]) / np.linalg.norm(logits[1]) < (2.8e-3 if kv_bits == 0 else 1.2e-2)
