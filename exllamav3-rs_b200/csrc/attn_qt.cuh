@@ -16,14 +16,15 @@
 // (attn_qdec.cuh) or fp16 tiles for every 64 (attn_paged.cuh).  Two CTAs per SM hide each other's barriers and waits; a producer
 // thread draws work units ahead and keeps the ring of code tiles full across units.
 //
-// What bounds it: latency.  A tile takes a CTA 8400 cycles, of which 2300 are issued instructions of two CTAs (issue slots 49 % busy;
-// stalls of a warp per issued instruction: instruction fetch 1.5, fixed latencies 1.4, tensor memory and shared memory 1.0 each,
-// barriers 0.7); the products take 1200, shared memory some 1600.  On the way, us, 4 sequences of 40 rows, contexts 1024 .. 32768,
-// whole call behind a work list of 8.7: one thread per key with products issued by a warp of keys 82, with an issuer 75, two threads
-// per key 61, references left alone up to a factor of sqrt(2) 50, values to 22 bits 54 (the mma.sync kernel: 72).  Scales applied to
-// the weights per group instead, which keeps codes exact with one rounding less, need four copies of the output: for up to 8 rows,
-// three CTAs per SM, 64 sequences of 5 rows took 176 to 202 us (the mma.sync kernel: 142): not kept.
-// Whole calls now, 4 bits, us: these 64 -> 47, 32 such sequences, 1024 .. 16384, 261 -> 191, 3 of 500 rows 106 -> 98; 8 bits 140 -> 134.
+// What bounds it: latency.  Twelve sequences of 40 rows over contexts of 1024 .. 32768, profiled: 23 tiles per CTA, some 6600 cycles each
+// with start and end, issue slots 57 % busy, 28 % of the warps an SM can hold, tensor pipe 18 %, DRAM 16 %; stalls of a warp per issued
+// instruction: shared memory 1.5, fixed latencies 1.3, branches 0.7, tensor memory and global loads 0.6, barriers 0.5, instruction
+// fetch 0.4.  On the way, us, 4 sequences of 40 rows, contexts 1024 .. 32768, whole call behind a work list of 8.7: one thread per
+// key with products issued by a warp of keys 82, with an issuer 75, two threads per key 61, references left alone up to a factor of
+// sqrt(2) 50, values to 22 bits 54 (the mma.sync kernel: 72).  Scales applied to the weights per group instead, which keeps codes exact
+// with one rounding less, need four copies of the output: for up to 8 rows, three CTAs per SM, 64 sequences of 5 rows took 176 to 202 us
+// (the mma.sync kernel: 142): not kept.
+// Whole calls now, 4 bits, us: these 72 -> 43, 32 such sequences 435 -> 248, 4 of 500 rows 428 -> 366, at 8 bits 632 -> 565.
 // Error against 64 bits: 40 rows, 4 bits 3.0e-4 -> 2.6e-4; 500 rows 4.8e-4 -> 4.2e-4, 8 bits 3.9e-4 -> 3.1e-4.  (With values rounded to
 // one fp16 and weights to another it was 3.4e-4: the largest weight is exact, its value was not.)
 // Every wait is bounded; a wait that runs out lets the others run out at once and sets the status word.

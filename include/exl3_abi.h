@@ -174,7 +174,8 @@ EXL3_API int exl3_paged_kv_cache_update(exl3_ctx* ctx, exl3_stream stream, const
                                const int32_t* cu_q, int bsz, int seq, int nkv, int hd, int pages, int pages_per_seq);
 
 /* exl3_shim_bighead_attn_paged (src/ffi.rs:84-96, csrc/exl3_shim.cpp:110-118 -> kernels/attention.cu:1716-2075).
- * Appends k,v (as above; kv_append may be 0 with k = v = NULL) then computes causal GQA attention of
+ * Appends k,v of all sequences (as above; kv_append may be 0 with k = v = NULL), then computes causal GQA attention (sequences may
+ * share pages: what one appends is there for all) of
  * q [bsz,q_len,nq,hd] over the first cache_seqlens[b]+kv_append cached keys; query i sees keys
  * j <= total - q_len + i.  sm_scale 0 = 1/sqrt(hd).  o like q.  kv_chunk_size is accepted and ignored (split sizes
  * are derived on the device from the real lengths).
