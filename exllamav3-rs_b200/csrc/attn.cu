@@ -409,16 +409,17 @@ int attn_pass(exl3_ctx* ctx, cudaStream_t st, AttnParams p, int total_rows, int 
     // quantised pools, whose units start with the rotation of their queries (24 sequences, contexts 512 .. 16384, 40 / 8
     // heads, one and two items: 4 bits, 5 rows 68 and 72 us, 40 rows 188 and 193; 8 bits 68 and 75, 188 and 196).
     static const int dec_items = getenv("EXL3_TUNE_DEC_ITEMS") ? atoi(getenv("EXL3_TUNE_DEC_ITEMS")) : 0;
-    // The tcgen05 kernel over codes: one item per slot while its blocks are few, less half of them, because each rounds its count up and
-    // items beyond the slots are a second wave; else two, which balance the blocks (us, one and two: 4 sequences of 65 rows, 512 .. 4096, 35
-    // and 37, of 100, 512 .. 4096, 32 and 44, 1024 .. 32768 110 and 98, of 500 506 and 368; one of 250 rows, 512 .. 4096, 25 and 35, of
-    // 500, 1024 .. 32768, 110 and 83; 16 of 250, 1024 .. 32768, 830 and 717; without and with the half: 3 of 125, 512 .. 2048, 34 and 28, one of
-    // 300 31 and 25, 5 of 40, 1024 .. 32768, 63 and 52).
+    // The tcgen05 kernel over codes: one item per slot; two, which balance the blocks, where these are not few and contexts may be long; and
+    // where they are few less half of them, because each rounds its count up and items beyond the slots are a second wave (us, one and two:
+    // 4 sequences of 65 rows, 512 .. 4096, 35 and 37, of 100, 512 .. 4096, 32 and 44, 1024 .. 32768 110 and 98, of 500 506 and 368; one of
+    // 250 rows, 512 .. 4096, 25 and 35, of 500, 1024 .. 32768, 110 and 83; 16 of 250, 1024 .. 32768, 830 and 717; 5 of a row and 2 of 640,
+    // 109 .. 218, 27 and 39; 3 of 410, 377 .. 1919, at 8 bits 86 and 92; without and with the half: 3 of 125, 512 .. 2048, 34 and 28, one of 300
+    // 31 and 25, 5 of 40, 1024 .. 32768, 63 and 52, but 2 of 205, 600 and 2000, 29 and 32).
     const int n_long = min_long(total_rows, p.bsz, max_rows / G);
     const long long qt_blocks = (long long)n_long * rb_max + (rows_lo == 0 ? p.bsz - n_long : 0);
-    const bool qt_few = use_qt && 3 * qt_blocks <= grid_x;
+    const bool qt_few = use_qt && 3 * qt_blocks <= grid_x, one_item = use_qdec || (use_qt && p.pps <= 8);
     const int target_items = dec_items && !use_tc ? grid_x * dec_items : qt_few ? grid_x - (int)qt_blocks / 2
-                             : grid_x * (use_tc ? (tc_items ? tc_items : 2) : (use_qdec ? 1 : 2));
+                             : grid_x * (use_tc ? (tc_items ? tc_items : 2) : (one_item ? 1 : 2));
     // items <= target + sum of row blocks (every (sequence, row block) rounds its split count up once); the row blocks are
     // bounded by bsz * rb_max and, usually much tighter for ragged batches, by total_rows * G / rows_per_cta + bsz
     const long long rb_sum = std::min((long long)p.bsz * rb_max, ((long long)total_rows * G + rows_per_cta - 1) / rows_per_cta + p.bsz);
@@ -546,9 +547,11 @@ int attn_impl(exl3_ctx* ctx, cudaStream_t st, AttnParams p, int total_rows, int 
     //    than 800 rows stay where they were.)
     //    Where contexts are short a unit is little more than its start and end, and a second wave of them costs as much as the first: by the
     //    block table, one page and more than a wave (6 of 300 rows without a context 20 and 29, 24 of 640 133 and 156, 4 of 300, one wave,
-    //    20 and 19; with contexts of 64 .. 128 26 and 34, 161 and 187, 26 and 24), or up to eight pages, more blocks than the other kernel has, and
-    //    a second or third wave that it does not need (128 .. 512, one of 800 rows 29 and 34, 5 of 300 34 and 42, 12 of 125 33 and 43;
-    //    but 5 of 800 86 and 71, 12 of 300 72 and 68, 24 of 65, as many blocks in either, 48 and 42).
+    //    20 and 19; with contexts of 64 .. 128 26 and 34, 161 and 187, 26 and 24), or up to five pages, more blocks than the other kernel has, and
+    //    a second or third wave that it does not need (128 .. 512, one of 800 rows 29 and 34, 5 of 300 34 and 42, 12 of 125 33 and 43; but 5 of
+    //    800 86 and 71, 12 of 300 72 and 68, 24 of 65, as many blocks in either, 48 and 42; with eight pages 3 of 410 92 and 85; beside
+    //    sequences of few rows, for which the other kernel needs a pass more, 5 of a row and 2 of 640 47 and 27, 40 and 2 of 240 without a
+    //    context 26 and 32, 0.87 in the mean of 700 such batches).
     //  * a ragged batch of both kinds in one pass instead of two, as long as the short ones have few keys, by the width of the block table:
     //    8 of a row and one of 100, two passes and one, 128 .. 1024 (5 pages) 25 and 20, 512 .. 4096 (17) 42 and 33, 1024 .. 32768 (129) 80 and
     //    94; 32 and one 39 and 30, 63 and 64, 168 and 223; at 8 bits 29 and 23, 47 and 43, 89 and 142; 44 and 38, 71 and 96, 171 and 359.
@@ -560,7 +563,7 @@ int attn_impl(exl3_ctx* ctx, cudaStream_t st, AttnParams p, int total_rows, int 
         return ((long long)n_long * ((max_rows + rows - 1) / rows) * p.nkv * (p.pps == 1 ? 1 : 2) + slots - 1) / slots;
     };
     const long long wq = waves(QT_ROWS, 2), w64 = waves(64, 3);
-    const bool cheap = p.pps == 1 ? wq > 1 : p.pps <= 8 && (max_rows + QT_ROWS - 1) / QT_ROWS > (max_rows + 63) / 64 && wq > w64 && wq <= 3;
+    const bool cheap = n_long >= p.bsz && (p.pps == 1 ? wq > 1 : p.pps <= 5 && (max_rows + QT_ROWS - 1) / QT_ROWS > (max_rows + 63) / 64 && wq > w64 && wq <= 3);
     const bool long_codes = codes && max_rows > dec_rows && (p.k_bits == 4 || max_rows <= 800) && (max_rows > 64 || p.cu_q || p.bsz == 1) && !cheap;
     const bool codes_alone = long_codes ? (long long)(p.bsz - n_long) * p.pps <= (p.k_bits == 4 ? 300 : 200)
                                         : codes && p.k_bits == 4 && max_rows > 32 && max_rows <= QT_ROWS && table >= 200 &&

@@ -807,7 +807,7 @@ def test_entries_over_one_block_table(ctx, bits):
     (4, [(12, 8), (4, 1), (2, 2)], 16, 3), (4, [(24, 7)], 0, 3), (4, [(4, 8), (8, 1)], 32, 3), (4, [(6, 9)], 64, 3),       # 33 to 48 rows: one block of 40, or blocks of 16
     (4, [(3, 1), (1, 10)], 0, 3), (4, [(3, 1), (1, 10)], 128, 7), (8, [(12, 1), (2, 13)], 0, 3), (8, [(12, 1), (2, 13)], 32, 7),      # both kinds in one pass and in two
     (4, [(3, 10)], 0, 3), (8, [(3, 13)], 0, 3), (4, [(1, 10)], 0, 3), (4, [(2, 0), (14, 13), (1, 3)], 0, 3),       # blocks of 40, one item per slot and two
-    (4, [(8, 25)], 0, 7), (4, [(6, 60)], 8, 7), (4, [(8, 25)], 9, 3), (8, [(2, 25), (1, 1)], 0, 3)])      # contexts too short for them, in a wider table, and few
+    (4, [(8, 25)], 0, 7), (4, [(6, 60)], 5, 7), (4, [(8, 25)], 6, 3), (8, [(2, 25), (1, 1)], 0, 3)])      # contexts too short for them, in a wider table, and few
 def test_attention_over_codes_of_mixed_batches(ctx, bits, mix, pages_wide, launches):
     """The rules that say which kernel takes a batch over 4- or 8-bit pools, on both sides: by the rows of its sequences, how many are
     short, and the block table's width.  Contexts around the tiles.  Bar: the repository's for quantised pools."""
